@@ -1,5 +1,5 @@
 // Bandwidth-bound kernels of the transformer step for sm_100a: RMSNorm fwd/bwd, RoPE, SwiGLU
-// fwd/bwd, cross-entropy fwd/bwd, dtype cast, embedding backward, multi-tensor AdamW.
+// fwd/bwd, cross-entropy fwd/bwd, dtype cast, embedding forward, multi-tensor AdamW.
 // All use 16-byte vector accesses, fp32 math, and grids sized as multiples of the 148 SMs.
 // They replace the ATen / Inductor-generated kernels the reference reaches for the same nodes
 // (autoparallel/_testing/models/llama3.py:187-213, 355-356, 396-397).
@@ -536,16 +536,6 @@ __global__ void embedding_fwd_kernel(const T* __restrict__ weight, const long lo
   for (int c = threadIdx.x; c < nvec; c += blockDim.x) dst[c] = src[c];
 }
 
-// ------------------------------------------------------------------------------------ embedding backward
-// out fp32 [rows, D] (zeroed by caller) += dy[token] for each token; one block per token.
-template <typename T>
-__global__ void embedding_bwd_kernel(const T* __restrict__ dy, const long long* __restrict__ ids, float* __restrict__ out,
-                                     int D) {
-  const long long tok = blockIdx.x;
-  const long long r = ids[tok];
-  for (int c = threadIdx.x; c < D; c += blockDim.x) atomicAdd(out + r * D + c, float(dy[tok * D + c]));
-}
-
 // ------------------------------------------------------------------------------------ AdamW
 // Multi-tensor: ``table`` lists chunks (tensor id, offset); each block handles one chunk.
 struct AdamTensor {
@@ -796,13 +786,6 @@ int apb_embedding_fwd(const void* weight, const long long* ids, void* out, long 
   if (tokens == 0) return 0;
   if ((D * (is_bf16 ? 2 : 4)) % 16) return 3;
   DISPATCH(is_bf16, embedding_fwd_kernel<T><<<(unsigned)tokens, 128, 0, st>>>((const T*)weight, ids, (T*)out, D, num_rows));
-  return cudaGetLastError() == cudaSuccess ? 0 : 4;
-}
-
-int apb_embedding_bwd(const void* dy, const long long* ids, float* out_f32, long long tokens, int D, int is_bf16,
-                      cudaStream_t st) {
-  if (tokens == 0) return 0;
-  DISPATCH(is_bf16, embedding_bwd_kernel<T><<<(unsigned)tokens, 256, 0, st>>>((const T*)dy, ids, out_f32, D));
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 

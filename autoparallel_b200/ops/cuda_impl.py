@@ -373,10 +373,10 @@ def _embedding(weight, ids):
 
 def _embedding_bwd(dy, ids, num_rows):
     dy = dy.contiguous()
-    out = torch.zeros(num_rows, dy.shape[-1], dtype=torch.float32, device=dy.device)
+    out = torch.empty(num_rows, dy.shape[-1], dtype=dy.dtype, device=dy.device)
     _C.embedding_bwd(dy, ids.contiguous(), out)
-    _count()
-    return out.to(dy.dtype)
+    _count(3 if ids.numel() >= 32 else 2)
+    return out
 
 
 # ----------------------------------------------------------------------------------- attention (library)
