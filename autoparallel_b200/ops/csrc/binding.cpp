@@ -41,12 +41,14 @@ int apb_embedding_bwd(const void* dy, const long long* ids, void* out, void* wor
                       int is_bf16, int num_sms, cudaStream_t st);
 int apb_embedding_fwd(const void* weight, const long long* ids, void* out, long long tokens, int D, long long num_rows,
                       int is_bf16, cudaStream_t st);
-int apb_moe_slots_max_experts(int threads);
-int apb_moe_slots(const long long* gate_idx, long long* slot, int num_blocks, int per_block, int E, int C, cudaStream_t st);
-int apb_moe_scatter(const void* src, const long long* slot, const float* w, void* buf, long long T, int k, int d, int E, int C, int nb,
-                    int is_bf16, cudaStream_t st);
-int apb_moe_gather(const void* buf, const long long* slot, const float* w, void* out, long long T, int k, int d, int E, int C, int nb,
-                   int is_bf16, cudaStream_t st);
+int apb_moe_slots_max_experts(int per_block);
+long long apb_moe_slots_workspace(int num_blocks, int per_block, int E, int num_sms);
+int apb_moe_slots(const long long* gate_idx, long long* slot, int* counts, int num_blocks, int per_block, int E, int C, int num_sms,
+                  cudaStream_t st);
+int apb_moe_scatter(const void* src, const long long* slot, const void* w, int w_bf16, long long* inv, void* buf, long long T, int k, int d,
+                    int E, int C, int nb, int is_bf16, cudaStream_t st);
+int apb_moe_gather(const void* buf, const long long* slot, const void* w, int w_bf16, void* out, long long T, int k, int d, int E, int C,
+                   int nb, int is_bf16, cudaStream_t st);
 int apb_moe_gate_grad(const void* buf, const long long* slot, const void* g, float* dw, long long T, int k, int d, int E, int C, int nb,
                       int is_bf16, cudaStream_t st);
 int apb_symm_header_bytes();
@@ -234,10 +236,7 @@ static void moe_check(const at::Tensor& x, const char* what) {
   TORCH_CHECK(x.is_cuda() && x.is_contiguous(), what, ": contiguous CUDA tensor expected");
 }
 
-int64_t moe_slots_max_experts(int64_t per_block) {
-  int threads = per_block >= 1024 ? 1024 : (int)((per_block + 31) / 32) * 32;
-  return apb_moe_slots_max_experts(threads);
-}
+int64_t moe_slots_max_experts(int64_t per_block) { return apb_moe_slots_max_experts((int)std::min<int64_t>(per_block, 1 << 30)); }
 
 void moe_slots(const at::Tensor& gate_idx, at::Tensor& slot, int64_t E, int64_t C, int64_t nb) {
   c10::cuda::CUDAGuard g(gate_idx.device());
@@ -247,32 +246,41 @@ void moe_slots(const at::Tensor& gate_idx, at::Tensor& slot, int64_t E, int64_t 
                   gate_idx.numel() == slot.numel() && nb > 0 && gate_idx.size(0) % nb == 0,
               "moe_slots: int64 [T, k] with T a multiple of the block count");
   const int64_t per_block = gate_idx.size(0) / nb * gate_idx.size(1);
-  check(apb_moe_slots((const long long*)gate_idx.data_ptr<int64_t>(), (long long*)slot.data_ptr<int64_t>(), (int)nb, (int)per_block,
-                      (int)E, (int)C, stream()),
+  at::Tensor counts = at::empty({(int64_t)apb_moe_slots_workspace((int)nb, (int)per_block, (int)E, num_sms())}, gate_idx.options().dtype(at::kInt));
+  check(apb_moe_slots((const long long*)gate_idx.data_ptr<int64_t>(), (long long*)slot.data_ptr<int64_t>(), counts.data_ptr<int>(), (int)nb,
+                      (int)per_block, (int)E, (int)C, num_sms(), stream()),
         "apb_moe_slots");
+}
+
+// gate weights: fp32 or bf16, used in the operand's precision
+bool gate_is_bf16(const at::Tensor& w, const at::Tensor& slot, const char* what) {
+  TORCH_CHECK((w.scalar_type() == at::kFloat || w.scalar_type() == at::kBFloat16) && w.numel() == slot.numel(), what,
+              ": fp32 or bf16 gate weights [T, k] expected");
+  return w.scalar_type() == at::kBFloat16;
 }
 
 void moe_scatter(const at::Tensor& src, const at::Tensor& slot, const at::Tensor& w, at::Tensor& buf, int64_t E, int64_t C, int64_t nb) {
   c10::cuda::CUDAGuard g(src.device());
   moe_check(src, "moe_scatter"); moe_check(slot, "moe_scatter"); moe_check(w, "moe_scatter"); moe_check(buf, "moe_scatter");
-  TORCH_CHECK(src.dim() == 2 && slot.dim() == 2 && slot.scalar_type() == at::kLong && w.scalar_type() == at::kFloat &&
-                  w.numel() == slot.numel() && slot.size(0) == src.size(0) && buf.scalar_type() == src.scalar_type() &&
-                  buf.numel() == E * nb * C * src.size(1),
-              "moe_scatter: src [T, d], slot [T, k] int64, w [T, k] fp32, buf [E, nb, C, d] of src's dtype");
-  check(apb_moe_scatter(src.data_ptr(), (const long long*)slot.data_ptr<int64_t>(), w.data_ptr<float>(), buf.data_ptr(), src.size(0),
-                        (int)slot.size(1), (int)src.size(1), (int)E, (int)C, (int)nb, is_bf16(src), stream()),
+  TORCH_CHECK(src.dim() == 2 && slot.dim() == 2 && slot.scalar_type() == at::kLong && slot.size(0) == src.size(0) &&
+                  buf.scalar_type() == src.scalar_type() && buf.numel() == E * nb * C * src.size(1),
+              "moe_scatter: src [T, d], slot [T, k] int64, buf [E, nb, C, d] of src's dtype");
+  at::Tensor inv = at::empty({E * nb * C}, slot.options());
+  check(apb_moe_scatter(src.data_ptr(), (const long long*)slot.data_ptr<int64_t>(), w.data_ptr(), gate_is_bf16(w, slot, "moe_scatter"),
+                        (long long*)inv.data_ptr<int64_t>(), buf.data_ptr(), src.size(0), (int)slot.size(1), (int)src.size(1), (int)E, (int)C,
+                        (int)nb, is_bf16(src), stream()),
         "apb_moe_scatter");
 }
 
 void moe_gather(const at::Tensor& buf, const at::Tensor& slot, const at::Tensor& w, at::Tensor& out) {
   c10::cuda::CUDAGuard g(buf.device());
   moe_check(buf, "moe_gather"); moe_check(slot, "moe_gather"); moe_check(w, "moe_gather"); moe_check(out, "moe_gather");
-  TORCH_CHECK(buf.dim() == 4 && slot.dim() == 2 && slot.scalar_type() == at::kLong && w.scalar_type() == at::kFloat &&
-                  w.numel() == slot.numel() && out.dim() == 2 && out.size(0) == slot.size(0) && out.size(1) == buf.size(3) &&
-                  out.scalar_type() == buf.scalar_type(),
-              "moe_gather: buf [E, nb, C, d], slot [T, k] int64, w [T, k] fp32, out [T, d] of buf's dtype");
-  check(apb_moe_gather(buf.data_ptr(), (const long long*)slot.data_ptr<int64_t>(), w.data_ptr<float>(), out.data_ptr(), slot.size(0),
-                       (int)slot.size(1), (int)buf.size(3), (int)buf.size(0), (int)buf.size(2), (int)buf.size(1), is_bf16(buf), stream()),
+  TORCH_CHECK(buf.dim() == 4 && slot.dim() == 2 && slot.scalar_type() == at::kLong && out.dim() == 2 && out.size(0) == slot.size(0) &&
+                  out.size(1) == buf.size(3) && out.scalar_type() == buf.scalar_type(),
+              "moe_gather: buf [E, nb, C, d], slot [T, k] int64, out [T, d] of buf's dtype");
+  check(apb_moe_gather(buf.data_ptr(), (const long long*)slot.data_ptr<int64_t>(), w.data_ptr(), gate_is_bf16(w, slot, "moe_gather"),
+                       out.data_ptr(), slot.size(0), (int)slot.size(1), (int)buf.size(3), (int)buf.size(0), (int)buf.size(2),
+                       (int)buf.size(1), is_bf16(buf), stream()),
         "apb_moe_gather");
 }
 

@@ -238,8 +238,13 @@ def _moe_slots(gate_idx, num_experts, capacity, num_blocks):
         return moe_ops._moe_slots(gate_idx, num_experts, capacity, num_blocks)
     slot = torch.empty_like(gate_idx, memory_format=torch.contiguous_format)
     _C.moe_slots(gate_idx.contiguous(), slot, num_experts, capacity, num_blocks)
-    _count()
+    _count(2)
     return slot
+
+
+def _gate_weights(w, dtype):
+    """The kernels apply the gate weight in the operand's precision (as the reference formula does) and read it as stored."""
+    return w.contiguous() if w.dtype in (torch.float32, torch.bfloat16) else w.to(dtype).contiguous()
 
 
 def _moe_scatter(src, slot, w, num_experts, capacity, num_blocks):
@@ -249,10 +254,9 @@ def _moe_scatter(src, slot, w, num_experts, capacity, num_blocks):
             and src.shape[0] > 0):
         _fallback("moe_index", f"moe_scatter {tuple(src.shape)} {src.dtype}")
         return moe_ops._moe_scatter(src, slot, w, num_experts, capacity, num_blocks)
-    buf = torch.zeros((num_experts, num_blocks, capacity, src.shape[1]), dtype=src.dtype, device=src.device)
-    # the gate weight is applied in the operand's precision (as the reference formula does), then widened for the kernel
-    _C.moe_scatter(src.contiguous(), slot.contiguous(), w.to(src.dtype).float().contiguous(), buf, num_experts, capacity, num_blocks)
-    _count()
+    buf = torch.empty((num_experts, num_blocks, capacity, src.shape[1]), dtype=src.dtype, device=src.device)
+    _C.moe_scatter(src.contiguous(), slot.contiguous(), _gate_weights(w, src.dtype), buf, num_experts, capacity, num_blocks)
+    _count(2)
     return buf
 
 
@@ -264,7 +268,7 @@ def _moe_gather(buf, slot, w):
         _fallback("moe_index", f"moe_gather {tuple(buf.shape)} {buf.dtype}")
         return moe_ops._moe_gather(buf, slot, w)
     out = torch.empty((slot.shape[0], buf.shape[3]), dtype=buf.dtype, device=buf.device)
-    _C.moe_gather(buf.contiguous(), slot.contiguous(), w.to(buf.dtype).float().contiguous(), out)
+    _C.moe_gather(buf.contiguous(), slot.contiguous(), _gate_weights(w, buf.dtype), out)
     _count()
     return out
 

@@ -137,7 +137,8 @@ def _scatter_setup(ctx, inputs, output):
 def _scatter_bwd(ctx, dbuf):
     src, slot, w = ctx.saved_tensors
     dsrc = ops.moe_gather(dbuf, slot, w)
-    dw = ops.moe_gate_grad(dbuf, slot, src).to(w.dtype)
+    # (the plain dispatch scatters with constant weights: nobody asks for their gradient, which reads the whole buffer)
+    dw = ops.moe_gate_grad(dbuf, slot, src).to(w.dtype) if ctx.needs_input_grad[2] else None
     return dsrc, None, dw, None, None, None
 
 

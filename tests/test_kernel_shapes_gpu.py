@@ -54,3 +54,47 @@ def test_embedding_gradient_of_an_unaligned_view(K):
     dy, idx = flat[1:].view(12, 16), torch.arange(12, device="cuda") % 5
     ref = torch.zeros(5, 16, dtype=torch.float64).index_add_(0, idx.cpu(), dy.double().cpu())
     assert _rel(lib.ops.embedding_bwd(dy, idx, 5), ref) <= 2**-8
+
+
+@pytest.mark.parametrize("T,k,E,C,nb,d", [
+    (8, 2, 4, 3, 1, 64),        # one chunk of assignments, drops
+    (2048, 8, 64, 300, 1, 40),  # 32 chunks of 512; rows of 80 bytes
+    (1000, 3, 16, 50, 8, 129),  # odd block sizes, rows that are no whole vectors, nine assignments past a warp
+    (512, 9, 500, 16, 1, 2304),  # more choices than one gather step, more experts than threads per group, wide rows
+    (70000, 8, 8, 4000, 1, 8),  # more assignments than two rounds of all CTAs
+])
+@pytest.mark.parametrize("dtype,wdtype", [(torch.bfloat16, torch.bfloat16), (torch.bfloat16, torch.float32), (torch.float32, torch.bfloat16)])
+def test_moe_dispatch_over_shapes(K, T, k, E, C, nb, d, dtype, wdtype):
+    lib, impl = K
+    from autoparallel_b200.ops import moe_ops
+
+    g = torch.Generator().manual_seed(T + k)
+    idx = (torch.rand(T, E, generator=g) + torch.linspace(0.3, 0, E)).topk(k).indices
+    x, w = torch.randn(T, d, generator=g).to(dtype), torch.rand(T, k, generator=g).to(wdtype)
+    before = dict(impl.library_fallbacks)
+    slot = lib.ops.moe_slots(idx.cuda(), E, C, nb)
+    rslot = moe_ops._moe_slots(idx, E, C, nb)
+    assert torch.equal(slot.cpu(), rslot)
+    buf = lib.ops.moe_scatter(x.cuda(), slot, w.cuda(), E, C, nb)
+    rbuf = moe_ops._moe_scatter(x, rslot, w, E, C, nb)
+    assert torch.equal(buf.cpu(), rbuf)  # one product per element, empty rows zero
+    flat, ec = moe_ops._buf_rows(rbuf.double())
+    picked = flat[moe_ops._rows(rslot, nb, ec)].view(T, k, -1)
+    tol = 2**-8 if dtype == torch.bfloat16 else 2**-20
+    assert _rel(lib.ops.moe_gather(buf, slot, w.cuda()), (picked * w.to(dtype).double().unsqueeze(2)).sum(1)) <= tol
+    assert _rel(lib.ops.moe_gate_grad(buf, slot, x.cuda()), (picked * x.double().unsqueeze(1)).sum(-1)) <= 2**-18
+    assert impl.library_fallbacks == before, "the kernels cover these shapes"
+
+
+def test_moe_dispatch_leaves_nothing_of_the_old_buffer(K):
+    """Every row of the buffer is written, also those no assignment names, whatever the memory held before."""
+    lib, _ = K
+    idx = torch.zeros(64, 1, dtype=torch.long, device="cuda")
+    slot = lib.ops.moe_slots(idx, 4, 128, 1)
+    x = torch.randn(64, 256, device="cuda", dtype=torch.bfloat16)
+    for _ in range(3):
+        junk = [torch.full((4 * 128 * 256,), float("nan"), device="cuda", dtype=torch.bfloat16),
+                torch.arange(4 * 128, device="cuda")]  # what the buffer and the row table may be allocated over
+        del junk
+        buf = lib.ops.moe_scatter(x, slot, torch.ones(64, 1, device="cuda", dtype=torch.bfloat16), 4, 128, 1)
+        assert torch.equal(buf[0, 0, :64], x) and not buf[0, 0, 64:].any() and not buf[1:].any()
