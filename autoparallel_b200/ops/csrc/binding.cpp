@@ -24,7 +24,8 @@ int apb_gemm_get_reserved_sms();
 int apb_gemm_fused_ctas(int fuse, int M, int N, int comm_ctas, int num_sms);
 int apb_rms_norm_fwd(const void* x, const void* w, void* y, float* rstd, long long rows, int D, float eps, int is_bf16,
                      cudaStream_t st);
-int apb_rms_norm_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx, void* dw, float* dw_acc,
+long long apb_rms_norm_bwd_workspace(long long rows, int D, int is_bf16, int num_sms);
+int apb_rms_norm_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx, void* dw, float* part,
                      long long rows, int D, int is_bf16, int num_sms, cudaStream_t st);
 int apb_cast(const void* src, void* dst, long long n, int src_bf16, int dst_bf16, int num_sms, cudaStream_t st);
 int apb_rope(const void* x, const float* cs, const float* sn, void* y, long long B, int S, int H, int D, int conj, int is_bf16,
@@ -159,11 +160,14 @@ void rms_norm_fwd(const at::Tensor& x, const at::Tensor& w, at::Tensor& y, at::T
 }
 
 void rms_norm_bwd(const at::Tensor& dy, const at::Tensor& x, const at::Tensor& w, const at::Tensor& rstd, at::Tensor& dx,
-                  at::Tensor& dw, at::Tensor& dw_acc) {
+                  at::Tensor& dw) {
   c10::cuda::CUDAGuard g(x.device());
   const int D = x.size(-1);
+  const int64_t rows = x.numel() / D;
+  const bool bf16 = is_bf16(x);
+  at::Tensor part = at::empty({(int64_t)apb_rms_norm_bwd_workspace(rows, D, bf16, num_sms())}, rstd.options());  // partial sums of dw
   check(apb_rms_norm_bwd(dy.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr<float>(), dx.data_ptr(), dw.data_ptr(),
-                         dw_acc.data_ptr<float>(), x.numel() / D, D, is_bf16(x), num_sms(), stream()),
+                         part.data_ptr<float>(), rows, D, bf16, num_sms(), stream()),
         "apb_rms_norm_bwd");
 }
 

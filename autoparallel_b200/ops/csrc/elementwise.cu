@@ -143,19 +143,34 @@ __device__ __forceinline__ void block_sum_multi(float (&v)[R], float* red) {
   for (int k = 0; k < R; ++k) v[k] = warp_sum(l < nw ? red[k * 32 + l] : 0.f);
 }
 
+// Where a backward block leaves its weight-gradient sums: its own row of fp32 partial sums, or (``stride`` 0) added with
+// atomics to one row that the caller zeroed.
+struct RmsDw {
+  float* base;
+  long long stride;  // floats between the blocks' rows
+  __device__ __forceinline__ void put(int col, const float (&v)[8]) const {
+    if (stride) {
+      float4* p = reinterpret_cast<float4*>(base + blockIdx.x * stride + col);
+      p[0] = make_float4(v[0], v[1], v[2], v[3]);
+      p[1] = make_float4(v[4], v[5], v[6], v[7]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) atomicAdd(base + col + i, v[i]);
+    }
+  }
+};
+
 // Backward.  One persistent block per SM (a single wave).  Every iteration takes ROWS rows at once and the loads of
 // the next iteration are issued before the current one is reduced and stored (two register sets that swap roles, so
 // nothing is copied): the row loop is bound by memory bandwidth rather than by one load-reduce-store round trip per
 // row.  The ROWS dot products share one block reduction.  Math per element: g*x once, then two fused multiply-adds
 // (weight-gradient partial and dot product); the second pass forms dx = g*(r*w) - x*(r*r*mean) with two more.
 // EXACT: D == blockDim.x * 8 * NVEC and rows % ROWS == 0, so no bounds predicate is needed anywhere.
-// dw partial sums per thread-owned columns are added into ``dw_acc`` (fp32 [D], zeroed by the caller) with one
-// atomicAdd per column per block.  Requires D <= blockDim.x * 8 * RMS_BWD_MAX_VEC.
+// Requires D <= blockDim.x * 8 * RMS_BWD_MAX_VEC.
 constexpr int RMS_BWD_MAX_VEC = 4;
 template <typename T, int NVEC, int ROWS, bool EXACT>
 __global__ void __launch_bounds__(512) rms_norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ w,
-                                                           const float* __restrict__ rstd, T* __restrict__ dx, float* __restrict__ dw_acc,
-                                                           long long rows, int D) {
+                                                           const float* __restrict__ rstd, T* __restrict__ dx, RmsDw dw, long long rows, int D) {
   __shared__ float red[32 * ROWS];
   float wreg[NVEC][8];
   float dwreg[NVEC][8];
@@ -245,32 +260,31 @@ __global__ void __launch_bounds__(512) rms_norm_bwd_kernel(const T* __restrict__
     row0 += step;
   }
 #pragma unroll
-  for (int j = 0; j < NVEC; ++j) {
-    if (EXACT || col[j] < D) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) atomicAdd(dw_acc + col[j] + i, dwreg[j][i]);
-    }
-  }
+  for (int j = 0; j < NVEC; ++j)
+    if (EXACT || col[j] < D) dw.put(col[j], dwreg[j]);
 }
 
-// Backward, bulk-copy form (the one the launcher prefers).  The rows of x and dy travel global -> shared memory as
-// untiled bulk copies (``cp.async.bulk``, completion on an mbarrier) through a ring of RMS_STAGES stages of ROWS rows,
-// issued two stages ahead by one thread, so the prefetch costs no registers and the copy engine keeps the memory
-// system busy while the block reduces and stores the current rows.  Each thread reads its 16-byte column groups from
-// shared memory twice (dot product / weight-gradient pass, then the dx pass) instead of holding them in registers.
-// One block per SM; waits are bounded: if a stage never arrives the block stops (its rows keep whatever dx held).
+// Backward, bulk-copy form (the one the launcher prefers).  Bound by memory: x and dy are read once, dx is written once.
+// One row per step and block; the rows travel global -> shared memory as untiled bulk copies (``cp.async.bulk``,
+// completion on an mbarrier) through a ring of RMS_STAGES stages, issued two steps ahead by one thread, so the prefetch
+// costs no registers.  Blocks are small and several share an SM: while one waits at its barrier the others work (a single
+// 512-thread block per SM taking four rows a step spent half its time in the reduction: 8192 x 4096 bf16 59 -> 33 us, 999 x 2048 20 -> 6 us, fp32 2047 x 2048 21 -> 10 us).
+// One block barrier per step: the partial sums of consecutive steps sit in alternating slots, and a stage is refilled
+// after the barrier of the following step, which every thread reaches only when it has read the stage for the last time.
+// Waits are bounded: if a stage never arrives the block stops (its rows keep whatever dx held).
 constexpr int RMS_STAGES = 3;
-template <typename T, int NVEC, int ROWS>
-__global__ void __launch_bounds__(512) rms_norm_bwd_bulk_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ w,
-                                                                const float* __restrict__ rstd, T* __restrict__ dx,
-                                                                float* __restrict__ dw_acc, long long rows, int D) {
+__host__ __device__ inline int rms_ring_bytes(int row_bytes) { return RMS_STAGES * 2 * row_bytes + 128; }
+template <typename T, int NVEC, int THREADS>
+__global__ void __launch_bounds__(THREADS, NVEC == 2 && THREADS == 512 ? 2 : 1) rms_norm_bwd_bulk_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ w,
+                                                                    const float* __restrict__ rstd, T* __restrict__ dx, RmsDw dw,
+                                                                    long long rows, int D) {
   extern __shared__ uint8_t rms_smem_raw[];
+  __shared__ uint64_t bars[RMS_STAGES];
+  __shared__ float red[2][THREADS / 32];
   __shared__ uint32_t abort_word;
+  constexpr bool KEEP = sizeof(T) == 2;  // the row stays in registers between the two passes (fp32: read from shared memory again)
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(rms_smem_raw) + 127) & ~uintptr_t(127));
   const int row_bytes = D * (int)sizeof(T);
-  const int stage_bytes = ROWS * row_bytes;  // per tensor
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + RMS_STAGES * 2 * stage_bytes);
-  float* red = reinterpret_cast<float*>(bars + RMS_STAGES);
   volatile uint32_t* abort_flag = &abort_word;
   if (threadIdx.x == 0) {
     for (int s_ = 0; s_ < RMS_STAGES; ++s_) mbar_init(&bars[s_], 1);
@@ -278,98 +292,107 @@ __global__ void __launch_bounds__(512) rms_norm_bwd_bulk_kernel(const T* __restr
     mbar_fence_init();
   }
   __syncthreads();
-
-  float wreg[NVEC][8], dwreg[NVEC][8];
-  int col[NVEC];
-#pragma unroll
-  for (int j = 0; j < NVEC; ++j) {
-    col[j] = (threadIdx.x + j * blockDim.x) * 8;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      dwreg[j][i] = 0.f;
-      wreg[j][i] = 0.f;
-    }
-    if (col[j] < D) {
-      Vec8<T> wv; wv.load(w + col[j]); wv.to_float(wreg[j]);
-    }
-  }
-  const float inv_d = 1.f / D;
-  const long long step = (long long)gridDim.x * ROWS;
-  const long long first = (long long)blockIdx.x * ROWS;
-  auto issue = [&](long long it) {  // one thread: start the copies of this block's iteration ``it``
-    const long long row0 = first + it * step;
-    if (row0 >= rows) return;
+  const long long step = gridDim.x, first = blockIdx.x;
+  auto issue = [&](long long it) {  // one thread: start the copies of this block's step ``it``
+    const long long row = first + it * step;
+    if (row >= rows) return;
     const int st = (int)(it % RMS_STAGES);
-    const long long nrows = rows - row0 < ROWS ? rows - row0 : ROWS;
-    const uint32_t bytes = (uint32_t)(nrows * row_bytes);
-    mbar_expect_tx(&bars[st], 2u * bytes);
-    bulk_load(smem + (2 * st) * stage_bytes, x + row0 * D, bytes, &bars[st]);
-    bulk_load(smem + (2 * st + 1) * stage_bytes, dy + row0 * D, bytes, &bars[st]);
+    mbar_expect_tx(&bars[st], 2u * row_bytes);
+    bulk_load(smem + (2 * st) * row_bytes, x + row * D, row_bytes, &bars[st]);
+    bulk_load(smem + (2 * st + 1) * row_bytes, dy + row * D, row_bytes, &bars[st]);
   };
   if (threadIdx.x == 0)
     for (int it = 0; it < RMS_STAGES - 1; ++it) issue(it);
 
-  long long it = 0;
-  for (long long row0 = first; row0 < rows; row0 += step, ++it) {
-    if (threadIdx.x == 0) issue(it + RMS_STAGES - 1);  // refills the stage every thread left at the end of the last iteration
-    const int st = (int)(it % RMS_STAGES);
-    if (!mbar_wait(&bars[st], (uint32_t)((it / RMS_STAGES) & 1), abort_flag)) {
-      *abort_flag = 1;
-      break;
-    }
-    const uint8_t* xs = smem + (2 * st) * stage_bytes;
-    const uint8_t* gs = xs + stage_bytes;
-    float dot[ROWS], r[ROWS];
-#pragma unroll
-    for (int k = 0; k < ROWS; ++k) {
-      dot[k] = 0.f;
-      const bool row_ok = row0 + k < rows;
-      r[k] = row_ok ? rstd[row0 + k] : 0.f;
-#pragma unroll
-      for (int j = 0; j < NVEC; ++j) {
-        if (row_ok && col[j] < D) {
-          Vec8<T> xv, gv;
-          xv.load(reinterpret_cast<const T*>(xs + k * row_bytes) + col[j]);
-          gv.load(reinterpret_cast<const T*>(gs + k * row_bytes) + col[j]);
-          float xf[8], gf[8]; xv.to_float(xf); gv.to_float(gf);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float gx = gf[i] * xf[i];
-            dwreg[j][i] = fmaf(gx, r[k], dwreg[j][i]);
-            dot[k] = fmaf(gx, wreg[j][i], dot[k]);
-          }
-        }
-      }
-    }
-    block_sum_multi<ROWS>(dot, red);
-#pragma unroll
-    for (int k = 0; k < ROWS; ++k) {
-      const long long row = row0 + k;
-      const float c = r[k] * r[k] * r[k] * dot[k] * inv_d;
-      if (row < rows) {
-#pragma unroll
-        for (int j = 0; j < NVEC; ++j) {
-          if (col[j] < D) {
-            Vec8<T> xv, gv;
-            xv.load(reinterpret_cast<const T*>(xs + k * row_bytes) + col[j]);
-            gv.load(reinterpret_cast<const T*>(gs + k * row_bytes) + col[j]);
-            float xf[8], gf[8], o[8]; xv.to_float(xf); gv.to_float(gf);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) o[i] = fmaf(gf[i], r[k] * wreg[j][i], -xf[i] * c);
-            Vec8<T> ov; ov.from_float(o); ov.store(dx + row * D + col[j]);
-          }
-        }
-      }
-    }
-    __syncthreads();  // every thread has read this stage for the last time: it may be refilled
-  }
+  Vec8<T> wv[NVEC];
+  float dwreg[NVEC][8];
+  int col[NVEC];
 #pragma unroll
   for (int j = 0; j < NVEC; ++j) {
-    if (col[j] < D) {
+    col[j] = (threadIdx.x + j * THREADS) * 8;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) atomicAdd(dw_acc + col[j] + i, dwreg[j][i]);
+    for (int i = 0; i < 8; ++i) dwreg[j][i] = 0.f;
+    if (col[j] < D) wv[j].load(w + col[j]);
+  }
+  const float inv_d = 1.f / D;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  long long it = 0;
+  float r_next = first < rows ? rstd[first] : 0.f;
+  for (long long row = first; row < rows; row += step, ++it) {
+    const int st = (int)(it % RMS_STAGES);
+    const float r = r_next;
+    if (row + step < rows) r_next = rstd[row + step];
+    if (!mbar_wait(&bars[st], (uint32_t)((it / RMS_STAGES) & 1), abort_flag)) *abort_flag = 1;
+    const T* xs = reinterpret_cast<const T*>(smem + (2 * st) * row_bytes);
+    const T* gs = reinterpret_cast<const T*>(smem + (2 * st + 1) * row_bytes);
+    Vec8<T> xk[KEEP ? NVEC : 1], gk[KEEP ? NVEC : 1];
+    float dot = 0.f;
+#pragma unroll
+    for (int j = 0; j < NVEC; ++j) {
+      if (col[j] < D) {
+        Vec8<T>& xv = xk[KEEP ? j : 0];
+        Vec8<T>& gv = gk[KEEP ? j : 0];
+        xv.load(xs + col[j]);
+        gv.load(gs + col[j]);
+        float xf[8], gf[8], wf[8]; xv.to_float(xf); gv.to_float(gf); wv[j].to_float(wf);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float gx = gf[i] * xf[i];
+          dwreg[j][i] = fmaf(gx, r, dwreg[j][i]);
+          dot = fmaf(gx, wf[i], dot);
+        }
+      }
+    }
+    dot = warp_sum(dot);
+    if (THREADS > 32) {
+      if (lane == 0) red[it & 1][warp] = dot;
+      __syncthreads();
+      dot = 0.f;
+#pragma unroll
+      for (int k = 0; k < THREADS / 32; ++k) dot += red[it & 1][k];
+    } else {
+      __syncwarp();
+    }
+    if (*abort_flag) break;  // (set before the barrier, so every thread leaves here)
+    if (threadIdx.x == 0) issue(it + RMS_STAGES - 1);
+    const float c = r * r * r * dot * inv_d;
+#pragma unroll
+    for (int j = 0; j < NVEC; ++j) {
+      if (col[j] < D) {
+        Vec8<T>& xv = xk[KEEP ? j : 0];
+        Vec8<T>& gv = gk[KEEP ? j : 0];
+        if (!KEEP) {
+          xv.load(xs + col[j]);
+          gv.load(gs + col[j]);
+        }
+        float xf[8], gf[8], wf[8], o[8]; xv.to_float(xf); gv.to_float(gf); wv[j].to_float(wf);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) o[i] = fmaf(gf[i], r * wf[i], -xf[i] * c);
+        Vec8<T> ov; ov.from_float(o); ov.store(dx + row * D + col[j]);
+      }
     }
   }
+#pragma unroll
+  for (int j = 0; j < NVEC; ++j)
+    if (col[j] < D) dw.put(col[j], dwreg[j]);
+}
+
+// dw = column sums of the blocks' partial rows: 32 columns per block, 32 groups of partial rows
+template <typename T>
+__global__ void __launch_bounds__(1024) rms_dw_kernel(const float* __restrict__ part, T* __restrict__ dw, int nparts, int D) {
+  __shared__ float red[32][33];
+  const int c = blockIdx.x * 32 + (threadIdx.x & 31), g = threadIdx.x >> 5;
+  float s = 0.f;
+  if (c < D) {
+#pragma unroll 8
+    for (int b = g; b < nparts; b += 32) s += part[(long long)b * D + c];
+  }
+  red[g][threadIdx.x & 31] = s;
+  __syncthreads();
+  s = warp_sum(red[threadIdx.x & 31][g]);
+  const int co = blockIdx.x * 32 + g;
+  if ((threadIdx.x & 31) == 0 && co < D) dw[co] = T(s);
 }
 
 template <typename T>
@@ -598,49 +621,64 @@ __global__ void adamw_kernel(const AdamTensor* __restrict__ tensors, const int2*
   }
 }
 
-// Launch configuration of rms_norm_bwd_kernel: as many threads as 8-element vectors in a row (up to
-// 1024) so each thread keeps ONE vector per operand in registers; that keeps the register count low
-// enough for several resident blocks per SM, which is what a latency-bound row loop needs.
+// Blocks of the backward launch: at most ``per_sm`` per SM and, below that, four rows each, so that few rows don't pay for
+// more partial rows of dw than they have rows worth summing; but never fewer blocks than rows or SMs allow.
+static inline int rms_grid(long long rows, int num_sms, int per_sm) {
+  const long long cap = (long long)num_sms * per_sm, quarter = (rows + 3) / 4;
+  long long g = quarter < cap ? quarter : cap;
+  const long long least = rows < num_sms ? rows : num_sms;
+  return (int)(g > least ? g : least);
+}
+// bulk form: rows short enough for three stages in shared memory and 16-byte aligned
+static inline bool rms_bulk(const void* dy, const void* x, int D, int elem) {
+  return rms_ring_bytes(D * elem) <= 200 * 1024 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dy)) % 16 == 0);
+}
+// Threads of a block of the bulk form: a warp per row up to D = 256, one vector per thread up to 256 threads, then two, then
+// 512 threads.  Blocks per SM: what shared memory holds, up to 768 threads' worth of rows in flight (1024 for the widest).
+struct RmsPlan {
+  int threads, nvec, per_sm;
+};
+static inline RmsPlan rms_plan(int D, int elem) {
+  const int vecs = D / 8;
+  RmsPlan p;
+  p.threads = vecs <= 32 ? 32 : vecs <= 64 ? 64 : vecs <= 128 ? 128 : vecs <= 512 ? 256 : 512;
+  const int nv = (vecs + p.threads - 1) / p.threads;
+  p.nvec = nv <= 2 ? nv : 4;
+  const int by_smem = 220 * 1024 / (rms_ring_bytes(D * elem) + 2048);
+  const int by_threads = p.threads == 32 ? 16 : p.threads == 512 ? (p.nvec == 2 ? 2 : 1) : 768 / p.threads;
+  p.per_sm = by_smem < 1 ? 1 : by_smem < by_threads ? by_smem : by_threads;
+  return p;
+}
+
+// Launches the row kernel; returns the number of blocks (= partial rows of dw when ``stride`` is not 0), < 0 on error.
 template <typename T>
-static inline int launch_rms_norm_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx, float* dw_acc,
-                                      long long rows, int D, int num_sms, cudaStream_t st) {
+static inline int launch_rms_norm_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx, float* dw_base,
+                                      long long stride, long long rows, int D, int num_sms, cudaStream_t st) {
+  const RmsDw dw{dw_base, stride};
+  if (rms_bulk(dy, x, D, (int)sizeof(T))) {
+    const int smem = rms_ring_bytes(D * (int)sizeof(T));
+    const RmsPlan plan = rms_plan(D, (int)sizeof(T));
+    const int grid = rms_grid(rows, num_sms, plan.per_sm);
+#define APB_RMS_BULK(NV, TH)                                                                                             \
+  if (plan.nvec == NV && plan.threads == TH) {                                                                           \
+    auto kern = rms_norm_bwd_bulk_kernel<T, NV, TH>;                                                                     \
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -4;         \
+    kern<<<grid, TH, smem, st>>>((const T*)dy, (const T*)x, (const T*)w, rstd, (T*)dx, dw, rows, D);                     \
+    return grid;                                                                                                         \
+  }
+    APB_RMS_BULK(1, 32)
+    APB_RMS_BULK(1, 64)
+    APB_RMS_BULK(1, 128)
+    APB_RMS_BULK(1, 256)
+    APB_RMS_BULK(2, 256)
+    APB_RMS_BULK(2, 512)
+    APB_RMS_BULK(4, 512)
+#undef APB_RMS_BULK
+  }
   int threads = 128;
   while (threads * 8 < D && threads < 512) threads *= 2;  // at most 512 threads: 128 registers each
   const int nvec = (D + threads * 8 - 1) / (threads * 8);
-  if (nvec > RMS_BWD_MAX_VEC) return 3;
-  // Preferred: the bulk-copy form, whenever three stages of at least one row of both tensors fit in shared memory.
-  {
-    const long long row_bytes = (long long)D * (long long)sizeof(T);
-    int rows_per_stage = 0;
-    for (int cand : {4, 2, 1})
-      if (RMS_STAGES * 2 * cand * row_bytes + 1024 <= 200 * 1024) {
-        rows_per_stage = cand;
-        break;
-      }
-    if (rows_per_stage > 0 && (reinterpret_cast<uintptr_t>(x) % 16 == 0) && (reinterpret_cast<uintptr_t>(dy) % 16 == 0)) {
-      const int smem = (int)(RMS_STAGES * 2 * rows_per_stage * row_bytes + 128 + RMS_STAGES * 8 + 32 * rows_per_stage * 4 + 128);
-      const long long iters = (rows + rows_per_stage - 1) / rows_per_stage;
-      const int grid = (int)(iters < num_sms ? iters : num_sms);
-#define APB_RMS_BULK(NV, RW)                                                                                                      \
-  {                                                                                                                               \
-    auto kern = rms_norm_bwd_bulk_kernel<T, NV, RW>;                                                                              \
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return 4;                   \
-    kern<<<grid, threads, smem, st>>>((const T*)dy, (const T*)x, (const T*)w, rstd, (T*)dx, dw_acc, rows, D);                     \
-    return 0;                                                                                                                     \
-  }
-#define APB_RMS_BULK_ROWS(NV)                                \
-  {                                                          \
-    if (rows_per_stage == 4) APB_RMS_BULK(NV, 4)             \
-    else if (rows_per_stage == 2) APB_RMS_BULK(NV, 2)        \
-    else APB_RMS_BULK(NV, 1)                                 \
-  }
-      if (nvec == 1) APB_RMS_BULK_ROWS(1)
-      else if (nvec == 2) APB_RMS_BULK_ROWS(2)
-      else APB_RMS_BULK_ROWS(4)
-#undef APB_RMS_BULK_ROWS
-#undef APB_RMS_BULK
-    }
-  }
+  if (nvec > RMS_BWD_MAX_VEC) return -3;
   const int per_sm = threads >= 512 ? 1 : (threads >= 256 ? 2 : 4);  // resident blocks at 128 registers per thread: one wave
   const long long cap = (long long)num_sms * per_sm;
   // rows per iteration: as many as the registers hold (16-byte vectors for bf16, two per vector for fp32)
@@ -650,15 +688,15 @@ static inline int launch_rms_norm_bwd(const void* dy, const void* x, const void*
     const long long iters = (rows + RW - 1) / RW;                                                                        \
     const int grid = (int)(iters < cap ? iters : cap);                                                                   \
     if (D == threads * 8 * NV && rows % RW == 0)                                                                         \
-      rms_norm_bwd_kernel<T, NV, RW, true><<<grid, threads, 0, st>>>((const T*)dy, (const T*)x, (const T*)w, rstd, (T*)dx, dw_acc, rows, D); \
+      rms_norm_bwd_kernel<T, NV, RW, true><<<grid, threads, 0, st>>>((const T*)dy, (const T*)x, (const T*)w, rstd, (T*)dx, dw, rows, D); \
     else                                                                                                                 \
-      rms_norm_bwd_kernel<T, NV, RW, false><<<grid, threads, 0, st>>>((const T*)dy, (const T*)x, (const T*)w, rstd, (T*)dx, dw_acc, rows, D); \
+      rms_norm_bwd_kernel<T, NV, RW, false><<<grid, threads, 0, st>>>((const T*)dy, (const T*)x, (const T*)w, rstd, (T*)dx, dw, rows, D); \
+    return grid;                                                                                                         \
   }
   if (nvec == 1) { if constexpr (wide) APB_RMS_BWD(1, 2) else APB_RMS_BWD(1, 4) }
   else if (nvec == 2) { if constexpr (wide) APB_RMS_BWD(2, 1) else APB_RMS_BWD(2, 2) }
   else APB_RMS_BWD(4, 1)  // (nvec 3 runs as 4 with the last vector masked)
 #undef APB_RMS_BWD
-  return 0;
 }
 
 static inline int grid_for(long long work_items, int threads, int num_sms) {
@@ -712,19 +750,23 @@ int apb_rms_norm_fwd(const void* x, const void* w, void* y, float* rstd, long lo
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 
-// dw_acc: fp32 [D] scratch, zeroed here; dw receives the cast result.
-int apb_rms_norm_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx, void* dw, float* dw_acc,
+// floats of workspace for apb_rms_norm_bwd: one partial row of dw per block, whichever form runs
+long long apb_rms_norm_bwd_workspace(long long rows, int D, int is_bf16, int num_sms) {
+  const int bulk = rms_grid(rows, num_sms, rms_plan(D, is_bf16 ? 2 : 4).per_sm);
+  const long long other = rows < 4ll * num_sms ? rows : 4ll * num_sms;
+  return (bulk > other ? bulk : other) * D;
+}
+
+int apb_rms_norm_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx, void* dw, float* part,
                      long long rows, int D, int is_bf16, int num_sms, cudaStream_t st) {
   if (D % 8) return 3;
   if (D > 512 * 8 * RMS_BWD_MAX_VEC) return 3;
-  cudaMemsetAsync(dw_acc, 0, sizeof(float) * D, st);
+  int n = 0;
   if (rows > 0) {
-    int e;
-    DISPATCH(is_bf16, e = launch_rms_norm_bwd<T>(dy, x, w, rstd, dx, dw_acc, rows, D, num_sms, st));
-    if (e) return e;
+    DISPATCH(is_bf16, n = launch_rms_norm_bwd<T>(dy, x, w, rstd, dx, part, D, rows, D, num_sms, st));
+    if (n < 0) return -n;
   }
-  if (is_bf16) cast_from_f32_kernel<bf16><<<grid_for(D / 8, 256, num_sms), 256, 0, st>>>(dw_acc, (bf16*)dw, D);
-  else cudaMemcpyAsync(dw, dw_acc, sizeof(float) * D, cudaMemcpyDeviceToDevice, st);
+  DISPATCH(is_bf16, rms_dw_kernel<T><<<(D + 31) / 32, 1024, 0, st>>>(part, (T*)dw, n, D));
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 
@@ -856,9 +898,9 @@ extern "C" int apb_rms_norm_bwd_noalloc(const void* dy, const void* x, const voi
   // the array keeps the previous call's sums: start from zero
   if (cudaMemsetAsync(acc, 0, sizeof(float) * D, st) != cudaSuccess) return APB_NOALLOC_ERR_LAUNCH;
   if (rows > 0) {
-    int e;
-    DISPATCH(is_bf16, e = launch_rms_norm_bwd<T>(dy, x, w, rstd, dx, acc, rows, D, num_sms, st));
-    if (e) return APB_NOALLOC_ERR_BAD_SHAPE;
+    int n;
+    DISPATCH(is_bf16, n = launch_rms_norm_bwd<T>(dy, x, w, rstd, dx, acc, 0, rows, D, num_sms, st));
+    if (n < 0) return APB_NOALLOC_ERR_BAD_SHAPE;
   }
   if (is_bf16) {
     cast_from_f32_kernel<bf16><<<grid_for(D / 8, 256, num_sms), 256, 0, st>>>(acc, (bf16*)dw, D);

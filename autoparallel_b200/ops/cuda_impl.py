@@ -27,7 +27,6 @@ from . import library as L
 _C = None
 _lock = threading.Lock()
 _status: dict[int, torch.Tensor] = {}
-_scratch: dict[tuple, torch.Tensor] = {}
 launch_count = 0  # kernels of this extension launched since import (bench bookkeeping)
 #: calls answered by a library kernel instead of this extension's, by kind
 library_fallbacks: dict[str, int] = {}
@@ -99,15 +98,6 @@ def check_status(device=None) -> None:
         if code != 0:
             t.zero_()
             raise RuntimeError(f"apb200 kernel status {code} on cuda:{idx}: {STATUS_NAMES.get(code, 'unknown')}")
-
-
-def _scratch_f32(device, n: int) -> torch.Tensor:
-    key = (torch.device(device).index or 0, "f32")
-    t = _scratch.get(key)
-    if t is None or t.numel() < n:
-        t = torch.empty(max(n, 16384), dtype=torch.float32, device=device)
-        _scratch[key] = t
-    return t
 
 
 def _count(n: int = 1) -> None:
@@ -318,8 +308,8 @@ def _rms_norm_bwd(dy, x, w, rstd):
     dy, x = dy.contiguous(), x.contiguous()
     dx = torch.empty_like(x)
     dw = torch.empty_like(w, dtype=x.dtype)
-    _C.rms_norm_bwd(dy, x, w.to(x.dtype).contiguous(), rstd.contiguous(), dx, dw, _scratch_f32(x.device, x.shape[-1]))
-    _count(3)
+    _C.rms_norm_bwd(dy, x, w.to(x.dtype).contiguous(), rstd.contiguous(), dx, dw)
+    _count(2)
     return dx, dw.to(w.dtype)
 
 

@@ -98,3 +98,25 @@ def test_moe_dispatch_leaves_nothing_of_the_old_buffer(K):
         del junk
         buf = lib.ops.moe_scatter(x, slot, torch.ones(64, 1, device="cuda", dtype=torch.bfloat16), 4, 128, 1)
         assert torch.equal(buf[0, 0, :64], x) and not buf[0, 0, 64:].any() and not buf[1:].any()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows", [1, 3, 149, 5000])
+@pytest.mark.parametrize("D", [8, 256, 264, 768, 1032, 2048, 4096, 5120, 8192, 16384])
+def test_rms_norm_gradients_over_row_widths(K, dtype, rows, D):
+    """One row, fewer rows than SMs, one more, several steps per block; widths on both sides of every block size and, in
+    fp32, past what the staged form holds."""
+    lib, _ = K
+    g = torch.Generator(device="cuda").manual_seed(rows + D)
+    x = torch.randn(rows, D, device="cuda", generator=g).to(dtype)
+    w = (1 + 0.1 * torch.randn(D, device="cuda", generator=g)).to(dtype)
+    dy = torch.randn(rows, D, device="cuda", generator=g).to(dtype)
+    _, rstd = lib.ops.rms_norm(x, w, 1e-5)
+    dx, dw = lib.ops.rms_norm_bwd(dy, x, w, rstd)
+    xd, wd, gd, rd = x.double(), w.double(), dy.double(), rstd.double().unsqueeze(-1)
+    xh = xd * rd
+    gw = gd * wd
+    # fp32 sums over a row (dx) and over the rows (dw): 2^-24 times the square root of their length, generously, then one rounding
+    tol = 2**-8 if dtype == torch.bfloat16 else 2**-24 * 16 * max(rows, D) ** 0.5
+    assert _rel(dx, rd * (gw - xh * (gw * xh).mean(-1, keepdim=True))) <= tol
+    assert _rel(dw, (gd * xh).sum(0)) <= tol
