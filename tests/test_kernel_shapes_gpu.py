@@ -120,3 +120,48 @@ def test_rms_norm_gradients_over_row_widths(K, dtype, rows, D):
     tol = 2**-8 if dtype == torch.bfloat16 else 2**-24 * 16 * max(rows, D) ** 0.5
     assert _rel(dx, rd * (gw - xh * (gw * xh).mean(-1, keepdim=True))) <= tol
     assert _rel(dw, (gd * xh).sum(0)) <= tol
+
+
+@pytest.mark.parametrize("M,N,K_", [
+    (256, 256, 64),     # one pair tile, one k-block
+    (4104, 4104, 64),   # every pair busy, both edges end inside a 32-row / 64-column store
+    (5000, 4136, 136),  # a row edge inside a warp's block, K past a k-block
+    (20000, 264, 8),    # a column tile of eight columns
+])
+@pytest.mark.parametrize("ta,tb", [(False, True), (True, False)])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("pair", [True, False])
+def test_gemm_stores_whole_tiles_and_nothing_else(K, M, N, K_, ta, tb, out_dtype, pair):
+    lib, impl = K
+    ext = impl.extension()
+    g = torch.Generator(device="cuda").manual_seed(M)
+    a = torch.randn((K_, M) if ta else (M, K_), device="cuda", generator=g).to(torch.bfloat16)
+    b = torch.randn((N, K_) if tb else (K_, N), device="cuda", generator=g).to(torch.bfloat16)
+    back = torch.full((M + 2, N + 64), 7.0, device="cuda", dtype=out_dtype)  # the result is a window of a wider matrix
+    c = back[1:M + 1, 32:N + 32]
+    prev = ext.gemm_get_pair_mode()
+    ext.gemm_set_pair_mode(pair)
+    try:
+        ext.gemm(a, b, c, ta, not tb, impl.status_buffer(a.device))
+        torch.cuda.synchronize()
+    finally:
+        ext.gemm_set_pair_mode(prev)
+    ref = (a.t() if ta else a).double() @ (b.t() if tb else b).double()
+    # fp32 accumulation of K products (2^-24 sqrt(K), generously), one rounding to bf16
+    assert _rel(c, ref) <= (2**-8 if out_dtype == torch.bfloat16 else 2**-24 * 8 * K_ ** 0.5)
+    back[1:M + 1, 32:N + 32] = 7.0
+    assert bool((back == 7.0).all()), "nothing outside the window is written"
+
+
+@pytest.mark.parametrize("E,M,N,K_", [(5, 160, 1408, 136), (3, 320, 72, 64), (4, 1000, 264, 72)])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+def test_grouped_gemm_keeps_group_edges(K, E, M, N, K_, out_dtype):
+    """M and N end inside a store block: the next group's first rows must not be overwritten."""
+    lib, _ = K
+    g = torch.Generator(device="cuda").manual_seed(M)
+    a = torch.randn(E, M, K_, device="cuda", generator=g).to(torch.bfloat16)
+    w = torch.randn(E, K_, N, device="cuda", generator=g).to(torch.bfloat16)
+    dy = torch.randn(E, M, N, device="cuda", generator=g).to(torch.bfloat16)
+    bf16 = out_dtype == torch.bfloat16
+    assert _rel(lib.ops.grouped_mm(a, w, False, out_dtype), a.double() @ w.double()) <= (2**-8 if bf16 else 2**-24 * 8 * K_ ** 0.5)
+    assert _rel(lib.ops.grouped_mm_wgrad(a, dy, out_dtype), a.double().transpose(1, 2) @ dy.double()) <= (2**-8 if bf16 else 2**-24 * 8 * M ** 0.5)
