@@ -165,3 +165,28 @@ def test_grouped_gemm_keeps_group_edges(K, E, M, N, K_, out_dtype):
     bf16 = out_dtype == torch.bfloat16
     assert _rel(lib.ops.grouped_mm(a, w, False, out_dtype), a.double() @ w.double()) <= (2**-8 if bf16 else 2**-24 * 8 * K_ ** 0.5)
     assert _rel(lib.ops.grouped_mm_wgrad(a, dy, out_dtype), a.double().transpose(1, 2) @ dy.double()) <= (2**-8 if bf16 else 2**-24 * 8 * M ** 0.5)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("V", [8, 1024, 4096 + 8, 8192, 16384 - 8, 16384, 16384 + 4096 + 8, 128256])
+def test_cross_entropy_over_row_widths(K, dtype, V):
+    """Rows below, at and past a full unrolled step of every block size; rows with masked (-inf and lowest) entries."""
+    lib, _ = K
+    g = torch.Generator(device="cuda").manual_seed(V)
+    rows = 5
+    logits = (3 * torch.randn(rows, V, device="cuda", generator=g)).to(dtype)
+    labels = torch.randint(0, V, (rows,), device="cuda", generator=g)
+    logits[1, : V // 2] = float("-inf")
+    logits[2, V // 2:] = torch.finfo(dtype).min
+    labels[1], labels[2] = V - 1, 0
+    loss, lse = lib.ops.cross_entropy(logits, labels)
+    ld = logits.double()
+    ref = torch.logsumexp(ld, -1)
+    picked = ld.gather(-1, labels.unsqueeze(-1)).squeeze(-1)
+    # the exponentials are the hardware's (2^-21 relative each); their sum is fp32, the values are of order 10
+    assert _rel(lse, ref) <= 2**-19 and (loss.double() - (ref - picked)).abs().max().item() <= 2**-19 * 16
+    dl = torch.randn(rows, device="cuda", generator=g)
+    d = lib.ops.cross_entropy_bwd(dl, logits, labels, lse)
+    p = torch.softmax(ld, -1)
+    p[torch.arange(rows), labels] -= 1
+    assert _rel(d, p * dl.double().unsqueeze(-1)) <= (2**-8 if dtype == torch.bfloat16 else 2**-18)
