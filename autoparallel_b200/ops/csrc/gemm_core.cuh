@@ -788,8 +788,15 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
+// The encoder is a driver call: unlike the runtime's calls it does not give a thread that has made none of those yet (an
+// autograd worker whose first work is a GEMM) the device's context, so the thread binds it once itself.
 inline EncodeTiledFn get_encode() {
   static EncodeTiledFn fn = nullptr;
+  static thread_local bool bound = false;
+  if (!bound) {
+    int dev = 0;
+    bound = cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess;
+  }
   if (fn == nullptr) {
     void* p = nullptr;
     cudaDriverEntryPointQueryResult q;
