@@ -11,6 +11,8 @@ int apb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, lo
                   int a_mn_major, int b_mn_major, int out_fp32, uint32_t* status, int num_sms, cudaStream_t stream);
 int apb_gemm_grouped_bf16(const void* A, const void* B, void* C, int G, int M, int N, int K, int a_mn_major, int b_mn_major,
                           int out_fp32, uint32_t* status, int num_sms, cudaStream_t stream);
+int apb_gemm_split(const void* A, const void* B, void* C, int G, int M, int N, int K, long long lda, long long ldb, long long ldc,
+                   int a_mn, int b_mn, int out_fp32, int bn, int s, uint32_t* status, cudaStream_t stream);
 void apb_gemm_set_pair_mode(int on);
 int apb_gemm_get_pair_mode();
 int apb_gemm_yield_request(int pairs, cudaStream_t stream);
@@ -127,6 +129,30 @@ void gemm_grouped(const at::Tensor& a, const at::Tensor& b, at::Tensor& c, bool 
   check(apb_gemm_grouped_bf16(a.data_ptr(), b.data_ptr(), c.data_ptr(), G, M, N, K, a_mn_major, b_mn_major, out_fp32,
                               reinterpret_cast<uint32_t*>(status.data_ptr()), num_sms(), stream()),
         "apb_gemm_grouped_bf16");
+}
+
+// The cluster split-k kernel (gemm_split.cu) with an explicit tile width and slice count; 2-d operands as in ``gemm`` or
+// contiguous 3-d stacks as in ``gemm_grouped``.
+void gemm_split(const at::Tensor& a, const at::Tensor& b, at::Tensor& c, bool a_mn_major, bool b_mn_major, int64_t bn, int64_t slices,
+                at::Tensor& status) {
+  c10::cuda::CUDAGuard g(a.device());
+  const int64_t d = c.dim();
+  TORCH_CHECK(a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16 && (d == 2 || d == 3) && a.dim() == d && b.dim() == d &&
+                  a.stride(-1) == 1 && b.stride(-1) == 1 && c.stride(-1) == 1,
+              "gemm_split: bf16 row-major operands, 2-d or 3-d");
+  TORCH_CHECK(d == 2 || (a.is_contiguous() && b.is_contiguous() && c.is_contiguous() && a.size(0) == c.size(0) && b.size(0) == c.size(0)),
+              "gemm_split: contiguous stacks required");
+  const int M = c.size(-2), N = c.size(-1);
+  const int K = a_mn_major ? a.size(-2) : a.size(-1);
+  TORCH_CHECK((a_mn_major ? a.size(-1) : a.size(-2)) == M && (b_mn_major ? b.size(-1) : b.size(-2)) == N &&
+                  (b_mn_major ? b.size(-2) : b.size(-1)) == K,
+              "gemm_split: shape mismatch");
+  const bool out_fp32 = c.scalar_type() == at::kFloat;
+  TORCH_CHECK(out_fp32 || c.scalar_type() == at::kBFloat16, "gemm_split: output must be bf16 or fp32");
+  check(apb_gemm_split(a.data_ptr(), b.data_ptr(), c.data_ptr(), d == 3 ? (int)c.size(0) : 0, M, N, K, a.stride(-2), b.stride(-2),
+                       c.stride(-2), a_mn_major, b_mn_major, out_fp32, (int)bn, (int)slices,
+                       reinterpret_cast<uint32_t*>(status.data_ptr()), stream()),
+        "apb_gemm_split");
 }
 
 // q [B,S,H,D], k / v [B,Sk,Hkv,D] -> out [B,S,H,D] bf16, lse [B,H,S] fp32.  Returns false (nothing launched) for
@@ -419,6 +445,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("dma_rs_sum", &dma_rs_sum);
   m.def("gemm", &gemm);
   m.def("gemm_grouped", &gemm_grouped);
+  m.def("gemm_split", &gemm_split);
   m.def("gemm_set_pair_mode", [](bool on) { apb_gemm_set_pair_mode(on ? 1 : 0); });
   m.def("gemm_yield_request", [](int64_t pairs) { check(apb_gemm_yield_request((int)pairs, stream()), "apb_gemm_yield_request"); });
   m.def("gemm_yield_outstanding", []() { return (int64_t)apb_gemm_yield_outstanding(); });

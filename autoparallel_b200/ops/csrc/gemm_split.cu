@@ -1,0 +1,383 @@
+// bf16 GEMM for shapes with few output tiles, sm_100a: one 128 x BN tile per thread-block cluster, the contraction split
+// over the cluster's CTAs.
+//
+//   C[M,N] = opA * opB, operands and layouts as in gemm_tcgen05.cu; grouped form: G stacked problems of one shape
+//
+// The persistent kernels give every CTA (pair) whole tiles of 128 or 256 x 256, so a product with fewer tiles than SMs
+// leaves most of the chip idle: 16 x 4096 x 4096 ran on 16 SMs, a router's weight gradient (64 x 2048, contracted over
+// 8192 tokens) on 8, each waiting for its own serial chain of loads.  Here BN (64, 128, 256) and the number of k-slices S
+// (1..8) are picked so that tiles x S fills the SMs.  Every CTA of a cluster accumulates its k-slice in TMEM, writes the
+// fp32 tile to its own shared memory (the load stages are free by then), and after one cluster barrier each CTA adds up
+// its share of the tile's rows from all S shared memories, in slice order, and stores it: no workspace, no atomics, no
+// second launch, the same result every time.
+//
+//   warp 0: TMA producer | warp 1: TMEM owner + MMA issuer | warps 2..5: TMEM -> shared memory | all: sum and store
+// Before -> after, us: 16 x 4096 x 4096 28 -> 12, 16 x 4096 x 14336 88 -> 27, 64 x 2048 x 2048 16 -> 8.6, 64 x 2048 x 8192 47 -> 16,
+// 512 x 256 x 256 7.4 -> 6.1, 999 x 1408 x 2048 18.8 -> 17.0.
+#include "gemm_core.cuh"
+
+namespace apb {
+
+constexpr int SPLIT_MAX = 8;  // portable cluster size
+constexpr int SPLIT_STAGE_TOTAL = 196608;  // 8 x 24 KB, 6 x 32 KB or 4 x 48 KB: deep enough for one CTA to hide the load latency
+constexpr int SPLIT_SMEM_BYTES = SPLIT_STAGE_TOTAL + 1024 + 256;
+
+__device__ __forceinline__ uint32_t cluster_size() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+
+template <bool A_MN, bool B_MN, int BN_T, bool GROUPED>
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
+gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
+  constexpr int B_BYTES = BN_T * BK * 2;
+  constexpr int ST = SPLIT_STAGE_TOTAL / (A_STAGE_BYTES + B_BYTES);
+  constexpr int LD = BN_T + 4;  // floats per row of the fp32 tile: rows start 16 bytes apart modulo the banks
+  static_assert(BM * LD * 4 <= SPLIT_STAGE_TOTAL, "the fp32 tile reuses the stages");
+  static_assert((2 * ST + 1) * 8 + 8 <= 256, "barrier block");
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* sA = smem;
+  uint8_t* sB = smem + ST * A_STAGE_BYTES;
+  float* tile = reinterpret_cast<float*>(smem);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + SPLIT_STAGE_TOTAL);
+  uint64_t* empty = full + ST;
+  uint64_t* tmem_full = empty + ST;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_full + 1);
+  volatile uint32_t* abort_flag = tmem_slot + 1;
+
+  const int S = (int)cluster_size(), slice = (int)cluster_ctarank();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int per_group = p.num_m_tiles * p.num_n_tiles;
+  const int t = blockIdx.x / S;
+  const int grp = GROUPED ? t / per_group : 0;
+  int tm, tn;
+  tile_coords(GROUPED ? t - grp * per_group : t, p.num_m_tiles, p.num_n_tiles, tm, tn);
+  const int m0 = tm * BM, n0 = tn * BN_T;
+  const int num_kb = (p.K + BK - 1) / BK;
+  const int kb0 = (int)((long long)num_kb * slice / S), kb1 = (int)((long long)num_kb * (slice + 1) / S);  // S <= num_kb: never empty
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < ST; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    mbar_init(tmem_full, 1);
+    *abort_flag = 0;
+    mbar_fence_init();
+    tma_prefetch_desc(&tmA);
+    tma_prefetch_desc(&tmB);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, BN_T);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  auto fail = [&](uint32_t code) {
+    atomicCAS(p.status, 0u, code);
+    *abort_flag = 1;
+  };
+
+  if (warp == 0) {
+    if (lane == 0) {
+      for (int kb = kb0, i = 0; kb < kb1; ++kb, ++i) {
+        const int stage = i % ST;
+        if (!mbar_wait(&empty[stage], ((i / ST) & 1) ^ 1, abort_flag)) {
+          fail(ST_TIMEOUT_EMPTY);
+          break;
+        }
+        auto load = [&](uint8_t* dst, const CUtensorMap* m, int x, int y) {
+          if (GROUPED) tma_load_3d(dst, m, &full[stage], x, y, grp);
+          else tma_load_2d(dst, m, &full[stage], x, y);
+        };
+        mbar_expect_tx(&full[stage], A_STAGE_BYTES + B_BYTES);
+        uint8_t* a_dst = sA + stage * A_STAGE_BYTES;
+        uint8_t* b_dst = sB + stage * B_BYTES;
+        if (!A_MN) {
+          load(a_dst, &tmA, kb * BK, m0);
+        } else {
+#pragma unroll
+          for (int c = 0; c < BM / 64; ++c) load(a_dst + c * CHUNK_BYTES, &tmA, m0 + c * 64, kb * BK);
+        }
+        if (!B_MN) {
+          load(b_dst, &tmB, kb * BK, n0);
+        } else {
+#pragma unroll
+          for (int c = 0; c < BN_T / 64; ++c) load(b_dst + c * CHUNK_BYTES, &tmB, n0 + c * 64, kb * BK);
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = make_idesc_bf16(BM, BN_T, A_MN ? 1u : 0u, B_MN ? 1u : 0u);
+      bool ok = true;
+      for (int kb = kb0, i = 0; kb < kb1; ++kb, ++i) {
+        const int stage = i % ST;
+        if (!mbar_wait(&full[stage], (i / ST) & 1, abort_flag)) {
+          fail(ST_TIMEOUT_FULL);
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t a_addr = smem_u32(sA + stage * A_STAGE_BYTES);
+        const uint32_t b_addr = smem_u32(sB + stage * B_BYTES);
+#pragma unroll
+        for (int k = 0; k < BK / UMMA_K; ++k) {
+          const uint64_t a_desc = A_MN ? make_smem_desc(a_addr + k * (UMMA_K * 128), CHUNK_BYTES, 1024)
+                                       : make_smem_desc(a_addr + k * (UMMA_K * 2), 16, 1024);
+          const uint64_t b_desc = B_MN ? make_smem_desc(b_addr + k * (UMMA_K * 128), CHUNK_BYTES, 1024)
+                                       : make_smem_desc(b_addr + k * (UMMA_K * 2), 16, 1024);
+          umma_f16(tmem_base, a_desc, b_desc, idesc, (i > 0 || k > 0) ? 1u : 0u);
+        }
+        umma_commit(&empty[stage]);
+      }
+      if (ok) umma_commit(tmem_full);
+    }
+    __syncwarp();
+  } else {
+    const int q = warp & 3;  // TMEM lane quarter this warp may read
+    // (the TMEM loads are warp-wide: the warp goes on together or not at all)
+    if (__all_sync(0xffffffffu, mbar_wait(tmem_full, 0, abort_flag))) {
+      tc_fence_after();
+      float* row = tile + (q * 32 + lane) * LD;
+#pragma unroll
+      for (int c = 0; c < BN_T / 32; ++c) {
+        uint32_t r[32];
+        tmem_ld_32x32(tmem_base + (uint32_t(q * 32) << 16) + c * 32, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          reinterpret_cast<uint4*>(row + c * 32)[i] = make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
+      }
+    } else {
+      fail(ST_TIMEOUT_TMEM_FULL);
+    }
+  }
+  tc_fence_before();
+  cluster_arrive();  // (also orders the threads of a cluster of one CTA)
+  cluster_wait();
+
+  if (*abort_flag == 0) {
+    const bool vec = p.out_fp32 ? (p.ldc & 3) == 0 : (p.ldc & 7) == 0;
+    const long long c_off = GROUPED ? (long long)grp * p.M * p.ldc : 0;
+    // eight columns per thread; the tile's vectors are dealt to the CTAs of the cluster in blocks of one per thread
+    for (int v = slice * GEMM_THREADS + threadIdx.x; v < BM * (BN_T / 8); v += S * GEMM_THREADS) {
+      const int r = v / (BN_T / 8), c = (v % (BN_T / 8)) * 8;
+      const long long row = m0 + r;
+      const int col = n0 + c;
+      if (row >= p.M || col >= p.N) continue;
+      float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+      const float* src = tile + r * LD + c;
+#pragma unroll 4
+      for (int s = 0; s < S; ++s) {
+        const uint32_t addr = map_to_cta(src, (uint32_t)s);
+        const float4 x = ld_cluster_f4(addr), y = ld_cluster_f4(addr + 16);
+        a.x += x.x; a.y += x.y; a.z += x.z; a.w += x.w;
+        b.x += y.x; b.y += y.y; b.z += y.z; b.w += y.w;
+      }
+      const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+      const long long off = c_off + row * p.ldc + col;
+      if (p.out_fp32) {
+        float* dst = reinterpret_cast<float*>(p.C) + off;
+        if (vec && col + 8 <= p.N) {
+          reinterpret_cast<float4*>(dst)[0] = a;
+          reinterpret_cast<float4*>(dst)[1] = b;
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            if (col + i < p.N) dst[i] = f[i];
+        }
+      } else {
+        __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + off;
+        if (vec && col + 8 <= p.N) {
+          *reinterpret_cast<uint4*>(dst) = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            if (col + i < p.N) dst[i] = __float2bfloat16(f[i]);
+        }
+      }
+    }
+  }
+  cluster_arrive();  // no CTA leaves while another may still read its tile
+  cluster_wait();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, BN_T);
+  }
+}
+
+}  // namespace apb
+
+using namespace apb;
+
+typedef void (*SplitKernel)(CUtensorMap, CUtensorMap, GemmParams);
+
+template <int BN_T, bool GROUPED>
+static SplitKernel split_kernel_of(int a_mn, int b_mn) {
+  if (!a_mn && !b_mn) return gemm_split_kernel<false, false, BN_T, GROUPED>;
+  if (!a_mn) return gemm_split_kernel<false, true, BN_T, GROUPED>;
+  if (!b_mn) return gemm_split_kernel<true, false, BN_T, GROUPED>;
+  return gemm_split_kernel<true, true, BN_T, GROUPED>;
+}
+
+template <bool GROUPED>
+static SplitKernel split_kernel_of(int bn, int a_mn, int b_mn) {
+  return bn == 64 ? split_kernel_of<64, GROUPED>(a_mn, b_mn) : bn == 128 ? split_kernel_of<128, GROUPED>(a_mn, b_mn)
+                                                                         : split_kernel_of<256, GROUPED>(a_mn, b_mn);
+}
+
+// Tile width and slice count for a product, or bn = 0 where the persistent kernels are expected to be faster.
+//
+// Only forms whose clusters are all resident at once: in a second wave every tile pays its fixed part again, and the
+// persistent kernels were faster in every such case of the sweeps (16 x 4096 x 4096 ... 8192 x 1024 x 4096, all widths and
+// slice counts).  The estimates (microseconds, one B200) are fitted to those sweeps: a fixed part that grows with the tile
+// (launch, prologue, TMEM -> shared memory -> C), then the longest of a chain of k-blocks, the operand traffic out of L2
+// (9.5 TB/s) and the operands out of memory (6.5 TB/s, less while few bytes are in flight), then the cluster's sum.
+// Over the sweeps the choice was always faster than the persistent kernels and within 20 % of the best form.
+struct SplitPlan {
+  int bn, s;
+};
+extern "C" int apb_gemm_resident_pairs(int num_sms);
+
+static SplitKernel split_kernel_any() { return gemm_split_kernel<false, false, 64, false>; }
+
+// CTAs of clusters of ``s`` that are resident at once (one CTA per SM; the partial ends of the GPCs are lost); asked once
+// per device and size.
+static int split_slots(int s, int num_sms) {
+  static int cached[64][SPLIT_MAX + 1];  // 0 = not asked yet; the answer is the same whoever asks
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && cached[dev][s] > 0) return cached[dev][s];
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(num_sms / s * s));
+  cfg.blockDim = dim3(GEMM_THREADS);
+  cfg.dynamicSmemBytes = SPLIT_SMEM_BYTES;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)s;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  SplitKernel kern = split_kernel_any();
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SPLIT_SMEM_BYTES) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
+    cudaGetLastError();
+    n = num_sms / s / 2;
+  }
+  if (dev >= 0 && dev < 64) cached[dev][s] = n * s;
+  return n * s;
+}
+
+static SplitPlan split_plan(int G, int M, int N, int K, int num_sms) {
+  const long long g = G > 0 ? G : 1;
+  const long long m_tiles = (M + BM - 1) / BM;
+  SplitPlan best{0, 0};
+  if (g * m_tiles * ((N + 255) / 256) > num_sms) return best;  // no width fits in one wave
+  const int kb = (K + BK - 1) / BK;
+  const bool pair = M >= 2 * BM && N >= BN;
+  const long long tiles = g * (pair ? (M + 2 * BM - 1) / (2 * BM) : m_tiles) * ((N + BN - 1) / BN);
+  const int units = pair ? apb_gemm_resident_pairs(num_sms) : num_sms;
+  const double now = 5.5 + (double)((tiles + units - 1) / units) * (0.5 + (pair ? 0.38 : 0.35) * kb);
+  const double operands = 2.0 * g * ((double)M * K + (double)N * K);
+  double t_best = 0.95 * now;  // (a clear gain only: the estimates are good to ten per cent or so)
+  for (int bn = 64; bn <= 256; bn *= 2) {
+    const double fixed = bn == 64 ? 5.6 : bn == 128 ? 7.0 : 9.0, per_kb = bn == 128 ? 0.20 : 0.27;
+    const long long t = g * m_tiles * ((N + bn - 1) / bn);
+    const double kb_bytes = 128.0 * ((M < BM ? M : BM) + (N < bn ? N : bn));
+    for (int s = 1; s <= SPLIT_MAX && s <= kb; ++s) {
+      if (t * s > num_sms) break;
+      if (t * s > split_slots(s, num_sms)) continue;
+      const int chain = (kb + s - 1) / s;
+      double flow = per_kb * chain;
+      const double l2 = (double)t * kb * kb_bytes / 9.5e6;
+      if (l2 > flow) flow = l2;
+      // megabytes in flight: the stages of all CTAs, rows and columns outside the matrices not counted
+      const double flight = 0.1875 * t * s * kb_bytes / (128.0 * (BM + bn));
+      const double from_memory = operands / (flight < 10.5 ? 0.62e6 * flight : 6.5e6);
+      if (from_memory > flow) flow = from_memory;
+      const double est = fixed + flow + (s > 1 ? 0.05 * s * bn / 64 : 0.0);
+      if (est < t_best) {
+        t_best = est;
+        best = SplitPlan{bn, s};
+      }
+    }
+  }
+  return best;
+}
+
+// One launch with the given tile width (64, 128, 256) and number of k-slices (1..8, at most one per 64 of K).  G > 0: grouped,
+// dense stacks (lda / ldb / ldc ignored).  Returns 0, or an argument / driver error (nothing launched).
+extern "C" int apb_gemm_split(const void* A, const void* B, void* C, int G, int M, int N, int K, long long lda, long long ldb, long long ldc,
+                              int a_mn, int b_mn, int out_fp32, int bn, int s, uint32_t* status, cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (bn != 64 && bn != 128 && bn != 256) return 3;
+  if (s < 1 || s > SPLIT_MAX || s > (K + BK - 1) / BK) return 3;
+  const bool grouped = G > 0;
+  if (grouped) {
+    lda = a_mn ? M : K;
+    ldb = b_mn ? N : K;
+    ldc = N;
+  }
+  if ((lda & 7) || (ldb & 7) ||
+      ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 15))
+    return 3;  // 16-byte bases and rows for TMA and for the vector stores
+  CUtensorMap tmA, tmB;
+  int e;
+  if (grouped) {
+    e = !a_mn ? make_map_3d(&tmA, A, (uint64_t)K, (uint64_t)M, (uint64_t)G, (uint64_t)lda, BM)
+              : make_map_3d(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)G, (uint64_t)lda, BK);
+    if (e) return e;
+    e = !b_mn ? make_map_3d(&tmB, B, (uint64_t)K, (uint64_t)N, (uint64_t)G, (uint64_t)ldb, bn)
+              : make_map_3d(&tmB, B, (uint64_t)N, (uint64_t)K, (uint64_t)G, (uint64_t)ldb, BK);
+  } else {
+    e = !a_mn ? make_map(&tmA, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda, BM) : make_map(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, BK);
+    if (e) return e;
+    e = !b_mn ? make_map(&tmB, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, bn) : make_map(&tmB, B, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, BK);
+  }
+  if (e) return e;
+  GemmParams p;
+  p.M = M; p.N = N; p.K = K; p.C = C; p.ldc = ldc; p.out_fp32 = out_fp32;
+  p.num_m_tiles = (M + BM - 1) / BM;
+  p.num_n_tiles = (N + bn - 1) / bn;
+  p.status = status;
+  p.groups = grouped ? G : 1;
+  const long long ctas = (long long)p.num_m_tiles * p.num_n_tiles * p.groups * s;
+  if (ctas > 0x7fffffffll / s) return 3;
+  SplitKernel kern = grouped ? split_kernel_of<true>(bn, a_mn, b_mn) : split_kernel_of<false>(bn, a_mn, b_mn);
+  // (the attribute belongs to the current device's instance of the kernel)
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SPLIT_SMEM_BYTES) != cudaSuccess) return 4;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)ctas);
+  cfg.blockDim = dim3(GEMM_THREADS);
+  cfg.dynamicSmemBytes = SPLIT_SMEM_BYTES;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)s;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, tmA, tmB, p) == cudaSuccess && cudaGetLastError() == cudaSuccess ? 0 : 4;
+}
+
+// The rule above and its launch: 0 = launched, -1 = the caller's kernels are the better choice (nothing launched), > 0 = error.
+extern "C" int apb_gemm_split_auto(const void* A, const void* B, void* C, int G, int M, int N, int K, long long lda, long long ldb,
+                                   long long ldc, int a_mn, int b_mn, int out_fp32, uint32_t* status, int num_sms, cudaStream_t stream) {
+  const SplitPlan plan = split_plan(G, M, N, K, num_sms);
+  if (plan.bn == 0) return -1;
+  return apb_gemm_split(A, B, C, G, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_fp32, plan.bn, plan.s, status, stream);
+}

@@ -147,12 +147,21 @@ extern "C" int apb_gemm_get_reserved_sms() { return g_reserved_sms; }
 extern "C" void apb_gemm_set_pair_mode(int on) { g_pair_mode = on ? 1 : 0; }
 extern "C" int apb_gemm_get_pair_mode() { return g_pair_mode; }
 
+// gemm_split.cu: products with few tiles; -1 = the kernels here are the better choice
+extern "C" int apb_gemm_split_auto(const void* A, const void* B, void* C, int G, int M, int N, int K, long long lda, long long ldb,
+                                   long long ldc, int a_mn, int b_mn, int out_fp32, uint32_t* status, int num_sms, cudaStream_t stream);
+
 // Returns 0 on success; >0 = argument / driver error (nothing launched).
 extern "C" int apb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
                              long long ldc, int a_mn_major, int b_mn_major, int out_fp32, uint32_t* status,
                              int num_sms, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (reinterpret_cast<uintptr_t>(C) & 15) return 3;
+  const int usable = num_sms - g_reserved_sms > 0 ? num_sms - g_reserved_sms : 1;
+  if (g_pair_mode) {
+    const int es = apb_gemm_split_auto(A, B, C, 0, M, N, K, lda, ldb, ldc, a_mn_major, b_mn_major, out_fp32, status, usable, stream);
+    if (es >= 0) return es;
+  }
   CUtensorMap tmA, tmB;
   const int e = make_operand_maps(&tmA, &tmB, A, B, M, N, K, lda, ldb, a_mn_major, b_mn_major);
   if (e) return e;  // TMA needs 16-byte aligned bases and row strides
@@ -201,7 +210,6 @@ extern "C" int apb_gemm_bf16(const void* A, const void* B, void* C, int M, int N
     return cudaGetLastError() == cudaSuccess ? 0 : 4;
   }
   const int tiles = p.num_m_tiles * p.num_n_tiles;
-  const int usable = num_sms - g_reserved_sms > 0 ? num_sms - g_reserved_sms : 1;
   const int grid = tiles < usable ? tiles : usable;
   auto launch = [&](auto kern) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_PLAIN_SMEM_BYTES);
@@ -222,6 +230,11 @@ extern "C" int apb_gemm_grouped_bf16(const void* A, const void* B, void* C, int 
   const int a_inner = a_mn_major ? M : K, b_inner = b_mn_major ? N : K;
   if ((a_inner & 7) || (b_inner & 7) || (N & 7)) return 3;  // 16-byte rows for TMA and for the vector stores
   if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) || (reinterpret_cast<uintptr_t>(C) & 15)) return 3;
+  const int usable = num_sms - g_reserved_sms > 0 ? num_sms - g_reserved_sms : 1;
+  if (g_pair_mode) {
+    const int es = apb_gemm_split_auto(A, B, C, G, M, N, K, 0, 0, 0, a_mn_major, b_mn_major, out_fp32, status, usable, stream);
+    if (es >= 0) return es;
+  }
   const bool pair = g_pair_mode && M >= 2 * BM && N >= BN;
   CUtensorMap tmA, tmB;
   int e = !a_mn_major ? make_map_3d(&tmA, A, (uint64_t)K, (uint64_t)M, (uint64_t)G, (uint64_t)K, BM)
@@ -255,7 +268,6 @@ extern "C" int apb_gemm_grouped_bf16(const void* A, const void* B, void* C, int 
     else launch(gemm_grouped_pair_kernel<true, true>, grid);
   } else {
     const long long tiles = (long long)G * p.num_m_tiles * p.num_n_tiles;
-    const int usable = num_sms - g_reserved_sms > 0 ? num_sms - g_reserved_sms : 1;
     const int grid = (int)(tiles < usable ? tiles : usable);
     if (!a_mn_major && !b_mn_major) launch(gemm_grouped_kernel<false, false>, grid);
     else if (!a_mn_major && b_mn_major) launch(gemm_grouped_kernel<false, true>, grid);

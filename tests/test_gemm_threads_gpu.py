@@ -1,4 +1,5 @@
 """The GEMM called from a thread that has done no CUDA work before."""
+import os
 import subprocess
 import sys
 
@@ -23,5 +24,6 @@ t.start(), t.join()
 torch.cuda.synchronize()
 assert torch.equal(out[0], ref)
 """
-    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300,
+                       cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
     assert r.returncode == 0, r.stderr[-2000:]

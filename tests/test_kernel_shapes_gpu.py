@@ -190,3 +190,41 @@ def test_cross_entropy_over_row_widths(K, dtype, V):
     p = torch.softmax(ld, -1)
     p[torch.arange(rows), labels] -= 1
     assert _rel(d, p * dl.double().unsqueeze(-1)) <= (2**-8 if dtype == torch.bfloat16 else 2**-18)
+
+
+@pytest.mark.parametrize("M,N,K_", [(1, 8, 8), (16, 4096, 4096), (64, 2048, 8192), (129, 264, 520), (1000, 1408, 2048), (300, 72, 1096)])
+@pytest.mark.parametrize("ta,tb", [(False, True), (False, False), (True, False), (True, True)])
+@pytest.mark.parametrize("bn,slices", [(0, 0), (64, 8), (64, 1), (128, 3), (256, 5), (256, 2)])
+def test_gemm_split_over_tiles_and_slices(K, M, N, K_, ta, tb, bn, slices):
+    """Tile widths and slice counts, ragged in every dimension, inside a wider matrix; (0, 0) = what the rule picks."""
+    lib, impl = K
+    ext = impl.extension()
+    if (ta and M % 8) or slices > (K_ + 63) // 64:
+        pytest.skip("not a form of this kernel")
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    a = torch.randn((K_, M) if ta else (M, K_), device="cuda", generator=g).to(torch.bfloat16)
+    b = torch.randn((N, K_) if tb else (K_, N), device="cuda", generator=g).to(torch.bfloat16)
+    ref = (a.t() if ta else a).double() @ (b.t() if tb else b).double()
+    for dtype in (torch.float32, torch.bfloat16):
+        back = torch.full((M + 2, N + 64), 7.0, device="cuda", dtype=dtype)
+        c = back[1:M + 1, 32:N + 32]
+        if bn:
+            ext.gemm_split(a, b, c, ta, not tb, bn, slices, impl.status_buffer(a.device))
+        else:
+            ext.gemm(a, b, c, ta, not tb, impl.status_buffer(a.device))
+        # fp32 accumulation of K products (2^-24 sqrt(K), generously), one rounding to bf16
+        assert _rel(c, ref) <= (2**-8 if dtype == torch.bfloat16 else 2**-24 * 8 * max(K_, 64) ** 0.5)
+        back[1:M + 1, 32:N + 32] = 7.0
+        assert bool((back == 7.0).all()), "nothing outside the window is written"
+
+
+@pytest.mark.parametrize("bn,slices", [(64, 2), (128, 1), (256, 3)])
+def test_grouped_gemm_split(K, bn, slices):
+    lib, impl = K
+    E, M, N, K_ = 3, 200, 328, 264
+    g = torch.Generator(device="cuda").manual_seed(bn)
+    a = torch.randn(E, M, K_, device="cuda", generator=g).to(torch.bfloat16)
+    w = torch.randn(E, K_, N, device="cuda", generator=g).to(torch.bfloat16)
+    c = torch.empty(E, M, N, device="cuda", dtype=torch.float32)
+    impl.extension().gemm_split(a, w, c, False, True, bn, slices, impl.status_buffer(a.device))
+    assert _rel(c, a.double() @ w.double()) <= 2**-24 * 8 * K_ ** 0.5
