@@ -228,3 +228,24 @@ def test_grouped_gemm_split(K, bn, slices):
     c = torch.empty(E, M, N, device="cuda", dtype=torch.float32)
     impl.extension().gemm_split(a, w, c, False, True, bn, slices, impl.status_buffer(a.device))
     assert _rel(c, a.double() @ w.double()) <= 2**-24 * 8 * K_ ** 0.5
+
+
+@pytest.mark.parametrize("M", [129, 136, 160, 248])
+@pytest.mark.parametrize("ta", [False, True])
+def test_pairs_with_less_than_two_full_row_tiles(K, M, ta):
+    """The odd CTA of a pair holds 1 to 120 rows; enough columns and groups that the persistent pair kernels run."""
+    lib, impl = K
+    if ta and M % 8:
+        pytest.skip("rows of 16 bytes")
+    E, N, K_ = 24, 1408, 192
+    g = torch.Generator(device="cuda").manual_seed(M)
+    a = torch.randn(*((E, K_, M) if ta else (E, M, K_)), device="cuda", generator=g).to(torch.bfloat16)
+    w = torch.randn(E, K_, N, device="cuda", generator=g).to(torch.bfloat16)
+    if ta:
+        got, ref = lib.ops.grouped_mm_wgrad(a, w, torch.float32), a.double().transpose(1, 2) @ w.double()
+    else:
+        got, ref = lib.ops.grouped_mm(a, w, False, torch.float32), a.double() @ w.double()
+    assert _rel(got, ref) <= 2**-24 * 8 * K_ ** 0.5  # fp32 accumulation of K products
+    x, y = a[0], torch.randn(K_, 20480, device="cuda", generator=g).to(torch.bfloat16)
+    out = lib.ops.gemm(x, y, ta, False, torch.float32)
+    assert _rel(out, (x.double().t() if ta else x.double()) @ y.double()) <= 2**-24 * 8 * K_ ** 0.5
