@@ -339,6 +339,75 @@ void adamw(const at::Tensor& table, const at::Tensor& chunks, int64_t num_chunks
         "apb_adamw");
 }
 
+// ------------------------------------------------------------------ whole operators: checks, allocation and launch in one call
+// What ops/cuda_impl.py asks for first; an empty result means "not this kernel's form" and is answered there.
+
+// [rows, last] with unit inner stride, rows of 16 bytes and an aligned base, as TMA needs it
+at::Tensor as2d(const at::Tensor& t) {
+  at::Tensor m = t.dim() == 2 ? t : t.reshape({-1, t.size(-1)});
+  if (m.stride(1) != 1 || m.stride(0) % 8 != 0 || reinterpret_cast<uintptr_t>(m.data_ptr()) % 16 != 0) m = m.contiguous();
+  return m;
+}
+
+c10::optional<at::Tensor> gemm_new(const at::Tensor& a, const at::Tensor& b, bool a_mn, bool b_mn, bool out_fp32, at::Tensor& status) {
+  if (a.scalar_type() != at::kBFloat16 || b.scalar_type() != at::kBFloat16) return c10::nullopt;
+  at::Tensor a2 = as2d(a), b2 = as2d(b);
+  const int64_t M = a2.size(a_mn ? 1 : 0), N = b2.size(b_mn ? 1 : 0);
+  if (a2.size(1) % 8 || b2.size(1) % 8 || N % 8) return c10::nullopt;
+  at::Tensor c = at::empty({M, N}, a2.options().dtype(out_fp32 ? at::kFloat : at::kBFloat16));
+  gemm(a2, b2, c, a_mn, b_mn, status);
+  return c;
+}
+
+// a[..., K] x (b[N, K] or b[K, N]) -> [..., N]
+c10::optional<at::Tensor> mm_nd(const at::Tensor& a, const at::Tensor& b, bool trans_b, bool out_fp32, at::Tensor& status) {
+  auto c = gemm_new(a, b, false, !trans_b, out_fp32, status);
+  if (!c.has_value() || a.dim() == 2) return c;
+  auto shape = a.sizes().vec();
+  shape.back() = c->size(1);
+  return c->view(shape);
+}
+
+std::tuple<at::Tensor, at::Tensor> rms_norm_new(const at::Tensor& x_, const at::Tensor& w, double eps) {
+  at::Tensor x = x_.contiguous(), y = at::empty_like(x);
+  at::Tensor rstd = at::empty(x.sizes().slice(0, x.dim() - 1), x.options().dtype(at::kFloat));
+  rms_norm_fwd(x, w.to(x.scalar_type()).contiguous(), y, rstd, eps);
+  return {y, rstd};
+}
+
+std::tuple<at::Tensor, at::Tensor> rms_norm_bwd_new(const at::Tensor& dy_, const at::Tensor& x_, const at::Tensor& w, const at::Tensor& rstd) {
+  at::Tensor dy = dy_.contiguous(), x = x_.contiguous(), dx = at::empty_like(x), dw = at::empty_like(w, x.scalar_type());
+  rms_norm_bwd(dy, x, w.to(x.scalar_type()).contiguous(), rstd.contiguous(), dx, dw);
+  return {dx, dw.to(w.scalar_type())};
+}
+
+at::Tensor rope_new(const at::Tensor& x_, const at::Tensor& cs, const at::Tensor& sn, bool conj) {
+  at::Tensor x = x_.contiguous(), y = at::empty_like(x);
+  rope(x, cs.to(at::kFloat).contiguous(), sn.to(at::kFloat).contiguous(), y, conj);
+  return y;
+}
+
+at::Tensor swiglu_new(const at::Tensor& a_, const at::Tensor& b_) {
+  at::Tensor a = a_.contiguous(), b = b_.contiguous(), y = at::empty_like(a);
+  swiglu_fwd(a, b, y);
+  return y;
+}
+
+std::tuple<at::Tensor, at::Tensor> swiglu_bwd_new(const at::Tensor& dy_, const at::Tensor& a_, const at::Tensor& b_) {
+  at::Tensor dy = dy_.contiguous(), a = a_.contiguous(), b = b_.contiguous(), da = at::empty_like(a), db = at::empty_like(b);
+  swiglu_bwd(dy, a, b, da, db);
+  return {da, db};
+}
+
+// fp32 <-> bf16 copy of a contiguous, aligned tensor
+c10::optional<at::Tensor> cast_new(const at::Tensor& x, bool to_bf16) {
+  if (x.scalar_type() != (to_bf16 ? at::kFloat : at::kBFloat16) || !x.is_contiguous() || reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 != 0)
+    return c10::nullopt;
+  at::Tensor out = at::empty_like(x, to_bf16 ? at::kBFloat16 : at::kFloat);
+  cast(x, out);
+  return out;
+}
+
 int64_t symm_header_bytes() { return apb_symm_header_bytes(); }
 
 // Bounded wait on a device flag (int32 tensor, element 0) that the caller may or may not ever raise.
@@ -457,12 +526,14 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_get_reserved_sms", []() { return (int64_t)apb_gemm_get_reserved_sms(); });
   m.def("gemm_get_pair_mode", []() { return apb_gemm_get_pair_mode() != 0; });
   m.def("attention_fwd", &attention_fwd);
-  m.def("rms_norm_fwd", &rms_norm_fwd);
-  m.def("rms_norm_bwd", &rms_norm_bwd);
-  m.def("cast", &cast);
-  m.def("rope", &rope);
-  m.def("swiglu_fwd", &swiglu_fwd);
-  m.def("swiglu_bwd", &swiglu_bwd);
+  m.def("mm", &gemm_new);
+  m.def("mm_nd", &mm_nd);
+  m.def("rms_norm", &rms_norm_new);
+  m.def("rms_norm_bwd", &rms_norm_bwd_new);
+  m.def("rope", &rope_new);
+  m.def("swiglu", &swiglu_new);
+  m.def("swiglu_bwd", &swiglu_bwd_new);
+  m.def("cast", &cast_new);
   m.def("xent_fwd", &xent_fwd);
   m.def("xent_bwd", &xent_bwd);
   m.def("embedding_bwd", &embedding_bwd);

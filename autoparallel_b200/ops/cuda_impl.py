@@ -23,6 +23,7 @@ import threading
 import torch
 
 from . import library as L
+from . import shadow
 
 _C = None
 _lock = threading.Lock()
@@ -81,7 +82,7 @@ def ensure_loaded() -> None:
 
 
 def status_buffer(device) -> torch.Tensor:
-    idx = torch.device(device).index or 0
+    idx = (device if isinstance(device, torch.device) else torch.device(device)).index or 0
     t = _status.get(idx)
     if t is None:
         t = torch.zeros(4, dtype=torch.int32, device=torch.device("cuda", idx))
@@ -140,13 +141,26 @@ def _gemm(a, b, trans_a, trans_b, out_dtype):
     return gemm_raw(a2, b2, bool(trans_a), not trans_b, out_dtype)
 
 
+_NATIVE_OUT = (torch.bfloat16, torch.float32)
+
+
 def _mm_nd(a, b, trans_b, out_dtype):
+    if out_dtype in _NATIVE_OUT and not _DIAG_LIBRARY_GEMM:
+        out = _C.mm_nd(a, b, trans_b, out_dtype is torch.float32, status_buffer(a.device))
+        if out is not None:
+            _count()
+            return out
     lead = a.shape[:-1]
     out = gemm_raw(_as2d(a), _as2d(b), False, not trans_b, out_dtype)
     return out.view(*lead, out.shape[-1])
 
 
 def _mm_wgrad(a, b, out_dtype):
+    if out_dtype in _NATIVE_OUT and not _DIAG_LIBRARY_GEMM:
+        out = _C.mm(a, b, True, True, out_dtype is torch.float32, status_buffer(a.device))
+        if out is not None:
+            _count()
+            return out
     return gemm_raw(_as2d(a), _as2d(b), True, True, out_dtype)
 
 
@@ -280,61 +294,41 @@ def _moe_gate_grad(buf, slot, g):
 def _dtype_cast(x, dtype):
     if x.dtype == dtype:
         return x
-    from . import shadow
-
     hit = shadow.lookup(x, dtype)  # the optimizer already wrote this parameter in ``dtype``
     if hit is not None:
         return hit
-    pair = {x.dtype, dtype}
-    if pair == {torch.float32, torch.bfloat16} and x.is_contiguous() and x.data_ptr() % 16 == 0:
-        out = torch.empty_like(x, dtype=dtype)
-        _C.cast(x, out)
-        _count()
-        return out
+    if dtype is torch.bfloat16 or (dtype is torch.float32 and x.dtype is torch.bfloat16):
+        out = _C.cast(x, dtype is torch.bfloat16)
+        if out is not None:
+            _count()
+            return out
     _fallback("cast", f"{x.dtype} -> {dtype}, contiguous={x.is_contiguous()}")
     return x.to(dtype)
 
 
 def _rms_norm(x, w, eps):
-    x = x.contiguous()
-    y = torch.empty_like(x)
-    rstd = torch.empty(x.shape[:-1], dtype=torch.float32, device=x.device)
-    _C.rms_norm_fwd(x, w.to(x.dtype).contiguous(), y, rstd, eps)
     _count()
-    return y, rstd
+    return _C.rms_norm(x, w, eps)
 
 
 def _rms_norm_bwd(dy, x, w, rstd):
-    dy, x = dy.contiguous(), x.contiguous()
-    dx = torch.empty_like(x)
-    dw = torch.empty_like(w, dtype=x.dtype)
-    _C.rms_norm_bwd(dy, x, w.to(x.dtype).contiguous(), rstd.contiguous(), dx, dw)
     _count(2)
-    return dx, dw.to(w.dtype)
+    return _C.rms_norm_bwd(dy, x, w, rstd)
 
 
 def _rope(x, cos, sin, conj):
-    x = x.contiguous()
-    y = torch.empty_like(x)
-    _C.rope(x, cos.float().contiguous(), sin.float().contiguous(), y, conj)
     _count()
-    return y
+    return _C.rope(x, cos, sin, conj)
 
 
 def _swiglu(a, b):
-    a, b = a.contiguous(), b.contiguous()
-    y = torch.empty_like(a)
-    _C.swiglu_fwd(a, b, y)
     _count()
-    return y
+    return _C.swiglu(a, b)
 
 
 def _swiglu_bwd(dy, a, b):
-    dy, a, b = dy.contiguous(), a.contiguous(), b.contiguous()
-    da, db = torch.empty_like(a), torch.empty_like(b)
-    _C.swiglu_bwd(dy, a, b, da, db)
     _count()
-    return da, db
+    return _C.swiglu_bwd(dy, a, b)
 
 
 def _cross_entropy(logits, labels):
