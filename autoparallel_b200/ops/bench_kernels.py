@@ -118,12 +118,12 @@ def main():
             w = torch.rand(T_, k_, device=dev)
             slot = torch.ops.apb200.moe_slots(gi, E_, C_, 1)
             buf = torch.ops.apb200.moe_scatter(x, slot, w, E_, C_, 1)
-            moved = 2 * T_ * k_ * d_ * 2
+            tokens = T_ * d_ * 2  # bytes of the token matrix
             for name, fn, ref, nb_ in (
                     ("moe_slots", lambda: torch.ops.apb200.moe_slots(gi, E_, C_, 1), lambda: moe_ops._moe_slots(gi, E_, C_, 1), T_ * k_ * 16),
                     ("moe_scatter", lambda: torch.ops.apb200.moe_scatter(x, slot, w, E_, C_, 1), lambda: moe_ops._moe_scatter(x, slot, w, E_, C_, 1),
-                     moved + E_ * C_ * d_ * 2),
-                    ("moe_gather", lambda: torch.ops.apb200.moe_gather(buf, slot, w), lambda: moe_ops._moe_gather(buf, slot, w), moved)):
+                     tokens + E_ * C_ * d_ * 2),
+                    ("moe_gather", lambda: torch.ops.apb200.moe_gather(buf, slot, w), lambda: moe_ops._moe_gather(buf, slot, w), (k_ + 1) * tokens)):
                 ms, best = time_fn(lambda: (), fn, iters=3, pool=2)
                 rec(f"{name} {T_}x{k_} E={E_} C={C_} d={d_} (kernel)", ms, best, nbytes=nb_)
                 ms, best = time_fn(lambda: (), ref, iters=3, pool=2)

@@ -138,8 +138,9 @@ __device__ __forceinline__ void store_row_chunk(const GemmParams& p, long long r
 // Epilogue of the plain GEMM for one warp's 32 rows and NCOL / 32 accumulator chunks: 128 bytes of every row at a time go
 // to the warp's staging block (128-byte swizzle, conflict free) and from there to C as one TMA store.  A thread owns a
 // row, so storing straight from registers puts 16-byte pieces of 32 different lines into every instruction, half a sector
-// each; a product with a short contraction was bound by that (weight gradients of 64 experts, 2048 x 1408 over 160 rows: 217 us before, 137 us now).
-// The store of a block overlaps the TMEM loads of the next (a second block per warp measured no better); out-of-range rows and columns are clipped by the tensor map.
+// each; a product with a short contraction was bound by that (weight gradients of 64 experts, 2048 x 1408 over 160 rows:
+// 217 us before, 137 us now).  The store of a block overlaps the TMEM loads of the next (a second block per warp measured no
+// better); out-of-range rows and columns are clipped by the tensor map.
 template <bool OUT_FP32, bool GROUPED>
 __device__ __forceinline__ void store_tile_tma(const CUtensorMap* tmC, uint8_t* stg, uint32_t taddr, int row0, int n0, int ncols, int M, int N,
                                                int grp, int lane) {

@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(256) moe_scatter_kernel(const T* __restrict__ 
 // Gather: bound by reading k rows per token.  ``tx`` threads (a power of two, 32..256) take a token, one vector each;
 // rows and weights of eight choices at a time are worked out once per token in shared memory and their loads are issued
 // together.
-// 371 -> 104 us, 3.5 TB/s (2-byte loads, one row address per element before).
+// 371 -> 104 us, 2.9 TB/s (2-byte loads, one row address per element before).
 constexpr int GATHER_K = 8;
 template <typename T, int W>
 __global__ void __launch_bounds__(256) moe_gather_kernel(const T* __restrict__ buf, const long long* __restrict__ slot, const void* __restrict__ w,
