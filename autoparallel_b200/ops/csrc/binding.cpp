@@ -344,7 +344,8 @@ void adamw(const at::Tensor& table, const at::Tensor& chunks, int64_t num_chunks
 
 // [rows, last] with unit inner stride, rows of 16 bytes and an aligned base, as TMA needs it
 at::Tensor as2d(const at::Tensor& t) {
-  at::Tensor m = t.dim() == 2 ? t : t.reshape({-1, t.size(-1)});
+  // (a single row is reshaped too: contiguous() does not look at its stride, which TMA does; the reshape makes it the width)
+  at::Tensor m = t.dim() == 2 && t.size(0) > 1 && t.size(1) > 0 ? t : t.reshape({-1, t.size(-1)});
   if (m.stride(1) != 1 || m.stride(0) % 8 != 0 || reinterpret_cast<uintptr_t>(m.data_ptr()) % 16 != 0) m = m.contiguous();
   return m;
 }

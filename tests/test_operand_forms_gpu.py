@@ -1,0 +1,50 @@
+"""Operand forms at the edge of what the kernels read - one row, views, empty sizes - against the CPU formulas."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def K():
+    from autoparallel_b200.ops import cuda_impl, library
+
+    cuda_impl.ensure_loaded()
+    yield library, cuda_impl
+    cuda_impl.check_status()
+
+
+def _rel(a, b):
+    a, b = a.double().cpu(), b.double().cpu()
+    assert a.shape == b.shape
+    return ((a - b).norm() / b.norm().clamp_min(1e-30)).item()
+
+
+BF16_TOL = 2**-8  # fp32 sums of a few hundred products, one rounding to bf16
+
+
+@pytest.mark.parametrize("row", [
+    lambda g: torch.randn(3, 67, generator=g)[0:1, :64],   # odd leading stride
+    lambda g: torch.randn(64, 1, generator=g).t(),         # strides (1, 1)
+    lambda g: torch.randn(1, 130, generator=g)[:, ::2][:, :64],  # every other element
+])
+def test_products_with_a_single_row_of_any_stride(K, row):
+    """``contiguous()`` ignores the stride of a dimension of size one; a tensor map does not."""
+    lib, impl = K
+    g = torch.Generator().manual_seed(0)
+    a, w, dy = row(g).bfloat16(), torch.randn(96, 64, generator=g).bfloat16(), torch.randn(1, 96, generator=g).bfloat16()
+    assert a.shape == (1, 64)
+    ad = torch.empty_strided(a.size(), a.stride(), dtype=a.dtype, device="cuda").copy_(a)
+    before = dict(impl.library_fallbacks)
+    assert _rel(lib.ops.mm_nd(ad, w.cuda(), True, torch.bfloat16), a.double() @ w.double().t()) <= BF16_TOL
+    assert _rel(lib.ops.mm_nd(dy.cuda(), w.cuda(), False, torch.bfloat16), dy.double() @ w.double()) <= BF16_TOL
+    assert _rel(lib.ops.mm_wgrad(dy.cuda(), ad, torch.float32), dy.double().t() @ a.double()) <= 2**-22  # one product per element
+    assert _rel(lib.ops.mm_wgrad(ad, dy.cuda(), torch.float32), a.double().t() @ dy.double()) <= 2**-22
+    assert impl.library_fallbacks == before
+
+
+def test_matrices_without_columns_stay_refused(K):
+    lib, _ = K
+    with pytest.raises(RuntimeError, match="cannot reshape tensor of 0 elements"):
+        lib.ops.mm_nd(torch.empty(4, 0, device="cuda", dtype=torch.bfloat16), torch.empty(8, 0, device="cuda", dtype=torch.bfloat16), True,
+                      torch.bfloat16)
