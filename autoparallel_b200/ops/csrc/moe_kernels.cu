@@ -273,8 +273,9 @@ static int slot_chunk(int num_blocks, int per_block, int num_sms) {
 // Largest expert count the slot kernel takes for ``per_block`` assignments per token block (48 KB of static-limit shared memory).
 extern "C" int apb_moe_slots_max_experts(int per_block) { return (48 * 1024 / 4) / ((slot_threads(per_block) >> 5) + 1); }
 
-// ints of workspace for apb_moe_slots
+// ints of workspace for apb_moe_slots; 0 for the sizes that it refuses
 extern "C" long long apb_moe_slots_workspace(int num_blocks, int per_block, int E, int num_sms) {
+  if (num_blocks <= 0 || per_block <= 0 || E <= 0) return 0;
   const int chunk = slot_chunk(num_blocks, per_block, num_sms);
   return (long long)num_blocks * ((per_block + chunk - 1) / chunk) * E;
 }

@@ -48,3 +48,9 @@ def test_matrices_without_columns_stay_refused(K):
     with pytest.raises(RuntimeError, match="cannot reshape tensor of 0 elements"):
         lib.ops.mm_nd(torch.empty(4, 0, device="cuda", dtype=torch.bfloat16), torch.empty(8, 0, device="cuda", dtype=torch.bfloat16), True,
                       torch.bfloat16)
+
+
+def test_slots_without_choices_stay_refused(K):
+    lib, _ = K
+    with pytest.raises(RuntimeError, match="apb_moe_slots"):
+        lib.ops.moe_slots(torch.empty(16, 0, device="cuda", dtype=torch.long), 4, 8, 1)
