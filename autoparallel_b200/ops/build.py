@@ -22,6 +22,10 @@ NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "--use_fast_math",
     "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
 ]
+# The C++ library is the shared one that torch has loaded.  A compiler that ships only libstdc++.a would put a second copy
+# into the extension; streams of one copy then use the locale of the other, and formatting the number in an error message
+# ends the process instead of raising.
+LINK_FLAGS = ["-nostdlib++", "-l:libstdc++.so.6", "-lm"]
 
 
 def so_path() -> str:
@@ -42,7 +46,7 @@ def _digest() -> str:
         with open(os.path.join(CSRC, f), "rb") as fh:
             h.update(f.encode())
             h.update(fh.read())
-    h.update(" ".join(NVCC_FLAGS).encode())
+    h.update(" ".join(NVCC_FLAGS + LINK_FLAGS).encode())
     return h.hexdigest()
 
 
@@ -92,7 +96,7 @@ def build(verbose: bool = False, force: bool = False) -> str:
     link = [cxx, "-shared", *objs, "-o", so_path()]
     for d in libdirs:
         link += [f"-L{d}", f"-Wl,-rpath,{d}"]
-    link += ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python", "-lcudart"]
+    link += ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python", "-lcudart", *LINK_FLAGS]
     r = subprocess.run(link, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"link failed: {' '.join(link)}\n{r.stderr}")

@@ -28,3 +28,10 @@ def test_slot_workspace_of_an_empty_dispatch():
         "print(f(1, 0, 8, 148), f(0, 16, 8, 148), f(1, 16, 0, 148), f(2, 1024, 8, 148) > 0)"
     )
     assert out == ["0", "0", "0", "True"]
+
+
+@needs_ext
+def test_the_extension_brings_no_cxx_library_of_its_own():
+    """With a static copy inside, an error with a number in its message ends the process (see ops/build.py)."""
+    with open(build.so_path(), "rb") as f:
+        assert b"\0libstdc++.so.6\0" in f.read()
