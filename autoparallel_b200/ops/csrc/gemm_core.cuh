@@ -857,6 +857,13 @@ inline int make_store_map(CUtensorMap* m, const void* ptr, uint64_t N, uint64_t 
   return r == CUDA_SUCCESS ? 0 : 2;
 }
 
+// C of an empty contraction (a weight gradient over no tokens): zeros.
+inline int zero_result(void* C, long long M, long long N, long long ldc, int out_fp32, cudaStream_t st) {
+  const size_t esz = out_fp32 ? 4 : 2, row = (size_t)N * esz;
+  const cudaError_t e = M == 1 || ldc == N ? cudaMemsetAsync(C, 0, row * (size_t)M, st) : cudaMemset2DAsync(C, (size_t)ldc * esz, 0, row, (size_t)M, st);
+  return e == cudaSuccess ? 0 : 4;
+}
+
 // Tensor maps of both operands for C[M,N] = opA * opB (see gemm_tcgen05.cu for the conventions).
 // ``pair``: the CTA-pair kernels load a K-major B in boxes of 128 rows (each CTA stages half of the tile columns).
 inline int make_operand_maps(CUtensorMap* tmA, CUtensorMap* tmB, const void* A, const void* B, int M, int N, int K,

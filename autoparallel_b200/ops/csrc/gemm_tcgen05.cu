@@ -155,8 +155,9 @@ extern "C" int apb_gemm_split_auto(const void* A, const void* B, void* C, int G,
 extern "C" int apb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
                              long long ldc, int a_mn_major, int b_mn_major, int out_fp32, uint32_t* status,
                              int num_sms, cudaStream_t stream) {
-  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (M <= 0 || N <= 0) return 0;
   if (reinterpret_cast<uintptr_t>(C) & 15) return 3;
+  if (K <= 0) return zero_result(C, M, N, ldc, out_fp32, stream);
   const int usable = num_sms - g_reserved_sms > 0 ? num_sms - g_reserved_sms : 1;
   if (g_pair_mode) {
     const int es = apb_gemm_split_auto(A, B, C, 0, M, N, K, lda, ldb, ldc, a_mn_major, b_mn_major, out_fp32, status, usable, stream);
@@ -226,10 +227,11 @@ extern "C" int apb_gemm_bf16(const void* A, const void* B, void* C, int M, int N
 // (K-major [rows=M or N, cols=K], or MN-major [rows=K, cols=M or N]); C is [G, M, N] bf16 or fp32.
 extern "C" int apb_gemm_grouped_bf16(const void* A, const void* B, void* C, int G, int M, int N, int K, int a_mn_major,
                                      int b_mn_major, int out_fp32, uint32_t* status, int num_sms, cudaStream_t stream) {
-  if (G <= 0 || M <= 0 || N <= 0 || K <= 0) return 0;
+  if (G <= 0 || M <= 0 || N <= 0) return 0;
   const int a_inner = a_mn_major ? M : K, b_inner = b_mn_major ? N : K;
   if ((a_inner & 7) || (b_inner & 7) || (N & 7)) return 3;  // 16-byte rows for TMA and for the vector stores
   if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) || (reinterpret_cast<uintptr_t>(C) & 15)) return 3;
+  if (K <= 0) return zero_result(C, (long long)G * M, N, N, out_fp32, stream);
   const int usable = num_sms - g_reserved_sms > 0 ? num_sms - g_reserved_sms : 1;
   if (g_pair_mode) {
     const int es = apb_gemm_split_auto(A, B, C, G, M, N, K, 0, 0, 0, a_mn_major, b_mn_major, out_fp32, status, usable, stream);

@@ -54,3 +54,32 @@ def test_slots_without_choices_stay_refused(K):
     lib, _ = K
     with pytest.raises(RuntimeError, match="apb_moe_slots"):
         lib.ops.moe_slots(torch.empty(16, 0, device="cuda", dtype=torch.long), 4, 8, 1)
+
+
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+def test_contractions_over_no_tokens_are_zero(K, out_dtype):
+    """A weight gradient when no token arrived (an expert's or a rank's share of a batch), over memory that held something else."""
+    lib, _ = K
+    a, b = torch.empty(0, 64, device="cuda", dtype=torch.bfloat16), torch.empty(0, 96, device="cuda", dtype=torch.bfloat16)
+    ga, gb = torch.empty(3, 0, 64, device="cuda", dtype=torch.bfloat16), torch.empty(3, 0, 96, device="cuda", dtype=torch.bfloat16)
+    for shape, f in [
+        ((64, 96), lambda: lib.ops.mm_wgrad(a, b, out_dtype)),
+        ((64, 96), lambda: lib.ops.mm_wgrad(a.view(2, 0, 64), b.view(2, 0, 96), out_dtype)),
+        ((64, 96), lambda: lib.ops.gemm(a, b, True, False, out_dtype)),
+        ((3, 64, 96), lambda: lib.ops.grouped_mm_wgrad(ga, gb, out_dtype)),
+        ((3, 8, 96), lambda: lib.ops.grouped_mm(ga.view(3, 64, 0)[:, :8], gb, False, out_dtype)),
+    ]:
+        for _ in range(2):
+            junk = torch.full(shape, float("nan"), device="cuda", dtype=out_dtype)
+            del junk  # (what the result is allocated over)
+            out = f()
+            assert out.shape == shape and out.dtype == out_dtype and not out.any()
+    assert lib.ops.mm_nd(a, torch.ones(96, 64, device="cuda", dtype=torch.bfloat16), True, out_dtype).shape == (0, 96)
+    # a window of a wider matrix: nothing beside it is touched
+    from autoparallel_b200.ops import cuda_impl
+
+    back = torch.full((6, 32), 7.0, device="cuda", dtype=out_dtype)
+    cuda_impl.extension().gemm(torch.empty(0, 4, device="cuda", dtype=torch.bfloat16), b[:, :16], back[1:5, 8:24], True, True, cuda_impl.status_buffer(back.device))
+    assert not back[1:5, 8:24].any()
+    back[1:5, 8:24] = 7.0
+    assert bool((back == 7.0).all())
