@@ -16,6 +16,8 @@
 // Rules for callers:
 //   * D (the normalised width) must be a multiple of 8 and at most APB_NOALLOC_MAX_D; larger
 //     widths are refused with APB_NOALLOC_ERR_TOO_LARGE and nothing is launched.
+//   * dy, x, w, dx and dw start on 16-byte boundaries (the kernels move 16 bytes at a time); others are refused with
+//     APB_NOALLOC_ERR_ALIGNMENT and nothing is launched.
 //   * The first call on each device looks up the array's device address (one-time set-up, done
 //     with that device current).  Make that first call outside of any stream capture.
 //   * All calls on one GPU share the one array.  It is cleared at the start of every call, so
@@ -36,6 +38,7 @@ extern "C" {
 #define APB_NOALLOC_ERR_LAUNCH 4      /* the CUDA launch itself failed */
 #define APB_NOALLOC_ERR_TOO_LARGE 7   /* D exceeds APB_NOALLOC_MAX_D */
 #define APB_NOALLOC_ERR_SETUP 8       /* the scratch array's address could not be obtained */
+#define APB_NOALLOC_ERR_ALIGNMENT 9   /* a base that is not on a 16-byte boundary */
 
 // dy, x, dx: [rows, D]; w, dw: [D] (bf16 if is_bf16 else fp32); rstd: fp32 [rows].
 int apb_rms_norm_bwd_noalloc(const void* dy, const void* x, const void* w, const float* rstd, void* dx, void* dw,

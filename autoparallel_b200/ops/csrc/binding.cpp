@@ -342,11 +342,18 @@ void adamw(const at::Tensor& table, const at::Tensor& chunks, int64_t num_chunks
 // ------------------------------------------------------------------ whole operators: checks, allocation and launch in one call
 // What ops/cuda_impl.py asks for first; an empty result means "not this kernel's form" and is answered there.
 
+// Dense and on the 16-byte base that the kernels' vector and bulk accesses need: contiguous() returns a dense view at an odd
+// offset as it is.
+at::Tensor dense(const at::Tensor& t) {
+  at::Tensor d = t.contiguous();
+  return reinterpret_cast<uintptr_t>(d.data_ptr()) % 16 == 0 ? d : d.clone(at::MemoryFormat::Contiguous);
+}
+
 // [rows, last] with unit inner stride, rows of 16 bytes and an aligned base, as TMA needs it
 at::Tensor as2d(const at::Tensor& t) {
   // (a single row is reshaped too: contiguous() does not look at its stride, which TMA does; the reshape makes it the width)
   at::Tensor m = t.dim() == 2 && t.size(0) > 1 && t.size(1) > 0 ? t : t.reshape({-1, t.size(-1)});
-  if (m.stride(1) != 1 || m.stride(0) % 8 != 0 || reinterpret_cast<uintptr_t>(m.data_ptr()) % 16 != 0) m = m.contiguous();
+  if (m.stride(1) != 1 || m.stride(0) % 8 != 0 || reinterpret_cast<uintptr_t>(m.data_ptr()) % 16 != 0) m = dense(m);
   return m;
 }
 
@@ -370,32 +377,32 @@ c10::optional<at::Tensor> mm_nd(const at::Tensor& a, const at::Tensor& b, bool t
 }
 
 std::tuple<at::Tensor, at::Tensor> rms_norm_new(const at::Tensor& x_, const at::Tensor& w, double eps) {
-  at::Tensor x = x_.contiguous(), y = at::empty_like(x);
+  at::Tensor x = dense(x_), y = at::empty_like(x);
   at::Tensor rstd = at::empty(x.sizes().slice(0, x.dim() - 1), x.options().dtype(at::kFloat));
-  rms_norm_fwd(x, w.to(x.scalar_type()).contiguous(), y, rstd, eps);
+  rms_norm_fwd(x, dense(w.to(x.scalar_type())), y, rstd, eps);
   return {y, rstd};
 }
 
 std::tuple<at::Tensor, at::Tensor> rms_norm_bwd_new(const at::Tensor& dy_, const at::Tensor& x_, const at::Tensor& w, const at::Tensor& rstd) {
-  at::Tensor dy = dy_.contiguous(), x = x_.contiguous(), dx = at::empty_like(x), dw = at::empty_like(w, x.scalar_type());
-  rms_norm_bwd(dy, x, w.to(x.scalar_type()).contiguous(), rstd.contiguous(), dx, dw);
+  at::Tensor dy = dense(dy_), x = dense(x_), dx = at::empty_like(x), dw = at::empty_like(w, x.scalar_type());
+  rms_norm_bwd(dy, x, dense(w.to(x.scalar_type())), rstd.contiguous(), dx, dw);
   return {dx, dw.to(w.scalar_type())};
 }
 
 at::Tensor rope_new(const at::Tensor& x_, const at::Tensor& cs, const at::Tensor& sn, bool conj) {
-  at::Tensor x = x_.contiguous(), y = at::empty_like(x);
-  rope(x, cs.to(at::kFloat).contiguous(), sn.to(at::kFloat).contiguous(), y, conj);
+  at::Tensor x = dense(x_), y = at::empty_like(x);
+  rope(x, dense(cs.to(at::kFloat)), dense(sn.to(at::kFloat)), y, conj);
   return y;
 }
 
 at::Tensor swiglu_new(const at::Tensor& a_, const at::Tensor& b_) {
-  at::Tensor a = a_.contiguous(), b = b_.contiguous(), y = at::empty_like(a);
+  at::Tensor a = dense(a_), b = dense(b_), y = at::empty_like(a);
   swiglu_fwd(a, b, y);
   return y;
 }
 
 std::tuple<at::Tensor, at::Tensor> swiglu_bwd_new(const at::Tensor& dy_, const at::Tensor& a_, const at::Tensor& b_) {
-  at::Tensor dy = dy_.contiguous(), a = a_.contiguous(), b = b_.contiguous(), da = at::empty_like(a), db = at::empty_like(b);
+  at::Tensor dy = dense(dy_), a = dense(a_), b = dense(b_), da = at::empty_like(a), db = at::empty_like(b);
   swiglu_bwd(dy, a, b, da, db);
   return {da, db};
 }

@@ -668,10 +668,8 @@ static inline int rms_grid(long long rows, int num_sms, int per_sm) {
   const long long least = rows < num_sms ? rows : num_sms;
   return (int)(g > least ? g : least);
 }
-// bulk form: rows short enough for three stages in shared memory and 16-byte aligned
-static inline bool rms_bulk(const void* dy, const void* x, int D, int elem) {
-  return rms_ring_bytes(D * elem) <= 200 * 1024 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dy)) % 16 == 0);
-}
+// bulk form: rows short enough for three stages in shared memory
+static inline bool rms_bulk(int D, int elem) { return rms_ring_bytes(D * elem) <= 200 * 1024; }
 // Threads of a block of the bulk form: a warp per row up to D = 256, one vector per thread up to 256 threads, then two, then
 // 512 threads.  Blocks per SM: what shared memory holds, up to 768 threads' worth of rows in flight (1024 for the widest).
 struct RmsPlan {
@@ -694,7 +692,7 @@ template <typename T>
 static inline int launch_rms_norm_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx, float* dw_base,
                                       long long stride, long long rows, int D, int num_sms, cudaStream_t st) {
   const RmsDw dw{dw_base, stride};
-  if (rms_bulk(dy, x, D, (int)sizeof(T))) {
+  if (rms_bulk(D, (int)sizeof(T))) {
     const int smem = rms_ring_bytes(D * (int)sizeof(T));
     const RmsPlan plan = rms_plan(D, (int)sizeof(T));
     const int grid = rms_grid(rows, num_sms, plan.per_sm);
@@ -744,6 +742,12 @@ static inline int grid_for(long long work_items, int threads, int num_sms) {
   return (int)(blocks < cap ? (blocks > 0 ? blocks : 1) : cap);
 }
 
+// All kernels here read and write 16-byte vectors: the entries refuse (3) a base that is not on such a boundary.
+template <typename... P>
+static inline bool aligned16(P... p) {
+  return ((reinterpret_cast<uintptr_t>(p) | ...) & 15) == 0;
+}
+
 }  // namespace apb
 
 using namespace apb;
@@ -762,6 +766,7 @@ extern "C" {
 
 int apb_rms_norm_fwd(const void* x, const void* w, void* y, float* rstd, long long rows, int D, float eps, int is_bf16,
                      cudaStream_t st) {
+  if (!aligned16(x, w, y)) return 3;
   if (D % 8) return 3;
   if (rows == 0) return 0;
   int dev = 0, sms = 148;
@@ -798,6 +803,7 @@ long long apb_rms_norm_bwd_workspace(long long rows, int D, int is_bf16, int num
 
 int apb_rms_norm_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx, void* dw, float* part,
                      long long rows, int D, int is_bf16, int num_sms, cudaStream_t st) {
+  if (!aligned16(dy, x, w, dx, part)) return 3;
   if (D % 8) return 3;
   if (D > 512 * 8 * RMS_BWD_MAX_VEC) return 3;
   int n = 0;
@@ -810,6 +816,7 @@ int apb_rms_norm_bwd(const void* dy, const void* x, const void* w, const float* 
 }
 
 int apb_cast(const void* src, void* dst, long long n, int src_bf16, int dst_bf16, int num_sms, cudaStream_t st) {
+  if (!aligned16(src, dst)) return 3;
   if (n == 0) return 0;
   const int grid = grid_for((n + 7) / 8, 256, num_sms);
   if (src_bf16 && !dst_bf16) cast_to_f32_kernel<bf16><<<grid, 256, 0, st>>>((const bf16*)src, (float*)dst, n);
@@ -820,6 +827,7 @@ int apb_cast(const void* src, void* dst, long long n, int src_bf16, int dst_bf16
 
 int apb_rope(const void* x, const float* cs, const float* sn, void* y, long long B, int S, int H, int D, int conj,
              int is_bf16, int num_sms, cudaStream_t st) {
+  if (!aligned16(x, cs, sn, y)) return 3;
   if (D % 8) return 3;
   const long long nvec = B * S * (D / 8);  // one thread per (position, 8-element group); the kernel walks the heads
   if (nvec == 0 || H == 0) return 0;
@@ -829,6 +837,7 @@ int apb_rope(const void* x, const float* cs, const float* sn, void* y, long long
 }
 
 int apb_swiglu_fwd(const void* a, const void* b, void* y, long long n, int is_bf16, int num_sms, cudaStream_t st) {
+  if (!aligned16(a, b, y)) return 3;
   if (n % 8) return 3;
   if (n == 0) return 0;
   DISPATCH(is_bf16, swiglu_fwd_kernel<T><<<grid_for(n / 8, 256, num_sms), 256, 0, st>>>((const T*)a, (const T*)b, (T*)y, n / 8));
@@ -837,6 +846,7 @@ int apb_swiglu_fwd(const void* a, const void* b, void* y, long long n, int is_bf
 
 int apb_swiglu_bwd(const void* dy, const void* a, const void* b, void* da, void* db, long long n, int is_bf16, int num_sms,
                    cudaStream_t st) {
+  if (!aligned16(dy, a, b, da, db)) return 3;
   if (n % 8) return 3;
   if (n == 0) return 0;
   DISPATCH(is_bf16, swiglu_bwd_kernel<T><<<grid_for(n / 8, 256, num_sms), 256, 0, st>>>((const T*)dy, (const T*)a, (const T*)b,
@@ -849,6 +859,7 @@ static int xent_threads(int V) { return V >= 512 * 8 * XENT_UNROLL ? 512 : (V >=
 
 int apb_xent_fwd(const void* logits, const long long* labels, float* loss, float* lse, long long rows, int V, int is_bf16,
                  cudaStream_t st) {
+  if (!aligned16(logits)) return 3;
   if (V % 8) return 3;
   if (rows == 0) return 0;
   const int threads = xent_threads(V);
@@ -858,6 +869,7 @@ int apb_xent_fwd(const void* logits, const long long* labels, float* loss, float
 
 int apb_xent_bwd(const float* dloss, const void* logits, const long long* labels, const float* lse, void* dlogits,
                  long long rows, int V, int is_bf16, cudaStream_t st) {
+  if (!aligned16(logits, dlogits)) return 3;
   if (V % 8) return 3;
   if (rows == 0) return 0;
   const int threads = xent_threads(V);
@@ -867,6 +879,7 @@ int apb_xent_bwd(const float* dloss, const void* logits, const long long* labels
 
 int apb_embedding_fwd(const void* weight, const long long* ids, void* out, long long tokens, int D, long long num_rows,
                       int is_bf16, cudaStream_t st) {
+  if (!aligned16(weight, out)) return 3;
   if (tokens == 0) return 0;
   if ((D * (is_bf16 ? 2 : 4)) % 16) return 3;
   DISPATCH(is_bf16, embedding_fwd_kernel<T><<<(unsigned)tokens, 128, 0, st>>>((const T*)weight, ids, (T*)out, D, num_rows));
@@ -928,6 +941,7 @@ extern "C" int apb_rms_norm_bwd_noalloc(const void* dy, const void* x, const voi
                                         long long rows, int D, int is_bf16, cudaStream_t st) {
   if (D <= 0 || rows < 0 || (D % 8) != 0) return APB_NOALLOC_ERR_BAD_SHAPE;
   if (D > APB_NOALLOC_MAX_D) return APB_NOALLOC_ERR_TOO_LARGE;
+  if (!aligned16(dy, x, w, dx, dw)) return APB_NOALLOC_ERR_ALIGNMENT;
   int dev = -1;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return APB_NOALLOC_ERR_SETUP;
   float* acc = g_noalloc_ptr[dev].load(std::memory_order_acquire);
@@ -960,6 +974,7 @@ extern "C" const char* apb_noalloc_strerror(int code) {
     case APB_NOALLOC_ERR_LAUNCH: return "CUDA launch failed";
     case APB_NOALLOC_ERR_TOO_LARGE: return "D exceeds APB_NOALLOC_MAX_D (16384): the built-in scratch array is too small";
     case APB_NOALLOC_ERR_SETUP: return "could not obtain the device address of the built-in scratch array";
+    case APB_NOALLOC_ERR_ALIGNMENT: return "dy, x, w, dx and dw must start on 16-byte boundaries";
     default: return "unknown error code";
   }
 }

@@ -106,11 +106,17 @@ def _count(n: int = 1) -> None:
     launch_count += n
 
 
+def _dense(t: torch.Tensor) -> torch.Tensor:
+    """``t`` contiguous and on a 16-byte base (``contiguous`` returns a dense view at an odd offset as it is)."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
+
+
 # ----------------------------------------------------------------------------------- GEMM family
 def _as2d(t: torch.Tensor) -> torch.Tensor:
     t2 = t.reshape(-1, t.shape[-1])
     if t2.stride(-1) != 1 or (t2.stride(0) % 8) != 0 or (t2.data_ptr() % 16) != 0:
-        t2 = t2.contiguous()
+        t2 = _dense(t2)
     return t2
 
 
@@ -206,7 +212,7 @@ def _grouped_mm(a, b, trans_b, out_dtype):
         _fallback("grouped_gemm", f"dtypes {a.dtype}/{b.dtype}, shapes {tuple(a.shape)} {tuple(b.shape)}")
         return ref(a, b, trans_b, out_dtype)
     c = torch.empty((a.shape[0], a.shape[1], n), dtype=out_dtype, device=a.device)
-    _C.gemm_grouped(a.contiguous(), b.contiguous(), c, False, not trans_b, status_buffer(a.device))
+    _C.gemm_grouped(_dense(a), _dense(b), c, False, not trans_b, status_buffer(a.device))
     _count()
     return c
 
@@ -219,7 +225,7 @@ def _grouped_mm_wgrad(a, b, out_dtype):
         _fallback("grouped_gemm", f"wgrad dtypes {a.dtype}/{b.dtype}, shapes {tuple(a.shape)} {tuple(b.shape)}")
         return ref(a, b, out_dtype)
     c = torch.empty((a.shape[0], a.shape[2], b.shape[2]), dtype=out_dtype, device=a.device)
-    _C.gemm_grouped(a.contiguous(), b.contiguous(), c, True, True, status_buffer(a.device))
+    _C.gemm_grouped(_dense(a), _dense(b), c, True, True, status_buffer(a.device))
     _count()
     return c
 
@@ -332,7 +338,7 @@ def _swiglu_bwd(dy, a, b):
 
 
 def _cross_entropy(logits, labels):
-    logits = logits.contiguous()
+    logits = _dense(logits)
     shape = logits.shape[:-1]
     loss = torch.empty(shape, dtype=torch.float32, device=logits.device)
     lse = torch.empty(shape, dtype=torch.float32, device=logits.device)
@@ -342,7 +348,7 @@ def _cross_entropy(logits, labels):
 
 
 def _cross_entropy_bwd(dloss, logits, labels, lse):
-    logits = logits.contiguous()
+    logits = _dense(logits)
     out = torch.empty_like(logits)
     _C.xent_bwd(dloss.float().contiguous(), logits, labels.contiguous(), lse.contiguous(), out)
     _count()
@@ -354,7 +360,7 @@ def _embedding(weight, ids):
         _fallback("embedding", f"table {weight.dtype} {tuple(weight.shape)}, ids {ids.dtype}")
         return torch.nn.functional.embedding(ids, weight)
     out = torch.empty((*ids.shape, weight.shape[1]), dtype=weight.dtype, device=weight.device)
-    _C.embedding_fwd(weight.contiguous(), ids.contiguous(), out)
+    _C.embedding_fwd(_dense(weight), ids.contiguous(), out)
     _count()
     return out
 
@@ -386,7 +392,7 @@ def attention_forward_own(q, k, v, causal, scale):
     """(out [B,S,H,D] bf16, lse [B,H,S] fp32) from this package's tcgen05 kernel, or None if it does not cover the shape."""
     if q.dtype != torch.bfloat16 or q.shape[-1] != 128:
         return None
-    q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
+    q, k, v = _dense(q), _dense(k), _dense(v)
     out = torch.empty_like(q)
     lse = torch.empty(q.shape[0], q.shape[2], q.shape[1], dtype=torch.float32, device=q.device)
     if not _C.attention_fwd(q, k, v, out, lse, bool(causal), float(scale), status_buffer(q.device)):

@@ -35,3 +35,40 @@ def test_the_extension_brings_no_cxx_library_of_its_own():
     """With a static copy inside, an error with a number in its message ends the process (see ops/build.py)."""
     with open(build.so_path(), "rb") as f:
         assert b"\0libstdc++.so.6\0" in f.read()
+
+
+@needs_ext
+def test_entries_refuse_bases_off_a_16_byte_boundary():
+    """The kernels move 16 bytes at a time; nothing is launched (there is no GPU here to launch on: that would be code 4)."""
+    out = _run("""
+V, LL, F, N = ctypes.c_void_p, ctypes.c_longlong, ctypes.c_float, None
+A = 1 << 20  # never read
+def entry(name, args, pointers):
+    f = getattr(so, name)
+    if not torch.cuda.is_available():
+        assert f(*args) == 4, (name, "an aligned call gets as far as the launch", f(*args))
+    for i in pointers:
+        bad = list(args)
+        bad[i] = V(A + 8)
+        print(f(*bad))
+p = V(A)
+entry("apb_rms_norm_fwd", [p, p, p, p, LL(4), 64, F(1e-5), 1, N], [0, 1, 2])
+entry("apb_rms_norm_bwd", [p, p, p, p, p, p, p, LL(4), 64, 1, 148, N], [0, 1, 2, 4])
+entry("apb_cast", [p, p, LL(64), 0, 1, 148, N], [0, 1])
+entry("apb_rope", [p, p, p, p, LL(1), 4, 2, 64, 0, 1, 148, N], [0, 1, 2, 3])
+entry("apb_swiglu_fwd", [p, p, p, LL(64), 1, 148, N], [0, 1, 2])
+entry("apb_swiglu_bwd", [p, p, p, p, p, LL(64), 1, 148, N], [0, 1, 2, 3, 4])
+entry("apb_xent_fwd", [p, p, p, p, LL(4), 64, 1, N], [0])
+entry("apb_xent_bwd", [p, p, p, p, p, LL(4), 64, 1, N], [1, 4])
+entry("apb_embedding_fwd", [p, p, p, LL(4), 64, LL(8), 1, N], [0, 2])
+""")
+    assert out == ["3"] * 26
+    out = _run("""
+V, LL = ctypes.c_void_p, ctypes.c_longlong
+p, bad = V(1 << 20), V((1 << 20) + 8)
+for i in (0, 1, 2, 4, 5):
+    a = [p] * 6
+    a[i] = bad
+    print(so.apb_rms_norm_bwd_noalloc(*a, LL(4), 64, 1, None))
+""")
+    assert out == ["9"] * 5

@@ -83,3 +83,52 @@ def test_contractions_over_no_tokens_are_zero(K, out_dtype):
     assert not back[1:5, 8:24].any()
     back[1:5, 8:24] = 7.0
     assert bool((back == 7.0).all())
+
+
+def _off(t, elements=1):
+    """``t`` as a dense view that starts ``elements`` past a 16-byte boundary."""
+    flat = torch.empty(t.numel() + 8, dtype=t.dtype, device="cuda")
+    v = flat[elements:elements + t.numel()].view(t.shape)
+    assert v.is_contiguous() and v.data_ptr() % 16 != 0
+    return v.copy_(t)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_dense_views_off_a_16_byte_boundary(K, dtype):
+    """``contiguous()`` returns such a view as it is; the kernels' accesses are 16 bytes wide."""
+    lib, _ = K
+    from autoparallel_b200.ops import library
+
+    g = torch.Generator().manual_seed(1)
+    r = lambda *s: torch.randn(*s, generator=g).to(dtype)  # noqa: E731
+    tol = BF16_TOL if dtype == torch.bfloat16 else 2**-16  # (fp32: the hardware exponential and reciprocal square root)
+    ref = library.reference_impls
+    x, w, dy = r(9, 64), r(64), r(9, 64)
+    cases = [
+        ("rms_norm", (x, w), (1e-5,)),
+        ("rms_norm_bwd", (dy, x, w), (torch.rand(9, generator=g) + 0.5,)),
+        ("rope", (r(2, 8, 4, 16), torch.randn(8, 8, generator=g), torch.randn(8, 8, generator=g)), (False,)),
+        ("swiglu", (x, dy), ()),
+        ("swiglu_bwd", (dy, x, r(9, 64)), ()),
+        ("cross_entropy", (x,), (torch.arange(9),)),
+        ("cross_entropy_bwd", (torch.rand(9, generator=g), x), (torch.arange(9), torch.logsumexp(x.float(), -1))),
+        ("embedding", (r(20, 64),), (torch.arange(9) % 5,)),
+        ("embedding_bwd", (dy,), (torch.arange(9) % 5, 20)),
+        ("dtype_cast", (x,), (torch.float32 if dtype == torch.bfloat16 else torch.bfloat16,)),
+    ]
+    if dtype == torch.bfloat16:
+        cases += [
+            ("mm_nd", (r(2, 9, 64), r(32, 64)), (True, dtype)),
+            ("mm_wgrad", (r(9, 64), r(9, 32)), (dtype,)),
+            ("gemm", (r(64, 24), r(32, 64)), (True, True, dtype)),
+            ("grouped_mm", (r(3, 9, 64), r(3, 64, 32)), (False, dtype)),
+            ("grouped_mm_wgrad", (r(3, 9, 64), r(3, 9, 32)), (dtype,)),
+        ]
+    for name, tensors, rest in cases:
+        want = ref[name](*tensors, *rest)
+        rest = [t.cuda() if isinstance(t, torch.Tensor) else t for t in rest]
+        for i in range(len(tensors)):  # each operand in turn, and a clean run beside it
+            args = [_off(t) if j == i else t.cuda() for j, t in enumerate(tensors)]
+            got = getattr(lib.ops, name)(*args, *rest)
+            for a, b in zip(got if isinstance(got, tuple) else (got,), want if isinstance(want, tuple) else (want,)):
+                assert _rel(a, b) <= tol, (name, i)
