@@ -8,10 +8,11 @@
 // call is an unbounded stall.  Such callers can still pass input and output buffers they own,
 // but they have nowhere to get the kernel's fp32 work buffer from.
 //
-// What it is: RMSNorm backward, exactly as apb_rms_norm_bwd computes it, except that the fp32
-// accumulator for the weight gradient lives in a fixed array inside the loaded library instead of
-// being passed in.  The array holds APB_NOALLOC_MAX_D floats (64 KiB) and is held by every GPU
-// that loads the library until the process exits.
+// What it is: RMSNorm backward by the kernels of apb_rms_norm_bwd, except that the fp32 partial
+// sums of the weight gradient live in a fixed array inside the loaded library instead of a
+// workspace that is passed in.  The array holds APB_NOALLOC_MAX_D floats (64 KiB: as many partial
+// rows of D as fit, which the blocks share with atomics) and is held by every GPU that loads the
+// library until the process exits.
 //
 // Rules for callers:
 //   * D (the normalised width) must be a multiple of 8 and at most APB_NOALLOC_MAX_D; larger

@@ -143,19 +143,21 @@ __device__ __forceinline__ void block_sum_multi(float (&v)[R], float* red) {
   for (int k = 0; k < R; ++k) v[k] = warp_sum(l < nw ? red[k * 32 + l] : 0.f);
 }
 
-// Where a backward block leaves its weight-gradient sums: its own row of fp32 partial sums, or (``stride`` 0) added with
-// atomics to one row that the caller zeroed.
+// Where a backward block leaves its weight-gradient sums: its own row of fp32 partial sums, or (``shared`` > 0) added with
+// atomics to one of ``shared`` rows that the caller zeroed.
 struct RmsDw {
   float* base;
-  long long stride;  // floats between the blocks' rows
+  long long D;
+  int shared;
   __device__ __forceinline__ void put(int col, const float (&v)[8]) const {
-    if (stride) {
-      float4* p = reinterpret_cast<float4*>(base + blockIdx.x * stride + col);
+    if (shared == 0) {
+      float4* p = reinterpret_cast<float4*>(base + blockIdx.x * D + col);
       p[0] = make_float4(v[0], v[1], v[2], v[3]);
       p[1] = make_float4(v[4], v[5], v[6], v[7]);
     } else {
+      float* p = base + (blockIdx.x % shared) * D + col;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) atomicAdd(base + col + i, v[i]);
+      for (int i = 0; i < 8; ++i) atomicAdd(p + i, v[i]);
     }
   }
 };
@@ -165,7 +167,8 @@ struct RmsDw {
 // nothing is copied): the row loop is bound by memory bandwidth rather than by one load-reduce-store round trip per
 // row.  The ROWS dot products share one block reduction.  Math per element: g*x once, then two fused multiply-adds
 // (weight-gradient partial and dot product); the second pass forms dx = g*(r*w) - x*(r*r*mean) with two more.
-// EXACT: D == blockDim.x * 8 * NVEC and rows % ROWS == 0, so no bounds predicate is needed anywhere.
+// EXACT: D == blockDim.x * 8 * NVEC and rows % ROWS == 0, so no bounds predicate is needed anywhere.  Runs for fp32 rows that the
+// ring of the form below does not hold.
 // Requires D <= blockDim.x * 8 * RMS_BWD_MAX_VEC.
 constexpr int RMS_BWD_MAX_VEC = 4;
 template <typename T, int NVEC, int ROWS, bool EXACT>
@@ -687,21 +690,29 @@ static inline RmsPlan rms_plan(int D, int elem) {
   return p;
 }
 
-// Launches the row kernel; returns the number of blocks (= partial rows of dw when ``stride`` is not 0), < 0 on error.
+// Blocks where they add to shared rows: an atomic per column and block, so a block takes four rows, eight where the rows are
+// long, unless that would leave more than three quarters of the SMs without any.
+static inline int rms_grid_shared(long long rows, int D, int num_sms, int per_sm) {
+  const long long cap = (long long)num_sms * per_sm, per_block = D < 2048 ? 4 : 8, least = rows < num_sms / 4 ? rows : num_sms / 4;
+  const long long g = (rows + per_block - 1) / per_block;
+  return (int)(g < least ? least : g < cap ? g : cap);
+}
+
+// Launches the row kernel; returns the number of partial rows of dw (its blocks, or ``shared``), < 0 on error.
 template <typename T>
 static inline int launch_rms_norm_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx, float* dw_base,
-                                      long long stride, long long rows, int D, int num_sms, cudaStream_t st) {
-  const RmsDw dw{dw_base, stride};
+                                      int shared, long long rows, int D, int num_sms, cudaStream_t st) {
+  const RmsDw dw{dw_base, D, shared};
   if (rms_bulk(D, (int)sizeof(T))) {
     const int smem = rms_ring_bytes(D * (int)sizeof(T));
     const RmsPlan plan = rms_plan(D, (int)sizeof(T));
-    const int grid = rms_grid(rows, num_sms, plan.per_sm);
+    const int grid = shared ? rms_grid_shared(rows, D, num_sms, plan.per_sm) : rms_grid(rows, num_sms, plan.per_sm);
 #define APB_RMS_BULK(NV, TH)                                                                                             \
   if (plan.nvec == NV && plan.threads == TH) {                                                                           \
     auto kern = rms_norm_bwd_bulk_kernel<T, NV, TH>;                                                                     \
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -4;         \
     kern<<<grid, TH, smem, st>>>((const T*)dy, (const T*)x, (const T*)w, rstd, (T*)dx, dw, rows, D);                     \
-    return grid;                                                                                                         \
+    return shared ? shared : grid;                                                                                       \
   }
     APB_RMS_BULK(1, 32)
     APB_RMS_BULK(1, 64)
@@ -712,28 +723,14 @@ static inline int launch_rms_norm_bwd(const void* dy, const void* x, const void*
     APB_RMS_BULK(4, 512)
 #undef APB_RMS_BULK
   }
-  int threads = 128;
-  while (threads * 8 < D && threads < 512) threads *= 2;  // at most 512 threads: 128 registers each
-  const int nvec = (D + threads * 8 - 1) / (threads * 8);
-  if (nvec > RMS_BWD_MAX_VEC) return -3;
-  const int per_sm = threads >= 512 ? 1 : (threads >= 256 ? 2 : 4);  // resident blocks at 128 registers per thread: one wave
-  const long long cap = (long long)num_sms * per_sm;
-  // rows per iteration: as many as the registers hold (16-byte vectors for bf16, two per vector for fp32)
-  constexpr bool wide = sizeof(T) == 4;
-#define APB_RMS_BWD(NV, RW)                                                                                              \
-  {                                                                                                                      \
-    const long long iters = (rows + RW - 1) / RW;                                                                        \
-    const int grid = (int)(iters < cap ? iters : cap);                                                                   \
-    if (D == threads * 8 * NV && rows % RW == 0)                                                                         \
-      rms_norm_bwd_kernel<T, NV, RW, true><<<grid, threads, 0, st>>>((const T*)dy, (const T*)x, (const T*)w, rstd, (T*)dx, dw, rows, D); \
-    else                                                                                                                 \
-      rms_norm_bwd_kernel<T, NV, RW, false><<<grid, threads, 0, st>>>((const T*)dy, (const T*)x, (const T*)w, rstd, (T*)dx, dw, rows, D); \
-    return grid;                                                                                                         \
+  // fp32 rows that the ring does not hold (D > 8512): a block of 512 threads keeps a row in registers
+  if constexpr (sizeof(T) == 4) {
+    const int grid = (int)(rows < num_sms ? rows : num_sms);
+    auto kern = D == 512 * 8 * RMS_BWD_MAX_VEC ? rms_norm_bwd_kernel<T, RMS_BWD_MAX_VEC, 1, true> : rms_norm_bwd_kernel<T, RMS_BWD_MAX_VEC, 1, false>;
+    kern<<<grid, 512, 0, st>>>((const T*)dy, (const T*)x, (const T*)w, rstd, (T*)dx, dw, rows, D);
+    return shared ? shared : grid;
   }
-  if (nvec == 1) { if constexpr (wide) APB_RMS_BWD(1, 2) else APB_RMS_BWD(1, 4) }
-  else if (nvec == 2) { if constexpr (wide) APB_RMS_BWD(2, 1) else APB_RMS_BWD(2, 2) }
-  else APB_RMS_BWD(4, 1)  // (nvec 3 runs as 4 with the last vector masked)
-#undef APB_RMS_BWD
+  return -3;
 }
 
 static inline int grid_for(long long work_items, int threads, int num_sms) {
@@ -794,11 +791,10 @@ int apb_rms_norm_fwd(const void* x, const void* w, void* y, float* rstd, long lo
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 
-// floats of workspace for apb_rms_norm_bwd: one partial row of dw per block, whichever form runs
+// floats of workspace for apb_rms_norm_bwd: one partial row of dw per block (the form for wide fp32 rows has one block per SM, as
+// the plan for such rows does)
 long long apb_rms_norm_bwd_workspace(long long rows, int D, int is_bf16, int num_sms) {
-  const int bulk = rms_grid(rows, num_sms, rms_plan(D, is_bf16 ? 2 : 4).per_sm);
-  const long long other = rows < 4ll * num_sms ? rows : 4ll * num_sms;
-  return (bulk > other ? bulk : other) * D;
+  return (long long)rms_grid(rows, num_sms, rms_plan(D, is_bf16 ? 2 : 4).per_sm) * D;
 }
 
 int apb_rms_norm_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx, void* dw, float* part,
@@ -808,7 +804,7 @@ int apb_rms_norm_bwd(const void* dy, const void* x, const void* w, const float* 
   if (D > 512 * 8 * RMS_BWD_MAX_VEC) return 3;
   int n = 0;
   if (rows > 0) {
-    DISPATCH(is_bf16, n = launch_rms_norm_bwd<T>(dy, x, w, rstd, dx, part, D, rows, D, num_sms, st));
+    DISPATCH(is_bf16, n = launch_rms_norm_bwd<T>(dy, x, w, rstd, dx, part, 0, rows, D, num_sms, st));
     if (n < 0) return -n;
   }
   DISPATCH(is_bf16, rms_dw_kernel<T><<<(D + 31) / 32, 1024, 0, st>>>(part, (T*)dw, n, D));
@@ -951,14 +947,20 @@ extern "C" int apb_rms_norm_bwd_noalloc(const void* dy, const void* x, const voi
     acc = g_noalloc_ptr[dev].load(std::memory_order_acquire);
   }
   const int num_sms = g_noalloc_sms[dev];
+  // The blocks share partial rows, one for sixteen of them as far as the array goes: all adding to one row would spend most of
+  // the time on its D addresses (16384 x 256 bf16: 197 us with one row, 20.6 with 37).
+  const int blocks = rms_grid_shared(rows, D, num_sms, rms_plan(D, is_bf16 ? 2 : 4).per_sm), most = APB_NOALLOC_MAX_D / D;
+  const int shared = blocks < 80 ? 1 : (blocks / 16 < most ? blocks / 16 : most);
   // the array keeps the previous call's sums: start from zero
-  if (cudaMemsetAsync(acc, 0, sizeof(float) * D, st) != cudaSuccess) return APB_NOALLOC_ERR_LAUNCH;
+  if (cudaMemsetAsync(acc, 0, sizeof(float) * shared * D, st) != cudaSuccess) return APB_NOALLOC_ERR_LAUNCH;
   if (rows > 0) {
     int n;
-    DISPATCH(is_bf16, n = launch_rms_norm_bwd<T>(dy, x, w, rstd, dx, acc, 0, rows, D, num_sms, st));
+    DISPATCH(is_bf16, n = launch_rms_norm_bwd<T>(dy, x, w, rstd, dx, acc, shared, rows, D, num_sms, st));
     if (n < 0) return APB_NOALLOC_ERR_BAD_SHAPE;
   }
-  if (is_bf16) {
+  if (shared > 1) {
+    DISPATCH(is_bf16, rms_dw_kernel<T><<<(D + 31) / 32, 1024, 0, st>>>(acc, (T*)dw, shared, D));
+  } else if (is_bf16) {
     cast_from_f32_kernel<bf16><<<grid_for(D / 8, 256, num_sms), 256, 0, st>>>(acc, (bf16*)dw, D);
   } else {
     if (cudaMemcpyAsync(dw, acc, sizeof(float) * D, cudaMemcpyDeviceToDevice, st) != cudaSuccess)

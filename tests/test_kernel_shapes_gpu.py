@@ -122,6 +122,32 @@ def test_rms_norm_gradients_over_row_widths(K, dtype, rows, D):
     assert _rel(dw, (gd * xh).sum(0)) <= tol
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,D", [(5, 8), (20000, 8), (148, 256), (9000, 256), (700, 2048), (5000, 4096), (600, 8192), (300, 10240), (200, 16384)])
+def test_allocation_free_rms_norm_gradients_over_shared_rows(K, dtype, rows, D):
+    """One partial row, several, the most that fit; each width that changes their number."""
+    import ctypes
+
+    from autoparallel_b200.ops import build
+
+    so = ctypes.CDLL(build.so_path())
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn(rows, D, device="cuda", generator=g).to(dtype)
+    w = (1 + 0.1 * torch.randn(D, device="cuda", generator=g)).to(dtype)
+    dy = torch.randn(rows, D, device="cuda", generator=g).to(dtype)
+    rstd = torch.rsqrt(x.float().pow(2).mean(-1) + 1e-5)
+    dx, dw = torch.empty_like(x), torch.empty_like(w)
+    p = [ctypes.c_void_p(t.data_ptr()) for t in (dy, x, w, rstd, dx, dw)]
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    assert so.apb_rms_norm_bwd_noalloc(*p, ctypes.c_longlong(rows), D, int(dtype == torch.bfloat16), st) == 0
+    xd, wd, gd, rd = x.double(), w.double(), dy.double(), rstd.double().unsqueeze(-1)
+    xh, gw = xd * rd, gd * wd
+    # as above: fp32 sums over a row (dx) and over the rows (dw), then one rounding
+    tol = 2**-8 if dtype == torch.bfloat16 else 2**-24 * 16 * max(rows, D) ** 0.5
+    assert _rel(dx, rd * (gw - xh * (gw * xh).mean(-1, keepdim=True))) <= tol
+    assert _rel(dw, (gd * xh).sum(0)) <= tol
+
+
 @pytest.mark.parametrize("M,N,K_", [
     (256, 256, 64),     # one pair tile, one k-block
     (4104, 4104, 64),   # every pair busy, both edges end inside a 32-row / 64-column store

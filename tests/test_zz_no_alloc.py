@@ -60,7 +60,7 @@ def test_matches_regular_entry_point_twice(lib, dtype):
         dx, dw = _call(lib, dy, x, w, rstd)
         torch.cuda.synchronize()
         assert torch.allclose(dx.float(), ref_dx.float(), rtol=tol, atol=tol)
-        # both paths add per-block partial sums with atomics, so order-of-summation noise only
+        # partial rows in the order of the blocks there, shared rows added to with atomics here: order-of-summation noise only
         assert torch.allclose(dw.float(), ref_dw.float(), rtol=tol, atol=tol * 8 if dtype == torch.bfloat16 else 1e-3)
 
 
