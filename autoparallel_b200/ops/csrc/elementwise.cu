@@ -168,11 +168,12 @@ struct RmsDw {
 // row.  The ROWS dot products share one block reduction.  Math per element: g*x once, then two fused multiply-adds
 // (weight-gradient partial and dot product); the second pass forms dx = g*(r*w) - x*(r*r*mean) with two more.
 // EXACT: D == blockDim.x * 8 * NVEC and rows % ROWS == 0, so no bounds predicate is needed anywhere.  Runs for fp32 rows that the
-// ring of the form below does not hold.
+// ring of the form below does not hold.  (512, 1): without the one the compiler settles on 32 registers and spills the row;
+// 16384 x 16384 fp32 2706 -> 1054 us.
 // Requires D <= blockDim.x * 8 * RMS_BWD_MAX_VEC.
 constexpr int RMS_BWD_MAX_VEC = 4;
 template <typename T, int NVEC, int ROWS, bool EXACT>
-__global__ void __launch_bounds__(512) rms_norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ w,
+__global__ void __launch_bounds__(512, 1) rms_norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ w,
                                                            const float* __restrict__ rstd, T* __restrict__ dx, RmsDw dw, long long rows, int D) {
   __shared__ float red[32 * ROWS];
   float wreg[NVEC][8];
