@@ -268,7 +268,8 @@ static void moe_check(const at::Tensor& x, const char* what) {
 
 int64_t moe_slots_max_experts(int64_t per_block) { return apb_moe_slots_max_experts((int)std::min<int64_t>(per_block, 1 << 30)); }
 
-void moe_slots(const at::Tensor& gate_idx, at::Tensor& slot, int64_t E, int64_t C, int64_t nb) {
+// Returns the number of kernels launched.
+int64_t moe_slots(const at::Tensor& gate_idx, at::Tensor& slot, int64_t E, int64_t C, int64_t nb) {
   c10::cuda::CUDAGuard g(gate_idx.device());
   moe_check(gate_idx, "moe_slots");
   moe_check(slot, "moe_slots");
@@ -276,10 +277,12 @@ void moe_slots(const at::Tensor& gate_idx, at::Tensor& slot, int64_t E, int64_t 
                   gate_idx.numel() == slot.numel() && nb > 0 && gate_idx.size(0) % nb == 0,
               "moe_slots: int64 [T, k] with T a multiple of the block count");
   const int64_t per_block = gate_idx.size(0) / nb * gate_idx.size(1);
-  at::Tensor counts = at::empty({(int64_t)apb_moe_slots_workspace((int)nb, (int)per_block, (int)E, num_sms())}, gate_idx.options().dtype(at::kInt));
+  const int64_t words = apb_moe_slots_workspace((int)nb, (int)per_block, (int)E, num_sms());  // counts of every chunk
+  at::Tensor counts = at::empty({words}, gate_idx.options().dtype(at::kInt));
   check(apb_moe_slots((const long long*)gate_idx.data_ptr<int64_t>(), (long long*)slot.data_ptr<int64_t>(), counts.data_ptr<int>(), (int)nb,
                       (int)per_block, (int)E, (int)C, num_sms(), stream()),
         "apb_moe_slots");
+  return words > nb * E ? 2 : 1;  // (one chunk per block needs no counts)
 }
 
 // gate weights: fp32 or bf16, used in the operand's precision

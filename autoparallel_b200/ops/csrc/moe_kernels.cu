@@ -262,9 +262,11 @@ static int launch_status() { return (int)cudaGetLastError(); }
 
 static int slot_threads(int per_block) { return per_block >= SLOT_THREADS ? SLOT_THREADS : ((per_block + 31) / 32) * 32; }
 
-// assignments per CTA: one round, more once that would be over two CTAs per SM (the prefix of every CTA reads all earlier counts)
+// assignments per CTA: one round, more once that would be over two CTAs per SM (the prefix of every CTA reads all earlier counts).
+// Up to two rounds stay with one CTA: a second round costs less than the count kernel's launch (1024 assignments: 4.2 us against 6.3).
 static int slot_chunk(int num_blocks, int per_block, int num_sms) {
   const int threads = slot_threads(per_block);
+  if (per_block <= 2 * threads) return per_block;
   const long long rounds = ((long long)num_blocks * per_block + 2ll * num_sms * threads - 1) / (2ll * num_sms * threads);
   const long long chunk = rounds * threads;
   return chunk < per_block ? (int)chunk : per_block;

@@ -247,8 +247,7 @@ def _moe_slots(gate_idx, num_experts, capacity, num_blocks):
         _fallback("moe_index", f"moe_slots {tuple(gate_idx.shape)} E={num_experts}")
         return moe_ops._moe_slots(gate_idx, num_experts, capacity, num_blocks)
     slot = torch.empty_like(gate_idx, memory_format=torch.contiguous_format)
-    _C.moe_slots(gate_idx.contiguous(), slot, num_experts, capacity, num_blocks)
-    _count(2)
+    _count(_C.moe_slots(gate_idx.contiguous(), slot, num_experts, capacity, num_blocks))
     return slot
 
 

@@ -86,6 +86,21 @@ def test_moe_dispatch_over_shapes(K, T, k, E, C, nb, d, dtype, wdtype):
     assert impl.library_fallbacks == before, "the kernels cover these shapes"
 
 
+@pytest.mark.parametrize("T,k,nb,launches", [(16, 2, 1, 1), (510, 1, 1, 1), (513, 1, 1, 1), (512, 2, 1, 1), (4096, 2, 8, 1), (513, 2, 1, 2), (2050, 2, 2, 2)])
+@pytest.mark.parametrize("E", [8, 372, 700])
+def test_moe_slots_around_one_and_two_rounds(K, T, k, nb, launches, E):
+    """One round, two rounds of one CTA, and the first sizes that are cut into chunks."""
+    lib, impl = K
+    from autoparallel_b200.ops import moe_ops
+
+    idx = torch.randint(0, E, (T, k), generator=torch.Generator().manual_seed(T))
+    idx[0] = idx[-1] = 3  # (one expert past its capacity wherever it is small)
+    before, fallbacks = impl.launch_count, dict(impl.library_fallbacks)
+    slot = lib.ops.moe_slots(idx.cuda(), E, 5, nb)
+    assert torch.equal(slot.cpu(), moe_ops._moe_slots(idx, E, 5, nb))
+    assert impl.launch_count - before == launches and impl.library_fallbacks == fallbacks
+
+
 def test_moe_dispatch_leaves_nothing_of_the_old_buffer(K):
     """Every row of the buffer is written, also those no assignment names, whatever the memory held before."""
     lib, _ = K
