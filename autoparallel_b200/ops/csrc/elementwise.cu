@@ -502,25 +502,26 @@ __global__ void swiglu_bwd_kernel(const T* __restrict__ dy, const T* __restrict_
 
 // ------------------------------------------------------------------------------------ cross-entropy
 // One block per row of V logits (V % 8 == 0).  Bound by memory: forward reads the logits once (online maximum and sum of
-// exponentials; loss = lse - logit[label]), backward reads and writes them once.  XENT_UNROLL independent 16- or 32-byte
-// loads per thread and step: with one load per step an SM had 32 KB in flight, too little for the latency (8192 x 128256 bf16 forward 392 -> 368 us; 8192 x 32064 backward 176 -> 161 us).  The
-// maximum moves once per step of all its vectors, not once per vector.
-constexpr int XENT_UNROLL = 4;
+// exponentials; loss = lse - logit[label]), backward reads and writes them once.  Two independent loads per thread and step
+// in most forms; four leave too much of a row to its end (``xent_fwd_threads`` has the times).
+// The maximum moves once per step of all its vectors, not once per vector.
+constexpr int XENT_UNROLL = 2;
 template <typename T>
-__global__ void __launch_bounds__(512) xent_fwd_kernel(const T* __restrict__ logits, const long long* __restrict__ labels,
-                                                       float* __restrict__ loss, float* __restrict__ lse, int V) {
+__global__ void __launch_bounds__(1024) xent_fwd_kernel(const T* __restrict__ logits, const long long* __restrict__ labels,
+                                                        float* __restrict__ loss, float* __restrict__ lse, int V) {
   __shared__ float red[32];
   const long long row = blockIdx.x;
   const T* lr = logits + row * V;
   float m = -INFINITY, s = 0.f;
   auto take = [&](const Vec8<T>* v, int n) {
+    float f[XENT_UNROLL][8];
     float lm = -INFINITY;
 #pragma unroll
     for (int k = 0; k < XENT_UNROLL; ++k) {
       if (k < n) {
-        float f[8]; v[k].to_float(f);
+        v[k].to_float(f[k]);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) lm = fmaxf(lm, f[i]);
+        for (int i = 0; i < 8; ++i) lm = fmaxf(lm, f[k][i]);
       }
     }
     const float nm = fmaxf(m, lm);
@@ -529,9 +530,8 @@ __global__ void __launch_bounds__(512) xent_fwd_kernel(const T* __restrict__ log
 #pragma unroll
     for (int k = 0; k < XENT_UNROLL; ++k) {
       if (k < n) {
-        float f[8]; v[k].to_float(f);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) acc += __expf(f[i] - ref);
+        for (int i = 0; i < 8; ++i) acc += __expf(f[k][i] - ref);
       }
     }
     s = s * __expf(m - ref) + acc;
@@ -545,7 +545,7 @@ __global__ void __launch_bounds__(512) xent_fwd_kernel(const T* __restrict__ log
     for (int k = 0; k < XENT_UNROLL; ++k) v[k].load(lr + c + k * step);
     take(v, XENT_UNROLL);
   }
-  for (; c < V; c += step) {
+  if (c < V) {  // (at most one vector is left)
     Vec8<T> v; v.load(lr + c);
     take(&v, 1);
   }
@@ -553,15 +553,15 @@ __global__ void __launch_bounds__(512) xent_fwd_kernel(const T* __restrict__ log
   s = (m == -INFINITY) ? 0.f : s * __expf(m - gm);
   s = block_sum(s, red);
   if (threadIdx.x == 0) {
-    const float l = gm + logf(s);
+    const float l = gm + __logf(s);
     lse[row] = l;
     loss[row] = l - float(lr[labels[row]]);
   }
 }
-template <typename T>
-__global__ void __launch_bounds__(512) xent_bwd_kernel(const float* __restrict__ dloss, const T* __restrict__ logits,
-                                                       const long long* __restrict__ labels, const float* __restrict__ lse,
-                                                       T* __restrict__ dlogits, int V) {
+template <typename T, bool PAIRS>
+__global__ void __launch_bounds__(1024) xent_bwd_kernel(const float* __restrict__ dloss, const T* __restrict__ logits,
+                                                        const long long* __restrict__ labels, const float* __restrict__ lse,
+                                                        T* __restrict__ dlogits, int V) {
   const long long row = blockIdx.x;
   const T* lr = logits + row * V;
   T* dr = dlogits + row * V;
@@ -575,16 +575,24 @@ __global__ void __launch_bounds__(512) xent_bwd_kernel(const float* __restrict__
   };
   const int step = blockDim.x * 8;
   int c = threadIdx.x * 8;
-  for (; c + (XENT_UNROLL - 1) * step < V; c += XENT_UNROLL * step) {
-    Vec8<T> v[XENT_UNROLL];
+  if (PAIRS) {
+    for (; c + step < V; c += 2 * step) {
+      Vec8<T> v[2];
 #pragma unroll
-    for (int k = 0; k < XENT_UNROLL; ++k) v[k].load(lr + c + k * step);
+      for (int k = 0; k < 2; ++k) v[k].load(lr + c + k * step);
 #pragma unroll
-    for (int k = 0; k < XENT_UNROLL; ++k) put(v[k], c + k * step);
-  }
-  for (; c < V; c += step) {
-    Vec8<T> v; v.load(lr + c);
-    put(v, c);
+      for (int k = 0; k < 2; ++k) put(v[k], c + k * step);
+    }
+    if (c < V) {
+      Vec8<T> v; v.load(lr + c);
+      put(v, c);
+    }
+  } else {
+#pragma unroll 1
+    for (; c < V; c += step) {
+      Vec8<T> v; v.load(lr + c);
+      put(v, c);
+    }
   }
 }
 
@@ -851,15 +859,24 @@ int apb_swiglu_bwd(const void* dy, const void* a, const void* b, void* da, void*
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 
-// a full step of the unrolled loop per thread where the row is long enough for one
-static int xent_threads(int V) { return V >= 512 * 8 * XENT_UNROLL ? 512 : (V >= 256 * 8 * XENT_UNROLL ? 256 : 128); }
+// Threads of a row's block.  Swept over 8 ... 256000 columns, 64 ... 8192 rows, both
+// types, one, two and four vectors a step, 128 ... 1024 threads, against one vector a step and 256 threads (from 8192 columns on 1024).
+// Forward: short rows waste large blocks on the reduction, long ones small blocks on latency; with at most two rows per SM the
+// row itself is the latency.  8192 rows of bf16: 4096 columns 18.6 -> 15.4 us, 32064 132 -> 87, 128256 392 -> 314.
+// Backward, bf16: two vectors a step (8192 x 32064 177 -> 158 us, 128256 646 -> 629).
+// Backward, fp32: one, and not unrolled (8192 x 128256 1285 us; 1352 where the compiler unrolls the loop, 1346 with four).
+static int xent_fwd_threads(long long rows, int V, bool is_bf16) {
+  if (rows <= 2 * 148) return V <= 8192 ? 256 : V <= 16384 ? 512 : 1024;
+  return V <= (is_bf16 ? 8192 : 4096) ? 128 : V < 36000 ? 256 : V < 140000 ? 512 : 1024;
+}
+static int xent_bwd_threads(int V, bool is_bf16) { return V < 8192 ? 256 : is_bf16 && V < 24000 ? 512 : 1024; }
 
 int apb_xent_fwd(const void* logits, const long long* labels, float* loss, float* lse, long long rows, int V, int is_bf16,
                  cudaStream_t st) {
   if (!aligned16(logits)) return 3;
   if (V % 8) return 3;
   if (rows == 0) return 0;
-  const int threads = xent_threads(V);
+  const int threads = xent_fwd_threads(rows, V, is_bf16);
   DISPATCH(is_bf16, xent_fwd_kernel<T><<<(unsigned)rows, threads, 0, st>>>((const T*)logits, labels, loss, lse, V));
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
@@ -869,8 +886,9 @@ int apb_xent_bwd(const float* dloss, const void* logits, const long long* labels
   if (!aligned16(logits, dlogits)) return 3;
   if (V % 8) return 3;
   if (rows == 0) return 0;
-  const int threads = xent_threads(V);
-  DISPATCH(is_bf16, xent_bwd_kernel<T><<<(unsigned)rows, threads, 0, st>>>(dloss, (const T*)logits, labels, lse, (T*)dlogits, V));
+  const int threads = xent_bwd_threads(V, is_bf16);
+  if (is_bf16) xent_bwd_kernel<bf16, true><<<(unsigned)rows, threads, 0, st>>>(dloss, (const bf16*)logits, labels, lse, (bf16*)dlogits, V);
+  else xent_bwd_kernel<float, false><<<(unsigned)rows, threads, 0, st>>>(dloss, (const float*)logits, labels, lse, (float*)dlogits, V);
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 

@@ -233,6 +233,29 @@ def test_cross_entropy_over_row_widths(K, dtype, V):
     assert _rel(d, p * dl.double().unsqueeze(-1)) <= (2**-8 if dtype == torch.bfloat16 else 2**-18)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("V", [8, 2048, 4096 + 8, 8192 + 8, 24000, 36000, 60008, 140008])
+def test_cross_entropy_with_more_rows_than_two_per_sm(K, dtype, V):
+    """The block sizes of long batches; a last vector that only some threads have."""
+    lib, _ = K
+    g = torch.Generator(device="cuda").manual_seed(V)
+    rows = 300
+    logits = (3 * torch.randn(rows, V, device="cuda", generator=g)).to(dtype)
+    labels = torch.randint(0, V, (rows,), device="cuda", generator=g)
+    logits[1, : V // 2] = float("-inf")
+    labels[1] = V - 1
+    loss, lse = lib.ops.cross_entropy(logits, labels)
+    dl = torch.randn(rows, device="cuda", generator=g)
+    d = lib.ops.cross_entropy_bwd(dl, logits, labels, lse)
+    ld = logits.double()
+    ref = torch.logsumexp(ld, -1)
+    # bounds as above
+    assert _rel(lse, ref) <= 2**-19 and (loss.double() - (ref - ld.gather(-1, labels.unsqueeze(-1)).squeeze(-1))).abs().max().item() <= 2**-19 * 16
+    p = torch.softmax(ld, -1)
+    p[torch.arange(rows), labels] -= 1
+    assert _rel(d, p * dl.double().unsqueeze(-1)) <= (2**-8 if dtype == torch.bfloat16 else 2**-18)
+
+
 @pytest.mark.parametrize("M,N,K_", [(1, 8, 8), (16, 4096, 4096), (64, 2048, 8192), (129, 264, 520), (1000, 1408, 2048), (300, 72, 1096)])
 @pytest.mark.parametrize("ta,tb", [(False, True), (False, False), (True, False), (True, True)])
 @pytest.mark.parametrize("bn,slices", [(0, 0), (64, 8), (64, 1), (128, 3), (256, 5), (256, 2)])
