@@ -39,7 +39,9 @@ int apb_xent_fwd(const void* logits, const long long* labels, float* loss, float
                  cudaStream_t st);
 int apb_xent_bwd(const float* dloss, const void* logits, const long long* labels, const float* lse, void* dlogits,
                  long long rows, int V, int is_bf16, cudaStream_t st);
-long long apb_embedding_bwd_workspace(long long tokens, long long num_rows, int D);
+int apb_embedding_bwd_sorts(long long tokens, long long num_rows, int D, int is_bf16);
+int apb_embedding_bwd_launches(long long tokens, long long num_rows, int D, int is_bf16);
+long long apb_embedding_bwd_workspace(long long tokens, long long num_rows, int D, int is_bf16);
 int apb_embedding_bwd(const void* dy, const long long* ids, void* out, void* workspace, long long tokens, long long num_rows, int D,
                       int is_bf16, int num_sms, cudaStream_t st);
 int apb_embedding_fwd(const void* weight, const long long* ids, void* out, long long tokens, int D, long long num_rows,
@@ -247,18 +249,19 @@ void embedding_fwd(const at::Tensor& weight, const at::Tensor& ids, at::Tensor& 
         "apb_embedding_fwd");
 }
 
-// out [num_rows, D] of dy's dtype receives every row (zeros where no token names it).
-void embedding_bwd(const at::Tensor& dy, const at::Tensor& ids, at::Tensor& out) {
+// out [num_rows, D] of dy's dtype receives every row (zeros where no token names it).  Returns the number of kernels launched.
+int64_t embedding_bwd(const at::Tensor& dy, const at::Tensor& ids, at::Tensor& out) {
   c10::cuda::CUDAGuard g(dy.device());
   const int64_t D = dy.size(-1), rows = out.size(0);
   TORCH_CHECK(dy.is_contiguous() && ids.is_contiguous() && out.is_contiguous() && out.dim() == 2 && out.size(1) == D &&
                   out.scalar_type() == dy.scalar_type() && ids.numel() * D == dy.numel(),
               "embedding_bwd: dy [..., D], ids [...], out [num_rows, D] of dy's dtype, all contiguous");
   const bool bf16 = is_bf16(dy);
-  at::Tensor ws = at::empty({(int64_t)apb_embedding_bwd_workspace(ids.numel(), rows, (int)D)}, dy.options().dtype(at::kByte));
+  at::Tensor ws = at::empty({(int64_t)apb_embedding_bwd_workspace(ids.numel(), rows, (int)D, bf16)}, dy.options().dtype(at::kByte));
   check(apb_embedding_bwd(dy.data_ptr(), (const long long*)ids.data_ptr<int64_t>(), out.data_ptr(), ws.data_ptr(), ids.numel(), rows,
                           (int)D, bf16, num_sms(), stream()),
         "apb_embedding_bwd");
+  return apb_embedding_bwd_launches(ids.numel(), rows, (int)D, bf16);
 }
 
 // Mixture-of-experts dispatch (ops/moe_ops.py): gate_idx / slot [T, k] int64, w [T, k] fp32, buf [E, nb, C, d], src / out / g [T, d].
@@ -548,6 +551,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("xent_fwd", &xent_fwd);
   m.def("xent_bwd", &xent_bwd);
   m.def("embedding_bwd", &embedding_bwd);
+  m.def("embedding_bwd_sorts", [](int64_t tokens, int64_t rows, int64_t D, bool bf16) { return apb_embedding_bwd_sorts(tokens, rows, (int)D, bf16) != 0; });
   m.def("embedding_fwd", &embedding_fwd);
   m.def("adamw", &adamw);
   m.def("moe_slots_max_experts", &moe_slots_max_experts);

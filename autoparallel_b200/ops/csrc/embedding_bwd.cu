@@ -1,21 +1,29 @@
 // Embedding table gradient for sm_100a: out[v, :] = sum of dy[t, :] over the tokens with ids[t] == v, zero rows included.
 //
-// Bound by memory: the table gradient is written once in its own type and dy is read once.  The tokens are grouped by row
-// first, so that every output row is summed in fp32 registers and stored once - no fp32 table, no zero fill of it, no
-// second pass that converts it, no atomics on row data.  8192 tokens of 4096 bf16, 128256 rows (1.05 GB written):
-// 278 us for the three kernels (246 of them the rows); the fp32 zero fill + atomics + cast that they replace took 841 us.
+// Two forms; ``apb_embedding_bwd_sorts`` says which one runs.
+//
+// Sorted, bound by memory: the table gradient is written once in its own type and dy is read once.  The tokens are grouped by row
+// first, so that every output row is summed in fp32 registers and stored once - no fp32 table, no zero fill of it, no second
+// pass that converts it, no atomics on row data.
 //
 //   emb_group_kernel    one cluster of 8 CTAs: counts per row (one atomic per warp and distinct id), segment starts, token
 //                       list sorted by row.  A cluster because its barrier orders the phases inside one launch; 8192
 //                       threads take a usual batch in one or two steps.
 //   emb_partial_kernel  rows with more than EMB_CHUNK tokens (frequent words, padding): one fp32 partial row per chunk, so
 //                       that no block walks a long list alone.
-//   emb_rows_kernel     every row: zeros, the sum of its tokens, or the sum of its chunks.
+//   emb_long_kernel     those rows, from their chunks: a slice of the columns per block.
+//   emb_rows_kernel     every other row: zeros or the sum of its tokens.
+//
+// Atomic: an fp32 table of zeros, one block per token, for bf16 a conversion.  Better where the table is small or the rows are
+// short (the grouping is a chain of latencies that a small table does not pay for), and for most fp32 tables, which the atomics
+// fill in place.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "ptx.cuh"
+
+extern "C" int apb_cast(const void* src, void* dst, long long n, int src_bf16, int dst_bf16, int num_sms, cudaStream_t st);  // elementwise.cu
 
 namespace apb {
 
@@ -31,11 +39,13 @@ struct EmbWs {
   int* perm;     // [T] tokens grouped by row
   int* rank;     // [T] arrival number of the token inside its row
   int2* desc;    // [max_chunks] {first entry in perm, tokens}
-  int* ctr;      // [2] entries and chunks handed out so far
+  int* ctr;      // [3] entries, chunks and long rows handed out so far
   float* part;   // [max_chunks, D]
+  int* longs;    // [max_longs] rows with more than EMB_CHUNK tokens
 };
 
-__host__ __device__ inline long long emb_max_chunks(long long T) { return T / EMB_CHUNK + T / (EMB_CHUNK + 1); }
+__host__ __device__ inline long long emb_max_longs(long long T) { return T / (EMB_CHUNK + 1); }
+__host__ __device__ inline long long emb_max_chunks(long long T) { return T / EMB_CHUNK + emb_max_longs(T); }
 static inline long long emb_round4(long long n) { return (n + 3) & ~3ll; }
 
 __global__ void __cluster_dims__(EMB_CTAS, 1, 1) __launch_bounds__(EMB_GROUP_THREADS)
@@ -43,7 +53,7 @@ emb_group_kernel(const long long* __restrict__ ids, EmbWs ws, int T, long long V
   const int tid = blockIdx.x * EMB_GROUP_THREADS + threadIdx.x, lane = threadIdx.x & 31;
   constexpr int nt = EMB_CTAS * EMB_GROUP_THREADS;
   for (long long v = tid; v < V; v += nt) ws.count[v] = 0;
-  if (tid < 2) ws.ctr[tid] = 0;
+  if (tid < 3) ws.ctr[tid] = 0;
   auto sync = [] {  // every phase reads what other CTAs of the cluster wrote in the one before
     __threadfence();
     cluster_arrive();
@@ -88,6 +98,13 @@ emb_group_kernel(const long long* __restrict__ ids, EmbWs ws, int T, long long V
     }
     const int s = __shfl_sync(0xffffffffu, cb, 31) + cs - c, b = __shfl_sync(0xffffffffu, nb, 31) + ns - n;
     if (first) ws.start[v] = s;
+    const unsigned longs = __ballot_sync(0xffffffffu, n > 0);
+    if (longs) {
+      int lb = 0;
+      if (lane == 0) lb = atomicAdd(ws.ctr + 2, __popc(longs));
+      lb = __shfl_sync(0xffffffffu, lb, 0);
+      if (n > 0) ws.longs[lb + __popc(longs & ((1u << lane) - 1u))] = (int)v;
+    }
     if (n > 0) {
       ws.chunk0[v] = b;
       for (int i = 0; i < n; ++i) ws.desc[b + i] = make_int2(s + i * EMB_CHUNK, min(EMB_CHUNK, c - i * EMB_CHUNK));
@@ -155,6 +172,20 @@ __device__ __forceinline__ void emb_sum(const T* __restrict__ dy, const int* lis
   }
 }
 
+// W floats of a partial row
+template <int W>
+__device__ __forceinline__ void emb_part_add(const float* p, float (&acc)[W]) {
+  if (W == 1) {
+    acc[0] += *p;
+  } else {
+#pragma unroll
+    for (int k = 0; k < W / 4; ++k) {
+      const float4 x = reinterpret_cast<const float4*>(p)[k];
+      acc[4 * k] += x.x; acc[4 * k + 1] += x.y; acc[4 * k + 2] += x.z; acc[4 * k + 3] += x.w;
+    }
+  }
+}
+
 template <typename T, int W>
 __global__ void __launch_bounds__(128) emb_partial_kernel(const T* __restrict__ dy, EmbWs ws, int D) {
   __shared__ int list[EMB_CHUNK];
@@ -170,6 +201,35 @@ __global__ void __launch_bounds__(128) emb_partial_kernel(const T* __restrict__ 
   }
 }
 
+// A block takes 32 W columns of a long row, each warp an eighth of its chunks.  (A block of the kernel below that summed all chunks and
+// all columns took 2.9 ms for 131072 tokens of one row, D = 4096; inside that kernel this code costs its other blocks registers.)
+template <typename T, int W>
+__global__ void __launch_bounds__(256) emb_long_kernel(EmbWs ws, T* __restrict__ out, int D) {
+  __shared__ float sum[8][32 * W];
+  const int slices = (D + 32 * W - 1) / (32 * W), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int items = ws.ctr[2] * slices;  // (at most T / 33 * D / 32)
+  for (int it = blockIdx.x; it < items; it += gridDim.x) {
+    const long long v = ws.longs[it / slices];
+    const int col = (it % slices * 32 + lane) * W, n = (ws.count[v] + EMB_CHUNK - 1) / EMB_CHUNK;
+    const float* p = ws.part + (long long)ws.chunk0[v] * D + col;
+    float acc[W] = {};
+    if (col < D) {
+#pragma unroll 8
+      for (int i = warp; i < n; i += 8) emb_part_add<W>(p + (long long)i * D, acc);
+    }
+#pragma unroll
+    for (int k = 0; k < W; ++k) sum[warp][k * 32 + lane] = acc[k];
+    __syncthreads();
+    if (warp == 0 && col < D) {
+      for (int g = 1; g < 8; ++g)
+#pragma unroll
+        for (int k = 0; k < W; ++k) acc[k] += sum[g][k * 32 + lane];
+      EmbVec<T, W>::store(out + v * D + col, acc);
+    }
+    __syncthreads();
+  }
+}
+
 // ``tx`` threads (a power of two, 32..256) walk a row, 256 / tx rows at a time; the block owns ``R`` consecutive rows
 template <typename T, int W>
 __global__ void __launch_bounds__(256) emb_rows_kernel(const T* __restrict__ dy, EmbWs ws, T* __restrict__ out, long long V, int D,
@@ -180,36 +240,72 @@ __global__ void __launch_bounds__(256) emb_rows_kernel(const T* __restrict__ dy,
   if ((int)threadIdx.x < nrows) {
     const int c = ws.count[row0 + threadIdx.x];
     cnt[threadIdx.x] = c;
-    from[threadIdx.x] = c == 0 ? 0 : (c > EMB_CHUNK ? ws.chunk0 : ws.start)[row0 + threadIdx.x];
+    from[threadIdx.x] = c == 0 ? 0 : ws.start[row0 + threadIdx.x];
   }
   __syncthreads();
   for (int r = threadIdx.x / tx; r < nrows; r += 256 / tx) {
     T* dst = out + (row0 + r) * D;
     const int c = cnt[r];
+    if (c > EMB_CHUNK) continue;
     for (int col = (threadIdx.x & (tx - 1)) * W; col < D; col += tx * W) {
       float acc[W] = {};
-      if (c > EMB_CHUNK) {
-        const float* p = ws.part + (long long)from[r] * D + col;
-        const int n = (c + EMB_CHUNK - 1) / EMB_CHUNK;
-#pragma unroll 4
-        for (int i = 0; i < n; ++i)
-#pragma unroll
-          for (int k = 0; k < W; ++k) acc[k] += p[(long long)i * D + k];
-      } else if (c > 0) {
-        emb_sum<T, W>(dy, ws.perm + from[r], c, D, col, acc);
-      }
+      if (c > 0) emb_sum<T, W>(dy, ws.perm + from[r], c, D, col, acc);
       EmbVec<T, W>::store(dst + col, acc);
     }
   }
 }
 
+// The other form: an fp32 table of zeros, one block per token that adds its row with atomics (a bf16 table is converted after).
+// ``U`` elements of a thread are loaded before the token's id is there: one in rows of up to 256, four in longer ones.
+template <typename T, int U>
+__global__ void __launch_bounds__(256) emb_atomic_kernel(const T* __restrict__ dy, const long long* __restrict__ ids, float* __restrict__ out,
+                                                         long long V, int D) {
+  const long long tok = blockIdx.x;
+  const long long r = ids[tok];
+  const bool ok = (unsigned long long)r < (unsigned long long)V;
+  const T* src = dy + tok * D;
+  if constexpr (U == 1) {  // (the loop below with one element makes a block half as long again: 524288 x 64 276 -> 390 us)
+    for (int c = threadIdx.x; c < D; c += blockDim.x) {
+      const float x = float(src[c]);
+      if (ok) atomicAdd(out + r * D + c, x);
+    }
+  } else {
+    for (int c = threadIdx.x; c < D; c += 256 * U) {
+      float x[U];
+#pragma unroll
+      for (int k = 0; k < U; ++k)
+        if (c + k * 256 < D) x[k] = float(src[c + k * 256]);
+      if (ok) {
+#pragma unroll
+        for (int k = 0; k < U; ++k)
+          if (c + k * 256 < D) atomicAdd(out + r * D + c + k * 256, x[k]);
+      }
+    }
+  }
+}
+
+template <typename T>
+static void emb_atomic(const void* dy, const long long* ids, float* out, long long tokens, long long V, int D, cudaStream_t st) {
+  if (D <= 256) emb_atomic_kernel<T, 1><<<(unsigned)tokens, 256, 0, st>>>((const T*)dy, ids, out, V, D);
+  else emb_atomic_kernel<T, 4><<<(unsigned)tokens, 256, 0, st>>>((const T*)dy, ids, out, V, D);
+}
+
+// (a memset of the same bytes takes 1 to 3 us more)
+__global__ void __launch_bounds__(256) emb_zero_kernel(float4* p, long long n) {
+  const long long i = (long long)blockIdx.x * 1024 + threadIdx.x;
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (i + k * 256 < n) p[i + k * 256] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
 template <typename T, int W>
 static void emb_launch(const void* dy, const EmbWs& ws, void* out, long long T_, long long V, int D, int num_sms, cudaStream_t st) {
-  const long long chunks = emb_max_chunks(T_);
   const int nvec = D / W;
-  if (chunks > 0) {
+  if (emb_max_longs(T_) > 0) {
     const int split = (nvec + 127) / 128;
-    emb_partial_kernel<T, W><<<dim3((unsigned)chunks, (unsigned)(split < 16 ? split : 16)), 128, 0, st>>>((const T*)dy, ws, D);
+    emb_partial_kernel<T, W><<<dim3((unsigned)emb_max_chunks(T_), (unsigned)(split < 16 ? split : 16)), 128, 0, st>>>((const T*)dy, ws, D);
+    const long long items = emb_max_longs(T_) * ((D + 32 * W - 1) / (32 * W));
+    emb_long_kernel<T, W><<<(unsigned)(items < 2 * num_sms ? items : 2 * num_sms), 256, 0, st>>>(ws, (T*)out, D);
   }
   int tx = 32;
   while (tx < nvec && tx < 256) tx *= 2;
@@ -232,7 +328,8 @@ static long long emb_carve(EmbWs* ws, void* base, long long T, long long V, int 
   const long long chunks = emb_max_chunks(T);
   ws->part = reinterpret_cast<float*>(take(chunks * D));
   ws->desc = reinterpret_cast<int2*>(take(2 * chunks));
-  ws->ctr = take(2);
+  ws->longs = take(emb_max_longs(T));
+  ws->ctr = take(3);
   ws->count = take(V);
   ws->start = take(V);
   ws->chunk0 = take(V);
@@ -245,7 +342,37 @@ static long long emb_carve(EmbWs* ws, void* base, long long T, long long V, int 
 
 using namespace apb;
 
-extern "C" long long apb_embedding_bwd_workspace(long long tokens, long long num_rows, int D) {
+// Estimates of both forms in microseconds, fitted to 405 sizes (1 ... 524288 tokens, 2 ... 1000000 rows of 16 ... 4096) in both types with
+// ids at random, by Zipf's law, half of them and all of them the same: bytes of the table and atomics, or the grouping and one
+// read of dy.  Sorting has to promise a tenth.  bf16, 8192 tokens at random, sorted / atomic: 32000 x 64 24.7 / 16.5 us, 8192 x 1024
+// 24.7 / 24.7, 32000 x 4096 82 / 263, 128256 x 4096 201 / 806; fp32: 128256 x 1024 123 / 92, 1024 x 4096 53 / 68.  Rows that are no whole vectors are slow to gather:
+// in fp32 nothing is left to gain.  Where it sorts, that was the slower form by more than 3 % in 8 of 3240 timings.
+extern "C" int apb_embedding_bwd_sorts(long long tokens, long long num_rows, int D, int is_bf16) {
+  const double T = (double)tokens, V = (double)num_rows, td = T * D, vd = V * D;
+  const bool vec = D % (is_bf16 ? 8 : 4) == 0;
+  double atomic, sorted;
+  if (is_bf16) {
+    atomic = 7 + vd * 10 / 4.2e6 + (td / 0.7e6 > 6.3e-4 * T ? td / 0.7e6 : 6.3e-4 * T);
+    sorted = 31 + (vec ? 5.6e-4 : 7.0e-4) * T + 1.0e-4 * V + vd * 2 / 4.3e6 + (vec ? 2.0e-7 : 6.0e-7) * td;
+  } else {
+    if (!vec) return 0;
+    atomic = 3 + vd * 4 / 5.4e6 + (td / 0.6e6 > 6.0e-4 * T ? td / 0.6e6 : 6.0e-4 * T);
+    sorted = 23 + 5.5e-4 * T + 1.2e-4 * V + vd * 4 / 5.6e6 + 2.3e-7 * td;
+  }
+  if (T >= 16 * V) sorted += 18;  // most lists are long, and summed in two steps
+  return sorted < 0.9 * atomic;
+}
+
+// kernels that a call launches
+extern "C" int apb_embedding_bwd_launches(long long tokens, long long num_rows, int D, int is_bf16) {
+  if (num_rows <= 0 || D <= 0) return 0;
+  if (apb_embedding_bwd_sorts(tokens, num_rows, D, is_bf16)) return emb_max_longs(tokens) > 0 ? 4 : 2;
+  return (num_rows * D % 4 == 0) + (tokens > 0) + (is_bf16 != 0);
+}
+
+// bytes of workspace
+extern "C" long long apb_embedding_bwd_workspace(long long tokens, long long num_rows, int D, int is_bf16) {
+  if (!apb_embedding_bwd_sorts(tokens, num_rows, D, is_bf16)) return is_bf16 ? num_rows * D * 4 : 0;
   EmbWs ws;
   return emb_carve(&ws, nullptr, tokens, num_rows, D);
 }
@@ -254,6 +381,19 @@ extern "C" long long apb_embedding_bwd_workspace(long long tokens, long long num
 extern "C" int apb_embedding_bwd(const void* dy, const long long* ids, void* out, void* workspace, long long tokens, long long num_rows,
                                  int D, int is_bf16, int num_sms, cudaStream_t st) {
   if (num_rows <= 0 || D <= 0) return 0;
+  if (!apb_embedding_bwd_sorts(tokens, num_rows, D, is_bf16)) {
+    if (tokens >= (1ll << 31) || (is_bf16 && (reinterpret_cast<uintptr_t>(out) & 15))) return 3;
+    float* acc = reinterpret_cast<float*>(is_bf16 ? workspace : out);
+    const long long n = num_rows * D;
+    if (n % 4 == 0 && (reinterpret_cast<uintptr_t>(acc) & 15) == 0) emb_zero_kernel<<<(unsigned)((n / 4 + 1023) / 1024), 256, 0, st>>>(reinterpret_cast<float4*>(acc), n / 4);
+    else if (cudaMemsetAsync(acc, 0, sizeof(float) * n, st) != cudaSuccess) return 4;
+    if (tokens > 0) {
+      if (is_bf16) emb_atomic<__nv_bfloat16>(dy, ids, acc, tokens, num_rows, D, st);
+      else emb_atomic<float>(dy, ids, acc, tokens, num_rows, D, st);
+    }
+    if (is_bf16) return apb_cast(acc, out, num_rows * D, 0, 1, num_sms, st);
+    return cudaGetLastError() == cudaSuccess ? 0 : 4;
+  }
   if (tokens >= (1ll << 30) || num_rows >= (1ll << 31)) return 3;
   EmbWs ws;
   emb_carve(&ws, workspace, tokens, num_rows, D);

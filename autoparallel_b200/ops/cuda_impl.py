@@ -367,8 +367,7 @@ def _embedding(weight, ids):
 def _embedding_bwd(dy, ids, num_rows):
     dy = dy.contiguous()
     out = torch.empty(num_rows, dy.shape[-1], dtype=dy.dtype, device=dy.device)
-    _C.embedding_bwd(dy, ids.contiguous(), out)
-    _count(3 if ids.numel() >= 32 else 2)
+    _count(_C.embedding_bwd(dy, ids.contiguous(), out))
     return out
 
 

@@ -48,6 +48,41 @@ def test_embedding_gradient_over_list_lengths(K, dtype, V, D, T, ids):
     assert torch.equal(out.cpu()[torch.bincount(idx, minlength=V) == 0], torch.zeros(int((torch.bincount(idx, minlength=V) == 0).sum()), D, dtype=dtype))
 
 
+@pytest.mark.parametrize("dtype,V,D,T,ids,sorts", [
+    (torch.bfloat16, 40000, 1024, 1, "same", True),      # one token of a long table
+    (torch.bfloat16, 40000, 1024, 32, "same", True),     # exactly one chunk, which is no long row
+    (torch.bfloat16, 40000, 1024, 33, "same", True),     # the shortest long row
+    (torch.bfloat16, 50257, 1000, 9000, "skewed", True),  # long and short lists, a last slice that is not full
+    (torch.bfloat16, 20000, 4096, 5000, "same", True),   # many chunks, several slices of the columns
+    (torch.bfloat16, 40000, 1025, 300, "random", True),  # rows that are no whole vectors
+    (torch.bfloat16, 100, 1024, 80000, "skewed", True),  # every row long
+    (torch.float32, 100, 1024, 80000, "skewed", True),
+    (torch.float32, 300, 1000, 60000, "same", True),
+    (torch.float32, 5, 1020, 60000, "random", True),
+    (torch.float32, 5, 1023, 60000, "random", False),    # fp32 rows that are no whole vectors
+    (torch.bfloat16, 1000, 256, 16384, "skewed", False),
+    (torch.bfloat16, 100000, 16, 513, "random", False),
+    (torch.float32, 50257, 1024, 300, "skewed", False),
+])
+def test_embedding_gradient_by_both_forms(K, dtype, V, D, T, ids, sorts):
+    lib, impl = K
+    assert impl.extension().embedding_bwd_sorts(T, V, D, dtype == torch.bfloat16) == sorts
+    g = torch.Generator(device="cuda").manual_seed(V + T)
+    idx = torch.randint(0, V, (T,), device="cuda", generator=g)
+    if ids == "same":
+        idx.fill_(V - 1)
+    elif ids == "skewed":
+        idx = (torch.rand(T, device="cuda", generator=g) ** 4 * V).long()
+    dy = torch.randn(T, D, device="cuda", generator=g).to(dtype)
+    out = lib.ops.embedding_bwd(dy, idx, V)
+    ref = torch.zeros(V, D, device="cuda", dtype=torch.float64).index_add_(0, idx, dy.double())
+    assert out.dtype == dtype and out.shape == (V, D)
+    err = ((out.double() - ref).norm() / ref.norm()).item()
+    # fp32 sums of at most T terms (each partial sum rounds once: 2^-24 sqrt(T) of the norm, bounded generously), then one rounding
+    assert err <= (2**-8 if dtype == torch.bfloat16 else 2**-24 * T ** 0.5 * 4)
+    assert not out[torch.bincount(idx, minlength=V) == 0].any()
+
+
 def test_embedding_gradient_of_an_unaligned_view(K):
     lib, _ = K
     flat = torch.randn(1 + 12 * 16, device="cuda").to(torch.bfloat16)
