@@ -46,10 +46,12 @@ constexpr int AG_NBUF = 4, AG_CHUNK = 8192;  // bounce ring of the gather warp: 
 constexpr int GEMM_FUSED_AG_SMEM_BYTES = GEMM_SMEM_BYTES + AG_NBUF * AG_CHUNK;
 constexpr int GEMM_AG_THREADS = GEMM_THREADS + 32;
 
-// CTA pairs take a product with more than one 128-row tile: also with 129 to 255 rows a pair's 256-row tile brings every
-// B tile into the SMs once (32 KB per SM and k-block), where two single CTAs load it twice (48 KB).  64 experts, 160 rows,
-// N = 1408, K = 2048: 95 -> 83 us.
-inline bool pair_shape(int M, int N) { return M > BM && N >= BN; }
+// CTA pairs take a product with at least one full pair tile.  Of those with 129 to 255 rows, whose odd CTA is partly idle, they take
+// the ones with a long contraction: the pair's tile brings every B tile into the SMs once (32 KB per SM and k-block) where two single
+// CTAs load it twice (48 KB), but starts 0.8 us later.  130 ... 255 rows, single against pair, geometric means over 256 < N <= 57344 and
+// groups of 4 ... 74: K = 64 0.88, 512 0.96, 1024 1.04, 1280 1.06, 2048 1.07, 4096 1.08, 8192 1.12; one column tile (N = 256) 0.89 to 0.99 below
+// K = 4096.  64 experts, 160 rows, N = 1408, K = 2048: 95 -> 83 us.
+inline bool pair_shape(int M, int N, int K) { return M >= 2 * BM ? N >= BN : M > BM && N > BN && K >= 1280; }
 
 enum : int { FUSE_NONE = 0, FUSE_GATHER_A = 1, FUSE_GATHER_B = 2, FUSE_REDUCE_SCATTER = 3 };
 

@@ -287,7 +287,7 @@ static SplitPlan split_plan(int G, int M, int N, int K, int num_sms) {
   SplitPlan best{0, 0};
   if (g * m_tiles * ((N + 255) / 256) > num_sms) return best;  // no width fits in one wave
   const int kb = (K + BK - 1) / BK;
-  const bool pair = pair_shape(M, N);
+  const bool pair = pair_shape(M, N, K);
   const long long tiles = g * (pair ? (M + 2 * BM - 1) / (2 * BM) : m_tiles) * ((N + BN - 1) / BN);
   const int units = pair ? apb_gemm_resident_pairs(num_sms) : num_sms;
   const double now = 5.5 + (double)((tiles + units - 1) / units) * (0.5 + (pair ? 0.38 : 0.35) * kb);

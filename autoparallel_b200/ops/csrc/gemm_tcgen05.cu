@@ -177,7 +177,7 @@ extern "C" int apb_gemm_bf16(const void* A, const void* B, void* C, int M, int N
     const int e3 = make_store_map(&tmC, C, (uint64_t)N, (uint64_t)M, 0, (uint64_t)ldc, out_fp32);
     if (e3) return e3;
   }
-  if (g_pair_mode && pair_shape(M, N)) {
+  if (g_pair_mode && pair_shape(M, N, K)) {
     // CTA pairs: B is loaded in boxes of 128 rows (each CTA stages half of the 256 tile columns)
     int e2 = 0;
     if (!b_mn_major) e2 = make_map(&tmB, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, BN / 2);
@@ -237,7 +237,7 @@ extern "C" int apb_gemm_grouped_bf16(const void* A, const void* B, void* C, int 
     const int es = apb_gemm_split_auto(A, B, C, G, M, N, K, 0, 0, 0, a_mn_major, b_mn_major, out_fp32, status, usable, stream);
     if (es >= 0) return es;
   }
-  const bool pair = g_pair_mode && pair_shape(M, N);
+  const bool pair = g_pair_mode && pair_shape(M, N, K);
   CUtensorMap tmA, tmB;
   int e = !a_mn_major ? make_map_3d(&tmA, A, (uint64_t)K, (uint64_t)M, (uint64_t)G, (uint64_t)K, BM)
                       : make_map_3d(&tmA, A, (uint64_t)M, (uint64_t)K, (uint64_t)G, (uint64_t)M, BK);

@@ -336,7 +336,7 @@ def test_pairs_with_less_than_two_full_row_tiles(K, M, ta):
     lib, impl = K
     if ta and M % 8:
         pytest.skip("rows of 16 bytes")
-    E, N, K_ = 24, 1408, 192
+    E, N, K_ = 24, 1408, 1288  # (a contraction long enough for pairs)
     g = torch.Generator(device="cuda").manual_seed(M)
     a = torch.randn(*((E, K_, M) if ta else (E, M, K_)), device="cuda", generator=g).to(torch.bfloat16)
     w = torch.randn(E, K_, N, device="cuda", generator=g).to(torch.bfloat16)
