@@ -13,6 +13,7 @@ int apb_gemm_grouped_bf16(const void* A, const void* B, void* C, int G, int M, i
                           int out_fp32, uint32_t* status, int num_sms, cudaStream_t stream);
 int apb_gemm_split(const void* A, const void* B, void* C, int G, int M, int N, int K, long long lda, long long ldb, long long ldc,
                    int a_mn, int b_mn, int out_fp32, int bn, int s, uint32_t* status, cudaStream_t stream);
+void apb_gemm_split_choice(int G, int M, int N, int K, int num_sms, int reserved, int* bn, int* s);
 void apb_gemm_set_pair_mode(int on);
 int apb_gemm_get_pair_mode();
 int apb_gemm_yield_request(int pairs, cudaStream_t stream);
@@ -529,6 +530,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm", &gemm);
   m.def("gemm_grouped", &gemm_grouped);
   m.def("gemm_split", &gemm_split);
+  m.def("gemm_split_choice", [](int64_t groups, int64_t M, int64_t N, int64_t K) {  // groups 0: a plain product
+    int bn = 0, s = 0;
+    apb_gemm_split_choice((int)groups, (int)M, (int)N, (int)K, num_sms(), apb_gemm_get_reserved_sms(), &bn, &s);
+    return std::make_tuple((int64_t)bn, (int64_t)s);
+  });
   m.def("gemm_set_pair_mode", [](bool on) { apb_gemm_set_pair_mode(on ? 1 : 0); });
   m.def("gemm_yield_request", [](int64_t pairs) { check(apb_gemm_yield_request((int)pairs, stream()), "apb_gemm_yield_request"); });
   m.def("gemm_yield_outstanding", []() { return (int64_t)apb_gemm_yield_outstanding(); });

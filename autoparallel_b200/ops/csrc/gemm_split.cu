@@ -12,8 +12,8 @@
 // second launch, the same result every time.
 //
 //   warp 0: TMA producer | warp 1: TMEM owner + MMA issuer | warps 2..5: TMEM -> shared memory | all: sum and store
-// Before -> after, us: 16 x 4096 x 4096 28 -> 12, 16 x 4096 x 14336 88 -> 27, 64 x 2048 x 2048 16 -> 8.6, 64 x 2048 x 8192 47 -> 16,
-// 512 x 256 x 256 7.4 -> 6.1, 999 x 1408 x 2048 18.8 -> 17.0.
+// Persistent kernels -> this one, us: 16 x 4096 x 4096 29 -> 13, 16 x 4096 x 14336 87 -> 25, 64 x 2048 x 2048 16.6 -> 8.6, 64 x 2048 x 8192 50 -> 15.6,
+// 512 x 256 x 256 7.0 -> 5.5, 160 x 8192 x 8192 55 -> 39; 478 products in profiles/gemm_split_rule_sweep.txt.
 #include "gemm_core.cuh"
 
 namespace apb {
@@ -239,12 +239,13 @@ static SplitKernel split_kernel_of(int bn, int a_mn, int b_mn) {
 
 // Tile width and slice count for a product, or bn = 0 where the persistent kernels are expected to be faster.
 //
-// Only forms whose clusters are all resident at once: in a second wave every tile pays its fixed part again, and the
-// persistent kernels were faster in every such case of the sweeps (16 x 4096 x 4096 ... 8192 x 1024 x 4096, all widths and
-// slice counts).  The estimates (microseconds, one B200) are fitted to those sweeps: a fixed part that grows with the tile
-// (launch, prologue, TMEM -> shared memory -> C), then the longest of a chain of k-blocks, the operand traffic out of L2
-// (9.5 TB/s) and the operands out of memory (6.5 TB/s, less while few bytes are in flight), then the cluster's sum.
-// Over the sweeps the choice was always faster than the persistent kernels and within 20 % of the best form.
+// Only forms whose clusters are all resident at once: in a second wave every tile pays its fixed part again.  The estimates
+// (microseconds, one B200) are fitted to sweeps: a fixed part that grows with the tile (launch, prologue, TMEM -> shared memory -> C),
+// then the longest of a chain of k-blocks, the operand traffic out of L2 (9.5 TB/s) and the operands out of memory (6.5 TB/s, less while
+// few bytes are in flight), then the cluster's sum.  They are good to ten per cent or so; where the sweeps showed them to flatter the
+// split, it is left out: forms with no more CTAs than the persistent kernels would use (twice as many where the contraction has
+// one or two blocks), slices of a single block, whole contractions in 256-wide tiles, and in 64-wide ones on most of the chip.
+// Of 260 random products that it splits, 3 were more than 2 % slower for it (contractions of 8, up to 0.6 us); the mean gain is 1.6.
 struct SplitPlan {
   int bn, s;
 };
@@ -281,25 +282,29 @@ static int split_slots(int s, int num_sms) {
   return n * s;
 }
 
-static SplitPlan split_plan(int G, int M, int N, int K, int num_sms) {
+static SplitPlan split_plan(int G, int M, int N, int K, int num_sms, int reserved) {
   const long long g = G > 0 ? G : 1;
   const long long m_tiles = (M + BM - 1) / BM;
+  const int usable = num_sms - reserved > 0 ? num_sms - reserved : 1;
   SplitPlan best{0, 0};
-  if (g * m_tiles * ((N + 255) / 256) > num_sms) return best;  // no width fits in one wave
+  if (g * m_tiles * ((N + 255) / 256) > usable) return best;  // no width fits in one wave
   const int kb = (K + BK - 1) / BK;
   const bool pair = pair_shape(M, N, K);
   const long long tiles = g * (pair ? (M + 2 * BM - 1) / (2 * BM) : m_tiles) * ((N + BN - 1) / BN);
-  const int units = pair ? apb_gemm_resident_pairs(num_sms) : num_sms;
+  int units = pair ? apb_gemm_resident_pairs(num_sms) - reserved / 2 : usable;  // as the launches have it
+  if (units < 1) units = 1;
   const double now = 5.5 + (double)((tiles + units - 1) / units) * (0.5 + (pair ? 0.38 : 0.35) * kb);
+  const long long ctas = (tiles < units ? tiles : units) * (pair ? 2 : 1) * (kb <= 2 ? 2 : 1);
   const double operands = 2.0 * g * ((double)M * K + (double)N * K);
-  double t_best = 0.95 * now;  // (a clear gain only: the estimates are good to ten per cent or so)
+  double t_best = 0.95 * now;  // (a clear gain only)
   for (int bn = 64; bn <= 256; bn *= 2) {
     const double fixed = bn == 64 ? 5.6 : bn == 128 ? 7.0 : 9.0, per_kb = bn == 128 ? 0.20 : 0.27;
     const long long t = g * m_tiles * ((N + bn - 1) / bn);
     const double kb_bytes = 128.0 * ((M < BM ? M : BM) + (N < bn ? N : bn));
     for (int s = 1; s <= SPLIT_MAX && s <= kb; ++s) {
-      if (t * s > num_sms) break;
-      if (t * s > split_slots(s, num_sms)) continue;
+      if (t * s > usable) break;
+      if (t * s > split_slots(s, num_sms) || t * s <= ctas) continue;
+      if (s > 1 ? kb < 2 * s : bn == 256 || (bn == 64 && t > 100)) continue;
       const int chain = (kb + s - 1) / s;
       double flow = per_kb * chain;
       const double l2 = (double)t * kb * kb_bytes / 9.5e6;
@@ -316,6 +321,13 @@ static SplitPlan split_plan(int G, int M, int N, int K, int num_sms) {
     }
   }
   return best;
+}
+
+// The rule above: tile width and slices, 0 and 0 where the persistent kernels run.
+extern "C" void apb_gemm_split_choice(int G, int M, int N, int K, int num_sms, int reserved, int* bn, int* s) {
+  const SplitPlan plan = split_plan(G, M, N, K, num_sms, reserved);
+  *bn = plan.bn;
+  *s = plan.s;
 }
 
 // One launch with the given tile width (64, 128, 256) and number of k-slices (1..8, at most one per 64 of K).  G > 0: grouped,
@@ -376,8 +388,9 @@ extern "C" int apb_gemm_split(const void* A, const void* B, void* C, int G, int 
 
 // The rule above and its launch: 0 = launched, -1 = the caller's kernels are the better choice (nothing launched), > 0 = error.
 extern "C" int apb_gemm_split_auto(const void* A, const void* B, void* C, int G, int M, int N, int K, long long lda, long long ldb,
-                                   long long ldc, int a_mn, int b_mn, int out_fp32, uint32_t* status, int num_sms, cudaStream_t stream) {
-  const SplitPlan plan = split_plan(G, M, N, K, num_sms);
+                                   long long ldc, int a_mn, int b_mn, int out_fp32, uint32_t* status, int num_sms, int reserved,
+                                   cudaStream_t stream) {
+  const SplitPlan plan = split_plan(G, M, N, K, num_sms, reserved);
   if (plan.bn == 0) return -1;
   return apb_gemm_split(A, B, C, G, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_fp32, plan.bn, plan.s, status, stream);
 }

@@ -149,7 +149,8 @@ extern "C" int apb_gemm_get_pair_mode() { return g_pair_mode; }
 
 // gemm_split.cu: products with few tiles; -1 = the kernels here are the better choice
 extern "C" int apb_gemm_split_auto(const void* A, const void* B, void* C, int G, int M, int N, int K, long long lda, long long ldb,
-                                   long long ldc, int a_mn, int b_mn, int out_fp32, uint32_t* status, int num_sms, cudaStream_t stream);
+                                   long long ldc, int a_mn, int b_mn, int out_fp32, uint32_t* status, int num_sms, int reserved,
+                                   cudaStream_t stream);
 
 // Returns 0 on success; >0 = argument / driver error (nothing launched).
 extern "C" int apb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
@@ -160,7 +161,7 @@ extern "C" int apb_gemm_bf16(const void* A, const void* B, void* C, int M, int N
   if (K <= 0) return zero_result(C, M, N, ldc, out_fp32, stream);
   const int usable = num_sms - g_reserved_sms > 0 ? num_sms - g_reserved_sms : 1;
   if (g_pair_mode) {
-    const int es = apb_gemm_split_auto(A, B, C, 0, M, N, K, lda, ldb, ldc, a_mn_major, b_mn_major, out_fp32, status, usable, stream);
+    const int es = apb_gemm_split_auto(A, B, C, 0, M, N, K, lda, ldb, ldc, a_mn_major, b_mn_major, out_fp32, status, num_sms, g_reserved_sms, stream);
     if (es >= 0) return es;
   }
   CUtensorMap tmA, tmB;
@@ -234,7 +235,7 @@ extern "C" int apb_gemm_grouped_bf16(const void* A, const void* B, void* C, int 
   if (K <= 0) return zero_result(C, (long long)G * M, N, N, out_fp32, stream);
   const int usable = num_sms - g_reserved_sms > 0 ? num_sms - g_reserved_sms : 1;
   if (g_pair_mode) {
-    const int es = apb_gemm_split_auto(A, B, C, G, M, N, K, 0, 0, 0, a_mn_major, b_mn_major, out_fp32, status, usable, stream);
+    const int es = apb_gemm_split_auto(A, B, C, G, M, N, K, 0, 0, 0, a_mn_major, b_mn_major, out_fp32, status, num_sms, g_reserved_sms, stream);
     if (es >= 0) return es;
   }
   const bool pair = g_pair_mode && pair_shape(M, N, K);

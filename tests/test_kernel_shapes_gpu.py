@@ -317,6 +317,34 @@ def test_gemm_split_over_tiles_and_slices(K, M, N, K_, ta, tb, bn, slices):
         assert bool((back == 7.0).all()), "nothing outside the window is written"
 
 
+@pytest.mark.parametrize("groups,M,N,K_,split", [
+    (0, 16, 4096, 4096, True),       # few rows
+    (0, 64, 2048, 8192, True),       # a router's weight gradient
+    (0, 512, 256, 256, True),        # four pair tiles
+    (16, 64, 704, 1024, True),       # a stack of small products
+    (0, 8192, 4096, 4096, False),    # more tiles than SMs
+    (64, 160, 1408, 2048, False),
+    (0, 300, 64, 64, False),         # one k-block, no more CTAs to be had than the persistent kernel uses
+    (0, 4858, 16, 80, False),
+])
+def test_which_products_are_split(K, groups, M, N, K_, split):
+    _, impl = K
+    ext = impl.extension()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    bn, s = ext.gemm_split_choice(groups, M, N, K_)
+    assert (bn != 0) == split
+    prev = ext.gemm_get_reserved_sms()
+    try:
+        for reserved in (0, 40, sms):
+            ext.gemm_set_reserved_sms(reserved)
+            bn, s = ext.gemm_split_choice(groups, M, N, K_)
+            if bn:
+                ctas = max(groups, 1) * -(-M // 128) * -(-N // bn) * s
+                assert ctas <= sms - reserved and (s == 1 or 2 * s <= -(-K_ // 64)) and (bn, s) != (256, 1)
+    finally:
+        ext.gemm_set_reserved_sms(prev)
+
+
 @pytest.mark.parametrize("bn,slices", [(64, 2), (128, 1), (256, 3)])
 def test_grouped_gemm_split(K, bn, slices):
     lib, impl = K
