@@ -338,7 +338,7 @@ template <bool A_MN, bool B_MN, int FUSE, bool PAIR = false, bool GROUPED = fals
 __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p,
                                          const FuseParams& f, int cta, int num_ctas, uint8_t* smem_raw,
                                          const CUtensorMap* tmC = nullptr) {
-  constexpr int STAGING = FUSE == FUSE_NONE ? STAGING_BYTES : 0;
+  constexpr int STAGING = FUSE == FUSE_NONE && ST_ARG == 0 ? STAGING_BYTES : 0;  // (fewer stages: to leave shared memory free)
   constexpr int ST = ST_ARG > 0 ? ST_ARG : (PAIR ? PAIR_STAGES : STAGES);
   constexpr int A_BYTES = A_STAGE_BYTES;                          // 128 rows of A per CTA
   constexpr int B_BYTES = PAIR ? B_STAGE_BYTES / 2 : B_STAGE_BYTES;  // PAIR: this CTA's 128 of the 256 B rows
@@ -698,7 +698,7 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
         rs_base = reinterpret_cast<float*>(f.peers.base[owner] + apbs::HEADER_BYTES) +
                   ((long long)f.rank * f.rows_per_rank + (row - (long long)owner * f.rows_per_rank)) * p.N;
       }
-      const bool via_tma = FUSE == FUSE_NONE && p.tma_store;
+      const bool via_tma = STAGING > 0 && p.tma_store;
       if (via_tma) {
         uint8_t* stg = smem + ST * (A_BYTES + B_BYTES) + (warp - 2) * STORE_BYTES;
         const int grp = GROUPED ? t / tiles_per_group : 0;
@@ -775,7 +775,7 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
         buf_phase ^= 1;
       }
     }
-    if (FUSE == FUSE_NONE && lane == 0) tma_store_wait_all();
+    if (STAGING > 0 && lane == 0) tma_store_wait_all();
   }
 
   tc_fence_before();

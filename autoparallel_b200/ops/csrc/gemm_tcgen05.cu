@@ -88,9 +88,12 @@ using namespace apb;
 
 // SMs that the GEMM kernels leave idle so that communication kernels launched on other streams (NCCL)
 // find a free SM right away: a persistent GEMM CTA owns its SM's shared memory for the whole kernel.
-// TMA stages of the CTA-pair GEMM: 6 fill the SM's shared memory; 5 or 4 leave 32 / 64 KB more for a
-// communication kernel's CTA to become resident beside a GEMM CTA.
+// TMA stages of the CTA-pair GEMM: 6 fill the SM's shared memory; 5 or 4 leave 32 / 64 KB more, and the epilogue's staging blocks,
+// for a communication kernel's CTA to become resident beside a GEMM CTA.
 static int g_pair_stages = 6;
+extern "C" int apb_gemm_pair_smem_bytes(int stages) {
+  return stages * (A_STAGE_BYTES + B_STAGE_BYTES / 2) + (stages == PAIR_STAGES ? STAGING_BYTES : 0) + 1024 + 256;
+}
 extern "C" void apb_gemm_set_pair_stages(int n) { g_pair_stages = n <= 4 ? 4 : (n == 5 ? 5 : 6); }
 extern "C" int apb_gemm_get_pair_stages() { return g_pair_stages; }
 // Dynamic tile scheduling of the CTA-pair GEMM (see gemm_core.cuh): off = every pair owns a fixed share.
@@ -160,7 +163,9 @@ extern "C" int apb_gemm_bf16(const void* A, const void* B, void* C, int M, int N
   if (reinterpret_cast<uintptr_t>(C) & 15) return 3;
   if (K <= 0) return zero_result(C, M, N, ldc, out_fp32, stream);
   const int usable = num_sms - g_reserved_sms > 0 ? num_sms - g_reserved_sms : 1;
-  if (g_pair_mode) {
+  // Pairs with dynamic tiles answer the requests for SMs, pairs with fewer stages leave shared memory free: those products stay theirs.
+  const bool keep_pairs = (g_dynamic_tiles || g_pair_stages != PAIR_STAGES) && pair_shape(M, N, K);
+  if (g_pair_mode && !keep_pairs) {
     const int es = apb_gemm_split_auto(A, B, C, 0, M, N, K, lda, ldb, ldc, a_mn_major, b_mn_major, out_fp32, status, num_sms, g_reserved_sms, stream);
     if (es >= 0) return es;
   }
@@ -187,7 +192,7 @@ extern "C" int apb_gemm_bf16(const void* A, const void* B, void* C, int M, int N
     int resident = apb_gemm_resident_pairs(num_sms) - g_reserved_sms / 2;
     if (resident < 1) resident = 1;
     const int pairs = tiles2 < resident ? tiles2 : resident;
-    const int smem2 = g_pair_stages * (A_STAGE_BYTES + B_STAGE_BYTES / 2) + STAGING_BYTES + 1024 + 256;
+    const int smem2 = apb_gemm_pair_smem_bytes(g_pair_stages);
     auto launch2 = [&](auto kern) {
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2);
       kern<<<2 * pairs, GEMM_THREADS, smem2, stream>>>(tmA, tmB, tmC, p);

@@ -72,3 +72,11 @@ for i in (0, 1, 2, 4, 5):
     print(so.apb_rms_norm_bwd_noalloc(*a, LL(4), 64, 1, None))
 """)
     assert out == ["9"] * 5
+
+
+@needs_ext
+def test_pair_gemm_with_fewer_stages_leaves_their_shared_memory():
+    """What the switch is for: room for a communication kernel's CTA beside a GEMM CTA (32 KB a stage, nothing else in their place)."""
+    out = _run("print(*[so.apb_gemm_pair_smem_bytes(s) for s in (4, 5, 6)])")
+    four, five, six = map(int, out)
+    assert (four, five) == (4 * 32768 + 1280, 5 * 32768 + 1280) and six <= 227 * 1024

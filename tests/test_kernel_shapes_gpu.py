@@ -345,6 +345,32 @@ def test_which_products_are_split(K, groups, M, N, K_, split):
         ext.gemm_set_reserved_sms(prev)
 
 
+@pytest.mark.parametrize("M,N,K_", [(512, 512, 2048), (300, 264, 520), (2000, 1544, 136)])
+@pytest.mark.parametrize("stages,dynamic", [(4, False), (5, False), (6, True)])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+def test_pairs_that_make_room_for_communication(K, M, N, K_, stages, dynamic, out_dtype):
+    """Fewer stages, and dynamic tiles that answer a request for SM pairs: also in products with few tiles, which would be split."""
+    lib, impl = K
+    ext = impl.extension()
+    g = torch.Generator(device="cuda").manual_seed(M)
+    a = torch.randn(M, K_, device="cuda", generator=g).to(torch.bfloat16)
+    b = torch.randn(N, K_, device="cuda", generator=g).to(torch.bfloat16)
+    prev = ext.gemm_get_pair_stages(), ext.gemm_get_dynamic_tiles()
+    ext.gemm_set_pair_stages(stages)
+    ext.gemm_set_dynamic_tiles(dynamic)
+    try:
+        if dynamic:
+            ext.gemm_yield_request(1)
+            assert ext.gemm_yield_outstanding() == 1
+        c = lib.ops.gemm(a, b, False, True, out_dtype)
+        assert ext.gemm_yield_outstanding() == 0  # (half of a launch of two pairs or more may go)
+    finally:
+        ext.gemm_set_pair_stages(prev[0])
+        ext.gemm_set_dynamic_tiles(prev[1])
+    # fp32 accumulation of K products (2^-24 sqrt(K), generously), one rounding to bf16
+    assert _rel(c, a.double() @ b.double().t()) <= (2**-8 if out_dtype == torch.bfloat16 else 2**-24 * 8 * K_ ** 0.5)
+
+
 @pytest.mark.parametrize("bn,slices", [(64, 2), (128, 1), (256, 3)])
 def test_grouped_gemm_split(K, bn, slices):
     lib, impl = K
