@@ -635,8 +635,11 @@ __global__ void adamw_kernel(const AdamTensor* __restrict__ tensors, const int2*
   const AdamTensor t = tensors[ch.x];
   const long long base = (long long)ch.y * ADAM_CHUNK;
   const long long end = min(base + (long long)ADAM_CHUNK, t.n);
+  // (any of the four may be a view at an odd offset: a gradient out of a flat buffer)
+  const bool vec = ((reinterpret_cast<uintptr_t>(t.p) | reinterpret_cast<uintptr_t>(t.g) | reinterpret_cast<uintptr_t>(t.m) |
+                     reinterpret_cast<uintptr_t>(t.v)) & 15) == 0;
   for (long long i = base + threadIdx.x * 4; i < end; i += blockDim.x * 4) {
-    if (i + 4 <= end && ((reinterpret_cast<uintptr_t>(t.p + i) & 15) == 0)) {
+    if (vec && i + 4 <= end) {
       float4 p = *reinterpret_cast<float4*>(t.p + i);
       const float4 g4 = *reinterpret_cast<const float4*>(t.g + i);
       float4 m = *reinterpret_cast<float4*>(t.m + i);

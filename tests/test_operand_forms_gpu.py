@@ -132,3 +132,27 @@ def test_dense_views_off_a_16_byte_boundary(K, dtype):
             got = getattr(lib.ops, name)(*args, *rest)
             for a, b in zip(got if isinstance(got, tuple) else (got,), want if isinstance(want, tuple) else (want,)):
                 assert _rel(a, b) <= tol, (name, i)
+
+
+@pytest.mark.parametrize("odd", ["param", "grad", "exp_avg", "exp_avg_sq"])
+def test_adamw_takes_views_off_a_16_byte_boundary(K, odd):
+    """A parameter, gradient or state out of a flat buffer: the same step as on tensors of their own."""
+    from autoparallel_b200.optim import AdamW
+
+    g = torch.Generator().manual_seed(2)
+    n = 70001  # two chunks of the kernel, and a tail
+    t = {k: torch.randn(n, generator=g) for k in ("param", "grad", "exp_avg")}
+    t["exp_avg_sq"] = torch.rand(n, generator=g)
+
+    def step(view):
+        v = {k: (_off(x) if view and k == odd else x.cuda()) for k, x in t.items()}
+        p = torch.nn.Parameter(v["param"])
+        opt = AdamW([p], lr=1e-2, betas=(0.9, 0.95), eps=1e-8, weight_decay=0.1)
+        p.grad = v["grad"]
+        opt._init_state(p)
+        opt.state[p]["exp_avg"], opt.state[p]["exp_avg_sq"] = v["exp_avg"], v["exp_avg_sq"]
+        opt.step()
+        return p.detach(), opt.state[p]["exp_avg"], opt.state[p]["exp_avg_sq"]
+
+    for a, b in zip(step(True), step(False)):
+        assert _rel(a, b) <= 2**-21  # (the vector and the scalar path round a product and sum differently, a few ulp)
