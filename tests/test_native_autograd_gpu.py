@@ -115,6 +115,37 @@ def test_transforms_stay_refused(ops):
         ops.mm_nd(fwd.make_dual(a.requires_grad_(), torch.ones_like(a)), w, True, torch.bfloat16)
 
 
+@pytest.mark.parametrize("name", NAMES)
+def test_every_recorded_call_refuses_transforms_and_forward_mode(ops, name):
+    """As the Python registration does.  (A dual tensor in a call that records nothing loses its tangent, on every device: what is
+    refused is the recorded form.)"""
+    import torch.autograd.forward_ad as fwd
+
+    (tensors, rest), _ = _case(name)
+    first, *others = [t.cuda() for t in tensors]
+    with pytest.raises(RuntimeError, match="functorch transforms"):
+        torch.func.grad(lambda t: _first(_op(ops, name)(t, *others, *rest)).float().sum())(first)
+    with pytest.raises((RuntimeError, NotImplementedError), match="jvp"), fwd.dual_level():
+        _op(ops, name)(fwd.make_dual(first.requires_grad_(), torch.ones_like(first)), *others, *rest)
+
+
+@pytest.mark.parametrize("shape", [(16, 64), (2, 8, 64)])
+def test_a_projection_changed_in_place_keeps_its_gradient_or_refuses(ops, shape):
+    g = torch.Generator(device="cuda").manual_seed(5)
+    a = torch.randn(*shape, device="cuda", generator=g).bfloat16()
+    w = torch.randn(32, 64, device="cuda", generator=g).bfloat16()
+    want = 2 * w.double().sum(0).expand(shape)
+    a.requires_grad_()
+    y = ops.mm_nd(a, w, True, torch.bfloat16)
+    try:
+        y.mul_(2)
+    except RuntimeError as e:
+        assert "view" in str(e)
+        return
+    (da,) = torch.autograd.grad(y.float().sum(), a)
+    assert ((da.double() - want).norm() / want.norm()).item() <= 2**-7
+
+
 def test_modes_below_autograd_still_see_the_operators(ops):
     from torch.utils._python_dispatch import TorchDispatchMode
 
