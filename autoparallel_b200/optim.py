@@ -87,7 +87,8 @@ class AdamW(torch.optim.Optimizer):
         return st
 
     def _table(self, gi: int, plist):
-        """Device table of (p, g, m, v, p_lp, n) records + chunk list; rebuilt if a pointer moved."""
+        """Device table of (p, g, m, v, p_lp, n) records + chunk list; rebuilt if a pointer moved.  ``None`` where the kernel's 16-byte
+        accesses, which go by the parameter's address, would meet a gradient or moment at an odd offset."""
         key = tuple((_local(p).data_ptr(), _local(p.grad).data_ptr()) for p in plist)
         cached = self._tables.get(gi)
         if cached is not None and cached[0] == key:
@@ -98,8 +99,10 @@ class AdamW(torch.optim.Optimizer):
             lp, lg = _local(p), _local(p.grad)
             n = lp.numel()
             lp_ptr = self._shadow_of(p).data_ptr() if self.emit_bf16 and lp.dtype == torch.float32 else 0
-            recs += struct.pack("<QQQQQq", lp.data_ptr(), lg.data_ptr(), _local(st["exp_avg"]).data_ptr(),
-                                _local(st["exp_avg_sq"]).data_ptr(), lp_ptr, n)
+            ptrs = lp.data_ptr(), lg.data_ptr(), _local(st["exp_avg"]).data_ptr(), _local(st["exp_avg_sq"]).data_ptr()
+            if (ptrs[1] | ptrs[2] | ptrs[3]) & 15 and not ptrs[0] & 15:
+                return None
+            recs += struct.pack("<QQQQQq", *ptrs, lp_ptr, n)
             chunks += [(ti, c) for c in range((n + self.CHUNK - 1) // self.CHUNK)]
         dev = _local(plist[0]).device
         # Gradients are fresh tensors every step, so the record table changes every step: stage it in
@@ -195,11 +198,14 @@ class AdamW(torch.optim.Optimizer):
                 and _local(p.grad).is_contiguous()
                 for p in plist
             )
-            if fast:
+            tabled = self._table(gi, plist) if fast else None
+            if fast and tabled is None and capturing:
+                raise RuntimeError("a captured optimizer step needs gradients and state on 16-byte boundaries")
+            if tabled is not None:
                 from .ops import cuda_impl
 
                 cuda_impl.ensure_loaded()
-                table, ch, n = self._table(gi, plist)
+                table, ch, n = tabled
                 if self.shadow_arena is not None:
                     self.shadow_arena.barrier()  # every rank has finished reading the old shards
                 hyper = self._hyper_buffers(gi, lp0.device)["dev"] if capturing else None
