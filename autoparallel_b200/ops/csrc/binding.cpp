@@ -265,7 +265,7 @@ int64_t embedding_bwd(const at::Tensor& dy, const at::Tensor& ids, at::Tensor& o
   return apb_embedding_bwd_launches(ids.numel(), rows, (int)D, bf16);
 }
 
-// Mixture-of-experts dispatch (ops/moe_ops.py): gate_idx / slot [T, k] int64, w [T, k] fp32, buf [E, nb, C, d], src / out / g [T, d].
+// Mixture-of-experts dispatch (ops/moe_ops.py): gate_idx / slot [T, k] int64, w [T, k] fp32 or bf16, buf [E, nb, C, d], src / out / g [T, d].
 static void moe_check(const at::Tensor& x, const char* what) {
   TORCH_CHECK(x.is_cuda() && x.is_contiguous(), what, ": contiguous CUDA tensor expected");
 }

@@ -272,7 +272,9 @@ __global__ void __launch_bounds__(512, 1) rms_norm_bwd_kernel(const T* __restric
 // One row per step and block; the rows travel global -> shared memory as untiled bulk copies (``cp.async.bulk``,
 // completion on an mbarrier) through a ring of RMS_STAGES stages, issued two steps ahead by one thread, so the prefetch
 // costs no registers.  Blocks are small and several share an SM: while one waits at its barrier the others work (a single
-// 512-thread block per SM taking four rows a step spent half its time in the reduction: 8192 x 4096 bf16 59 -> 33 us, 999 x 2048 20 -> 6 us, fp32 2047 x 2048 21 -> 10 us).
+// 512-thread block per SM taking four rows a step spent half its time in the reduction).  This kernel alone, before -> after: 8192 x 4096
+// bf16 59 -> 33 us, 999 x 2048 20 -> 6, fp32 2047 x 2048 21 -> 10; with the weight gradient's column sums (before: a cleared row, atomics and a
+// cast) 59 -> 36, 24 -> 11, 24 -> 14.
 // One block barrier per step: the partial sums of consecutive steps sit in alternating slots, and a stage is refilled
 // after the barrier of the following step, which every thread reaches only when it has read the stage for the last time.
 // Waits are bounded: if a stage never arrives the block stops (its rows keep whatever dx held).

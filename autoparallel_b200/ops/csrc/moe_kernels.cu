@@ -2,7 +2,7 @@
 //
 //   moe_slots     arrival rank of every (token, choice) inside its expert, per token block, in token-major order
 //                 -> row of the block's [E * C] buffer, or E * C for an assignment beyond the capacity
-//   moe_scatter   buf[e, blk, c, :] = w[t, j] * src[t, :]            (buffer [E, nb, C, d], zero-filled by the caller)
+//   moe_scatter   buf[e, blk, c, :] = w[t, j] * src[t, :]            (buffer [E, nb, C, d]; every row is written here, the empty ones with zeros)
 //   moe_gather    out[t, :] = sum_j w[t, j] * buf[slot[t, j], :]     (dropped assignments contribute nothing)
 //   moe_gate_grad dw[t, j] = < buf[slot[t, j], :], g[t, :] >
 //
