@@ -201,24 +201,17 @@ class AdamW(torch.optim.Optimizer):
             tabled = self._table(gi, plist) if fast else None
             if fast and tabled is None and capturing:
                 raise RuntimeError("a captured optimizer step needs gradients and state on 16-byte boundaries")
+            if self.shadow_arena is not None:  # (on both paths: a gradient's address may differ from rank to rank)
+                self.shadow_arena.barrier()  # every rank has finished reading the old shards
             if tabled is not None:
                 from .ops import cuda_impl
 
                 cuda_impl.ensure_loaded()
                 table, ch, n = tabled
-                if self.shadow_arena is not None:
-                    self.shadow_arena.barrier()  # every rank has finished reading the old shards
                 hyper = self._hyper_buffers(gi, lp0.device)["dev"] if capturing else None
                 cuda_impl.extension().adamw(table, ch, n, group["lr"], b1, b2, group["eps"], group["weight_decay"], bc1, bc2,
                                             self.grad_scale, hyper)
                 cuda_impl._count()
-                if self.shadow_arena is not None:
-                    self.shadow_arena.barrier()  # the new shards are complete on every rank before anyone pulls
-                if self.emit_bf16:
-                    from .ops import shadow
-
-                    for p in plist:
-                        shadow.publish(_local(p), self._shadow_of(p))
             else:
                 for p in plist:
                     st = self.state[p]
@@ -229,9 +222,13 @@ class AdamW(torch.optim.Optimizer):
                     upd = (m / bc1) / ((v / bc2).sqrt() + group["eps"])
                     lp.mul_(1 - group["lr"] * group["weight_decay"]).add_(upd.to(lp.dtype), alpha=-group["lr"])
                     if self.emit_bf16 and lp.dtype == torch.float32:
-                        from .ops import shadow
+                        self._shadow_of(p).copy_(lp)
+            if self.shadow_arena is not None:
+                self.shadow_arena.barrier()  # the new shards are complete on every rank before anyone pulls
+            if self.emit_bf16:
+                from .ops import shadow
 
-                        sh = self._shadow_of(p)
-                        sh.copy_(lp)
-                        shadow.publish(lp, sh)
+                for p in plist:
+                    if _local(p).dtype == torch.float32:
+                        shadow.publish(_local(p), self._shadow_of(p))
         return loss

@@ -180,6 +180,28 @@ def test_adamw_bf16_shadow_replaces_the_cast_until_the_parameter_changes():
     shadow.clear()
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_adamw_brackets_every_path_with_arena_barriers(dtype):
+    """Two barriers a step on the elementwise path too: whether a rank's gradients reach the kernel depends on their addresses."""
+    from autoparallel_b200.ops import shadow
+    from autoparallel_b200.optim import AdamW
+
+    shadow.clear()
+    p = torch.nn.Parameter(torch.randn(40).to(dtype))
+    seen = []
+
+    class Arena:
+        def barrier(self):
+            seen.append(p.detach().clone())
+
+    opt = AdamW([p], lr=1e-2, emit_bf16=True, shadow_arena=Arena())
+    before = p.detach().clone()
+    p.grad = torch.randn_like(p)
+    opt.step()
+    assert len(seen) == 2 and torch.equal(seen[0], before) and torch.equal(seen[1], p.detach()) and not torch.equal(before, p.detach())
+    shadow.clear()
+
+
 def test_yarn_rope_tables_keep_fast_pairs_and_stretch_slow_ones():
     from autoparallel_b200.models.llama3 import rope_tables
 
