@@ -151,6 +151,11 @@ class AdamW(torch.optim.Optimizer):
             if gi not in self._tables:
                 raise RuntimeError("run one eager optimizer step before capturing (the pointer table is sized by it)")
 
+    def load_state_dict(self, state_dict) -> None:
+        super().load_state_dict(state_dict)
+        # the moments are other tensors now, which the key (parameters and gradients) does not show: no key matches from here
+        self._tables = {gi: (None, *entry[1:]) for gi, entry in self._tables.items()}
+
     @torch.no_grad()
     def advance_for_replay(self) -> None:
         """Before replaying a captured step: count the step and hand the kernel this step's learning rate and bias

@@ -1,4 +1,6 @@
 """Operand forms at the edge of what the kernels read - one row, views, empty sizes - against the CPU formulas."""
+import copy
+
 import pytest
 import torch
 
@@ -132,6 +134,32 @@ def test_dense_views_off_a_16_byte_boundary(K, dtype):
             got = getattr(lib.ops, name)(*args, *rest)
             for a, b in zip(got if isinstance(got, tuple) else (got,), want if isinstance(want, tuple) else (want,)):
                 assert _rel(a, b) <= tol, (name, i)
+
+
+def test_adamw_steps_on_the_loaded_state(K):
+    """Parameters and gradients keep their addresses when a state is loaded; the moments are other tensors."""
+    from autoparallel_b200.optim import AdamW
+
+    g = torch.Generator().manual_seed(3)
+    p0, g0 = torch.randn(1000, generator=g), torch.randn(1000, generator=g)
+
+    def make(first):
+        p = torch.nn.Parameter(p0.cuda())
+        opt = AdamW([p], lr=1e-2)
+        p.grad = (first * g0).cuda()
+        opt.step()
+        with torch.no_grad():
+            p.copy_(p0)
+            p.grad.copy_(g0)
+        return p, opt
+
+    p, opt = make(1.0)
+    q, other = make(-3.0)
+    opt.load_state_dict(copy.deepcopy(other.state_dict()))
+    opt.step(), other.step()
+    assert torch.equal(p, q)
+    for k in ("exp_avg", "exp_avg_sq"):
+        assert torch.equal(opt.state[p][k], other.state[q][k])
 
 
 @pytest.mark.parametrize("odd", ["param", "grad", "exp_avg", "exp_avg_sq"])
