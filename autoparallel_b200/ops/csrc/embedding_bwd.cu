@@ -10,9 +10,9 @@
 //                       list sorted by row.  A cluster because its barrier orders the phases inside one launch; 8192
 //                       threads take a usual batch in one or two steps.
 //   emb_partial_kernel  rows with more than EMB_CHUNK tokens (frequent words, padding): one fp32 partial row per chunk, so
-//                       that no block walks a long list alone.
-//   emb_long_kernel     those rows, from their chunks: a slice of the columns per block.
-//   emb_rows_kernel     every other row: zeros or the sum of its tokens.
+//                       that no block walks a long list alone.  Of rows with more than EMB_DIRECT chunks the last block of a group adds
+//                       the group up, and the last group the row.
+//   emb_rows_kernel     every other row: zeros, the sum of its tokens, or of its chunks.
 //
 // Atomic: an fp32 table of zeros, one block per token, for bf16 a conversion.  Better where the table is small or the rows are
 // short (the grouping is a chain of latencies that a small table does not pay for), and for most fp32 tables, which the atomics
@@ -28,6 +28,8 @@ extern "C" int apb_cast(const void* src, void* dst, long long n, int src_bf16, i
 namespace apb {
 
 constexpr int EMB_CHUNK = 32;
+constexpr int EMB_DIRECT = 32;  // most chunks of a row that emb_rows_kernel adds up
+constexpr int EMB_GROUP = 16;   // chunks of a longer one that are added up by one block
 constexpr int EMB_CTAS = 8, EMB_GROUP_THREADS = 1024;
 constexpr int EMB_ROWS = 8;  // most rows of one block of emb_rows_kernel
 
@@ -38,10 +40,10 @@ struct EmbWs {
   int* chunk0;   // [V] first chunk of the row (rows with more than EMB_CHUNK tokens)
   int* perm;     // [T] tokens grouped by row
   int* rank;     // [T] arrival number of the token inside its row
-  int2* desc;    // [max_chunks] {first entry in perm, tokens}
-  int* ctr;      // [3] entries, chunks and long rows handed out so far
+  int4* desc;    // [max_chunks] {first entry in perm, tokens, row, number of the chunk in the row}
+  int* ctr;      // [2] entries and chunks handed out so far
+  int* done;     // [2, max_chunks, column slices] finished chunks of the group that starts here, finished groups of the row
   float* part;   // [max_chunks, D]
-  int* longs;    // [max_longs] rows with more than EMB_CHUNK tokens
 };
 
 __host__ __device__ inline long long emb_max_longs(long long T) { return T / (EMB_CHUNK + 1); }
@@ -49,11 +51,12 @@ __host__ __device__ inline long long emb_max_chunks(long long T) { return T / EM
 static inline long long emb_round4(long long n) { return (n + 3) & ~3ll; }
 
 __global__ void __cluster_dims__(EMB_CTAS, 1, 1) __launch_bounds__(EMB_GROUP_THREADS)
-emb_group_kernel(const long long* __restrict__ ids, EmbWs ws, int T, long long V) {
+emb_group_kernel(const long long* __restrict__ ids, EmbWs ws, int T, long long V, long long ndone) {
   const int tid = blockIdx.x * EMB_GROUP_THREADS + threadIdx.x, lane = threadIdx.x & 31;
   constexpr int nt = EMB_CTAS * EMB_GROUP_THREADS;
   for (long long v = tid; v < V; v += nt) ws.count[v] = 0;
-  if (tid < 3) ws.ctr[tid] = 0;
+  for (long long i = tid; i < ndone; i += nt) ws.done[i] = 0;
+  if (tid < 2) ws.ctr[tid] = 0;
   auto sync = [] {  // every phase reads what other CTAs of the cluster wrote in the one before
     __threadfence();
     cluster_arrive();
@@ -98,16 +101,9 @@ emb_group_kernel(const long long* __restrict__ ids, EmbWs ws, int T, long long V
     }
     const int s = __shfl_sync(0xffffffffu, cb, 31) + cs - c, b = __shfl_sync(0xffffffffu, nb, 31) + ns - n;
     if (first) ws.start[v] = s;
-    const unsigned longs = __ballot_sync(0xffffffffu, n > 0);
-    if (longs) {
-      int lb = 0;
-      if (lane == 0) lb = atomicAdd(ws.ctr + 2, __popc(longs));
-      lb = __shfl_sync(0xffffffffu, lb, 0);
-      if (n > 0) ws.longs[lb + __popc(longs & ((1u << lane) - 1u))] = (int)v;
-    }
     if (n > 0) {
       ws.chunk0[v] = b;
-      for (int i = 0; i < n; ++i) ws.desc[b + i] = make_int2(s + i * EMB_CHUNK, min(EMB_CHUNK, c - i * EMB_CHUNK));
+      for (int i = 0; i < n; ++i) ws.desc[b + i] = make_int4(s + i * EMB_CHUNK, min(EMB_CHUNK, c - i * EMB_CHUNK), (int)v, i);
     }
   }
   sync();
@@ -172,61 +168,68 @@ __device__ __forceinline__ void emb_sum(const T* __restrict__ dy, const int* lis
   }
 }
 
-// W floats of a partial row
+// acc += n partial rows that lie ``stride`` floats apart, written by other blocks of this launch
 template <int W>
-__device__ __forceinline__ void emb_part_add(const float* p, float (&acc)[W]) {
-  if (W == 1) {
-    acc[0] += *p;
-  } else {
+__device__ __forceinline__ void emb_part_sum(const float* p, int n, long long stride, float (&acc)[W]) {
+#pragma unroll 8
+  for (int i = 0; i < n; ++i, p += stride) {
+    if constexpr (W == 1) {
+      acc[0] += __ldcg(p);
+    } else {
 #pragma unroll
-    for (int k = 0; k < W / 4; ++k) {
-      const float4 x = reinterpret_cast<const float4*>(p)[k];
-      acc[4 * k] += x.x; acc[4 * k + 1] += x.y; acc[4 * k + 2] += x.z; acc[4 * k + 3] += x.w;
+      for (int k = 0; k < W / 4; ++k) {
+        const float4 x = __ldcg(reinterpret_cast<const float4*>(p) + k);
+        acc[4 * k] += x.x; acc[4 * k + 1] += x.y; acc[4 * k + 2] += x.z; acc[4 * k + 3] += x.w;
+      }
     }
   }
 }
 
+// What the block has written is visible to the one that finds itself the last of ``n``; true there, in all threads.
+__device__ __forceinline__ bool emb_last(int* counter, int n) {
+  __shared__ int last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(counter, 1) == n - 1;
+  __syncthreads();
+  __threadfence();
+  return last != 0;
+}
+
+// A block takes a slice of the columns of one chunk.  In rows of many chunks the blocks that finish last add up, in the order of the
+// chunks and in two steps: one block of the kernel below that added all chunks of a row took 2.9 ms for 131072 tokens of one row,
+// D = 4096.  Rows of up to 32 chunks are left to that kernel, which adds them beside the stores of the table's other rows: 8192 tokens by
+// Zipf's law, 128256 x 4096, 222 us with the sums here, 228 with a launch of their own, 206 so.
 template <typename T, int W>
-__global__ void __launch_bounds__(128) emb_partial_kernel(const T* __restrict__ dy, EmbWs ws, int D) {
+__global__ void __launch_bounds__(128) emb_partial_kernel(const T* __restrict__ dy, EmbWs ws, T* __restrict__ out, long long max_chunks, int D) {
   __shared__ int list[EMB_CHUNK];
-  if ((int)blockIdx.x >= ws.ctr[1]) return;
-  const int2 d = ws.desc[blockIdx.x];
+  const int b = blockIdx.x, slices = gridDim.y, step = slices * 128 * W, col0 = (blockIdx.y * 128 + threadIdx.x) * W;
+  if (b >= ws.ctr[1]) return;
+  const int4 d = ws.desc[b];
+  const int n = (ws.count[d.z] + EMB_CHUNK - 1) / EMB_CHUNK;  // chunks of the row
   if ((int)threadIdx.x < d.y) list[threadIdx.x] = ws.perm[d.x + threadIdx.x];
   __syncthreads();
-  for (int col = (blockIdx.y * 128 + threadIdx.x) * W; col < D; col += gridDim.y * 128 * W) {
+  for (int col = col0; col < D; col += step) {
     float acc[W] = {};
     emb_sum<T, W>(dy, list, d.y, D, col, acc);
 #pragma unroll
-    for (int k = 0; k < W; ++k) ws.part[(long long)blockIdx.x * D + col + k] = acc[k];
+    for (int k = 0; k < W; ++k) ws.part[(long long)b * D + col + k] = acc[k];
   }
-}
-
-// A block takes 32 W columns of a long row, each warp an eighth of its chunks.  (A block of the kernel below that summed all chunks and
-// all columns took 2.9 ms for 131072 tokens of one row, D = 4096; inside that kernel this code costs its other blocks registers.)
-template <typename T, int W>
-__global__ void __launch_bounds__(256) emb_long_kernel(EmbWs ws, T* __restrict__ out, int D) {
-  __shared__ float sum[8][32 * W];
-  const int slices = (D + 32 * W - 1) / (32 * W), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int items = ws.ctr[2] * slices;  // (at most T / 33 * D / 32)
-  for (int it = blockIdx.x; it < items; it += gridDim.x) {
-    const long long v = ws.longs[it / slices];
-    const int col = (it % slices * 32 + lane) * W, n = (ws.count[v] + EMB_CHUNK - 1) / EMB_CHUNK;
-    const float* p = ws.part + (long long)ws.chunk0[v] * D + col;
+  if (n <= EMB_DIRECT) return;
+  const int g = d.w / EMB_GROUP, row0 = b - d.w, first = row0 + g * EMB_GROUP, members = min(EMB_GROUP, n - g * EMB_GROUP);
+  if (!emb_last(ws.done + (long long)first * slices + blockIdx.y, members)) return;
+  for (int col = col0; col < D; col += step) {
     float acc[W] = {};
-    if (col < D) {
-#pragma unroll 8
-      for (int i = warp; i < n; i += 8) emb_part_add<W>(p + (long long)i * D, acc);
-    }
-#pragma unroll
-    for (int k = 0; k < W; ++k) sum[warp][k * 32 + lane] = acc[k];
-    __syncthreads();
-    if (warp == 0 && col < D) {
-      for (int g = 1; g < 8; ++g)
-#pragma unroll
-        for (int k = 0; k < W; ++k) acc[k] += sum[g][k * 32 + lane];
-      EmbVec<T, W>::store(out + v * D + col, acc);
-    }
-    __syncthreads();
+    emb_part_sum<W>(ws.part + (long long)first * D + col, members, D, acc);
+#pragma unroll  // (the group's first row takes the sum: nobody else reads these columns of it any more)
+    for (int k = 0; k < W; ++k) ws.part[(long long)first * D + col + k] = acc[k];
+  }
+  const int groups = (n + EMB_GROUP - 1) / EMB_GROUP;
+  if (!emb_last(ws.done + (max_chunks + row0) * slices + blockIdx.y, groups)) return;
+  for (int col = col0; col < D; col += step) {
+    float acc[W] = {};
+    emb_part_sum<W>(ws.part + (long long)row0 * D + col, groups, (long long)EMB_GROUP * D, acc);
+    EmbVec<T, W>::store(out + (long long)d.z * D + col, acc);
   }
 }
 
@@ -240,16 +243,25 @@ __global__ void __launch_bounds__(256) emb_rows_kernel(const T* __restrict__ dy,
   if ((int)threadIdx.x < nrows) {
     const int c = ws.count[row0 + threadIdx.x];
     cnt[threadIdx.x] = c;
-    from[threadIdx.x] = c == 0 ? 0 : ws.start[row0 + threadIdx.x];
+    from[threadIdx.x] = c == 0 ? 0 : (c > EMB_CHUNK ? ws.chunk0 : ws.start)[row0 + threadIdx.x];
   }
   __syncthreads();
   for (int r = threadIdx.x / tx; r < nrows; r += 256 / tx) {
     T* dst = out + (row0 + r) * D;
     const int c = cnt[r];
-    if (c > EMB_CHUNK) continue;
+    if (c > EMB_CHUNK * EMB_DIRECT) continue;
     for (int col = (threadIdx.x & (tx - 1)) * W; col < D; col += tx * W) {
       float acc[W] = {};
-      if (c > 0) emb_sum<T, W>(dy, ws.perm + from[r], c, D, col, acc);
+      if (c > EMB_CHUNK) {
+        const float* p = ws.part + (long long)from[r] * D + col;
+        const int n = (c + EMB_CHUNK - 1) / EMB_CHUNK;
+#pragma unroll 4
+        for (int i = 0; i < n; ++i)
+#pragma unroll
+          for (int k = 0; k < W; ++k) acc[k] += p[(long long)i * D + k];
+      } else if (c > 0) {
+        emb_sum<T, W>(dy, ws.perm + from[r], c, D, col, acc);
+      }
       EmbVec<T, W>::store(dst + col, acc);
     }
   }
@@ -298,15 +310,20 @@ __global__ void __launch_bounds__(256) emb_zero_kernel(float4* p, long long n) {
     if (i + k * 256 < n) p[i + k * 256] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
+// column slices of emb_partial_kernel, ``w`` elements per thread
+static int emb_slices(int D, int w) {
+  const int n = (D / w + 127) / 128;
+  return n < 16 ? n : 16;
+}
+
 template <typename T, int W>
-static void emb_launch(const void* dy, const EmbWs& ws, void* out, long long T_, long long V, int D, int num_sms, cudaStream_t st) {
-  const int nvec = D / W;
-  if (emb_max_longs(T_) > 0) {
-    const int split = (nvec + 127) / 128;
-    emb_partial_kernel<T, W><<<dim3((unsigned)emb_max_chunks(T_), (unsigned)(split < 16 ? split : 16)), 128, 0, st>>>((const T*)dy, ws, D);
-    const long long items = emb_max_longs(T_) * ((D + 32 * W - 1) / (32 * W));
-    emb_long_kernel<T, W><<<(unsigned)(items < 2 * num_sms ? items : 2 * num_sms), 256, 0, st>>>(ws, (T*)out, D);
-  }
+static void emb_launch(const void* dy, const long long* ids, const EmbWs& ws, void* out, long long T_, long long V, int D, int num_sms,
+                       cudaStream_t st) {
+  const int nvec = D / W, slices = emb_slices(D, W);
+  const long long chunks = emb_max_chunks(T_);
+  emb_group_kernel<<<EMB_CTAS, EMB_GROUP_THREADS, 0, st>>>(ids, ws, (int)T_, V, 2 * chunks * slices);
+  if (emb_max_longs(T_) > 0)
+    emb_partial_kernel<T, W><<<dim3((unsigned)chunks, (unsigned)slices), 128, 0, st>>>((const T*)dy, ws, (T*)out, chunks, D);
   int tx = 32;
   while (tx < nvec && tx < 256) tx *= 2;
   // rows per block: eight where the table is long (one 64-KB store stream per block), fewer where it would leave SMs idle,
@@ -327,9 +344,9 @@ static long long emb_carve(EmbWs* ws, void* base, long long T, long long V, int 
   };
   const long long chunks = emb_max_chunks(T);
   ws->part = reinterpret_cast<float*>(take(chunks * D));
-  ws->desc = reinterpret_cast<int2*>(take(2 * chunks));
-  ws->longs = take(emb_max_longs(T));
-  ws->ctr = take(3);
+  ws->desc = reinterpret_cast<int4*>(take(4 * chunks));
+  ws->done = take(2 * chunks * emb_slices(D, 1));  // (the most of all forms)
+  ws->ctr = take(2);
   ws->count = take(V);
   ws->start = take(V);
   ws->chunk0 = take(V);
@@ -366,7 +383,7 @@ extern "C" int apb_embedding_bwd_sorts(long long tokens, long long num_rows, int
 // kernels that a call launches
 extern "C" int apb_embedding_bwd_launches(long long tokens, long long num_rows, int D, int is_bf16) {
   if (num_rows <= 0 || D <= 0) return 0;
-  if (apb_embedding_bwd_sorts(tokens, num_rows, D, is_bf16)) return emb_max_longs(tokens) > 0 ? 4 : 2;
+  if (apb_embedding_bwd_sorts(tokens, num_rows, D, is_bf16)) return emb_max_longs(tokens) > 0 ? 3 : 2;
   return (num_rows * D % 4 == 0) + (tokens > 0) + (is_bf16 != 0);
 }
 
@@ -397,15 +414,14 @@ extern "C" int apb_embedding_bwd(const void* dy, const long long* ids, void* out
   if (tokens >= (1ll << 30) || num_rows >= (1ll << 31)) return 3;
   EmbWs ws;
   emb_carve(&ws, workspace, tokens, num_rows, D);
-  emb_group_kernel<<<EMB_CTAS, EMB_GROUP_THREADS, 0, st>>>(ids, ws, (int)tokens, num_rows);
   const int w = is_bf16 ? 8 : 4;
   const bool vec = D % w == 0 && ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
   if (is_bf16) {
-    if (vec) emb_launch<__nv_bfloat16, 8>(dy, ws, out, tokens, num_rows, D, num_sms, st);
-    else emb_launch<__nv_bfloat16, 1>(dy, ws, out, tokens, num_rows, D, num_sms, st);
+    if (vec) emb_launch<__nv_bfloat16, 8>(dy, ids, ws, out, tokens, num_rows, D, num_sms, st);
+    else emb_launch<__nv_bfloat16, 1>(dy, ids, ws, out, tokens, num_rows, D, num_sms, st);
   } else {
-    if (vec) emb_launch<float, 4>(dy, ws, out, tokens, num_rows, D, num_sms, st);
-    else emb_launch<float, 1>(dy, ws, out, tokens, num_rows, D, num_sms, st);
+    if (vec) emb_launch<float, 4>(dy, ids, ws, out, tokens, num_rows, D, num_sms, st);
+    else emb_launch<float, 1>(dy, ids, ws, out, tokens, num_rows, D, num_sms, st);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }

@@ -55,6 +55,9 @@ def test_embedding_gradient_over_list_lengths(K, dtype, V, D, T, ids):
     (torch.bfloat16, 50257, 1000, 9000, "skewed", True),  # long and short lists, a last slice that is not full
     (torch.bfloat16, 20000, 4096, 5000, "same", True),   # many chunks, several slices of the columns
     (torch.bfloat16, 40000, 1025, 300, "random", True),  # rows that are no whole vectors
+    (torch.bfloat16, 40000, 1024, 1024, "same", True),   # the longest row of the rows kernel
+    (torch.bfloat16, 40000, 1024, 1025, "same", True),   # one chunk more: three groups of blocks
+    (torch.bfloat16, 40000, 1025, 1600, "same", True),   # the same in rows that are no whole vectors
     (torch.bfloat16, 100, 1024, 80000, "skewed", True),  # every row long
     (torch.float32, 100, 1024, 80000, "skewed", True),
     (torch.float32, 300, 1000, 60000, "same", True),
