@@ -501,7 +501,8 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
+      const uint32_t full_pair = PAIR ? map_to_cta(full, 0) : 0u;  // the even CTA's barriers
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -552,7 +553,7 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
           uint8_t* a_dst = sA + stage * A_BYTES;
           uint8_t* b_dst = sB + stage * B_BYTES;
           // one load helper for the four cases (pair or not, 2-D or grouped 3-D)
-          const uint32_t full_addr = PAIR ? map_to_cta(&full[stage], 0) : 0u;
+          const uint32_t full_addr = full_pair + stage * 8;
           auto load = [&](uint8_t* dst, const CUtensorMap* tm_, int x, int y) {
             if (PAIR) {
               if (GROUPED) tma_load_3d_pair(dst, tm_, full_addr, x, y, grp);
@@ -588,8 +589,13 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && half == 0) {
+    // One elected thread, descriptors as offsets from one base: the issue of a k-block cost about 300 ns before, more than its MMAs take.
+    // 64 x 1280 x 2048 x 1408 387 -> 343 us, 8192 x 4096 x 4096 NN 194 -> 173, 2048 x 4096 x 4096 NN 59 -> 51.
+    if (half == 0 && elect_one()) {
       constexpr uint32_t idesc = make_idesc_bf16(TM, BN, A_MN ? 1u : 0u, B_MN ? 1u : 0u);
+      const uint64_t a_desc = make_smem_desc(smem_u32(sA), A_MN ? CHUNK_BYTES : 16, 1024);
+      const uint64_t b_desc = make_smem_desc(smem_u32(sB), B_MN ? CHUNK_BYTES : 16, 1024);
+      const uint32_t empty_even = PAIR ? map_to_cta(empty, 0) : 0u, empty_odd = PAIR ? map_to_cta(empty, 1) : 0u;
       int stage = 0;
       uint32_t phase = 0;
       int buf = 0;
@@ -612,21 +618,18 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
             break;
           }
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(sA + stage * A_BYTES);
-          const uint32_t b_addr = smem_u32(sB + stage * B_BYTES);
+          const uint64_t a_stage = a_desc + desc_offset(stage * A_BYTES), b_stage = b_desc + desc_offset(stage * B_BYTES);
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k) {
-            const uint64_t a_desc = A_MN ? make_smem_desc(a_addr + k * (UMMA_K * 128), CHUNK_BYTES, 1024)
-                                         : make_smem_desc(a_addr + k * (UMMA_K * 2), 16, 1024);
-            const uint64_t b_desc = B_MN ? make_smem_desc(b_addr + k * (UMMA_K * 128), CHUNK_BYTES, 1024)
-                                         : make_smem_desc(b_addr + k * (UMMA_K * 2), 16, 1024);
-            if (PAIR) umma_f16_pair(d_tmem, a_desc, b_desc, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-            else umma_f16(d_tmem, a_desc, b_desc, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            const uint64_t ad = a_stage + desc_offset(k * (A_MN ? UMMA_K * 128 : UMMA_K * 2));
+            const uint64_t bd = b_stage + desc_offset(k * (B_MN ? UMMA_K * 128 : UMMA_K * 2));
+            if (PAIR) umma_f16_pair(d_tmem, ad, bd, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            else umma_f16(d_tmem, ad, bd, idesc, (kb > 0 || k > 0) ? 1u : 0u);
           }
           // stage reusable once these MMAs have read it (PAIR: in both CTAs)
           if (PAIR) {
-            umma_commit_pair(map_to_cta(&empty[stage], 0));
-            umma_commit_pair(map_to_cta(&empty[stage], 1));
+            umma_commit_pair(empty_even + stage * 8);
+            umma_commit_pair(empty_odd + stage * 8);
           } else {
             umma_commit(&empty[stage]);
           }

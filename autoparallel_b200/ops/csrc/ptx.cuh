@@ -34,6 +34,8 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// One thread of a converged warp, the same one at every call.  Producer and MMA roles are taken with it: TMA and tcgen05 instructions want
+// uniform operands, and a branch on a lane number (which could hold several threads) makes each of them several times as slow to issue.
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
   asm volatile(
@@ -71,7 +73,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 }
 // Bounded wait.  Returns false after kWaitLimitNs or once *abort_flag is set by another role.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag) {
-  if (mbar_try_wait(bar, parity)) return true;
+  if (__builtin_expect(mbar_try_wait(bar, parity), 1)) return true;
   const unsigned long long t0 = globaltimer_ns();
   for (uint32_t i = 1;; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
@@ -267,6 +269,9 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr, uint32_t 
   d |= static_cast<uint64_t>(2) << 61;  // SWIZZLE_128B
   return d;
 }
+
+// Added to a descriptor, moves its start by ``bytes`` (a multiple of 16; the address stays below 256 KB, so nothing carries out of its field).
+__device__ __forceinline__ constexpr uint64_t desc_offset(uint32_t bytes) { return bytes >> 4; }
 
 // Instruction descriptor for kind::f16 with bf16 A/B, fp32 D.
 __host__ __device__ constexpr uint32_t make_idesc_bf16(uint32_t m, uint32_t n, uint32_t a_mn_major, uint32_t b_mn_major) {
