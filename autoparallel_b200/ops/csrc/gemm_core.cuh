@@ -9,7 +9,7 @@
 //                 the epilogues' "accumulator free" arrivals go to the even CTA's barriers; "stage
 //                 free" and "accumulator full" are committed by the MMA thread to each CTA's barrier
 //                 separately (two plain commits; no multicast anywhere).
-//   warp 0: TMA producer | warp 1: TMEM owner + MMA issuer | warps 2..5: epilogue
+//   warp 0: TMA producer | warp 1: TMEM owner + MMA issuer | warps 2..9 (2..5 in the fused kernels and with fewer stages): epilogue
 //   warp 6 (gather-fused kernels only): copy engine driver, see gather_comm_warp
 //
 // FUSE selects what the CTA does beyond a plain GEMM:
@@ -35,8 +35,10 @@ constexpr int B_STAGE_BYTES = BN * BK * 2;
 constexpr int CHUNK_BYTES = BK * 128;  // one [BK x 64-element] MN-major box
 constexpr int GEMM_THREADS = 192;
 constexpr int GEMM_SMEM_BYTES = STAGES * (A_STAGE_BYTES + B_STAGE_BYTES) + 1024 /*align*/ + 256 /*barriers*/;
-constexpr int STORE_BYTES = 4096;  // per epilogue warp: 32 rows x 128 bytes of C, the box of one TMA store (plain GEMM)
-constexpr int STAGING_BYTES = 4 * STORE_BYTES;
+constexpr int STORE_BYTES = 4096;  // per epilogue warp: 32 rows x 128 bytes of C (plain GEMM)
+constexpr int EPI_WARPS = 8;       // plain GEMM: two warps per TMEM lane quarter, each half of the tile's columns
+constexpr int GEMM_PLAIN_THREADS = 64 + 32 * EPI_WARPS;
+constexpr int STAGING_BYTES = EPI_WARPS * STORE_BYTES;
 constexpr int GEMM_PLAIN_SMEM_BYTES = GEMM_SMEM_BYTES + STAGING_BYTES;
 static_assert(GEMM_PLAIN_SMEM_BYTES + 1024 + 512 <= 233472, "a communication kernel's CTA (no shared memory to speak of) still fits beside a GEMM CTA");
 constexpr int PAIR_STAGES = 6;  // 6 x (16 KB of A + 16 KB of B) = the same 192 KB as 4 x 48 KB
@@ -55,6 +57,18 @@ inline bool pair_shape(int M, int N, int K) { return M >= 2 * BM ? N >= BN : M >
 
 enum : int { FUSE_NONE = 0, FUSE_GATHER_A = 1, FUSE_GATHER_B = 2, FUSE_REDUCE_SCATTER = 3 };
 
+// Division of 0 <= n < 2^31 by a number that the host knows, as a multiplication and a shift (Granlund and Montgomery, "Division by invariant
+// integers using multiplication", 1994).
+struct FastDiv {
+  uint32_t d = 1, mul = 1, shift = 0;
+  FastDiv() = default;
+  __host__ explicit FastDiv(uint32_t div) : d(div) {
+    while ((1ull << shift) < d) ++shift;
+    mul = (uint32_t)((((1ull << shift) - d) << 32) / d + 1);
+  }
+  __device__ __forceinline__ int div(int n) const { return (int)((__umulhi(mul, (uint32_t)n) + (uint32_t)n) >> shift); }
+};
+
 struct GemmParams {
   int M, N, K;
   void* C;
@@ -66,7 +80,9 @@ struct GemmParams {
   // dynamic tile scheduling (DYN): {next tile, pairs that have left, SM-pair requests, pairs that gave up their SMs};
   // all but the requests are zero between launches
   int* tile_counter = nullptr;
-  int tma_store = 0;  // C leaves through shared memory and TMA stores (plain GEMM; needs 16-byte rows)
+  // plain GEMM: divisors of the tile order, see plain_tile
+  FastDiv div_group, div_tiles, div_tail;
+  int vec_store = 0;  // C leaves through shared memory in whole 128-byte lines (plain GEMM; needs 16-byte rows)
 };
 
 struct FuseParams {
@@ -94,6 +110,22 @@ __device__ __forceinline__ void tile_coords(int t, int num_m, int num_n, int& tm
   const int r = t % per_group;
   tm = first_m + r % gsz;
   tn = r / gsz;
+}
+
+// The same order for the plain GEMM, tile ``t`` of all groups: every warp of the epilogue walks it, and three integer divisions with their
+// remainders are several hundred cycles of a tile.
+inline void set_tile_order(GemmParams& p, int num_m) {
+  p.div_group = FastDiv((uint32_t)GROUP_M * p.num_n_tiles);
+  p.div_tiles = FastDiv((uint32_t)num_m * p.num_n_tiles);
+  p.div_tail = FastDiv(num_m % GROUP_M ? num_m % GROUP_M : GROUP_M);
+}
+__device__ __forceinline__ void plain_tile(const GemmParams& p, int num_m, bool grouped, int t, int& grp, int& tm, int& tn) {
+  grp = grouped ? p.div_tiles.div(t) : 0;
+  if (grouped) t -= grp * (int)p.div_tiles.d;
+  const int g = p.div_group.div(t), first_m = g * GROUP_M, r = t - g * (int)p.div_group.d;
+  const bool tail = num_m - first_m < GROUP_M;
+  tn = tail ? p.div_tail.div(r) : r / GROUP_M;
+  tm = first_m + r - tn * (tail ? (int)p.div_tail.d : GROUP_M);
 }
 
 __device__ __forceinline__ void red_add_v4_sys(float* addr, float a, float b, float c, float d) {
@@ -137,50 +169,63 @@ __device__ __forceinline__ void store_row_chunk(const GemmParams& p, long long r
   }
 }
 
-// Epilogue of the plain GEMM for one warp's 32 rows and NCOL / 32 accumulator chunks: 128 bytes of every row at a time go
-// to the warp's staging block (128-byte swizzle, conflict free) and from there to C as one TMA store.  A thread owns a
-// row, so storing straight from registers puts 16-byte pieces of 32 different lines into every instruction, half a sector
-// each; a product with a short contraction was bound by that (weight gradients of 64 experts, 2048 x 1408 over 160 rows:
-// 217 us before, 137 us now).  The store of a block overlaps the TMEM loads of the next (a second block per warp measured no
-// better); out-of-range rows and columns are clipped by the tensor map.
-template <bool OUT_FP32, bool GROUPED>
-__device__ __forceinline__ void store_tile_tma(const CUtensorMap* tmC, uint8_t* stg, uint32_t taddr, int row0, int n0, int ncols, int M, int N,
-                                               int grp, int lane) {
-  constexpr int CC = OUT_FP32 ? 32 : 64;  // columns of 128 bytes
+// Epilogue of the plain GEMM for one warp's 32 rows and ``ncols`` columns: 128 bytes of every row at a time go to the warp's staging block
+// (128-byte swizzle, conflict free) and from there to C with eight lanes to a row, so that every store instruction writes whole lines; a
+// thread owns a row in TMEM, and storing straight from registers puts 16-byte pieces of 32 lines into every instruction.  ``release`` is
+// called as soon as the last block is in registers.
+// A product with a short contraction is bound by this chain.  TMA stores from the staging block (the form before) wait in the queue of
+// the tile's loads, 1500 to 2000 cycles for each block before it can be written again.  Two warps per lane quarter, because one warp's
+// chain of dependent instructions (900 cycles a block) fills neither the load-store unit nor the memory.  Weight gradients of 64 experts,
+// 2048 x 1408 over 160 rows: 162 us with TMA stores, 130 with four warps and these stores, 93 with eight (the result alone takes 64).
+template <bool OUT_FP32, typename Release>
+__device__ __forceinline__ void store_tile(void* C, long long ldc, uint8_t* stg, uint32_t taddr, int row0, int n0, int ncols, int M, int N, int lane,
+                                           Release release) {
+  constexpr int CC = OUT_FP32 ? 32 : 64, PER = OUT_FP32 ? 4 : 8;  // columns of 128 and of 16 bytes
+  const int used = row0 < M ? min(ncols, N - n0) : 0;             // (rows and columns past the matrix are not read)
+  if (used <= 0) {
+    release();
+    return;
+  }
+  const int unit = lane & 7, sub = lane >> 3;
+  const long long row_bytes = ldc * (OUT_FP32 ? 4 : 2);
+  uint8_t* dst0 = reinterpret_cast<uint8_t*>(C) + (row0 + sub) * row_bytes + (long long)(n0 + unit * PER) * (OUT_FP32 ? 4 : 2);
 #pragma unroll 1
-  for (int c = 0; c < ncols; c += CC) {
+  for (int c = 0; c < used; c += CC) {
     uint4 v[8];
     uint32_t r[32];
     tmem_ld_32x32(taddr + c, r);
-    tmem_ld_wait();
     if (OUT_FP32) {
+      tmem_ld_wait_for(r);
 #pragma unroll
       for (int i = 0; i < 8; ++i) v[i] = make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
     } else {
-      auto pack8 = [&](int i) {
-        return make_uint4(pack_bf16(__uint_as_float(r[8 * i + 0]), __uint_as_float(r[8 * i + 1])),
-                          pack_bf16(__uint_as_float(r[8 * i + 2]), __uint_as_float(r[8 * i + 3])),
-                          pack_bf16(__uint_as_float(r[8 * i + 4]), __uint_as_float(r[8 * i + 5])),
-                          pack_bf16(__uint_as_float(r[8 * i + 6]), __uint_as_float(r[8 * i + 7])));
+      uint32_t r2[32];
+      tmem_ld_32x32(taddr + c + 32, r2);
+      tmem_ld_wait_for(r);
+      tmem_ld_wait_for(r2);
+      auto pack8 = [](const uint32_t* x) {
+        return make_uint4(pack_bf16(__uint_as_float(x[0]), __uint_as_float(x[1])), pack_bf16(__uint_as_float(x[2]), __uint_as_float(x[3])),
+                          pack_bf16(__uint_as_float(x[4]), __uint_as_float(x[5])), pack_bf16(__uint_as_float(x[6]), __uint_as_float(x[7])));
       };
 #pragma unroll
-      for (int i = 0; i < 4; ++i) v[i] = pack8(i);
-      tmem_ld_32x32(taddr + c + 32, r);
-      tmem_ld_wait();
-#pragma unroll
-      for (int i = 0; i < 4; ++i) v[4 + i] = pack8(i);
+      for (int i = 0; i < 4; ++i) {
+        v[i] = pack8(r + 8 * i);
+        v[4 + i] = pack8(r2 + 8 * i);
+      }
     }
-    if (lane == 0) tma_store_wait_read();  // the block's previous store has been read out
-    __syncwarp();
+    if (c + CC >= used) release();
+    __syncwarp();  // the block before has been read out
 #pragma unroll
     for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(stg + lane * 128 + ((i ^ (lane & 7)) << 4)) = v[i];
-    fence_proxy_async_smem();
     __syncwarp();
-    if (lane == 0 && row0 < M && n0 + c < N) {
-      if (GROUPED) tma_store_3d(tmC, stg, n0 + c, row0, grp);
-      else tma_store_2d(tmC, stg, n0 + c, row0);
-      tma_store_commit();
+    const bool in_cols = n0 + c + unit * PER < N;  // (N is a number of whole vectors: rows are)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int row = i * 4 + sub;
+      const uint4 x = *reinterpret_cast<const uint4*>(stg + row * 128 + ((unit ^ (row & 7)) << 4));
+      if (in_cols && row0 + row < M) *reinterpret_cast<uint4*>(dst0 + i * 4 * row_bytes) = x;
     }
+    dst0 += 128;
   }
 }
 
@@ -336,9 +381,10 @@ __device__ __forceinline__ void gather_comm_warp(const GemmParams& p, const Fuse
 constexpr int TILE_RING = 4;
 template <bool A_MN, bool B_MN, int FUSE, bool PAIR = false, bool GROUPED = false, int ST_ARG = 0, bool DYN = false>
 __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p,
-                                         const FuseParams& f, int cta, int num_ctas, uint8_t* smem_raw,
-                                         const CUtensorMap* tmC = nullptr) {
+                                         const FuseParams& f, int cta, int num_ctas, uint8_t* smem_raw) {
   constexpr int STAGING = FUSE == FUSE_NONE && ST_ARG == 0 ? STAGING_BYTES : 0;  // (fewer stages: to leave shared memory free)
+  constexpr int EPI = STAGING > 0 ? EPI_WARPS : 4;
+  constexpr int EPI_COLS = BN * 4 / EPI;  // columns of the tile per epilogue warp
   constexpr int ST = ST_ARG > 0 ? ST_ARG : (PAIR ? PAIR_STAGES : STAGES);
   constexpr int A_BYTES = A_STAGE_BYTES;                          // 128 rows of A per CTA
   constexpr int B_BYTES = PAIR ? B_STAGE_BYTES / 2 : B_STAGE_BYTES;  // PAIR: this CTA's 128 of the 256 B rows
@@ -352,13 +398,13 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
   uint64_t* full = bars;                     // [ST]  PAIR: the even CTA's are used
   uint64_t* empty = bars + ST;               // [ST]
   uint64_t* tmem_full = bars + 2 * ST;       // [2]
-  uint64_t* tmem_empty = bars + 2 * ST + 2;  // [2]   PAIR: the even CTA's are used (256 arrivals)
+  uint64_t* tmem_empty = bars + 2 * ST + 2;  // [2]   one arrival per epilogue warp; PAIR: of both CTAs, on the even CTA's
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * ST + 4);
   volatile uint32_t* abort_flag = tmem_slot + 1;
   uint64_t* ring_bars = bars + 2 * ST + 6;   // [AG_NBUF], gather-fused kernels only
   static_assert(!DYN || (PAIR && FUSE == FUSE_NONE), "dynamic tiles: CTA pairs, plain GEMM");
   uint64_t* tile_ready = bars + 2 * ST + 10;  // [TILE_RING] DYN: entry published (1 arrival, in each CTA)
-  uint64_t* tile_free = tile_ready + TILE_RING;  // [TILE_RING] DYN: entry read by all 10 readers of the pair (even CTA's)
+  uint64_t* tile_free = tile_ready + TILE_RING;  // [TILE_RING] DYN: entry read by all readers of the pair (even CTA's)
   volatile int* tile_ring = reinterpret_cast<volatile int*>(tile_free + TILE_RING);  // [TILE_RING]
   static_assert((2 * PAIR_STAGES + 10 + 2 * TILE_RING) * 8 + TILE_RING * 4 <= 256, "barrier block");
   constexpr bool GATHER = FUSE == FUSE_GATHER_A || FUSE == FUSE_GATHER_B;
@@ -383,8 +429,12 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
     if (f.rows_per_shard % BN == 0 && p.num_n_tiles == (f.rows_per_shard / BN) * f.n) shard_n_tiles = f.rows_per_shard / BN;
     else n_rot = (f.rank * f.rows_per_shard) / BN;
   }
-  auto map_tile = [&](int t, int& tm, int& tn) {
-    if (GROUPED) t %= tiles_per_group;
+  auto map_tile = [&](int t, int& grp, int& tm, int& tn) {
+    if (FUSE == FUSE_NONE) {
+      plain_tile(p, num_m_units, GROUPED, t, grp, tm, tn);
+      return;
+    }
+    grp = 0;
     if (shard_n_tiles > 0) {
       const int per_shard = num_m_units * shard_n_tiles;
       const int s = t / per_shard;
@@ -467,12 +517,12 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tmem_full[b], 1);
-      mbar_init(&tmem_empty[b], PAIR ? 256 : 128);
+      mbar_init(&tmem_empty[b], PAIR ? 2 * EPI : EPI);
     }
     if (DYN)
       for (int b = 0; b < TILE_RING; ++b) {
         mbar_init(&tile_ready[b], 1);
-        mbar_init(&tile_free[b], 10);  // odd CTA: producer + 4 epilogue warps; even CTA: MMA thread + 4 epilogue warps
+        mbar_init(&tile_free[b], 2 * (EPI + 1));  // odd CTA: producer + epilogue warps; even CTA: MMA thread + epilogue warps
       }
     if (GATHER)
       for (int b = 0; b < AG_NBUF; ++b) mbar_init(&ring_bars[b], 1);
@@ -517,11 +567,10 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
       int tile_it = 0;
       for (int t = (DYN && half == 0) ? fetch_tile(tile_it) : read_tile(tile_it); t >= 0 && ok;
            t = (DYN && half == 0) ? fetch_tile(tile_it) : read_tile(tile_it)) {
-        int tm, tn;
-        map_tile(t, tm, tn);
+        int grp, tm, tn;
+        map_tile(t, grp, tm, tn);
         // rows of A and of B that THIS CTA stages
         const int m0 = tm * TM + (int)half * BM, n0 = tn * BN + (int)half * B_ROWS;
-        const int grp = GROUPED ? t / tiles_per_group : 0;
         if ((FUSE == FUSE_GATHER_A && !A_MN) || (FUSE == FUSE_GATHER_B && !B_MN)) {
           // the tile's rows of the gathered operand must have landed
           const int r0 = (FUSE == FUSE_GATHER_A) ? m0 : n0;
@@ -658,8 +707,10 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
       gather_comm_warp(p, f, cta, num_ctas, ring, abort_flag);
     }
   } else {
-    // ------------------------------------------------------------------ epilogue (warps 2..5)
+    // ------------------------------------------------------------------ epilogue (warps 2..)
     const int q = warp & 3;  // TMEM lane quarter this warp may read
+    const int col0 = ((warp - 2) >> 2) * EPI_COLS;  // first of its columns
+    const uint32_t tmem_empty_even = PAIR ? map_to_cta(tmem_empty, 0) : 0u;
     int buf = 0;
     uint32_t buf_phase = 0;
     int tile_it = 0;
@@ -669,18 +720,19 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
       return __shfl_sync(0xffffffffu, t, 0);
     };
     for (int t = next_epi_tile(); t >= 0; t = next_epi_tile()) {
-      int tm, tn;
-      map_tile(t, tm, tn);
+      int grp, tm, tn;
+      map_tile(t, grp, tm, tn);
       const long long cta_row0 = (long long)tm * TM + (long long)half * BM;  // first of this CTA's 128 rows
-      if (!mbar_wait(&tmem_full[buf], buf_phase, abort_flag)) {
+      // (the TMEM loads are warp-wide: the warp goes on together or not at all)
+      if (!__all_sync(0xffffffffu, mbar_wait(&tmem_full[buf], buf_phase, abort_flag))) {
         atomicCAS(p.status, 0u, (uint32_t)ST_TIMEOUT_TMEM_FULL);
         *abort_flag = 1;
         break;
       }
       tc_fence_after();
       const long long row = cta_row0 + q * 32 + lane;
-      const int n0 = tn * BN;
-      const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + buf * BN;
+      const int n0 = tn * BN + col0;
+      const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + buf * BN + col0;
       float* rs_base = nullptr;
       if (FUSE == FUSE_REDUCE_SCATTER) {
         const int owner = (int)(cta_row0 / f.rows_per_rank);
@@ -701,15 +753,24 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
         rs_base = reinterpret_cast<float*>(f.peers.base[owner] + apbs::HEADER_BYTES) +
                   ((long long)f.rank * f.rows_per_rank + (row - (long long)owner * f.rows_per_rank)) * p.N;
       }
-      const bool via_tma = STAGING > 0 && p.tma_store;
-      if (via_tma) {
+      auto release = [&]() {  // this warp has read its rows of the accumulator
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          if (PAIR) mbar_arrive_cluster_plain(tmem_empty_even + buf * 8);
+          else mbar_arrive(&tmem_empty[buf]);
+        }
+      };
+      const bool staged = STAGING > 0 && p.vec_store;
+      if (staged) {
         uint8_t* stg = smem + ST * (A_BYTES + B_BYTES) + (warp - 2) * STORE_BYTES;
-        const int grp = GROUPED ? t / tiles_per_group : 0;
-        if (p.out_fp32) store_tile_tma<true, GROUPED>(tmC, stg, taddr, (int)cta_row0 + q * 32, n0, BN, p.M, p.N, grp, lane);
-        else store_tile_tma<false, GROUPED>(tmC, stg, taddr, (int)cta_row0 + q * 32, n0, BN, p.M, p.N, grp, lane);
+        const long long c_off = GROUPED ? (long long)grp * p.M * p.ldc : 0;
+        const int r0 = (int)cta_row0 + q * 32;
+        if (p.out_fp32) store_tile<true>(reinterpret_cast<float*>(p.C) + c_off, p.ldc, stg, taddr, r0, n0, EPI_COLS, p.M, p.N, lane, release);
+        else store_tile<false>(reinterpret_cast<__nv_bfloat16*>(p.C) + c_off, p.ldc, stg, taddr, r0, n0, EPI_COLS, p.M, p.N, lane, release);
       }
 #pragma unroll 1
-      for (int c = 0; c < BN / 32 && !via_tma; ++c) {
+      for (int c = 0; c < EPI_COLS / 32 && !staged; ++c) {
         uint32_t r[32];
         tmem_ld_32x32(taddr + c * 32, r);
         tmem_ld_wait();
@@ -768,17 +829,14 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
           __syncwarp();
           continue;
         }
-        store_row_chunk(p, row, col, r, GROUPED ? (long long)(t / tiles_per_group) * p.M * p.ldc : 0);
+        store_row_chunk(p, row, col, r, GROUPED ? (long long)grp * p.M * p.ldc : 0);
       }
-      tc_fence_before();
-      if (PAIR) mbar_arrive_cluster(map_to_cta(&tmem_empty[buf], 0));
-      else mbar_arrive(&tmem_empty[buf]);
+      if (!staged) release();
       if (++buf == 2) {
         buf = 0;
         buf_phase ^= 1;
       }
     }
-    if (STAGING > 0 && lane == 0) tma_store_wait_all();
   }
 
   tc_fence_before();
@@ -843,21 +901,6 @@ inline int make_map_3d(CUtensorMap* m, const void* ptr, uint64_t inner, uint64_t
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? 0 : 2;
-}
-
-// Tensor map of C for TMA stores: boxes of 128 bytes x 32 rows, 128-byte swizzle; groups = 0 for a plain matrix.
-inline int make_store_map(CUtensorMap* m, const void* ptr, uint64_t N, uint64_t M, uint64_t groups, uint64_t ldc, int out_fp32) {
-  EncodeTiledFn enc = get_encode();
-  if (!enc) return 1;
-  const uint64_t esz = out_fp32 ? 4 : 2;
-  cuuint64_t dims[3] = {N, M, groups};
-  cuuint64_t strides[2] = {ldc * esz, ldc * esz * M};
-  cuuint32_t box[3] = {(cuuint32_t)(128 / esz), 32, 1};
-  cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = enc(m, out_fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, groups ? 3 : 2, const_cast<void*>(ptr), dims,
-                   strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : 2;
 }

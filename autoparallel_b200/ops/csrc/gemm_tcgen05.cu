@@ -18,40 +18,36 @@
 namespace apb {
 
 template <bool A_MN, bool B_MN>
-__global__ void __launch_bounds__(GEMM_THREADS, 1)
-gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                 const __grid_constant__ CUtensorMap tmC, GemmParams p) {
+__global__ void __launch_bounds__(GEMM_PLAIN_THREADS, 1)
+gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
   FuseParams f{};
-  gemm_cta<A_MN, B_MN, FUSE_NONE>(tmA, tmB, p, f, blockIdx.x, gridDim.x, smem_raw, &tmC);
+  gemm_cta<A_MN, B_MN, FUSE_NONE>(tmA, tmB, p, f, blockIdx.x, gridDim.x, smem_raw);
 }
 
 template <bool A_MN, bool B_MN, int ST = 0, bool DYN = false>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
-gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                      const __grid_constant__ CUtensorMap tmC, GemmParams p) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ST == 0 ? GEMM_PLAIN_THREADS : GEMM_THREADS, 1)
+gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
   FuseParams f{};
-  gemm_cta<A_MN, B_MN, FUSE_NONE, true, false, ST, DYN>(tmA, tmB, p, f, blockIdx.x, gridDim.x, smem_raw, &tmC);
+  gemm_cta<A_MN, B_MN, FUSE_NONE, true, false, ST, DYN>(tmA, tmB, p, f, blockIdx.x, gridDim.x, smem_raw);
 }
 
 // Grouped GEMM: G problems of one shape (the expert projections of a capacity-based MoE layer).
 template <bool A_MN, bool B_MN>
-__global__ void __launch_bounds__(GEMM_THREADS, 1)
-gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                    const __grid_constant__ CUtensorMap tmC, GemmParams p) {
+__global__ void __launch_bounds__(GEMM_PLAIN_THREADS, 1)
+gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
   FuseParams f{};
-  gemm_cta<A_MN, B_MN, FUSE_NONE, false, true>(tmA, tmB, p, f, blockIdx.x, gridDim.x, smem_raw, &tmC);
+  gemm_cta<A_MN, B_MN, FUSE_NONE, false, true>(tmA, tmB, p, f, blockIdx.x, gridDim.x, smem_raw);
 }
 
 template <bool A_MN, bool B_MN>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
-gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                         const __grid_constant__ CUtensorMap tmC, GemmParams p) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_PLAIN_THREADS, 1)
+gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
   FuseParams f{};
-  gemm_cta<A_MN, B_MN, FUSE_NONE, true, true>(tmA, tmB, p, f, blockIdx.x, gridDim.x, smem_raw, &tmC);
+  gemm_cta<A_MN, B_MN, FUSE_NONE, true, true>(tmA, tmB, p, f, blockIdx.x, gridDim.x, smem_raw);
 }
 
 static int g_pair_mode = 1;  // 0: one CTA per tile, 1: CTA pairs where the shape allows (default)
@@ -68,7 +64,7 @@ extern "C" int apb_gemm_resident_pairs(int num_sms) {
   using namespace apb;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(num_sms & ~1));
-  cfg.blockDim = dim3(GEMM_THREADS);
+  cfg.blockDim = dim3(GEMM_PLAIN_THREADS);
   cfg.dynamicSmemBytes = GEMM_PLAIN_SMEM_BYTES;
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeClusterDimension;
@@ -177,25 +173,22 @@ extern "C" int apb_gemm_bf16(const void* A, const void* B, void* C, int M, int N
   p.num_m_tiles = (M + BM - 1) / BM;
   p.num_n_tiles = (N + BN - 1) / BN;
   p.status = status;
-  CUtensorMap tmC = tmA;  // (not read unless the TMA store is on)
-  p.tma_store = (ldc * (out_fp32 ? 4 : 2)) % 16 == 0;
-  if (p.tma_store) {
-    const int e3 = make_store_map(&tmC, C, (uint64_t)N, (uint64_t)M, 0, (uint64_t)ldc, out_fp32);
-    if (e3) return e3;
-  }
+  p.vec_store = ldc % (out_fp32 ? 4 : 8) == 0 && N % (out_fp32 ? 4 : 8) == 0;
   if (g_pair_mode && pair_shape(M, N, K)) {
     // CTA pairs: B is loaded in boxes of 128 rows (each CTA stages half of the 256 tile columns)
     int e2 = 0;
     if (!b_mn_major) e2 = make_map(&tmB, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, BN / 2);
     if (e2) return e2;
     const int tiles2 = ((M + 2 * BM - 1) / (2 * BM)) * p.num_n_tiles;
+    set_tile_order(p, (M + 2 * BM - 1) / (2 * BM));
     int resident = apb_gemm_resident_pairs(num_sms) - g_reserved_sms / 2;
     if (resident < 1) resident = 1;
     const int pairs = tiles2 < resident ? tiles2 : resident;
     const int smem2 = apb_gemm_pair_smem_bytes(g_pair_stages);
+    const int threads2 = g_pair_stages == PAIR_STAGES ? GEMM_PLAIN_THREADS : GEMM_THREADS;
     auto launch2 = [&](auto kern) {
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2);
-      kern<<<2 * pairs, GEMM_THREADS, smem2, stream>>>(tmA, tmB, tmC, p);
+      kern<<<2 * pairs, threads2, smem2, stream>>>(tmA, tmB, p);
     };
 #define APB_LAUNCH_PAIR(ST)                                                              \
   do {                                                                                   \
@@ -216,11 +209,12 @@ extern "C" int apb_gemm_bf16(const void* A, const void* B, void* C, int M, int N
     else APB_LAUNCH_PAIR(0);
     return cudaGetLastError() == cudaSuccess ? 0 : 4;
   }
+  set_tile_order(p, p.num_m_tiles);
   const int tiles = p.num_m_tiles * p.num_n_tiles;
   const int grid = tiles < usable ? tiles : usable;
   auto launch = [&](auto kern) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_PLAIN_SMEM_BYTES);
-    kern<<<grid, GEMM_THREADS, GEMM_PLAIN_SMEM_BYTES, stream>>>(tmA, tmB, tmC, p);
+    kern<<<grid, GEMM_PLAIN_THREADS, GEMM_PLAIN_SMEM_BYTES, stream>>>(tmA, tmB, p);
   };
   if (!a_mn_major && !b_mn_major) launch(gemm_bf16_kernel<false, false>);
   else if (!a_mn_major && b_mn_major) launch(gemm_bf16_kernel<false, true>);
@@ -257,14 +251,12 @@ extern "C" int apb_gemm_grouped_bf16(const void* A, const void* B, void* C, int 
   p.num_n_tiles = (N + BN - 1) / BN;
   p.status = status;
   p.groups = G;
-  CUtensorMap tmC;
-  p.tma_store = 1;  // (N % 8 == 0: rows of 16-byte vectors in both output types)
-  e = make_store_map(&tmC, C, (uint64_t)N, (uint64_t)M, (uint64_t)G, (uint64_t)N, out_fp32);
-  if (e) return e;
+  p.vec_store = 1;  // (N % 8 == 0: rows of 16-byte vectors in both output types)
   auto launch = [&](auto kern, int grid) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_PLAIN_SMEM_BYTES);
-    kern<<<grid, GEMM_THREADS, GEMM_PLAIN_SMEM_BYTES, stream>>>(tmA, tmB, tmC, p);
+    kern<<<grid, GEMM_PLAIN_THREADS, GEMM_PLAIN_SMEM_BYTES, stream>>>(tmA, tmB, p);
   };
+  set_tile_order(p, pair ? (M + 2 * BM - 1) / (2 * BM) : p.num_m_tiles);
   if (pair) {
     const long long tiles2 = (long long)G * ((M + 2 * BM - 1) / (2 * BM)) * p.num_n_tiles;
     int resident = apb_gemm_resident_pairs(num_sms) - g_reserved_sms / 2;

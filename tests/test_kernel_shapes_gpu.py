@@ -405,3 +405,39 @@ def test_pairs_with_less_than_two_full_row_tiles(K, M, ta):
     x, y = a[0], torch.randn(K_, 20480, device="cuda", generator=g).to(torch.bfloat16)
     out = lib.ops.gemm(x, y, ta, False, torch.float32)
     assert _rel(out, (x.double().t() if ta else x.double()) @ y.double()) <= 2**-24 * 8 * K_ ** 0.5
+
+
+@pytest.mark.parametrize("out", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("G,M,N,Kd", [
+    (0, 4361, 1800, 72),   # pairs: groups of 16 tile rows and one of 2, a last tile row of 9 rows, a last column tile of 8 columns
+    (0, 100, 40000, 72),   # one CTA per tile, more tiles than SMs
+    (3, 2600, 1032, 40),   # grouped: several groups per CTA pair, one k-block that is not full
+    (70, 160, 520, 1288),  # grouped, an odd CTA with 32 rows
+])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (True, True)])
+def test_gemm_tiles_land_where_they_belong(K, G, M, N, Kd, a_mn, b_mn, out):
+    """Whole numbers: every sum is exact.  The plain product writes into the middle of a wider matrix, whose margins stay."""
+    _, impl = K
+    ext = impl.extension()
+    if a_mn and M % 8:
+        M += 8 - M % 8  # (rows of 16 bytes)
+    gen = torch.Generator(device="cuda").manual_seed(M + N)
+    lead = (G,) if G else ()
+    a = torch.randint(-1, 2, (*lead, M, Kd), device="cuda", generator=gen).to(torch.bfloat16)
+    b = torch.randint(-1, 2, (*lead, N, Kd), device="cuda", generator=gen).to(torch.bfloat16)
+    ref = (a.float() @ b.float().transpose(-1, -2)).to(out)
+    a = a.transpose(-1, -2).contiguous() if a_mn else a
+    b = b.transpose(-1, -2).contiguous() if b_mn else b
+    if G:
+        c = torch.full((G, M, N), 99.0, device="cuda", dtype=out)
+        ext.gemm_grouped(a, b, c, a_mn, b_mn, impl.status_buffer(c.device))
+        assert torch.equal(c, ref)
+        return
+    for pad in (8, 1):  # rows of whole 16-byte vectors, and rows that are not
+        wide = torch.full((M + 2, N + 8 + pad), 99.0, device="cuda", dtype=out)
+        flat = wide.view(-1)
+        c = flat[8:8 + (M - 1) * wide.shape[1] + N].as_strided((M, N), (wide.shape[1], 1))  # (starts on a 16-byte boundary)
+        ext.gemm(a, b, c, a_mn, b_mn, impl.status_buffer(c.device))
+        assert torch.equal(c, ref)
+        c.fill_(99.0)
+        assert bool((wide == 99.0).all())
