@@ -169,7 +169,7 @@ __device__ __forceinline__ void store_row_chunk(const GemmParams& p, long long r
   }
 }
 
-// Epilogue of the plain GEMM for one warp's 32 rows and ``ncols`` columns: 128 bytes of every row at a time go to the warp's staging block
+// Epilogue of the plain GEMM for one warp's 32 rows and ``ncols`` columns (a multiple of 64): 128 bytes of every row at a time go to the warp's staging block
 // (128-byte swizzle, conflict free) and from there to C with eight lanes to a row, so that every store instruction writes whole lines; a
 // thread owns a row in TMEM, and storing straight from registers puts 16-byte pieces of 32 lines into every instruction.  ``release`` is
 // called as soon as the last block is in registers.

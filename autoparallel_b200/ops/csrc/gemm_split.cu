@@ -11,7 +11,9 @@
 // its share of the tile's rows from all S shared memories, in slice order, and stores it: no workspace, no atomics, no
 // second launch, the same result every time.
 //
-//   warp 0: TMA producer | warp 1: TMEM owner + MMA issuer | warps 2..5: TMEM -> shared memory | all: sum and store
+// A cluster of one CTA has nothing to add and stores its tile from TMEM (store_tile).
+//
+//   warp 0: TMA producer | warp 1: TMEM owner + MMA issuer | warps 2..9 (64 columns: 2..5): TMEM -> shared memory (or C) | all: sum and store
 // Persistent kernels -> this one, us: 16 x 4096 x 4096 29 -> 13, 16 x 4096 x 14336 87 -> 25, 64 x 2048 x 2048 16.6 -> 8.6, 64 x 2048 x 8192 50 -> 15.6,
 // 512 x 256 x 256 7.0 -> 5.5, 160 x 8192 x 8192 55 -> 39; 478 products in profiles/gemm_split_rule_sweep.txt.
 #include "gemm_core.cuh"
@@ -20,6 +22,7 @@ namespace apb {
 
 constexpr int SPLIT_MAX = 8;  // portable cluster size
 constexpr int SPLIT_STAGE_TOTAL = 196608;  // 8 x 24 KB, 6 x 32 KB or 4 x 48 KB: deep enough for one CTA to hide the load latency
+constexpr int SPLIT_THREADS = GEMM_PLAIN_THREADS;
 constexpr int SPLIT_SMEM_BYTES = SPLIT_STAGE_TOTAL + 1024 + 256;
 
 __device__ __forceinline__ uint32_t cluster_size() {
@@ -34,10 +37,11 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
 }
 
 template <bool A_MN, bool B_MN, int BN_T, bool GROUPED>
-__global__ void __launch_bounds__(GEMM_THREADS, 1)
+__global__ void __launch_bounds__(SPLIT_THREADS, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
   constexpr int B_BYTES = BN_T * BK * 2;
   constexpr int ST = SPLIT_STAGE_TOTAL / (A_STAGE_BYTES + B_BYTES);
+  constexpr int HALVES = BN_T >= 128 ? EPI_WARPS / 4 : 1, COLS = BN_T / HALVES;  // warps per lane quarter, and their columns: blocks of 64
   constexpr int LD = BN_T + 4;  // floats per row of the fp32 tile: rows start 16 bytes apart modulo the banks
   static_assert(BM * LD * 4 <= SPLIT_STAGE_TOTAL, "the fp32 tile reuses the stages");
   static_assert((2 * ST + 1) * 8 + 8 <= 256, "barrier block");
@@ -60,28 +64,39 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   int tm, tn;
   tile_coords(GROUPED ? t - grp * per_group : t, p.num_m_tiles, p.num_n_tiles, tm, tn);
   const int m0 = tm * BM, n0 = tn * BN_T;
+  const int rows = min(BM, p.M - m0);  // of the tile that are inside the matrix
+  const bool solo = S == 1 && p.vec_store;
   const int num_kb = (p.K + BK - 1) / BK;
   const int kb0 = (int)((long long)num_kb * slice / S), kb1 = (int)((long long)num_kb * (slice + 1) / S);  // S <= num_kb: never empty
 
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < ST; ++s) {
-      mbar_init(&full[s], 1);
-      mbar_init(&empty[s], 1);
+  // The producer goes on as soon as it has set up the barriers; the others wait for them and for the TMEM columns, whose allocation
+  // (half a microsecond) the first loads hide.
+  uint32_t tmem_base = 0;
+  if (warp == 0) {
+    if (elect_one()) {
+      for (int s = 0; s < ST; ++s) {
+        mbar_init(&full[s], 1);
+        mbar_init(&empty[s], 1);
+      }
+      mbar_init(tmem_full, 1);
+      *abort_flag = 0;
+      mbar_fence_init();
     }
-    mbar_init(tmem_full, 1);
-    *abort_flag = 0;
-    mbar_fence_init();
-    tma_prefetch_desc(&tmA);
-    tma_prefetch_desc(&tmB);
+    __syncwarp();
+    named_arrive(1, SPLIT_THREADS);
+  } else {
+    if (warp == 1) {
+      tmem_alloc(tmem_slot, BN_T);
+      tmem_relinquish();
+    } else if (warp == 2 && lane == 0) {
+      tma_prefetch_desc(&tmA);
+      tma_prefetch_desc(&tmB);
+    }
+    tc_fence_before();
+    named_sync(1, SPLIT_THREADS);
+    tc_fence_after();
+    tmem_base = *tmem_slot;
   }
-  if (warp == 1) {
-    tmem_alloc(tmem_slot, BN_T);
-    tmem_relinquish();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
   auto fail = [&](uint32_t code) {
     atomicCAS(p.status, 0u, code);
     *abort_flag = 1;
@@ -156,77 +171,104 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       if (ok) umma_commit(tmem_full);
     }
     __syncwarp();
-  } else {
+  } else if (warp < 2 + 4 * HALVES) {
     const int q = warp & 3;  // TMEM lane quarter this warp may read
+    const int col0 = ((warp - 2) >> 2) * COLS;  // first of its columns
     // (the TMEM loads are warp-wide: the warp goes on together or not at all)
-    if (__all_sync(0xffffffffu, mbar_wait(tmem_full, 0, abort_flag))) {
+    if (!__all_sync(0xffffffffu, mbar_wait(tmem_full, 0, abort_flag))) {
+      fail(ST_TIMEOUT_TMEM_FULL);
+    } else if (solo) {
       tc_fence_after();
-      float* row = tile + (q * 32 + lane) * LD;
+      uint8_t* stg = smem + (warp - 2) * STORE_BYTES;
+      const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + col0;
+      const long long c_off = GROUPED ? (long long)grp * p.M * p.ldc : 0;
+      auto nothing = []() {};
+      if (p.out_fp32) store_tile<true>(reinterpret_cast<float*>(p.C) + c_off, p.ldc, stg, taddr, m0 + q * 32, n0 + col0, COLS, p.M, p.N, lane, nothing);
+      else store_tile<false>(reinterpret_cast<__nv_bfloat16*>(p.C) + c_off, p.ldc, stg, taddr, m0 + q * 32, n0 + col0, COLS, p.M, p.N, lane, nothing);
+    } else if (q * 32 < rows) {
+      tc_fence_after();
+      float* row = tile + (q * 32 + lane) * LD + col0;
 #pragma unroll
-      for (int c = 0; c < BN_T / 32; ++c) {
+      for (int c = 0; c < COLS / 32; ++c) {
         uint32_t r[32];
-        tmem_ld_32x32(tmem_base + (uint32_t(q * 32) << 16) + c * 32, r);
-        tmem_ld_wait();
+        tmem_ld_32x32(tmem_base + (uint32_t(q * 32) << 16) + col0 + c * 32, r);
+        tmem_ld_wait_for(r);
 #pragma unroll
         for (int i = 0; i < 8; ++i)
           reinterpret_cast<uint4*>(row + c * 32)[i] = make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
       }
-    } else {
-      fail(ST_TIMEOUT_TMEM_FULL);
     }
+  }
+  if (solo) {  // nothing to add up: the warps have stored the tile from TMEM
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+      tc_fence_after();
+      tmem_dealloc(tmem_base, BN_T);
+    }
+    return;
   }
   tc_fence_before();
+  __syncwarp();
   cluster_arrive();  // (also orders the threads of a cluster of one CTA)
-  cluster_wait();
-
-  if (*abort_flag == 0) {
-    const bool vec = p.out_fp32 ? (p.ldc & 3) == 0 : (p.ldc & 7) == 0;
-    const long long c_off = GROUPED ? (long long)grp * p.M * p.ldc : 0;
-    // eight columns per thread; the tile's vectors are dealt to the CTAs of the cluster in blocks of one per thread
-    for (int v = slice * GEMM_THREADS + threadIdx.x; v < BM * (BN_T / 8); v += S * GEMM_THREADS) {
-      const int r = v / (BN_T / 8), c = (v % (BN_T / 8)) * 8;
-      const long long row = m0 + r;
-      const int col = n0 + c;
-      if (row >= p.M || col >= p.N) continue;
-      float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-      const float* src = tile + r * LD + c;
-#pragma unroll 4
-      for (int s = 0; s < S; ++s) {
-        const uint32_t addr = map_to_cta(src, (uint32_t)s);
-        const float4 x = ld_cluster_f4(addr), y = ld_cluster_f4(addr + 16);
-        a.x += x.x; a.y += x.y; a.z += x.z; a.w += x.w;
-        b.x += y.x; b.y += y.y; b.z += y.z; b.w += y.w;
-      }
-      const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-      const long long off = c_off + row * p.ldc + col;
-      if (p.out_fp32) {
-        float* dst = reinterpret_cast<float*>(p.C) + off;
-        if (vec && col + 8 <= p.N) {
-          reinterpret_cast<float4*>(dst)[0] = a;
-          reinterpret_cast<float4*>(dst)[1] = b;
-        } else {
-#pragma unroll
-          for (int i = 0; i < 8; ++i)
-            if (col + i < p.N) dst[i] = f[i];
-        }
-      } else {
-        __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + off;
-        if (vec && col + 8 <= p.N) {
-          *reinterpret_cast<uint4*>(dst) = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
-        } else {
-#pragma unroll
-          for (int i = 0; i < 8; ++i)
-            if (col + i < p.N) dst[i] = __float2bfloat16(f[i]);
-        }
-      }
-    }
-  }
-  cluster_arrive();  // no CTA leaves while another may still read its tile
   cluster_wait();
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, BN_T);
   }
+
+  // The sum: four columns per thread and row, the rows of a thread a whole stride apart, two at a time so that their loads are under way
+  // together (the other CTAs' shared memory gives 16 bytes a cycle and SM, with a round trip of hundreds of cycles).  The loops stay small on
+  // purpose: eight rows at a time, unrolled, were slower in every product (64 x 1408 x 2048 6.9 us against 5.8): the code is fetched once
+  // per launch.  128 x 128 tiles in two slices: sum and store 2.8 -> 1.6 us, in one 2.8 + 0.8 -> 1.2 (TMEM to C).
+  if (*abort_flag == 0) {
+    constexpr int VPR = BN_T / 4, RSTEP = SPLIT_THREADS / VPR;  // threads per row, rows per pass of the CTA
+    static_assert(RSTEP * VPR == SPLIT_THREADS, "whole rows");
+    const int c = (threadIdx.x % VPR) * 4, col = n0 + c, step = S * RSTEP;
+    const bool whole = (p.ldc & 3) == 0 && col + 4 <= p.N;
+    const int esz = p.out_fp32 ? 4 : 2;
+    const uint32_t src0 = smem_u32(tile) + c * 4;
+    uint8_t* dst0 = reinterpret_cast<uint8_t*>(p.C) + ((GROUPED ? (long long)grp * p.M * p.ldc : 0) + (long long)m0 * p.ldc + col) * esz;
+    const long long ld_bytes = p.ldc * esz;
+    auto add = [](float4& a, const float4& x) { a.x += x.x; a.y += x.y; a.z += x.z; a.w += x.w; };
+    auto store = [&](int r, const float4& v) {
+      uint8_t* dst = dst0 + r * ld_bytes;
+      if (whole) {
+        if (p.out_fp32) *reinterpret_cast<float4*>(dst) = v;
+        else *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+      } else {
+        const float f[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if (col + i >= p.N) break;
+          if (p.out_fp32) reinterpret_cast<float*>(dst)[i] = f[i];
+          else reinterpret_cast<__nv_bfloat16*>(dst)[i] = __float2bfloat16(f[i]);
+        }
+      }
+    };
+#pragma unroll 1
+    for (int r = slice * RSTEP + threadIdx.x / VPR; r < rows && col < p.N; r += 2 * step) {
+      const uint32_t src = src0 + r * (LD * 4);
+      float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+      if (r + step < rows) {
+#pragma unroll 2
+        for (int s = 0; s < S; ++s) {
+          const uint32_t from = map_to_cta(src, (uint32_t)s);
+          const float4 x = ld_cluster_f4(from), y = ld_cluster_f4(from + step * (LD * 4));
+          add(a, x);
+          add(b, y);
+        }
+        store(r + step, b);
+      } else {
+#pragma unroll 4
+        for (int s = 0; s < S; ++s) add(a, ld_cluster_f4(map_to_cta(src, (uint32_t)s)));
+      }
+      store(r, a);
+    }
+  }
+  __syncwarp();
+  cluster_arrive_relaxed();  // no CTA leaves while another may still read its tile
+  cluster_wait();
 }
 
 }  // namespace apb
@@ -274,7 +316,7 @@ static int split_slots(int s, int num_sms) {
   if (dev >= 0 && dev < 64 && cached[dev][s] > 0) return cached[dev][s];
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(num_sms / s * s));
-  cfg.blockDim = dim3(GEMM_THREADS);
+  cfg.blockDim = dim3(SPLIT_THREADS);
   cfg.dynamicSmemBytes = SPLIT_SMEM_BYTES;
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeClusterDimension;
@@ -378,6 +420,7 @@ extern "C" int apb_gemm_split(const void* A, const void* B, void* C, int G, int 
   p.num_n_tiles = (N + bn - 1) / bn;
   p.status = status;
   p.groups = grouped ? G : 1;
+  p.vec_store = ldc % (out_fp32 ? 4 : 8) == 0 && N % (out_fp32 ? 4 : 8) == 0;
   const long long ctas = (long long)p.num_m_tiles * p.num_n_tiles * p.groups * s;
   if (ctas > 0x7fffffffll / s) return 3;
   SplitKernel kern = grouped ? split_kernel_of<true>(bn, a_mn, b_mn) : split_kernel_of<false>(bn, a_mn, b_mn);
@@ -385,7 +428,7 @@ extern "C" int apb_gemm_split(const void* A, const void* B, void* C, int G, int 
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SPLIT_SMEM_BYTES) != cudaSuccess) return 4;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)ctas);
-  cfg.blockDim = dim3(GEMM_THREADS);
+  cfg.blockDim = dim3(SPLIT_THREADS);
   cfg.dynamicSmemBytes = SPLIT_SMEM_BYTES;
   cfg.stream = stream;
   cudaLaunchAttribute attr;

@@ -46,6 +46,10 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// Named barrier of ``threads`` threads of the CTA: ``arrive`` goes on at once, ``sync`` waits for all.
+__device__ __forceinline__ void named_arrive(int id, int threads) { asm volatile("barrier.cta.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ void named_sync(int id, int threads) { asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+
 // ----------------------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
@@ -159,11 +163,18 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   return r;
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+// without the release: for a barrier that only says that reads of other CTAs' shared memory are over (a release waits for global stores too)
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // shared::cluster address of ``p`` (a shared-memory pointer of this CTA) as seen in CTA ``rank``
 __device__ __forceinline__ uint32_t map_to_cta(const void* p, uint32_t rank) {
   uint32_t a;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr), "r"(rank));
   return a;
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
