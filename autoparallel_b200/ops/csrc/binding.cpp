@@ -3,8 +3,12 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
+#include <torch/library.h>
 
+#include <array>
+#include <atomic>
 #include <cstdint>
+#include <mutex>
 
 extern "C" {
 int apb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc,
@@ -518,9 +522,246 @@ void dma_rs_sum(const at::Tensor& src, at::Tensor& dst, const std::vector<int64_
         "apb_dma_rs_sum");
 }
 
+// ------------------------------------------------------------------ the operators' CUDA entries
+// Registered over the Python entries once the extension is loaded, so that an operator call - from a graph, from the autograd engine's
+// threads - runs no Python on its way to the kernel: 6 to 9 us of host time per call, and the interpreter's lock.  Every function takes the
+// forms that its counterpart in ops/cuda_impl.py gives to this extension, under the same conditions; all others, and what the flags there
+// ask for, go to that Python function.
+struct Native {
+  py::object table;  // operator name -> function of ops/cuda_impl.py
+  bool diag_library_gemm = false, moe_kernels = true;
+  std::atomic<bool> shadows{false};  // low-precision copies of parameters may exist: casts ask Python for them
+  std::atomic<int64_t> launches{0};
+};
+Native& native() {
+  static Native* n = new Native;  // (never destroyed: its Python object must not outlive the interpreter's end)
+  return *n;
+}
+
+template <typename R, typename... A>
+R in_python(const char* op, const A&... args) {
+  py::gil_scoped_acquire gil;
+  return py::cast<R>(native().table[op](args...));
+}
+py::object py_dtype(at::ScalarType t) { return py::reinterpret_borrow<py::object>(reinterpret_cast<PyObject*>(torch::getTHPDtype(t))); }
+
+// The word that bounded waits report to, one per device: made by Python at the first use on a device and shared with it.
+at::Tensor& status_of(const at::Tensor& t) {
+  static std::array<at::Tensor, 64> words;
+  static std::array<std::atomic<bool>, 64> known{};
+  static std::mutex m;
+  const int dev = t.get_device();
+  TORCH_CHECK(dev >= 0 && dev < 64, "unexpected device index ", dev);
+  if (!known[dev].load(std::memory_order_acquire)) {
+    at::Tensor w = in_python<at::Tensor>("status_buffer", t.device());
+    std::lock_guard<std::mutex> g(m);
+    if (!known[dev].load(std::memory_order_relaxed)) {
+      words[dev] = w;
+      known[dev].store(true, std::memory_order_release);
+    }
+  }
+  return words[dev];
+}
+void count(int64_t n = 1) { native().launches.fetch_add(n, std::memory_order_relaxed); }
+bool float_or_bf16(at::ScalarType t) { return t == at::kBFloat16 || t == at::kFloat; }
+
+using at::Tensor;
+using Two = std::tuple<Tensor, Tensor>;
+
+Tensor op_mm_nd(const Tensor& a, const Tensor& b, bool trans_b, at::ScalarType dtype) {
+  if (float_or_bf16(dtype) && !native().diag_library_gemm) {
+    auto c = mm_nd(a, b, trans_b, dtype == at::kFloat, status_of(a));
+    if (c.has_value()) {
+      count();
+      return *c;
+    }
+  }
+  py::gil_scoped_acquire gil;
+  return in_python<Tensor>("mm_nd", a, b, trans_b, py_dtype(dtype));
+}
+Tensor op_mm_wgrad(const Tensor& a, const Tensor& b, at::ScalarType dtype) {
+  if (float_or_bf16(dtype) && !native().diag_library_gemm) {
+    auto c = gemm_new(a, b, true, true, dtype == at::kFloat, status_of(a));
+    if (c.has_value()) {
+      count();
+      return *c;
+    }
+  }
+  py::gil_scoped_acquire gil;
+  return in_python<Tensor>("mm_wgrad", a, b, py_dtype(dtype));
+}
+bool grouped_ok(const Tensor& a, const Tensor& b, at::ScalarType dtype) {
+  return a.dim() == 3 && b.dim() == 3 && a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16 && a.size(2) % 8 == 0 &&
+         b.size(2) % 8 == 0 && float_or_bf16(dtype);
+}
+Tensor op_grouped_mm(const Tensor& a, const Tensor& b, bool trans_b, at::ScalarType dtype) {
+  if (grouped_ok(a, b, dtype) && b.size(trans_b ? 1 : 2) % 8 == 0) {
+    Tensor c = at::empty({a.size(0), a.size(1), b.size(trans_b ? 1 : 2)}, a.options().dtype(dtype));
+    gemm_grouped(dense(a), dense(b), c, false, !trans_b, status_of(a));
+    count();
+    return c;
+  }
+  py::gil_scoped_acquire gil;
+  return in_python<Tensor>("grouped_mm", a, b, trans_b, py_dtype(dtype));
+}
+Tensor op_grouped_wgrad(const Tensor& a, const Tensor& b, at::ScalarType dtype) {
+  if (grouped_ok(a, b, dtype)) {
+    Tensor c = at::empty({a.size(0), a.size(2), b.size(2)}, a.options().dtype(dtype));
+    gemm_grouped(dense(a), dense(b), c, true, true, status_of(a));
+    count();
+    return c;
+  }
+  py::gil_scoped_acquire gil;
+  return in_python<Tensor>("grouped_mm_wgrad", a, b, py_dtype(dtype));
+}
+Tensor op_cast(const Tensor& x, at::ScalarType dtype) {
+  if (x.scalar_type() == dtype) return x;
+  if (!native().shadows.load(std::memory_order_relaxed) && (dtype == at::kBFloat16 || (dtype == at::kFloat && x.scalar_type() == at::kBFloat16))) {
+    auto y = cast_new(x, dtype == at::kBFloat16);
+    if (y.has_value()) {
+      count();
+      return *y;
+    }
+  }
+  py::gil_scoped_acquire gil;
+  return in_python<Tensor>("dtype_cast", x, py_dtype(dtype));
+}
+Two op_rms_norm(const Tensor& x, const Tensor& w, double eps) {
+  count();
+  return rms_norm_new(x, w, eps);
+}
+Two op_rms_norm_bwd(const Tensor& dy, const Tensor& x, const Tensor& w, const Tensor& rstd) {
+  count(2);
+  return rms_norm_bwd_new(dy, x, w, rstd);
+}
+Tensor op_rope(const Tensor& x, const Tensor& cos, const Tensor& sin, bool conj) {
+  count();
+  return rope_new(x, cos, sin, conj);
+}
+Tensor op_swiglu(const Tensor& a, const Tensor& b) {
+  count();
+  return swiglu_new(a, b);
+}
+Two op_swiglu_bwd(const Tensor& dy, const Tensor& a, const Tensor& b) {
+  count();
+  return swiglu_bwd_new(dy, a, b);
+}
+Two op_xent(const Tensor& logits_, const Tensor& labels) {
+  Tensor logits = dense(logits_);
+  const auto shape = logits.sizes().slice(0, logits.dim() - 1);
+  Tensor loss = at::empty(shape, logits.options().dtype(at::kFloat)), lse = at::empty(shape, loss.options());
+  xent_fwd(logits, labels.contiguous(), loss, lse);
+  count();
+  return {loss, lse};
+}
+Tensor op_xent_bwd(const Tensor& dloss, const Tensor& logits_, const Tensor& labels, const Tensor& lse) {
+  Tensor logits = dense(logits_), out = at::empty_like(logits);
+  xent_bwd(dloss.to(at::kFloat).contiguous(), logits, labels.contiguous(), lse.contiguous(), out);
+  count();
+  return out;
+}
+Tensor op_embedding(const Tensor& weight, const Tensor& ids) {
+  if (weight.dim() == 2 && float_or_bf16(weight.scalar_type()) && weight.size(1) * weight.element_size() % 16 == 0 && ids.scalar_type() == at::kLong) {
+    auto shape = ids.sizes().vec();
+    shape.push_back(weight.size(1));
+    Tensor out = at::empty(shape, weight.options());
+    embedding_fwd(dense(weight), ids.contiguous(), out);
+    count();
+    return out;
+  }
+  py::gil_scoped_acquire gil;
+  return in_python<Tensor>("embedding", weight, ids);
+}
+Tensor op_embedding_bwd(const Tensor& dy_, const Tensor& ids, int64_t rows) {
+  Tensor dy = dy_.contiguous(), out = at::empty({rows, dy.size(-1)}, dy.options());
+  count(embedding_bwd(dy, ids.contiguous(), out));
+  return out;
+}
+
+bool moe_ok(std::initializer_list<const Tensor*> ts) {
+  if (!native().moe_kernels) return false;
+  for (const Tensor* t : ts)
+    if (!t->is_cuda()) return false;
+  return true;
+}
+Tensor gate_weights(const Tensor& w, at::ScalarType dtype) { return (float_or_bf16(w.scalar_type()) ? w : w.to(dtype)).contiguous(); }
+Tensor op_moe_slots(const Tensor& idx, int64_t E, int64_t C, int64_t nb) {
+  if (moe_ok({&idx}) && idx.scalar_type() == at::kLong && idx.dim() == 2 && nb > 0 && idx.size(0) > 0 && idx.size(0) % nb == 0 &&
+      E <= moe_slots_max_experts(idx.size(0) / nb * idx.size(1)) && E * C < (int64_t(1) << 31)) {
+    Tensor slot = at::empty_like(idx, at::MemoryFormat::Contiguous);
+    count(moe_slots(idx.contiguous(), slot, E, C, nb));
+    return slot;
+  }
+  return in_python<Tensor>("moe_slots", idx, E, C, nb);
+}
+Tensor op_moe_scatter(const Tensor& src, const Tensor& slot, const Tensor& w, int64_t E, int64_t C, int64_t nb) {
+  if (moe_ok({&src, &slot, &w}) && float_or_bf16(src.scalar_type()) && src.dim() == 2 && nb > 0 && src.size(0) > 0 && src.size(0) % nb == 0) {
+    Tensor buf = at::empty({E, nb, C, src.size(1)}, src.options());
+    moe_scatter(src.contiguous(), slot.contiguous(), gate_weights(w, src.scalar_type()), buf, E, C, nb);
+    count(2);
+    return buf;
+  }
+  return in_python<Tensor>("moe_scatter", src, slot, w, E, C, nb);
+}
+Tensor op_moe_gather(const Tensor& buf, const Tensor& slot, const Tensor& w) {
+  if (moe_ok({&buf, &slot, &w}) && float_or_bf16(buf.scalar_type()) && buf.dim() == 4 && buf.size(1) > 0 && slot.dim() == 2 && slot.size(0) > 0 &&
+      slot.size(0) % buf.size(1) == 0) {
+    Tensor out = at::empty({slot.size(0), buf.size(3)}, buf.options());
+    moe_gather(buf.contiguous(), slot.contiguous(), gate_weights(w, buf.scalar_type()), out);
+    count();
+    return out;
+  }
+  return in_python<Tensor>("moe_gather", buf, slot, w);
+}
+Tensor op_moe_gate_grad(const Tensor& buf, const Tensor& slot, const Tensor& g) {
+  if (moe_ok({&buf, &slot, &g}) && float_or_bf16(buf.scalar_type()) && buf.dim() == 4 && g.scalar_type() == buf.scalar_type() && buf.size(1) > 0 &&
+      slot.dim() == 2 && slot.size(0) > 0 && slot.size(0) % buf.size(1) == 0) {
+    Tensor dw = at::empty(slot.sizes(), buf.options().dtype(at::kFloat));
+    moe_gate_grad(buf.contiguous(), slot.contiguous(), g.contiguous(), dw);
+    count();
+    return dw;
+  }
+  return in_python<Tensor>("moe_gate_grad", buf, slot, g);
+}
+
+// Once per process, after the Python functions are known.  The dispatcher warns when a kernel takes another's place, which here is meant.
+void register_native(py::dict table, bool diag_library_gemm, bool moe_kernels) {
+  static torch::Library* lib = nullptr;
+  if (lib != nullptr) return;
+  native().table = std::move(table);
+  native().diag_library_gemm = diag_library_gemm;
+  native().moe_kernels = moe_kernels;
+  struct Quiet : c10::WarningHandler {
+    void process(const c10::Warning&) override {}
+  } quiet;
+  c10::WarningUtils::WarningHandlerGuard guard(&quiet);
+  lib = new torch::Library(torch::Library::IMPL, "apb200", c10::DispatchKey::CUDA, __FILE__, __LINE__);
+  lib->impl("mm_nd", op_mm_nd);
+  lib->impl("mm_wgrad", op_mm_wgrad);
+  lib->impl("grouped_mm", op_grouped_mm);
+  lib->impl("grouped_mm_wgrad", op_grouped_wgrad);
+  lib->impl("dtype_cast", op_cast);
+  lib->impl("rms_norm", op_rms_norm);
+  lib->impl("rms_norm_bwd", op_rms_norm_bwd);
+  lib->impl("rope", op_rope);
+  lib->impl("swiglu", op_swiglu);
+  lib->impl("swiglu_bwd", op_swiglu_bwd);
+  lib->impl("cross_entropy", op_xent);
+  lib->impl("cross_entropy_bwd", op_xent_bwd);
+  lib->impl("embedding", op_embedding);
+  lib->impl("embedding_bwd", op_embedding_bwd);
+  lib->impl("moe_slots", op_moe_slots);
+  lib->impl("moe_scatter", op_moe_scatter);
+  lib->impl("moe_gather", op_moe_gather);
+  lib->impl("moe_gate_grad", op_moe_gate_grad);
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  m.def("register_native", &register_native);
+  m.def("native_launches", []() { return native().launches.load(std::memory_order_relaxed); });
+  m.def("native_shadows", [](bool on) { native().shadows.store(on, std::memory_order_relaxed); });
   m.def("dma_flag_bytes", []() { return (int64_t)apb_dma_flag_bytes(); });
   m.def("dma_ring_max", []() { return (int64_t)apb_dma_ring_max(); });
   m.def("dma_barrier", &dma_barrier);

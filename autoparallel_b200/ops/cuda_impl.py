@@ -28,7 +28,7 @@ from . import shadow
 _C = None
 _lock = threading.Lock()
 _status: dict[int, torch.Tensor] = {}
-launch_count = 0  # kernels of this extension launched since import (bench bookkeeping)
+_launches = 0  # kernels of this extension launched from Python; ``launch_count`` adds those of the native entries
 #: calls answered by a library kernel instead of this extension's, by kind
 library_fallbacks: dict[str, int] = {}
 _DIAG_LIBRARY_GEMM = os.environ.get("APB200_DIAG_LIBRARY_GEMM") == "1"
@@ -57,6 +57,12 @@ STATUS_NAMES = {
 }
 
 
+def __getattr__(name):
+    if name == "launch_count":  # kernels of this extension launched since import (bench bookkeeping)
+        return _launches + (_C.native_launches() if _C is not None else 0)
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
+
+
 def extension():
     return _C
 
@@ -77,8 +83,12 @@ def ensure_loaded() -> None:
                     "(or __graft_entry__.build())"
                 )
             build.build()
-        _C = importlib.import_module("autoparallel_b200.ops._C")
+        ext = importlib.import_module("autoparallel_b200.ops._C")
+        _C = ext
         _register()
+        # from here on calls reach the native entries (csrc/binding.cpp), which come back here for what they do not take
+        ext.register_native({**L._cuda_table, "status_buffer": status_buffer}, _DIAG_LIBRARY_GEMM, _MOE_KERNELS)
+        shadow.on_change(ext.native_shadows)
 
 
 def status_buffer(device) -> torch.Tensor:
@@ -102,8 +112,8 @@ def check_status(device=None) -> None:
 
 
 def _count(n: int = 1) -> None:
-    global launch_count
-    launch_count += n
+    global _launches
+    _launches += n
 
 
 def _dense(t: torch.Tensor) -> torch.Tensor:

@@ -17,10 +17,20 @@ import torch
 #: reference to the shard: while it is alive nothing else can own that address)
 _shadows: dict[int, tuple] = {}
 hits = 0  # casts answered from a shadow (for tests and launch accounting)
+_listener = None  # told whether there may be shadows
+
+
+def on_change(fn) -> None:
+    """``fn(bool)``: called now and whenever the first shadow appears or all are dropped (the native cast asks here only while some exist)."""
+    global _listener
+    _listener = fn
+    fn(bool(_shadows))
 
 
 def publish(param_local: torch.Tensor, shadow: torch.Tensor) -> None:
     """Called by the optimizer after it has written ``shadow`` = ``param_local`` in low precision."""
+    if not _shadows and _listener is not None:
+        _listener(True)
     _shadows[param_local.data_ptr()] = (shadow, param_local._version, weakref.ref(param_local))
 
 
@@ -43,3 +53,5 @@ def lookup(x: torch.Tensor, dtype: torch.dtype):
 
 def clear() -> None:
     _shadows.clear()
+    if _listener is not None:
+        _listener(False)

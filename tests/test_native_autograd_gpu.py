@@ -162,3 +162,86 @@ def test_modes_below_autograd_still_see_the_operators(ops):
         y = ops.rms_norm(x, w, 1e-5)[0]
         y.backward(torch.ones_like(y))
     assert "apb200.rms_norm.default" in seen and "apb200.rms_norm_bwd.default" in seen
+
+
+def _entry_cases():
+    r = lambda *s, dt=torch.bfloat16: torch.randn(*s, device="cuda").to(dt)
+    f32, bf, f16 = torch.float32, torch.bfloat16, torch.float16
+    idx = torch.randint(0, 6, (24, 2), device="cuda")
+    slot = torch.randperm(48, device="cuda").clamp_(max=6 * 5).view(24, 2)  # every row once, the other assignments dropped
+    return [
+        ("mm_nd", (r(2, 5, 64), r(48, 64), True, bf)),
+        ("mm_nd", (r(2, 5, 64)[:, ::2], r(64, 48), False, f32)),
+        ("mm_nd", (r(4, 64), r(48, 64), True, f16)),             # a result type of the library's
+        ("mm_nd", (r(4, 60, dt=f32), r(7, 60, dt=f32), True, f32)),  # operands of the library's
+        ("mm_nd", (r(4, 64), r(50, 64), True, bf)),              # a width that is no whole vector
+        ("mm_wgrad", (r(3, 8, 64), r(3, 8, 40), f32)),
+        ("mm_wgrad", (r(24, 62), r(24, 40), bf)),
+        ("grouped_mm", (r(3, 9, 64), r(3, 64, 40), False, bf)),
+        ("grouped_mm", (r(3, 9, 64), r(3, 42, 64), True, bf)),
+        ("grouped_mm_wgrad", (r(3, 9, 64), r(3, 9, 40).transpose(1, 2).contiguous().transpose(1, 2), f32)),
+        ("grouped_mm_wgrad", (r(3, 9, 63), r(3, 9, 40), f32)),
+        ("dtype_cast", (r(7, 16, dt=f32), bf)),
+        ("dtype_cast", (r(7, 16, dt=f32)[:, 1:], bf)),
+        ("dtype_cast", (r(7, 16), f32)),
+        ("dtype_cast", (r(7, 16), f16)),
+        ("dtype_cast", (torch.arange(9, device="cuda"), f32)),
+        ("rms_norm", (r(2, 3, 64)[:, :2], r(64, dt=f32), 1e-5)),
+        ("rms_norm_bwd", (r(6, 64), r(6, 64), r(64, dt=f32), r(6, dt=f32).abs())),
+        ("rope", (r(2, 6, 4, 32), r(6, 16), r(6, 16), True)),
+        ("swiglu", (r(6, 64).t().contiguous().t(), r(6, 64))),
+        ("swiglu_bwd", (r(6, 64), r(6, 64).t().contiguous().t(), r(6, 64))),
+        ("cross_entropy", (r(2, 5, 64)[:, 1:], torch.randint(0, 64, (2, 4), device="cuda"))),
+        ("cross_entropy_bwd", (r(2, 4), r(2, 4, 64), torch.randint(0, 64, (2, 4), device="cuda"), r(2, 4, dt=f32))),
+        ("embedding", (r(9, 64), torch.randint(0, 9, (2, 4), device="cuda"))),
+        ("embedding", (r(9, 63), torch.randint(0, 9, (2, 4), device="cuda"))),
+        ("embedding_bwd", (r(2, 4, 64, dt=f32), torch.randint(0, 9, (2, 4), device="cuda"), 9)),
+        ("moe_slots", (idx, 6, 5, 2)),
+        ("moe_slots", (idx, 9000, 5, 2)),                        # more experts than the kernel counts
+        ("moe_scatter", (r(24, 16), slot, r(24, 2, dt=f32), 6, 5, 1)),
+        ("moe_scatter", (r(24, 16, dt=f16), slot, r(24, 2, dt=f16), 6, 5, 1)),
+        ("moe_gather", (r(6, 1, 5, 16), slot, r(24, 2, dt=f16))),
+        ("moe_gather", (r(6, 1, 5, 16, dt=f16), slot, r(24, 2, dt=f16))),
+        ("moe_gate_grad", (r(6, 1, 5, 16), slot, r(24, 16))),
+        ("moe_gate_grad", (r(6, 1, 5, 16), slot, r(24, 16, dt=f32))),
+    ]
+
+
+def test_native_entries_answer_as_the_python_ones():
+    """Every form: the same values, launches and library calls as the function of ops/cuda_impl.py that the entry stands for."""
+    from autoparallel_b200.ops import cuda_impl, library, moe_ops  # noqa: F401
+
+    cuda_impl.ensure_loaded()
+    torch.manual_seed(0)
+    for name, args in _entry_cases():
+        results = []
+        for fn in (getattr(library.ops, name), library._cuda_table[name]):
+            launches, calls = cuda_impl.launch_count, dict(cuda_impl.library_fallbacks)
+            out = fn(*args)
+            out = out if isinstance(out, tuple) else (out,)
+            library_calls = {k: v - calls.get(k, 0) for k, v in cuda_impl.library_fallbacks.items() if v != calls.get(k, 0)}
+            results.append((out, cuda_impl.launch_count - launches, library_calls))
+        (a, la, fa), (b, lb, fb) = results
+        assert la == lb and fa == fb, name
+        for x, y in zip(a, b, strict=True):
+            assert x.dtype == y.dtype and x.shape == y.shape and x.stride() == y.stride(), name
+            if name == "embedding_bwd":  # (atomics in this form)
+                assert torch.allclose(x, y, atol=1e-5), name
+            else:
+                assert torch.equal(x, y), name
+
+
+def test_native_cast_hands_out_the_optimizers_copy():
+    from autoparallel_b200.ops import library, shadow
+
+    p, copy = torch.randn(8, 16, device="cuda"), torch.zeros(8, 16, device="cuda", dtype=torch.bfloat16)
+    shadow.clear()
+    assert torch.equal(library.ops.dtype_cast(p, torch.bfloat16), p.bfloat16())
+    shadow.publish(p, copy)
+    try:
+        assert library.ops.dtype_cast(p, torch.bfloat16).data_ptr() == copy.data_ptr()
+        p.mul_(2)  # no longer what was copied
+        assert torch.equal(library.ops.dtype_cast(p, torch.bfloat16), p.bfloat16())
+    finally:
+        shadow.clear()
+    assert torch.equal(library.ops.dtype_cast(p, torch.bfloat16), p.bfloat16())
