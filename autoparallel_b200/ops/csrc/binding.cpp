@@ -58,7 +58,7 @@ int apb_moe_slots(const long long* gate_idx, long long* slot, int* counts, int n
 int apb_moe_scatter(const void* src, const long long* slot, const void* w, int w_bf16, long long* inv, void* buf, long long T, int k, int d,
                     int E, int C, int nb, int is_bf16, cudaStream_t st);
 int apb_moe_gather(const void* buf, const long long* slot, const void* w, int w_bf16, void* out, long long T, int k, int d, int E, int C,
-                   int nb, int is_bf16, cudaStream_t st);
+                   int nb, int is_bf16, int num_sms, cudaStream_t st);
 int apb_moe_gate_grad(const void* buf, const long long* slot, const void* g, float* dw, long long T, int k, int d, int E, int C, int nb,
                       int is_bf16, cudaStream_t st);
 int apb_symm_header_bytes();
@@ -321,7 +321,7 @@ void moe_gather(const at::Tensor& buf, const at::Tensor& slot, const at::Tensor&
               "moe_gather: buf [E, nb, C, d], slot [T, k] int64, out [T, d] of buf's dtype");
   check(apb_moe_gather(buf.data_ptr(), (const long long*)slot.data_ptr<int64_t>(), w.data_ptr(), gate_is_bf16(w, slot, "moe_gather"),
                        out.data_ptr(), slot.size(0), (int)slot.size(1), (int)buf.size(3), (int)buf.size(0), (int)buf.size(2),
-                       (int)buf.size(1), is_bf16(buf), stream()),
+                       (int)buf.size(1), is_bf16(buf), num_sms(), stream()),
         "apb_moe_gather");
 }
 

@@ -124,6 +124,16 @@ def test_moe_dispatch_over_shapes(K, T, k, E, C, nb, d, dtype, wdtype):
     assert impl.library_fallbacks == before, "the kernels cover these shapes"
 
 
+@pytest.mark.parametrize("T,k,E,C,nb,d", [
+    (96, 40, 64, 50, 1, 264),   # more choices than lanes, a second piece of a row that is not full
+    (9600, 2, 8, 2600, 1, 520),  # one warp takes all columns of its token
+    (3, 1, 4, 1, 1, 8),         # fewer tokens than warps of a block
+])
+@pytest.mark.parametrize("dtype,wdtype", [(torch.bfloat16, torch.bfloat16), (torch.float32, torch.float32)])
+def test_moe_gather_over_warps_and_choices(K, T, k, E, C, nb, d, dtype, wdtype):
+    test_moe_dispatch_over_shapes(K, T, k, E, C, nb, d, dtype, wdtype)
+
+
 @pytest.mark.parametrize("T,k,nb,launches", [(16, 2, 1, 1), (510, 1, 1, 1), (513, 1, 1, 1), (512, 2, 1, 1), (4096, 2, 8, 1), (513, 2, 1, 2), (2050, 2, 2, 2)])
 @pytest.mark.parametrize("E", [8, 372, 700])
 def test_moe_slots_around_one_and_two_rounds(K, T, k, nb, launches, E):
