@@ -422,6 +422,8 @@ def test_pairs_with_less_than_two_full_row_tiles(K, M, ta):
     (0, 4361, 1800, 72),   # pairs: groups of 16 tile rows and one of 2, a last tile row of 9 rows, a last column tile of 8 columns
     (0, 100, 40000, 72),   # one CTA per tile, more tiles than SMs
     (3, 2600, 1032, 40),   # grouped: several groups per CTA pair, one k-block that is not full
+    (0, 5000, 5128, 6552),  # rounds larger than L2: contractions in turn forwards and backwards, a last k-block that is not full
+    (0, 128, 39000, 26000),  # the same with one CTA per tile
     (70, 160, 520, 1288),  # grouped, an odd CTA with 32 rows
 ])
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (True, True)])
