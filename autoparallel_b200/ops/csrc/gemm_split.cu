@@ -293,13 +293,18 @@ static SplitKernel split_kernel_of(int bn, int a_mn, int b_mn) {
 
 // Tile width and slice count for a product, or bn = 0 where the persistent kernels are expected to be faster.
 //
-// Only forms whose clusters are all resident at once: in a second wave every tile pays its fixed part again.  The estimates
-// (microseconds, one B200) are fitted to sweeps: a fixed part that grows with the tile (launch, prologue, TMEM -> shared memory -> C),
-// then the longest of a chain of k-blocks, the operand traffic out of L2 (9.5 TB/s) and the operands out of memory (6.5 TB/s, less while
-// few bytes are in flight), then the cluster's sum.  They are good to ten per cent or so; where the sweeps showed them to flatter the
-// split, it is left out: forms with no more CTAs than the persistent kernels would use (twice as many where the contraction has
-// one or two blocks), slices of a single block, whole contractions in 256-wide tiles, and in 64-wide ones on most of the chip.
-// Of 260 random products that it splits, 3 were more than 2 % slower for it (contractions of 8, up to 0.6 us); the mean gain is 1.6.
+// Only forms whose clusters are all resident at once: in a second wave every tile pays its fixed part again.  The estimates (microseconds, one
+// B200) are fitted to a sweep of 1221 products with every form that fits, 1 <= M <= 4096, 64 <= N, K <= 8192, all layouts: a fixed part
+// (launch, prologue, the way out of TMEM), then the longest of a chain of k-blocks, the operand traffic out of L2 (15 TB/s) and the operands
+// out of memory (8.6 TB/s, less while few bytes are in flight), a round trip more where the chain is longer than the stages, then what
+// comes through the other CTAs' shared memory (19 GB/s and CTA).  They are good to 13 per cent; the form they pick takes 1.4 % more than
+// the best one in the geometric mean (the estimates of the kernels before: 5.4 %), and 28 of the 1221 products are more than 3 % slower than
+// by those (by 0.2 to 0.6 us but for three).  Left out, because the sweeps showed the estimates to flatter them: forms with no more CTAs
+// than the persistent kernels would use (twice as many where the contraction has one or two blocks), slices of a single block, whole
+// contractions in 256-wide tiles, and in 64-wide ones on most of the chip.
+//
+// Contractions of up to 16 blocks (K <= 1024) keep the estimates fitted to the kernels as they were: the new ones would give them fewer
+// slices, that is longer chains of fp32 sums, for 0.1 to 0.4 us each, and the loss of a small decoder came out further from 64 bits.
 struct SplitPlan {
   int bn, s;
 };
@@ -347,12 +352,16 @@ static SplitPlan split_plan(int G, int M, int N, int K, int num_sms, int reserve
   const long long tiles = g * (pair ? (M + 2 * BM - 1) / (2 * BM) : m_tiles) * ((N + BN - 1) / BN);
   int units = pair ? apb_gemm_resident_pairs(num_sms) - reserved / 2 : usable;  // as the launches have it
   if (units < 1) units = 1;
-  const double now = 5.5 + (double)((tiles + units - 1) / units) * (0.5 + (pair ? 0.38 : 0.35) * kb);
+  const bool brief = kb <= 16;
+  const double waves = (double)((tiles + units - 1) / units);
+  const double now = brief ? 5.5 + waves * (0.5 + (pair ? 0.38 : 0.35) * kb)
+                           : pair ? 3.35 + waves * (0.49 + 0.45 * kb) : 3.2 + waves * (0.87 + 0.33 * kb);
   const long long ctas = (tiles < units ? tiles : units) * (pair ? 2 : 1) * (kb <= 2 ? 2 : 1);
   const double operands = 2.0 * g * ((double)M * K + (double)N * K);
-  double t_best = 0.95 * now;  // (a clear gain only)
+  double t_best = brief ? 0.95 * now : now;
   for (int bn = 64; bn <= 256; bn *= 2) {
-    const double fixed = bn == 64 ? 5.6 : bn == 128 ? 7.0 : 9.0, per_kb = bn == 128 ? 0.20 : 0.27;
+    const double per_kb = brief ? (bn == 128 ? 0.20 : 0.27) : bn == 64 ? 0.23 : bn == 128 ? 0.26 : 0.39;
+    const int stages = SPLIT_STAGE_TOTAL / (A_STAGE_BYTES + bn * BK * 2);
     const long long t = g * m_tiles * ((N + bn - 1) / bn);
     const double kb_bytes = 128.0 * ((M < BM ? M : BM) + (N < bn ? N : bn));
     for (int s = 1; s <= SPLIT_MAX && s <= kb; ++s) {
@@ -361,13 +370,24 @@ static SplitPlan split_plan(int G, int M, int N, int K, int num_sms, int reserve
       if (s > 1 ? kb < 2 * s : bn == 256 || (bn == 64 && t > 100)) continue;
       const int chain = (kb + s - 1) / s;
       double flow = per_kb * chain;
-      const double l2 = (double)t * kb * kb_bytes / 9.5e6;
+      const double l2 = (double)t * kb * kb_bytes / (brief ? 9.5e6 : 14.7e6);
       if (l2 > flow) flow = l2;
       // megabytes in flight: the stages of all CTAs, rows and columns outside the matrices not counted
       const double flight = 0.1875 * t * s * kb_bytes / (128.0 * (BM + bn));
-      const double from_memory = operands / (flight < 10.5 ? 0.62e6 * flight : 6.5e6);
+      const double most = brief ? 6.5e6 : 8.6e6, grows = (brief ? 0.62e6 : 0.684e6) * flight;
+      const double from_memory = operands / (grows < most ? grows : most);
       if (from_memory > flow) flow = from_memory;
-      const double est = fixed + flow + (s > 1 ? 0.05 * s * bn / 64 : 0.0);
+      if (brief) {
+        const double est = (bn == 64 ? 5.6 : bn == 128 ? 7.0 : 9.0) + flow + (s > 1 ? 0.05 * s * bn / 64 : 0.0);
+        if (est < t_best) {
+          t_best = est;
+          best = SplitPlan{bn, s};
+        }
+        continue;
+      }
+      const double fixed = s > 1 ? (bn == 256 ? 3.8 : 4.1) : (bn == 64 ? 3.5 : 4.0);
+      const double shared = s > 1 ? 4.0 * (M < BM ? M : BM) * (N < bn ? N : bn) * (s - 1) / s / 18.7e3 + 0.034 * s : 0.0;
+      const double est = fixed + flow + (chain > stages ? 0.31 : 0.0) + shared;
       if (est < t_best) {
         t_best = est;
         best = SplitPlan{bn, s};
