@@ -113,8 +113,6 @@ __device__ __forceinline__ void tile_coords(int t, int num_m, int num_n, int& tm
   tn = r / gsz;
 }
 
-// The same order for the plain GEMM, tile ``t`` of all groups: every warp of the epilogue walks it, and three integer divisions with their
-// remainders are several hundred cycles of a tile.
 // Rounds of tiles (``units`` at a time) that read more than L2 holds go through the contraction in turn forwards and backwards, so that a
 // round begins with what the one before read last - mostly the same rows of A.  Memory traffic is power, and at the power cap power is
 // time (sustained, us, always forwards -> in turn): 14336 x 4096 x 8192 800 -> 755, 8192 x 8192 x 8192 867 -> 841, 8192 x 4096 x 14336
@@ -129,6 +127,8 @@ inline void set_tile_order(GemmParams& p, int num_m, int tile_m, int units) {
   p.div_tiles = FastDiv((uint32_t)num_m * p.num_n_tiles);
   p.div_tail = FastDiv(num_m % GROUP_M ? num_m % GROUP_M : GROUP_M);
 }
+// The order of tile_coords for the plain GEMM, tile ``t`` of all groups: every warp of the epilogue walks it, and three integer divisions with their
+// remainders are several hundred cycles of a tile.
 __device__ __forceinline__ void plain_tile(const GemmParams& p, int num_m, bool grouped, int t, int& grp, int& tm, int& tn) {
   grp = grouped ? p.div_tiles.div(t) : 0;
   if (grouped) t -= grp * (int)p.div_tiles.d;
