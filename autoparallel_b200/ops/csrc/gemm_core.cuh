@@ -82,7 +82,6 @@ struct GemmParams {
   int* tile_counter = nullptr;
   // plain GEMM: divisors of the tile order, see plain_tile
   FastDiv div_group, div_tiles, div_tail;
-  int alternate = 0;  // odd rounds of tiles run through the contraction backwards
   int vec_store = 0;  // C leaves through shared memory in whole 128-byte lines (plain GEMM; needs 16-byte rows)
 };
 
@@ -113,22 +112,17 @@ __device__ __forceinline__ void tile_coords(int t, int num_m, int num_n, int& tm
   tn = r / gsz;
 }
 
-// Rounds of tiles (``units`` at a time) that read more than L2 holds go through the contraction in turn forwards and backwards, so that a
-// round begins with what the one before read last - mostly the same rows of A.  Memory traffic is power, and at the power cap power is
-// time (sustained, us, always forwards -> in turn): 14336 x 4096 x 8192 800 -> 755, 8192 x 8192 x 8192 867 -> 841, 8192 x 4096 x 14336
-// 757 -> 747, 8192 x 4096 x 128256 7513 -> 7414.  Rounds that fit gain nothing or lose (8192 x 128256 x 4096, 43 MB a round: 6446 -> 6625).
-// The order depends on the tile alone: the same product gives the same bits at every launch.
-constexpr long long ROUND_BYTES_IN_L2 = 64ll << 20;
-inline void set_tile_order(GemmParams& p, int num_m, int tile_m, int units) {
-  const long long rows = num_m < GROUP_M ? num_m : GROUP_M, cols = (units + rows - 1) / rows;
-  const long long round = (rows * tile_m + (cols < p.num_n_tiles ? cols : p.num_n_tiles) * BN) * 2ll * p.K;
-  p.alternate = round > ROUND_BYTES_IN_L2 && (long long)num_m * p.num_n_tiles > units;
+// The order of tile_coords for the plain GEMM, tile ``t`` of all groups: every warp of the epilogue walks it, and three integer divisions with their
+// remainders are several hundred cycles of a tile.
+//
+// Every tile goes through the contraction forwards, so that its bits depend neither on the launch (reserved SMs, pairs that are resident, tiles
+// handed out at run time) nor on where the tile lies: equal rows give equal results.  Backwards in every other round, for what L2 still holds
+// of the round before, saves power and with it time in rounds of more than 64 MB (8B feed-forward block 3 %), and gives that up.
+inline void set_tile_order(GemmParams& p, int num_m) {
   p.div_group = FastDiv((uint32_t)GROUP_M * p.num_n_tiles);
   p.div_tiles = FastDiv((uint32_t)num_m * p.num_n_tiles);
   p.div_tail = FastDiv(num_m % GROUP_M ? num_m % GROUP_M : GROUP_M);
 }
-// The order of tile_coords for the plain GEMM, tile ``t`` of all groups: every warp of the epilogue walks it, and three integer divisions with their
-// remainders are several hundred cycles of a tile.
 __device__ __forceinline__ void plain_tile(const GemmParams& p, int num_m, bool grouped, int t, int& grp, int& tm, int& tn) {
   grp = grouped ? p.div_tiles.div(t) : 0;
   if (grouped) t -= grp * (int)p.div_tiles.d;
@@ -592,9 +586,8 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
             break;
           }
         }
-        const bool backwards = FUSE == FUSE_NONE && p.alternate && ((DYN ? t / num_units : tile_it - 1) & 1);
         for (int kb0 = 0; kb0 < num_kb; ++kb0) {
-          const int kb = FUSE == FUSE_NONE ? (backwards ? num_kb - 1 - kb0 : kb0) : (kb0 + k_rot) % num_kb;
+          const int kb = FUSE == FUSE_NONE ? kb0 : (kb0 + k_rot) % num_kb;
           if ((FUSE == FUSE_GATHER_B && B_MN) || (FUSE == FUSE_GATHER_A && A_MN)) {
             const int r0 = kb * BK;
             const int s0 = r0 / f.rows_per_shard, s1 = (min(r0 + BK, p.K) - 1) / f.rows_per_shard;

@@ -183,7 +183,7 @@ extern "C" int apb_gemm_bf16(const void* A, const void* B, void* C, int M, int N
     int resident = apb_gemm_resident_pairs(num_sms) - g_reserved_sms / 2;
     if (resident < 1) resident = 1;
     const int pairs = tiles2 < resident ? tiles2 : resident;
-    set_tile_order(p, (M + 2 * BM - 1) / (2 * BM), 2 * BM, pairs);
+    set_tile_order(p, (M + 2 * BM - 1) / (2 * BM));
     const int smem2 = apb_gemm_pair_smem_bytes(g_pair_stages);
     const int threads2 = g_pair_stages == PAIR_STAGES ? GEMM_PLAIN_THREADS : GEMM_THREADS;
     auto launch2 = [&](auto kern) {
@@ -211,7 +211,7 @@ extern "C" int apb_gemm_bf16(const void* A, const void* B, void* C, int M, int N
   }
   const int tiles = p.num_m_tiles * p.num_n_tiles;
   const int grid = tiles < usable ? tiles : usable;
-  set_tile_order(p, p.num_m_tiles, BM, grid);
+  set_tile_order(p, p.num_m_tiles);
   auto launch = [&](auto kern) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_PLAIN_SMEM_BYTES);
     kern<<<grid, GEMM_PLAIN_THREADS, GEMM_PLAIN_SMEM_BYTES, stream>>>(tmA, tmB, p);
@@ -261,7 +261,7 @@ extern "C" int apb_gemm_grouped_bf16(const void* A, const void* B, void* C, int 
     int resident = apb_gemm_resident_pairs(num_sms) - g_reserved_sms / 2;
     if (resident < 1) resident = 1;
     const int grid = 2 * (int)(tiles2 < resident ? tiles2 : resident);
-    set_tile_order(p, (M + 2 * BM - 1) / (2 * BM), 2 * BM, grid / 2);
+    set_tile_order(p, (M + 2 * BM - 1) / (2 * BM));
     if (!a_mn_major && !b_mn_major) launch(gemm_grouped_pair_kernel<false, false>, grid);
     else if (!a_mn_major && b_mn_major) launch(gemm_grouped_pair_kernel<false, true>, grid);
     else if (a_mn_major && !b_mn_major) launch(gemm_grouped_pair_kernel<true, false>, grid);
@@ -269,7 +269,7 @@ extern "C" int apb_gemm_grouped_bf16(const void* A, const void* B, void* C, int 
   } else {
     const long long tiles = (long long)G * p.num_m_tiles * p.num_n_tiles;
     const int grid = (int)(tiles < usable ? tiles : usable);
-    set_tile_order(p, p.num_m_tiles, BM, grid);
+    set_tile_order(p, p.num_m_tiles);
     if (!a_mn_major && !b_mn_major) launch(gemm_grouped_kernel<false, false>, grid);
     else if (!a_mn_major && b_mn_major) launch(gemm_grouped_kernel<false, true>, grid);
     else if (a_mn_major && !b_mn_major) launch(gemm_grouped_kernel<true, false>, grid);

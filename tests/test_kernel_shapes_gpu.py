@@ -422,7 +422,7 @@ def test_pairs_with_less_than_two_full_row_tiles(K, M, ta):
     (0, 4361, 1800, 72),   # pairs: groups of 16 tile rows and one of 2, a last tile row of 9 rows, a last column tile of 8 columns
     (0, 100, 40000, 72),   # one CTA per tile, more tiles than SMs
     (3, 2600, 1032, 40),   # grouped: several groups per CTA pair, one k-block that is not full
-    (0, 5000, 5128, 6552),  # rounds larger than L2: contractions in turn forwards and backwards, a last k-block that is not full
+    (0, 5000, 5128, 6552),  # a long contraction, rounds of tiles that read 70 MB, a last k-block that is not full
     (0, 128, 39000, 26000),  # the same with one CTA per tile
     (70, 160, 520, 1288),  # grouped, an odd CTA with 32 rows
 ])
@@ -453,3 +453,32 @@ def test_gemm_tiles_land_where_they_belong(K, G, M, N, Kd, a_mn, b_mn, out):
         assert torch.equal(c, ref)
         c.fill_(99.0)
         assert bool((wide == 99.0).all())
+
+
+@pytest.mark.parametrize("pair", [True, False])
+def test_gemm_bits_do_not_depend_on_the_launch(K, pair):
+    """Products whose rounds of tiles read more than L2 holds: equal rows and columns of the operands give equal results wherever they lie,
+    and reserved SMs or tiles handed out at run time change no bit."""
+    _, impl = K
+    ext = impl.extension()
+    M, N, K_, rows, cols = 5120, 5120, 8192, 512, 512
+    g = torch.Generator(device="cuda").manual_seed(1)
+    a = torch.randn(rows, K_, device="cuda", generator=g).to(torch.bfloat16).repeat(M // rows, 1)
+    b = torch.randn(cols, K_, device="cuda", generator=g).to(torch.bfloat16).repeat(N // cols, 1)
+    prev = ext.gemm_get_pair_mode(), ext.gemm_get_reserved_sms(), ext.gemm_get_dynamic_tiles()
+    ext.gemm_set_pair_mode(pair)
+    try:
+        first = None
+        for reserved, dynamic in ((0, False), (16, False), (50, False), (0, True), (16, True)):
+            ext.gemm_set_reserved_sms(reserved)
+            ext.gemm_set_dynamic_tiles(dynamic)
+            c = torch.empty(M, N, device="cuda")
+            ext.gemm(a, b, c, False, False, impl.status_buffer(c.device))
+            blocks = c.view(M // rows, rows, N // cols, cols)
+            assert torch.equal(blocks, blocks[:1, :, :1].expand_as(blocks)), (reserved, dynamic)
+            first = c if first is None else first
+            assert torch.equal(c, first), (reserved, dynamic)
+    finally:
+        ext.gemm_set_pair_mode(prev[0])
+        ext.gemm_set_reserved_sms(prev[1])
+        ext.gemm_set_dynamic_tiles(prev[2])
