@@ -9,6 +9,7 @@
 #include <atomic>
 #include <cstdint>
 #include <mutex>
+#include <string>
 
 extern "C" {
 int apb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc,
@@ -525,10 +526,19 @@ void dma_rs_sum(const at::Tensor& src, at::Tensor& dst, const std::vector<int64_
 // ------------------------------------------------------------------ the operators' CUDA entries
 // Registered over the Python entries once the extension is loaded, so that an operator call - from a graph, from the autograd engine's
 // threads - runs no Python on its way to the kernel: 6 to 9 us of host time per call, and the interpreter's lock.  Every function takes the
-// forms that its counterpart in ops/cuda_impl.py gives to this extension, under the same conditions; all others, and what the flags there
-// ask for, go to that Python function.
+// forms that its counterpart in ops/cuda_impl.py gives to this extension, under the same conditions; all others, what the flags there
+// ask for, and every call of an operator for which register_cuda_impl has installed another function go to the table of ops/library.py.
+enum Entry : int {
+  MM_ND, MM_WGRAD, GROUPED_MM, GROUPED_MM_WGRAD, DTYPE_CAST, RMS_NORM, RMS_NORM_BWD, ROPE, SWIGLU, SWIGLU_BWD, CROSS_ENTROPY, CROSS_ENTROPY_BWD,
+  EMBEDDING, EMBEDDING_BWD, MOE_SLOTS, MOE_SCATTER, MOE_GATHER, MOE_GATE_GRAD, NUM_ENTRIES
+};
+constexpr const char* ENTRY_NAMES[NUM_ENTRIES] = {
+    "mm_nd", "mm_wgrad", "grouped_mm", "grouped_mm_wgrad", "dtype_cast", "rms_norm", "rms_norm_bwd", "rope", "swiglu", "swiglu_bwd", "cross_entropy",
+    "cross_entropy_bwd", "embedding", "embedding_bwd", "moe_slots", "moe_scatter", "moe_gather", "moe_gate_grad"};
 struct Native {
-  py::object table;  // operator name -> function of ops/cuda_impl.py
+  py::object table;  // operator name -> Python function, as it is at the time of a call
+  py::object status_buffer;
+  std::atomic<uint32_t> installed{0};  // bit per entry: the table's function is not the one of ops/cuda_impl.py
   bool diag_library_gemm = false, moe_kernels = true;
   std::atomic<bool> shadows{false};  // low-precision copies of parameters may exist: casts ask Python for them
   std::atomic<int64_t> launches{0};
@@ -538,10 +548,12 @@ Native& native() {
   return *n;
 }
 
+bool ours(Entry e) { return (native().installed.load(std::memory_order_relaxed) >> e & 1u) == 0; }
+
 template <typename R, typename... A>
-R in_python(const char* op, const A&... args) {
+R in_python(Entry e, const A&... args) {
   py::gil_scoped_acquire gil;
-  return py::cast<R>(native().table[op](args...));
+  return py::cast<R>(native().table[ENTRY_NAMES[e]](args...));
 }
 py::object py_dtype(at::ScalarType t) { return py::reinterpret_borrow<py::object>(reinterpret_cast<PyObject*>(torch::getTHPDtype(t))); }
 
@@ -553,7 +565,10 @@ at::Tensor& status_of(const at::Tensor& t) {
   const int dev = t.get_device();
   TORCH_CHECK(dev >= 0 && dev < 64, "unexpected device index ", dev);
   if (!known[dev].load(std::memory_order_acquire)) {
-    at::Tensor w = in_python<at::Tensor>("status_buffer", t.device());
+    at::Tensor w = [&]() {
+      py::gil_scoped_acquire gil;
+      return py::cast<at::Tensor>(native().status_buffer(t.device()));
+    }();
     std::lock_guard<std::mutex> g(m);
     if (!known[dev].load(std::memory_order_relaxed)) {
       words[dev] = w;
@@ -569,7 +584,7 @@ using at::Tensor;
 using Two = std::tuple<Tensor, Tensor>;
 
 Tensor op_mm_nd(const Tensor& a, const Tensor& b, bool trans_b, at::ScalarType dtype) {
-  if (float_or_bf16(dtype) && !native().diag_library_gemm) {
+  if (ours(MM_ND) && float_or_bf16(dtype) && !native().diag_library_gemm) {
     auto c = mm_nd(a, b, trans_b, dtype == at::kFloat, status_of(a));
     if (c.has_value()) {
       count();
@@ -577,10 +592,10 @@ Tensor op_mm_nd(const Tensor& a, const Tensor& b, bool trans_b, at::ScalarType d
     }
   }
   py::gil_scoped_acquire gil;
-  return in_python<Tensor>("mm_nd", a, b, trans_b, py_dtype(dtype));
+  return in_python<Tensor>(MM_ND, a, b, trans_b, py_dtype(dtype));
 }
 Tensor op_mm_wgrad(const Tensor& a, const Tensor& b, at::ScalarType dtype) {
-  if (float_or_bf16(dtype) && !native().diag_library_gemm) {
+  if (ours(MM_WGRAD) && float_or_bf16(dtype) && !native().diag_library_gemm) {
     auto c = gemm_new(a, b, true, true, dtype == at::kFloat, status_of(a));
     if (c.has_value()) {
       count();
@@ -588,35 +603,35 @@ Tensor op_mm_wgrad(const Tensor& a, const Tensor& b, at::ScalarType dtype) {
     }
   }
   py::gil_scoped_acquire gil;
-  return in_python<Tensor>("mm_wgrad", a, b, py_dtype(dtype));
+  return in_python<Tensor>(MM_WGRAD, a, b, py_dtype(dtype));
 }
 bool grouped_ok(const Tensor& a, const Tensor& b, at::ScalarType dtype) {
   return a.dim() == 3 && b.dim() == 3 && a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16 && a.size(2) % 8 == 0 &&
          b.size(2) % 8 == 0 && float_or_bf16(dtype);
 }
 Tensor op_grouped_mm(const Tensor& a, const Tensor& b, bool trans_b, at::ScalarType dtype) {
-  if (grouped_ok(a, b, dtype) && b.size(trans_b ? 1 : 2) % 8 == 0) {
+  if (ours(GROUPED_MM) && grouped_ok(a, b, dtype) && b.size(trans_b ? 1 : 2) % 8 == 0) {
     Tensor c = at::empty({a.size(0), a.size(1), b.size(trans_b ? 1 : 2)}, a.options().dtype(dtype));
     gemm_grouped(dense(a), dense(b), c, false, !trans_b, status_of(a));
     count();
     return c;
   }
   py::gil_scoped_acquire gil;
-  return in_python<Tensor>("grouped_mm", a, b, trans_b, py_dtype(dtype));
+  return in_python<Tensor>(GROUPED_MM, a, b, trans_b, py_dtype(dtype));
 }
 Tensor op_grouped_wgrad(const Tensor& a, const Tensor& b, at::ScalarType dtype) {
-  if (grouped_ok(a, b, dtype)) {
+  if (ours(GROUPED_MM_WGRAD) && grouped_ok(a, b, dtype)) {
     Tensor c = at::empty({a.size(0), a.size(2), b.size(2)}, a.options().dtype(dtype));
     gemm_grouped(dense(a), dense(b), c, true, true, status_of(a));
     count();
     return c;
   }
   py::gil_scoped_acquire gil;
-  return in_python<Tensor>("grouped_mm_wgrad", a, b, py_dtype(dtype));
+  return in_python<Tensor>(GROUPED_MM_WGRAD, a, b, py_dtype(dtype));
 }
 Tensor op_cast(const Tensor& x, at::ScalarType dtype) {
-  if (x.scalar_type() == dtype) return x;
-  if (!native().shadows.load(std::memory_order_relaxed) && (dtype == at::kBFloat16 || (dtype == at::kFloat && x.scalar_type() == at::kBFloat16))) {
+  if (x.scalar_type() == dtype && ours(DTYPE_CAST)) return x;
+  if (ours(DTYPE_CAST) && !native().shadows.load(std::memory_order_relaxed) && (dtype == at::kBFloat16 || (dtype == at::kFloat && x.scalar_type() == at::kBFloat16))) {
     auto y = cast_new(x, dtype == at::kBFloat16);
     if (y.has_value()) {
       count();
@@ -624,29 +639,35 @@ Tensor op_cast(const Tensor& x, at::ScalarType dtype) {
     }
   }
   py::gil_scoped_acquire gil;
-  return in_python<Tensor>("dtype_cast", x, py_dtype(dtype));
+  return in_python<Tensor>(DTYPE_CAST, x, py_dtype(dtype));
 }
 Two op_rms_norm(const Tensor& x, const Tensor& w, double eps) {
+  if (!ours(RMS_NORM)) return in_python<Two>(RMS_NORM, x, w, eps);
   count();
   return rms_norm_new(x, w, eps);
 }
 Two op_rms_norm_bwd(const Tensor& dy, const Tensor& x, const Tensor& w, const Tensor& rstd) {
+  if (!ours(RMS_NORM_BWD)) return in_python<Two>(RMS_NORM_BWD, dy, x, w, rstd);
   count(2);
   return rms_norm_bwd_new(dy, x, w, rstd);
 }
 Tensor op_rope(const Tensor& x, const Tensor& cos, const Tensor& sin, bool conj) {
+  if (!ours(ROPE)) return in_python<Tensor>(ROPE, x, cos, sin, conj);
   count();
   return rope_new(x, cos, sin, conj);
 }
 Tensor op_swiglu(const Tensor& a, const Tensor& b) {
+  if (!ours(SWIGLU)) return in_python<Tensor>(SWIGLU, a, b);
   count();
   return swiglu_new(a, b);
 }
 Two op_swiglu_bwd(const Tensor& dy, const Tensor& a, const Tensor& b) {
+  if (!ours(SWIGLU_BWD)) return in_python<Two>(SWIGLU_BWD, dy, a, b);
   count();
   return swiglu_bwd_new(dy, a, b);
 }
 Two op_xent(const Tensor& logits_, const Tensor& labels) {
+  if (!ours(CROSS_ENTROPY)) return in_python<Two>(CROSS_ENTROPY, logits_, labels);
   Tensor logits = dense(logits_);
   const auto shape = logits.sizes().slice(0, logits.dim() - 1);
   Tensor loss = at::empty(shape, logits.options().dtype(at::kFloat)), lse = at::empty(shape, loss.options());
@@ -655,13 +676,14 @@ Two op_xent(const Tensor& logits_, const Tensor& labels) {
   return {loss, lse};
 }
 Tensor op_xent_bwd(const Tensor& dloss, const Tensor& logits_, const Tensor& labels, const Tensor& lse) {
+  if (!ours(CROSS_ENTROPY_BWD)) return in_python<Tensor>(CROSS_ENTROPY_BWD, dloss, logits_, labels, lse);
   Tensor logits = dense(logits_), out = at::empty_like(logits);
   xent_bwd(dloss.to(at::kFloat).contiguous(), logits, labels.contiguous(), lse.contiguous(), out);
   count();
   return out;
 }
 Tensor op_embedding(const Tensor& weight, const Tensor& ids) {
-  if (weight.dim() == 2 && float_or_bf16(weight.scalar_type()) && weight.size(1) * weight.element_size() % 16 == 0 && ids.scalar_type() == at::kLong) {
+  if (ours(EMBEDDING) && weight.dim() == 2 && float_or_bf16(weight.scalar_type()) && weight.size(1) * weight.element_size() % 16 == 0 && ids.scalar_type() == at::kLong) {
     auto shape = ids.sizes().vec();
     shape.push_back(weight.size(1));
     Tensor out = at::empty(shape, weight.options());
@@ -670,9 +692,10 @@ Tensor op_embedding(const Tensor& weight, const Tensor& ids) {
     return out;
   }
   py::gil_scoped_acquire gil;
-  return in_python<Tensor>("embedding", weight, ids);
+  return in_python<Tensor>(EMBEDDING, weight, ids);
 }
 Tensor op_embedding_bwd(const Tensor& dy_, const Tensor& ids, int64_t rows) {
+  if (!ours(EMBEDDING_BWD)) return in_python<Tensor>(EMBEDDING_BWD, dy_, ids, rows);
   Tensor dy = dy_.contiguous(), out = at::empty({rows, dy.size(-1)}, dy.options());
   count(embedding_bwd(dy, ids.contiguous(), out));
   return out;
@@ -686,49 +709,59 @@ bool moe_ok(std::initializer_list<const Tensor*> ts) {
 }
 Tensor gate_weights(const Tensor& w, at::ScalarType dtype) { return (float_or_bf16(w.scalar_type()) ? w : w.to(dtype)).contiguous(); }
 Tensor op_moe_slots(const Tensor& idx, int64_t E, int64_t C, int64_t nb) {
-  if (moe_ok({&idx}) && idx.scalar_type() == at::kLong && idx.dim() == 2 && nb > 0 && idx.size(0) > 0 && idx.size(0) % nb == 0 &&
+  if (ours(MOE_SLOTS) && moe_ok({&idx}) && idx.scalar_type() == at::kLong && idx.dim() == 2 && nb > 0 && idx.size(0) > 0 && idx.size(0) % nb == 0 &&
       E <= moe_slots_max_experts(idx.size(0) / nb * idx.size(1)) && E * C < (int64_t(1) << 31)) {
     Tensor slot = at::empty_like(idx, at::MemoryFormat::Contiguous);
     count(moe_slots(idx.contiguous(), slot, E, C, nb));
     return slot;
   }
-  return in_python<Tensor>("moe_slots", idx, E, C, nb);
+  return in_python<Tensor>(MOE_SLOTS, idx, E, C, nb);
 }
 Tensor op_moe_scatter(const Tensor& src, const Tensor& slot, const Tensor& w, int64_t E, int64_t C, int64_t nb) {
-  if (moe_ok({&src, &slot, &w}) && float_or_bf16(src.scalar_type()) && src.dim() == 2 && nb > 0 && src.size(0) > 0 && src.size(0) % nb == 0) {
+  if (ours(MOE_SCATTER) && moe_ok({&src, &slot, &w}) && float_or_bf16(src.scalar_type()) && src.dim() == 2 && nb > 0 && src.size(0) > 0 && src.size(0) % nb == 0) {
     Tensor buf = at::empty({E, nb, C, src.size(1)}, src.options());
     moe_scatter(src.contiguous(), slot.contiguous(), gate_weights(w, src.scalar_type()), buf, E, C, nb);
     count(2);
     return buf;
   }
-  return in_python<Tensor>("moe_scatter", src, slot, w, E, C, nb);
+  return in_python<Tensor>(MOE_SCATTER, src, slot, w, E, C, nb);
 }
 Tensor op_moe_gather(const Tensor& buf, const Tensor& slot, const Tensor& w) {
-  if (moe_ok({&buf, &slot, &w}) && float_or_bf16(buf.scalar_type()) && buf.dim() == 4 && buf.size(1) > 0 && slot.dim() == 2 && slot.size(0) > 0 &&
+  if (ours(MOE_GATHER) && moe_ok({&buf, &slot, &w}) && float_or_bf16(buf.scalar_type()) && buf.dim() == 4 && buf.size(1) > 0 && slot.dim() == 2 && slot.size(0) > 0 &&
       slot.size(0) % buf.size(1) == 0) {
     Tensor out = at::empty({slot.size(0), buf.size(3)}, buf.options());
     moe_gather(buf.contiguous(), slot.contiguous(), gate_weights(w, buf.scalar_type()), out);
     count();
     return out;
   }
-  return in_python<Tensor>("moe_gather", buf, slot, w);
+  return in_python<Tensor>(MOE_GATHER, buf, slot, w);
 }
 Tensor op_moe_gate_grad(const Tensor& buf, const Tensor& slot, const Tensor& g) {
-  if (moe_ok({&buf, &slot, &g}) && float_or_bf16(buf.scalar_type()) && buf.dim() == 4 && g.scalar_type() == buf.scalar_type() && buf.size(1) > 0 &&
+  if (ours(MOE_GATE_GRAD) && moe_ok({&buf, &slot, &g}) && float_or_bf16(buf.scalar_type()) && buf.dim() == 4 && g.scalar_type() == buf.scalar_type() && buf.size(1) > 0 &&
       slot.dim() == 2 && slot.size(0) > 0 && slot.size(0) % buf.size(1) == 0) {
     Tensor dw = at::empty(slot.sizes(), buf.options().dtype(at::kFloat));
     moe_gate_grad(buf.contiguous(), slot.contiguous(), g.contiguous(), dw);
     count();
     return dw;
   }
-  return in_python<Tensor>("moe_gate_grad", buf, slot, g);
+  return in_python<Tensor>(MOE_GATE_GRAD, buf, slot, g);
+}
+
+// What register_cuda_impl installed for ``name``: ``on`` if it is not the function that the native entry stands for.
+void native_installed(const std::string& name, bool on) {
+  for (int e = 0; e < NUM_ENTRIES; ++e)
+    if (name == ENTRY_NAMES[e]) {
+      if (on) native().installed.fetch_or(1u << e, std::memory_order_relaxed);
+      else native().installed.fetch_and(~(1u << e), std::memory_order_relaxed);
+    }
 }
 
 // Once per process, after the Python functions are known.  The dispatcher warns when a kernel takes another's place, which here is meant.
-void register_native(py::dict table, bool diag_library_gemm, bool moe_kernels) {
+void register_native(py::dict table, py::object status_buffer, bool diag_library_gemm, bool moe_kernels) {
   static torch::Library* lib = nullptr;
   if (lib != nullptr) return;
   native().table = std::move(table);
+  native().status_buffer = std::move(status_buffer);
   native().diag_library_gemm = diag_library_gemm;
   native().moe_kernels = moe_kernels;
   struct Quiet : c10::WarningHandler {
@@ -736,30 +769,31 @@ void register_native(py::dict table, bool diag_library_gemm, bool moe_kernels) {
   } quiet;
   c10::WarningUtils::WarningHandlerGuard guard(&quiet);
   lib = new torch::Library(torch::Library::IMPL, "apb200", c10::DispatchKey::CUDA, __FILE__, __LINE__);
-  lib->impl("mm_nd", op_mm_nd);
-  lib->impl("mm_wgrad", op_mm_wgrad);
-  lib->impl("grouped_mm", op_grouped_mm);
-  lib->impl("grouped_mm_wgrad", op_grouped_wgrad);
-  lib->impl("dtype_cast", op_cast);
-  lib->impl("rms_norm", op_rms_norm);
-  lib->impl("rms_norm_bwd", op_rms_norm_bwd);
-  lib->impl("rope", op_rope);
-  lib->impl("swiglu", op_swiglu);
-  lib->impl("swiglu_bwd", op_swiglu_bwd);
-  lib->impl("cross_entropy", op_xent);
-  lib->impl("cross_entropy_bwd", op_xent_bwd);
-  lib->impl("embedding", op_embedding);
-  lib->impl("embedding_bwd", op_embedding_bwd);
-  lib->impl("moe_slots", op_moe_slots);
-  lib->impl("moe_scatter", op_moe_scatter);
-  lib->impl("moe_gather", op_moe_gather);
-  lib->impl("moe_gate_grad", op_moe_gate_grad);
+  lib->impl(ENTRY_NAMES[MM_ND], op_mm_nd);
+  lib->impl(ENTRY_NAMES[MM_WGRAD], op_mm_wgrad);
+  lib->impl(ENTRY_NAMES[GROUPED_MM], op_grouped_mm);
+  lib->impl(ENTRY_NAMES[GROUPED_MM_WGRAD], op_grouped_wgrad);
+  lib->impl(ENTRY_NAMES[DTYPE_CAST], op_cast);
+  lib->impl(ENTRY_NAMES[RMS_NORM], op_rms_norm);
+  lib->impl(ENTRY_NAMES[RMS_NORM_BWD], op_rms_norm_bwd);
+  lib->impl(ENTRY_NAMES[ROPE], op_rope);
+  lib->impl(ENTRY_NAMES[SWIGLU], op_swiglu);
+  lib->impl(ENTRY_NAMES[SWIGLU_BWD], op_swiglu_bwd);
+  lib->impl(ENTRY_NAMES[CROSS_ENTROPY], op_xent);
+  lib->impl(ENTRY_NAMES[CROSS_ENTROPY_BWD], op_xent_bwd);
+  lib->impl(ENTRY_NAMES[EMBEDDING], op_embedding);
+  lib->impl(ENTRY_NAMES[EMBEDDING_BWD], op_embedding_bwd);
+  lib->impl(ENTRY_NAMES[MOE_SLOTS], op_moe_slots);
+  lib->impl(ENTRY_NAMES[MOE_SCATTER], op_moe_scatter);
+  lib->impl(ENTRY_NAMES[MOE_GATHER], op_moe_gather);
+  lib->impl(ENTRY_NAMES[MOE_GATE_GRAD], op_moe_gate_grad);
 }
 
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("register_native", &register_native);
+  m.def("native_installed", &native_installed);
   m.def("native_launches", []() { return native().launches.load(std::memory_order_relaxed); });
   m.def("native_shadows", [](bool on) { native().shadows.store(on, std::memory_order_relaxed); });
   m.def("dma_flag_bytes", []() { return (int64_t)apb_dma_flag_bytes(); });

@@ -86,8 +86,11 @@ def ensure_loaded() -> None:
         ext = importlib.import_module("autoparallel_b200.ops._C")
         _C = ext
         _register()
-        # from here on calls reach the native entries (csrc/binding.cpp), which come back here for what they do not take
-        ext.register_native({**L._cuda_table, "status_buffer": status_buffer}, _DIAG_LIBRARY_GEMM, _MOE_KERNELS)
+        # from here on calls reach the native entries (csrc/binding.cpp), which come back to the table for what they do not take and
+        # for operators that get another function
+        own = dict(L._cuda_table)
+        L.on_install(lambda name, fn: ext.native_installed(name, fn is not own.get(name)))
+        ext.register_native(L._cuda_table, status_buffer, _DIAG_LIBRARY_GEMM, _MOE_KERNELS)
         shadow.on_change(ext.native_shadows)
 
 

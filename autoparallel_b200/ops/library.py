@@ -278,9 +278,20 @@ for _name in _CPU_IMPLS:
     lib.impl(_name, _make_cuda_entry(_name), "CUDA")
 
 
+_on_install = None  # told of every function that is installed once the extension is loaded
+
+
+def on_install(fn) -> None:
+    """``fn(name, wrapper)``: called whenever a wrapper is installed (the native entries then hand that operator's calls to it)."""
+    global _on_install
+    _on_install = fn
+
+
 def register_cuda_impl(name: str, fn) -> None:
-    """Install the sm_100a kernel wrapper for ``apb200::<name>``."""
+    """Install the sm_100a kernel wrapper for ``apb200::<name>``: what the operator's next call on CUDA tensors runs."""
     _cuda_table[name] = fn
+    if _on_install is not None:
+        _on_install(name, fn)
 
 
 # --------------------------------------------------------------------------------------

@@ -245,3 +245,33 @@ def test_native_cast_hands_out_the_optimizers_copy():
     finally:
         shadow.clear()
     assert torch.equal(library.ops.dtype_cast(p, torch.bfloat16), p.bfloat16())
+
+
+@pytest.mark.parametrize("name", [
+    "mm_nd", "mm_wgrad", "grouped_mm", "grouped_mm_wgrad", "dtype_cast", "rms_norm", "rms_norm_bwd", "rope", "swiglu", "swiglu_bwd", "cross_entropy",
+    "cross_entropy_bwd", "embedding", "embedding_bwd", "moe_slots", "moe_scatter", "moe_gather", "moe_gate_grad"])
+def test_an_installed_wrapper_is_what_the_next_call_runs(name):
+    """register_cuda_impl after the extension is loaded: the operator runs the function, and the kernel again once its own is back."""
+    from autoparallel_b200.ops import cuda_impl, library, register_cuda_impl
+
+    cuda_impl.ensure_loaded()
+    torch.manual_seed(0)
+    own = library._cuda_table[name]
+    args = next(a for n, a in _entry_cases() if n == name)
+    want = getattr(library.ops, name)(*args)
+    calls = []
+
+    def mine(*a):
+        calls.append(len(a))
+        return own(*a)
+
+    def equal(x, y):
+        x, y = (x, y) if isinstance(x, tuple) else ((x,), (y,))
+        return all(torch.allclose(p, q, atol=1e-5) if name == "embedding_bwd" else torch.equal(p, q) for p, q in zip(x, y, strict=True))  # (atomics)
+
+    register_cuda_impl(name, mine)
+    try:
+        assert equal(getattr(library.ops, name)(*args), want) and calls == [len(args)]
+    finally:
+        register_cuda_impl(name, own)
+    assert equal(getattr(library.ops, name)(*args), want) and calls == [len(args)]
