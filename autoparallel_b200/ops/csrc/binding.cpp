@@ -8,8 +8,10 @@
 #include <array>
 #include <atomic>
 #include <cstdint>
+#include <map>
 #include <mutex>
 #include <string>
+#include <vector>
 
 extern "C" {
 int apb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc,
@@ -85,6 +87,10 @@ int apb_dma_rs_sum(const void* src, void* dst, const unsigned long long* bases, 
                    int rank, int n, int num_ctas, uint32_t* status, cudaStream_t st);
 int apb_attention_fwd(const void* q, const void* k, const void* v, void* out, float* lse, int B, int S, int Sk, int H, int Hkv,
                       int D, int causal, float scale, uint32_t* status, cudaStream_t stream);
+int apb_gemm_footprint(int i, int* out);
+int apb_gemm_split_footprint(int i, int* out);
+int apb_symm_footprint(int mode, int* out);
+int apb_dma_sum_footprint(int n, int* out);
 int apb_adamw(const void* tensors_dev, const void* chunks_dev, int num_chunks, float lr, float beta1, float beta2, float eps,
               float wd, float bc1, float bc2, float grad_scale, const float* hyper_dev, cudaStream_t st);
 }
@@ -523,6 +529,25 @@ void dma_rs_sum(const at::Tensor& src, at::Tensor& dst, const std::vector<int64_
         "apb_dma_rs_sum");
 }
 
+// (threads, registers per thread, bytes of shared memory) of a CTA of every kernel of a kind: "gemm", "split", and the communication kernels
+// that are meant to become resident beside one of those, "beside".
+std::map<std::string, std::vector<std::array<int, 3>>> kernel_footprints() {
+  std::map<std::string, std::vector<std::array<int, 3>>> all;
+  auto add = [&](const char* kind, int (*of)(int, int*), int i) {
+    std::array<int, 3> out;
+    const int err = of(i, out.data());
+    if (err < 0) return false;
+    check(err, "kernel_footprint");
+    all[kind].push_back(out);
+    return true;
+  };
+  for (int i = 0; add("gemm", apb_gemm_footprint, i); ++i) {}
+  for (int i = 0; add("split", apb_gemm_split_footprint, i); ++i) {}
+  for (int mode : {0, 2}) add("beside", apb_symm_footprint, mode);  // (the reduce-scatter keeps the loads from all peers in registers)
+  for (int n = 2; add("beside", apb_dma_sum_footprint, n); ++n) {}
+  return all;
+}
+
 // ------------------------------------------------------------------ the operators' CUDA entries
 // Registered over the Python entries once the extension is loaded, so that an operator call - from a graph, from the autograd engine's
 // threads - runs no Python on its way to the kernel: 6 to 9 us of host time per call, and the interpreter's lock.  Every function takes the
@@ -792,6 +817,7 @@ void register_native(py::dict table, py::object status_buffer, bool diag_library
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  m.def("kernel_footprints", &kernel_footprints);
   m.def("register_native", &register_native);
   m.def("native_installed", &native_installed);
   m.def("native_launches", []() { return native().launches.load(std::memory_order_relaxed); });

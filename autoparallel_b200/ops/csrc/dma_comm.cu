@@ -21,6 +21,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "footprint.cuh"
 #include "symm_proto.cuh"
 
 namespace apbd {
@@ -63,7 +64,7 @@ __global__ void arena_wait_kernel(unsigned long long my_base, int rank, int n, i
 // out[i] = scale * (own[i] + sum over the n-1 peer slots), fp32, 16 bytes per thread per step.  ``slots`` is
 // [n][elems] in the owner's staging entry; slot ``rank`` is unused (the owner's partial is read in place).
 template <int N>
-__global__ void __launch_bounds__(256) slot_sum_kernel(const float4* __restrict__ own, const float4* __restrict__ slots, float4* __restrict__ out,
+__global__ void __launch_bounds__(256, 4) slot_sum_kernel(const float4* __restrict__ own, const float4* __restrict__ slots, float4* __restrict__ out,
                                                        long long vecs, long long slot_vecs, int rank, float scale) {
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < vecs; i += stride) {
@@ -175,6 +176,17 @@ int apb_dma_rs_sum(const void* src, void* dst, const unsigned long long* bases, 
 #undef APB_SUM
   arena_signal_kernel<<<1, 32, 0, st>>>(l, rank, n, ARENA_OFF_CONSUMED, entry * MAX_RANKS + rank, seq);
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
+}
+
+// Footprint of the sum over the slots of ``n`` ranks.
+int apb_dma_sum_footprint(int n, int* out) {
+#define APB_SUM(NN) \
+  case NN: return apb::kernel_footprint((const void*)slot_sum_kernel<NN>, 256, 0, out);
+  switch (n) {
+    APB_SUM(2) APB_SUM(3) APB_SUM(4) APB_SUM(5) APB_SUM(6) APB_SUM(7) APB_SUM(8)
+    default: return -1;
+  }
+#undef APB_SUM
 }
 
 }  // extern "C"

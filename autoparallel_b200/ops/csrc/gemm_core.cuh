@@ -24,6 +24,8 @@
 //                   rank's staging area in peer memory (16-byte stores over NVLink); the owner
 //                   sums the n slots once every rank has signalled completion
 #pragma once
+#include "footprint.cuh"
+#include "footprint.cuh"
 #include "ptx.cuh"
 #include "symm_proto.cuh"
 
@@ -40,7 +42,13 @@ constexpr int EPI_WARPS = 8;       // plain GEMM: two warps per TMEM lane quarte
 constexpr int GEMM_PLAIN_THREADS = 64 + 32 * EPI_WARPS;
 constexpr int STAGING_BYTES = EPI_WARPS * STORE_BYTES;
 constexpr int GEMM_PLAIN_SMEM_BYTES = GEMM_SMEM_BYTES + STAGING_BYTES;
-static_assert(GEMM_PLAIN_SMEM_BYTES + 1024 + 512 <= 233472, "a communication kernel's CTA (no shared memory to speak of) still fits beside a GEMM CTA");
+// A communication kernel on another stream becomes resident beside a GEMM CTA if the SM has room for both.  A launch bound of two CTAs holds the
+// plain and the split kernels to 96 registers (without it ptxas takes 142 to 159), which leaves a CTA of 512 threads and 64 registers.
+// With the epilogue's eight stores of a block written as one loop the bound cost 64 x 2048 x 1408 x 160 87 -> 93 us; in two groups of four with
+// one running address it is 84 (96 registers, 20 products with short contractions: 0.98 of the time without the bound).
+constexpr int GEMM_MIN_CTAS = 2, GEMM_REGISTERS = SM_REGISTERS / (GEMM_MIN_CTAS * GEMM_PLAIN_THREADS) / 8 * 8;
+static_assert(GEMM_PLAIN_THREADS * GEMM_REGISTERS + BESIDE_REGISTERS <= SM_REGISTERS, "registers for a communication kernel's CTA beside a GEMM CTA");
+static_assert(GEMM_PLAIN_SMEM_BYTES + BESIDE_SMEM_BYTES + 2 * CTA_SMEM_RESERVED <= SM_SMEM_BYTES, "shared memory for one, too");
 constexpr int PAIR_STAGES = 6;  // 6 x (16 KB of A + 16 KB of B) = the same 192 KB as 4 x 48 KB
 constexpr int EPI_STAGE_FLOATS = 32 * 33;  // per epilogue warp: one 32x32 fp32 block, padded
 constexpr int GEMM_FUSED_RS_SMEM_BYTES = GEMM_SMEM_BYTES + 4 * EPI_STAGE_FLOATS * 4;
@@ -223,11 +231,20 @@ __device__ __forceinline__ void store_tile(void* C, long long ldc, uint8_t* stg,
     for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(stg + lane * 128 + ((i ^ (lane & 7)) << 4)) = v[i];
     __syncwarp();
     const bool in_cols = n0 + c + unit * PER < N;  // (N is a number of whole vectors: rows are)
+    uint8_t* dst = dst0;  // (four lines under way, and one address stepped through the rows: see GEMM_REGISTERS)
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int row = i * 4 + sub;
-      const uint4 x = *reinterpret_cast<const uint4*>(stg + row * 128 + ((unit ^ (row & 7)) << 4));
-      if (in_cols && row0 + row < M) *reinterpret_cast<uint4*>(dst0 + i * 4 * row_bytes) = x;
+    for (int h = 0; h < 8; h += 4) {
+      uint4 x[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int row = (h + i) * 4 + sub;
+        x[i] = *reinterpret_cast<const uint4*>(stg + row * 128 + ((unit ^ (row & 7)) << 4));
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (in_cols && row0 + (h + i) * 4 + sub < M) *reinterpret_cast<uint4*>(dst) = x[i];
+        dst += 4 * row_bytes;
+      }
     }
     dst0 += 128;
   }

@@ -37,7 +37,7 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
 }
 
 template <bool A_MN, bool B_MN, int BN_T, bool GROUPED>
-__global__ void __launch_bounds__(SPLIT_THREADS, 1)
+__global__ void __launch_bounds__(SPLIT_THREADS, GEMM_MIN_CTAS)
 gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
   constexpr int B_BYTES = BN_T * BK * 2;
   constexpr int ST = SPLIT_STAGE_TOTAL / (A_STAGE_BYTES + B_BYTES);
@@ -188,7 +188,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     } else if (q * 32 < rows) {
       tc_fence_after();
       float* row = tile + (q * 32 + lane) * LD + col0;
-#pragma unroll
+#pragma unroll (COLS > 64 ? 2 : 4)  // (the registers of four loads are more than a communication kernel's CTA leaves)
       for (int c = 0; c < COLS / 32; ++c) {
         uint32_t r[32];
         tmem_ld_32x32(tmem_base + (uint32_t(q * 32) << 16) + col0 + c * 32, r);
@@ -468,4 +468,12 @@ extern "C" int apb_gemm_split_auto(const void* A, const void* B, void* C, int G,
   const SplitPlan plan = split_plan(G, M, N, K, num_sms, reserved);
   if (plan.bn == 0) return -1;
   return apb_gemm_split(A, B, C, G, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_fp32, plan.bn, plan.s, status, stream);
+}
+
+// Footprint of the ``i``-th kernel of this file; -1 past the last.
+extern "C" int apb_gemm_split_footprint(int i, int* out) {
+  if (i < 0 || i >= 24) return -1;
+  const int bn = 64 << (i % 3), a_mn = i / 3 & 1, b_mn = i / 6 & 1;
+  const SplitKernel kern = i < 12 ? split_kernel_of<false>(bn, a_mn, b_mn) : split_kernel_of<true>(bn, a_mn, b_mn);
+  return kernel_footprint((const void*)kern, SPLIT_THREADS, SPLIT_SMEM_BYTES, out);
 }

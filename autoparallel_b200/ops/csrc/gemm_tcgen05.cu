@@ -18,7 +18,7 @@
 namespace apb {
 
 template <bool A_MN, bool B_MN>
-__global__ void __launch_bounds__(GEMM_PLAIN_THREADS, 1)
+__global__ void __launch_bounds__(GEMM_PLAIN_THREADS, GEMM_MIN_CTAS)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
   FuseParams f{};
@@ -26,7 +26,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 }
 
 template <bool A_MN, bool B_MN, int ST = 0, bool DYN = false>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ST == 0 ? GEMM_PLAIN_THREADS : GEMM_THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ST == 0 ? GEMM_PLAIN_THREADS : GEMM_THREADS, ST == 0 ? GEMM_MIN_CTAS : 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
   FuseParams f{};
@@ -35,7 +35,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 
 // Grouped GEMM: G problems of one shape (the expert projections of a capacity-based MoE layer).
 template <bool A_MN, bool B_MN>
-__global__ void __launch_bounds__(GEMM_PLAIN_THREADS, 1)
+__global__ void __launch_bounds__(GEMM_PLAIN_THREADS, GEMM_MIN_CTAS)
 gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
   FuseParams f{};
@@ -43,7 +43,7 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 }
 
 template <bool A_MN, bool B_MN>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_PLAIN_THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_PLAIN_THREADS, GEMM_MIN_CTAS)
 gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
   FuseParams f{};
@@ -276,4 +276,17 @@ extern "C" int apb_gemm_grouped_bf16(const void* A, const void* B, void* C, int 
     else launch(gemm_grouped_kernel<true, true>, grid);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
+}
+
+// Footprint of the ``i``-th plain kernel that fills its SM's shared memory; -1 past the last.
+extern "C" int apb_gemm_footprint(int i, int* out) {
+#define APB_LAYOUTS(KERN, ...) \
+  (const void*)KERN<false, false __VA_ARGS__>, (const void*)KERN<false, true __VA_ARGS__>, (const void*)KERN<true, false __VA_ARGS__>, (const void*)KERN<true, true __VA_ARGS__>
+#define APB_COMMA ,
+  static const void* const kernels[] = {APB_LAYOUTS(gemm_bf16_kernel), APB_LAYOUTS(gemm_bf16_pair_kernel), APB_LAYOUTS(gemm_bf16_pair_kernel, APB_COMMA 0 APB_COMMA true),
+                                        APB_LAYOUTS(gemm_grouped_kernel), APB_LAYOUTS(gemm_grouped_pair_kernel)};
+#undef APB_LAYOUTS
+#undef APB_COMMA
+  if (i < 0 || i >= (int)(sizeof(kernels) / sizeof(kernels[0]))) return -1;
+  return kernel_footprint(kernels[i], GEMM_PLAIN_THREADS, GEMM_PLAIN_SMEM_BYTES, out);
 }

@@ -21,6 +21,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "footprint.cuh"
 #include "symm_proto.cuh"
 
 namespace apbs {
@@ -65,8 +66,12 @@ __device__ __forceinline__ uint4 multimem_sum_bf16x8(const void* mc_addr) {
   return v;
 }
 
+// 64 registers at most (two CTAs' worth), so that a CTA fits beside a GEMM CTA; the reduce-scatter keeps 121 for the loads from all peers
+// and starts on SMs that no GEMM holds.
+constexpr int COLL_THREADS = 512;
+static_assert(2 * apb::BESIDE_REGISTERS <= apb::SM_REGISTERS, "the launch bound of two CTAs");
 template <int MODE>
-__global__ void __launch_bounds__(512) symm_collective_kernel(CollParams p) {
+__global__ void __launch_bounds__(COLL_THREADS, MODE == REDUCE_SCATTER ? 1 : 2) symm_collective_kernel(CollParams p) {
   uint8_t* my_ws = p.peers.base[p.rank];
   uint8_t* my_stage = my_ws + HEADER_BYTES;
   const int n = p.n;
@@ -243,11 +248,18 @@ int apb_symm_collective(int mode, const unsigned long long* peer_ptrs, int rank,
   p.outer = outer; p.inner_bytes = inner_bytes; p.elem_kind = elem_kind; p.scale = scale; p.status = status; p.target0 = target0; p.target1 = target1;
   p.mc_stage = (mode == REDUCE_SCATTER && multicast_base != 0ull)
                    ? reinterpret_cast<const uint8_t*>(multicast_base) + HEADER_BYTES : nullptr;
-  if (mode == ALL_GATHER) symm_collective_kernel<ALL_GATHER><<<num_ctas, 512, 0, st>>>(p);
-  else if (mode == REDUCE_SCATTER) symm_collective_kernel<REDUCE_SCATTER><<<num_ctas, 512, 0, st>>>(p);
-  else if (mode == ALL_TO_ALL) symm_collective_kernel<ALL_TO_ALL><<<num_ctas, 512, 0, st>>>(p);
+  if (mode == ALL_GATHER) symm_collective_kernel<ALL_GATHER><<<num_ctas, COLL_THREADS, 0, st>>>(p);
+  else if (mode == REDUCE_SCATTER) symm_collective_kernel<REDUCE_SCATTER><<<num_ctas, COLL_THREADS, 0, st>>>(p);
+  else if (mode == ALL_TO_ALL) symm_collective_kernel<ALL_TO_ALL><<<num_ctas, COLL_THREADS, 0, st>>>(p);
   else return 3;
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
+}
+
+// Footprint of the collective of this mode.
+int apb_symm_footprint(int mode, int* out) {
+  const void* kern = mode == ALL_GATHER ? (const void*)symm_collective_kernel<ALL_GATHER>
+                     : mode == REDUCE_SCATTER ? (const void*)symm_collective_kernel<REDUCE_SCATTER> : (const void*)symm_collective_kernel<ALL_TO_ALL>;
+  return apb::kernel_footprint(kern, COLL_THREADS, 0, out);
 }
 
 }  // extern "C"

@@ -482,3 +482,16 @@ def test_gemm_bits_do_not_depend_on_the_launch(K, pair):
         ext.gemm_set_pair_mode(prev[0])
         ext.gemm_set_reserved_sms(prev[1])
         ext.gemm_set_dynamic_tiles(prev[2])
+
+
+def test_communication_kernels_fit_beside_a_gemm_cta(K):
+    """Threads, registers (in units of 256 per warp) and shared memory (1 KB more per CTA than it asks for) of an SM."""
+    kinds = K[1].extension().kernel_footprints()
+    sm = torch.cuda.get_device_properties(0)
+    registers = lambda threads, per_thread: threads // 32 * (-(-32 * per_thread // 256) * 256)
+    for kind in ("gemm", "split"):
+        for gemm in kinds[kind]:
+            for other in kinds["beside"]:
+                assert gemm[0] + other[0] <= sm.max_threads_per_multi_processor
+                assert registers(*gemm[:2]) + registers(*other[:2]) <= sm.regs_per_multiprocessor, (kind, gemm, other)
+                assert gemm[2] + other[2] + 2 * 1024 <= sm.shared_memory_per_multiprocessor, (kind, gemm, other)
