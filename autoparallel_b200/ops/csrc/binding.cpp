@@ -584,7 +584,7 @@ py::object py_dtype(at::ScalarType t) { return py::reinterpret_borrow<py::object
 
 // The word that bounded waits report to, one per device: made by Python at the first use on a device and shared with it.
 at::Tensor& status_of(const at::Tensor& t) {
-  static std::array<at::Tensor, 64> words;
+  static auto& words = *new std::array<at::Tensor, 64>;  // (never destroyed, like Native)
   static std::array<std::atomic<bool>, 64> known{};
   static std::mutex m;
   const int dev = t.get_device();

@@ -98,8 +98,8 @@ def status_buffer(device) -> torch.Tensor:
     idx = (device if isinstance(device, torch.device) else torch.device(device)).index or 0
     t = _status.get(idx)
     if t is None:
-        t = torch.zeros(4, dtype=torch.int32, device=torch.device("cuda", idx))
-        _status[idx] = t
+        # (the native entries keep the word they get: threads that come here together must leave with the same one)
+        t = _status.setdefault(idx, torch.zeros(4, dtype=torch.int32, device=torch.device("cuda", idx)))
     return t
 
 

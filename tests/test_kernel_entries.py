@@ -3,8 +3,12 @@ import ctypes
 import os
 import subprocess
 import sys
+import threading
+import time
+from concurrent.futures import ThreadPoolExecutor
 
 import pytest
+import torch
 
 from autoparallel_b200.ops import build
 
@@ -80,3 +84,24 @@ def test_pair_gemm_with_fewer_stages_leaves_their_shared_memory():
     out = _run("print(*[so.apb_gemm_pair_smem_bytes(s) for s in (4, 5, 6)])")
     four, five, six = map(int, out)
     assert (four, five) == (4 * 32768 + 1280, 5 * 32768 + 1280) and six <= 227 * 1024
+
+
+def test_one_status_word_per_device_whichever_thread_is_first(monkeypatch):
+    """Both sides of the binding keep the word they got first: two threads at the first use of a device must get the same one."""
+    from autoparallel_b200.ops import cuda_impl
+
+    together = threading.Barrier(2)
+
+    def zeros(*shape, **kw):  # (stands in for the device; slow enough for the other thread to come past the look-up)
+        time.sleep(0.3)
+        return torch.empty(*shape, dtype=kw["dtype"])
+
+    def first_use(_):
+        together.wait(timeout=10)
+        return cuda_impl.status_buffer(torch.device("cuda", 0))
+
+    monkeypatch.setattr(cuda_impl, "_status", {})
+    monkeypatch.setattr(cuda_impl.torch, "zeros", zeros)
+    with ThreadPoolExecutor(2) as pool:
+        first, second = pool.map(first_use, range(2))
+    assert first is second is cuda_impl.status_buffer(torch.device("cuda", 0))
