@@ -14,9 +14,11 @@
 // A cluster of one CTA has nothing to add and stores its tile from TMEM (store_tile).
 //
 //   warp 0: TMA producer | warp 1: TMEM owner + MMA issuer | warps 2..9 (64 columns: 2..5): TMEM -> shared memory (or C) | all: sum and store
-// Persistent kernels -> this one, us: 16 x 4096 x 4096 29 -> 13, 16 x 4096 x 14336 87 -> 25, 64 x 2048 x 2048 16.6 -> 8.6, 64 x 2048 x 8192 50 -> 15.6,
-// 512 x 256 x 256 7.0 -> 5.5, 160 x 8192 x 8192 55 -> 39; 478 products in profiles/gemm_split_rule_sweep.txt.
+// Persistent kernels -> this one, us: 16 x 4096 x 4096 27 -> 10.4, 16 x 4096 x 14336 84 -> 23.5, 64 x 2048 x 2048 15.6 -> 6.6, 64 x 2048 x 8192 46 -> 11.5,
+// 512 x 256 x 256 5.8 -> 4.9, 160 x 8192 x 8192 45 -> 37; 1221 products in profiles/gemm_split_estimate_sweep.txt.
 #include "gemm_core.cuh"
+
+#include <mutex>
 
 namespace apb {
 
@@ -293,18 +295,18 @@ static SplitKernel split_kernel_of(int bn, int a_mn, int b_mn) {
 
 // Tile width and slice count for a product, or bn = 0 where the persistent kernels are expected to be faster.
 //
-// Only forms whose clusters are all resident at once: in a second wave every tile pays its fixed part again.  The estimates (microseconds, one
-// B200) are fitted to a sweep of 1221 products with every form that fits, 1 <= M <= 4096, 64 <= N, K <= 8192, all layouts: a fixed part
-// (launch, prologue, the way out of TMEM), then the longest of a chain of k-blocks, the operand traffic out of L2 (15 TB/s) and the operands
-// out of memory (8.6 TB/s, less while few bytes are in flight), a round trip more where the chain is longer than the stages, then what
-// comes through the other CTAs' shared memory (19 GB/s and CTA).  They are good to 13 per cent; the form they pick takes 1.4 % more than
-// the best one in the geometric mean (the estimates of the kernels before: 5.4 %), and 28 of the 1221 products are more than 3 % slower than
-// by those (by 0.2 to 0.6 us but for three).  Left out, because the sweeps showed the estimates to flatter them: forms with no more CTAs
-// than the persistent kernels would use (twice as many where the contraction has one or two blocks), slices of a single block, whole
-// contractions in 256-wide tiles, and in 64-wide ones on most of the chip.
+// Only forms whose clusters are all resident at once: in a second wave every tile pays its fixed part again.  Left out as well, because the
+// sweeps showed the estimates to flatter them: forms with no more CTAs than the persistent kernels would use (twice as many where the contraction
+// has one or two blocks), slices of a single block, whole contractions in 256-wide tiles, and in 64-wide ones on most of the chip.
 //
-// Contractions of up to 16 blocks (K <= 1024) keep the estimates fitted to the kernels as they were: the new ones would give them fewer
-// slices, that is longer chains of fp32 sums, for 0.1 to 0.4 us each, and the loss of a small decoder came out further from 64 bits.
+// Two sets of estimates (SplitCosts, microseconds on one B200).  FITTED, to a sweep of 1221 products with every form that fits, 1 <= M <= 4096,
+// 64 <= N, K <= 8192, all layouts (profiles/gemm_split_estimate_sweep.txt), picks the form for contractions of more than 16 blocks.  EARLIER,
+// fitted to the kernels before their single-thread roles were elected, bounds the length of a slice's chain of fp32 sums: the tensor cores'
+// rounding error grows in proportion to it, 2.1 times at twice the length (fp32 results, 64 x 1 in place of 128 x 2, 1160 <= K <= 2800), and
+// without the bound one product in a hundred got a longer chain than it had, up to twice.  Contractions of up to 16 blocks (K <= 1024) keep the
+// form that EARLIER gives them: FITTED would gain 0.1 to 0.4 us each, most of it by fewer slices.
+// On the products of the sweep with K > 1024 the forms picked take 2.4 % more than the best one in the geometric mean (without the bound 2.3,
+// by EARLIER alone 7.4).
 struct SplitPlan {
   int bn, s;
 };
@@ -312,36 +314,57 @@ extern "C" int apb_gemm_resident_pairs(int num_sms);
 
 static SplitKernel split_kernel_any() { return gemm_split_kernel<false, false, 64, false>; }
 
-// CTAs of clusters of ``s`` that are resident at once (one CTA per SM; the partial ends of the GPCs are lost); asked once
-// per device and size.
-static int split_slots(int s, int num_sms) {
-  static int cached[64][SPLIT_MAX + 1];  // 0 = not asked yet; the answer is the same whoever asks
+// CTAs of clusters of 1 ... SPLIT_MAX that are resident at once on the current device (one CTA per SM; the partial ends of the GPCs are
+// lost); asked once per device.
+static void ask_slots(int* slots, int num_sms) {
+  SplitKernel kern = split_kernel_any();
+  const bool opted_in = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SPLIT_SMEM_BYTES) == cudaSuccess;
+  for (int s = 1; s <= SPLIT_MAX; ++s) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(num_sms / s * s));
+    cfg.blockDim = dim3(SPLIT_THREADS);
+    cfg.dynamicSmemBytes = SPLIT_SMEM_BYTES;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)s;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (!opted_in || cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
+      cudaGetLastError();
+      n = num_sms / s / 2;
+    }
+    slots[s] = n * s;
+  }
+}
+static const int* split_slots(int num_sms) {
+  constexpr int DEVICES = 64;
+  static int slots[DEVICES][SPLIT_MAX + 1];
+  static std::once_flag asked[DEVICES];
+  static const int none[SPLIT_MAX + 1] = {0};
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev >= 0 && dev < 64 && cached[dev][s] > 0) return cached[dev][s];
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(num_sms / s * s));
-  cfg.blockDim = dim3(SPLIT_THREADS);
-  cfg.dynamicSmemBytes = SPLIT_SMEM_BYTES;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = (unsigned)s;
-  attr.val.clusterDim.y = 1;
-  attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  int n = 0;
-  SplitKernel kern = split_kernel_any();
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SPLIT_SMEM_BYTES) != cudaSuccess ||
-      cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
-    cudaGetLastError();
-    n = num_sms / s / 2;
-  }
-  if (dev >= 0 && dev < 64) cached[dev][s] = n * s;
-  return n * s;
+  if (dev < 0 || dev >= DEVICES) return none;  // (the persistent kernels)
+  std::call_once(asked[dev], ask_slots, slots[dev], num_sms);
+  return slots[dev];
 }
 
-static SplitPlan split_plan(int G, int M, int N, int K, int num_sms, int reserved) {
+// What a form is expected to take: a fixed part (launch, prologue, the way out of TMEM), then the longest of a chain of k-blocks, the operand
+// traffic out of L2 and the operands out of memory (less while few bytes are in flight; the sweep's operands were partly in L2, which its rates
+// include), a round trip more where the chain is longer than the stages, then what comes through the other CTAs' shared memory.
+struct SplitCosts {
+  double pair_launch, pair_wave, pair_kb, single_launch, single_wave, single_kb, margin;  // the persistent kernels, and what a form has to beat
+  double per_kb[3], one_slice[3], more_slices[3];                                          // by tile width: 64, 128, 256
+  double l2, memory, memory_per_mb;                                                        // bytes per us; the last per megabyte in flight
+  double long_chain, sum_width, sum_byte, sum_slice;                                       // us; per slice and 64 columns, per byte, per slice
+};
+constexpr SplitCosts EARLIER = {5.5, 0.5, 0.38, 5.5, 0.5, 0.35, 0.95, {0.27, 0.20, 0.27}, {5.6, 7.0, 9.0}, {5.6, 7.0, 9.0}, 9.5e6, 6.5e6, 0.62e6, 0.0, 0.05, 0.0, 0.0};
+constexpr SplitCosts FITTED = {3.35, 0.49, 0.45, 3.2, 0.87, 0.33, 1.0, {0.23, 0.26, 0.39}, {3.5, 4.0, 4.0}, {4.1, 4.1, 3.8}, 14.7e6, 8.6e6, 0.684e6, 0.31, 0.0, 1 / 18.7e3, 0.034};
+
+// The fastest form by ``costs`` with at most ``max_chain`` k-blocks to a slice; the persistent kernels have them all.
+static SplitPlan split_pick(const SplitCosts& costs, int max_chain, int G, int M, int N, int K, int num_sms, int reserved) {
   const long long g = G > 0 ? G : 1;
   const long long m_tiles = (M + BM - 1) / BM;
   const int usable = num_sms - reserved > 0 ? num_sms - reserved : 1;
@@ -352,42 +375,32 @@ static SplitPlan split_plan(int G, int M, int N, int K, int num_sms, int reserve
   const long long tiles = g * (pair ? (M + 2 * BM - 1) / (2 * BM) : m_tiles) * ((N + BN - 1) / BN);
   int units = pair ? apb_gemm_resident_pairs(num_sms) - reserved / 2 : usable;  // as the launches have it
   if (units < 1) units = 1;
-  const bool brief = kb <= 16;
   const double waves = (double)((tiles + units - 1) / units);
-  const double now = brief ? 5.5 + waves * (0.5 + (pair ? 0.38 : 0.35) * kb)
-                           : pair ? 3.35 + waves * (0.49 + 0.45 * kb) : 3.2 + waves * (0.87 + 0.33 * kb);
+  const double now = pair ? costs.pair_launch + waves * (costs.pair_wave + costs.pair_kb * kb) : costs.single_launch + waves * (costs.single_wave + costs.single_kb * kb);
   const long long ctas = (tiles < units ? tiles : units) * (pair ? 2 : 1) * (kb <= 2 ? 2 : 1);
   const double operands = 2.0 * g * ((double)M * K + (double)N * K);
-  double t_best = brief ? 0.95 * now : now;
-  for (int bn = 64; bn <= 256; bn *= 2) {
-    const double per_kb = brief ? (bn == 128 ? 0.20 : 0.27) : bn == 64 ? 0.23 : bn == 128 ? 0.26 : 0.39;
+  const int* slots = split_slots(num_sms);
+  double t_best = kb <= max_chain ? costs.margin * now : 1e30;
+  for (int w = 0; w < 3; ++w) {
+    const int bn = 64 << w;
     const int stages = SPLIT_STAGE_TOTAL / (A_STAGE_BYTES + bn * BK * 2);
     const long long t = g * m_tiles * ((N + bn - 1) / bn);
-    const double kb_bytes = 128.0 * ((M < BM ? M : BM) + (N < bn ? N : bn));
+    const double rows = M < BM ? M : BM, cols = N < bn ? N : bn, kb_bytes = 128.0 * (rows + cols);
     for (int s = 1; s <= SPLIT_MAX && s <= kb; ++s) {
       if (t * s > usable) break;
-      if (t * s > split_slots(s, num_sms) || t * s <= ctas) continue;
+      if (t * s > slots[s] || t * s <= ctas) continue;
       if (s > 1 ? kb < 2 * s : bn == 256 || (bn == 64 && t > 100)) continue;
       const int chain = (kb + s - 1) / s;
-      double flow = per_kb * chain;
-      const double l2 = (double)t * kb * kb_bytes / (brief ? 9.5e6 : 14.7e6);
+      if (chain > max_chain) continue;
+      double flow = costs.per_kb[w] * chain;
+      const double l2 = (double)t * kb * kb_bytes / costs.l2;
       if (l2 > flow) flow = l2;
       // megabytes in flight: the stages of all CTAs, rows and columns outside the matrices not counted
-      const double flight = 0.1875 * t * s * kb_bytes / (128.0 * (BM + bn));
-      const double most = brief ? 6.5e6 : 8.6e6, grows = (brief ? 0.62e6 : 0.684e6) * flight;
-      const double from_memory = operands / (grows < most ? grows : most);
+      const double grows = costs.memory_per_mb * 0.1875 * t * s * kb_bytes / (128.0 * (BM + bn));
+      const double from_memory = operands / (grows < costs.memory ? grows : costs.memory);
       if (from_memory > flow) flow = from_memory;
-      if (brief) {
-        const double est = (bn == 64 ? 5.6 : bn == 128 ? 7.0 : 9.0) + flow + (s > 1 ? 0.05 * s * bn / 64 : 0.0);
-        if (est < t_best) {
-          t_best = est;
-          best = SplitPlan{bn, s};
-        }
-        continue;
-      }
-      const double fixed = s > 1 ? (bn == 256 ? 3.8 : 4.1) : (bn == 64 ? 3.5 : 4.0);
-      const double shared = s > 1 ? 4.0 * (M < BM ? M : BM) * (N < bn ? N : bn) * (s - 1) / s / 18.7e3 + 0.034 * s : 0.0;
-      const double est = fixed + flow + (chain > stages ? 0.31 : 0.0) + shared;
+      double est = (s > 1 ? costs.more_slices[w] : costs.one_slice[w]) + flow + (chain > stages ? costs.long_chain : 0.0);
+      if (s > 1) est += costs.sum_width * s * bn / 64 + costs.sum_byte * 4.0 * rows * cols * (s - 1) / s + costs.sum_slice * s;
       if (est < t_best) {
         t_best = est;
         best = SplitPlan{bn, s};
@@ -395,6 +408,13 @@ static SplitPlan split_plan(int G, int M, int N, int K, int num_sms, int reserve
     }
   }
   return best;
+}
+
+static SplitPlan split_plan(int G, int M, int N, int K, int num_sms, int reserved) {
+  const int kb = (K + BK - 1) / BK;
+  const SplitPlan earlier = split_pick(EARLIER, kb, G, M, N, K, num_sms, reserved);
+  if (kb <= 16) return earlier;
+  return split_pick(FITTED, earlier.bn ? (kb + earlier.s - 1) / earlier.s : kb, G, M, N, K, num_sms, reserved);
 }
 
 // The rule above: tile width and slices, 0 and 0 where the persistent kernels run.

@@ -495,3 +495,21 @@ def test_communication_kernels_fit_beside_a_gemm_cta(K):
                 assert gemm[0] + other[0] <= sm.max_threads_per_multi_processor
                 assert registers(*gemm[:2]) + registers(*other[:2]) <= sm.regs_per_multiprocessor, (kind, gemm, other)
                 assert gemm[2] + other[2] + 2 * 1024 <= sm.shared_memory_per_multiprocessor, (kind, gemm, other)
+
+
+@pytest.mark.parametrize("groups,M,N,K_,bn,slices", [(0, 2514, 256, 1096, 128, 2), (0, 2615, 176, 3416, 256, 4), (4, 1470, 200, 2024, 256, 2), (0, 155, 472, 7304, 128, 8),
+                                                     (0, 121, 10624, 2360, 256, 2)])
+def test_a_faster_form_has_no_longer_chains(K, groups, M, N, K_, bn, slices):
+    """The error of an fp32 result grows with the blocks that one chain of sums runs through; the form that the rule picks is as exact as
+    the one given, which it took before the kernels got faster (a tenth for the order of the sums)."""
+    _, impl = K
+    ext = impl.extension()
+    g = torch.Generator(device="cuda").manual_seed(M)
+    lead = (groups,) if groups else ()
+    a = torch.randn(*lead, M, K_, device="cuda", generator=g).to(torch.bfloat16)
+    b = torch.randn(*lead, N, K_, device="cuda", generator=g).to(torch.bfloat16)
+    ref = a.double() @ b.double().transpose(-1, -2)
+    c, given = torch.empty(*lead, M, N, device="cuda"), torch.empty(*lead, M, N, device="cuda")
+    (ext.gemm_grouped if groups else ext.gemm)(a, b, c, False, False, impl.status_buffer(a.device))
+    ext.gemm_split(a, b, given, False, False, bn, slices, impl.status_buffer(a.device))
+    assert _rel(c, ref) <= 1.1 * _rel(given, ref)
