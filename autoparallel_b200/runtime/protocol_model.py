@@ -169,11 +169,11 @@ class TileCounters:
             self.requests += max(0, min(pairs, cap - self.requests))
 
 
-def run_dynamic_gemm(counters: TileCounters, num_tiles: int, num_pairs: int, readers: int = 10, ring: int = 4,
+def run_dynamic_gemm(counters: TileCounters, num_tiles: int, num_pairs: int, readers: int = 18, ring: int = 4,
                      jitter: float = 0.0, seed: int = 0) -> dict:
     """One launch: per CTA pair a fetching thread (the even CTA's producer) publishes tile indices through a
-    ``ring``-entry ring that ``readers`` consumer threads (odd CTA's producer, MMA thread, eight epilogue
-    warps) read and release.  Returns, per pair, the tiles each reader saw; the caller checks that every
+    ``ring``-entry ring that ``readers`` consumer threads (odd CTA's producer, MMA thread, the eight epilogue
+    warps of each CTA) read and release.  Returns, per pair, the tiles each reader saw; the caller checks that every
     tile was handled exactly once and by all readers of one pair alike."""
     rng = random.Random(seed)
     seen = {p: [[] for _ in range(readers)] for p in range(num_pairs)}

@@ -88,7 +88,7 @@ def test_dynamic_tiles_are_each_handled_once_even_when_pairs_leave(requests):
     for launch in range(2):
         c.request(requests)
         asked = c.requests
-        seen = pm.run_dynamic_gemm(c, num_tiles, num_pairs, readers=10, jitter=1e-4, seed=launch)
+        seen = pm.run_dynamic_gemm(c, num_tiles, num_pairs, readers=18, jitter=1e-4, seed=launch)
         tiles = []
         for p in range(num_pairs):
             assert all(s == seen[p][0] for s in seen[p])  # producer, MMA and epilogue roles agree
