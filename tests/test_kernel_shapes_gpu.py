@@ -513,3 +513,26 @@ def test_a_faster_form_has_no_longer_chains(K, groups, M, N, K_, bn, slices):
     (ext.gemm_grouped if groups else ext.gemm)(a, b, c, False, False, impl.status_buffer(a.device))
     ext.gemm_split(a, b, given, False, False, bn, slices, impl.status_buffer(a.device))
     assert _rel(c, ref) <= 1.1 * _rel(given, ref)
+
+
+@pytest.mark.parametrize("M,N,K_", [(129, 265, 520), (1, 7, 1024), (260, 130, 72)])
+@pytest.mark.parametrize("bn,slices", [(64, 1), (64, 2), (128, 1), (128, 7), (256, 1), (256, 4)])
+@pytest.mark.parametrize("out", [torch.bfloat16, torch.float32])
+def test_gemm_split_rows_that_are_no_whole_vectors(K, M, N, K_, bn, slices, out):
+    """Leading dimensions that are multiples of four, of two and odd, columns past the last whole vector: element by element, for one slice
+    as for more.  Whole numbers: every sum is exact."""
+    _, impl = K
+    ext = impl.extension()
+    if slices > (K_ + 63) // 64:
+        pytest.skip("not a form of this kernel")
+    gen = torch.Generator(device="cuda").manual_seed(M + N)
+    a = torch.randint(-1, 2, (M, K_), device="cuda", generator=gen).to(torch.bfloat16)
+    b = torch.randint(-1, 2, (N, K_), device="cuda", generator=gen).to(torch.bfloat16)
+    ref = (a.float() @ b.float().t()).to(out)
+    for ld in (-(-N // 8) * 8 + 4, -(-N // 8) * 8 + 2, -(-N // 8) * 8 + 1):
+        flat = torch.full((8 + M * ld + 8,), 99.0, device="cuda", dtype=out)
+        c = flat[8:].as_strided((M, N), (ld, 1))  # (starts on a 16-byte boundary)
+        ext.gemm_split(a, b, c, False, False, bn, slices, impl.status_buffer(c.device))
+        assert torch.equal(c, ref), ld
+        c.fill_(99.0)
+        assert bool((flat == 99.0).all()), ld
