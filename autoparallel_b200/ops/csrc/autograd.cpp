@@ -5,7 +5,7 @@
 // kernel's entry and its gradient node is a C++ one.  What that costs on the host per call (forward alone / forward that
 // records a gradient): 18 -> 8 us / 38 -> 10 us, the CUDA entry apart.
 // CPU, meta and fake CPU tensors (planning) keep the Python registration.  Everything below autograd - dispatch modes, fake
-// tensors, functionalisation, the CUDA entries of ops/cuda_impl.py - is reached as before, by redispatch; functorch
+// tensors, functionalisation, the CUDA entries at the end of binding.cpp - is reached as before, by redispatch; functorch
 // transforms and forward-mode differentiation of a recorded call are refused by the C++ function itself as they are by the Python
 // one; a dual tensor in a call that records nothing loses its tangent, as it does there.
 #include <ATen/core/dispatch/Dispatcher.h>

@@ -58,9 +58,9 @@ constexpr int GEMM_AG_THREADS = GEMM_THREADS + 32;
 
 // CTA pairs take a product with at least one full pair tile.  Of those with 129 to 255 rows, whose odd CTA is partly idle, they take
 // the ones with a long contraction: the pair's tile brings every B tile into the SMs once (32 KB per SM and k-block) where two single
-// CTAs load it twice (48 KB), but starts 0.8 us later.  130 ... 255 rows, single against pair, geometric means over 256 < N <= 57344 and
-// groups of 4 ... 74: K = 64 0.88, 512 0.96, 1024 1.04, 1280 1.06, 2048 1.07, 4096 1.08, 8192 1.12; one column tile (N = 256) 0.89 to 0.99 below
-// K = 4096.  64 experts, 160 rows, N = 1408, K = 2048: 95 -> 83 us.
+// CTAs load it twice (48 KB), but starts later.  130 ... 255 rows, single against pair, geometric means over 256 < N <= 57344 and groups of 4 ... 74:
+// K = 64 0.92, 512 1.05 (0.96 to 1.17), 1024 1.05 (0.99 to 1.15), 1280 1.08, 2048 1.11, 4096 1.12, 8192 1.12; one column tile (N = 256) 0.89, 0.95,
+// 0.98, 1.00, 1.05, 1.09, 1.10.  64 experts, 160 rows, N = 1408, K = 2048, weights [N, K]: 116 -> 97 us.
 inline bool pair_shape(int M, int N, int K) { return M >= 2 * BM ? N >= BN : M > BM && N > BN && K >= 1280; }
 
 enum : int { FUSE_NONE = 0, FUSE_GATHER_A = 1, FUSE_GATHER_B = 2, FUSE_REDUCE_SCATTER = 3 };
@@ -125,7 +125,7 @@ __device__ __forceinline__ void tile_coords(int t, int num_m, int num_n, int& tm
 //
 // Every tile goes through the contraction forwards, so that its bits depend neither on the launch (reserved SMs, pairs that are resident, tiles
 // handed out at run time) nor on where the tile lies: equal rows give equal results.  Backwards in every other round, for what L2 still holds
-// of the round before, saves power and with it time in rounds of more than 64 MB (8B feed-forward block 3 %), and gives that up.
+// of the round before, saves power and with it time where a round reads more than L2 holds (8B feed-forward block 0 to 3 %), and gives that up.
 inline void set_tile_order(GemmParams& p, int num_m) {
   p.div_group = FastDiv((uint32_t)GROUP_M * p.num_n_tiles);
   p.div_tiles = FastDiv((uint32_t)num_m * p.num_n_tiles);
@@ -188,7 +188,8 @@ __device__ __forceinline__ void store_row_chunk(const GemmParams& p, long long r
 // A product with a short contraction is bound by this chain.  TMA stores from the staging block (the form before) wait in the queue of
 // the tile's loads, 1500 to 2000 cycles for each block before it can be written again.  Two warps per lane quarter, because one warp's
 // chain of dependent instructions (900 cycles a block) fills neither the load-store unit nor the memory.  Weight gradients of 64 experts,
-// 2048 x 1408 over 160 rows: 162 us with TMA stores, 130 with four warps and these stores, 93 with eight (the result alone takes 64).
+// 2048 x 1408 over 160 rows: 162 us with TMA stores, 130 with four warps and these stores, 93 with eight, 84 with the stores in groups of four (the
+// result alone takes 64).
 template <bool OUT_FP32, typename Release>
 __device__ __forceinline__ void store_tile(void* C, long long ldc, uint8_t* stg, uint32_t taddr, int row0, int n0, int ncols, int M, int N, int lane,
                                            Release release) {
@@ -392,7 +393,7 @@ __device__ __forceinline__ void gather_comm_warp(const GemmParams& p, const Fuse
 // DYN (CTA pairs, FUSE_NONE): tiles are handed out at run time.  The even CTA's producer thread takes the
 // next tile index from a global counter and publishes it through a four-entry ring in BOTH CTAs'
 // shared memory (remote store + remote mbarrier arrive); the odd CTA's producer, the MMA thread and
-// the eight epilogue warps of the pair read it there and release the entry on the even CTA's
+// the sixteen epilogue warps of the pair read it there and release the entry on the even CTA's
 // barrier.  A pair that starts late or shares its SMs with another kernel (a communication kernel on
 // another stream) simply takes fewer tiles, so nothing waits for the slowest pair's fixed share.
 // Before each fetch the producer also looks at a request counter: a collective that is about to launch on

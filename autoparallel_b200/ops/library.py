@@ -6,8 +6,10 @@ namespace.  A schema is defined once here; three implementations hang off it:
 * ``CPU``  – a plain PyTorch fp32 restatement (the numerics oracle of the test-suite and
   what planner tests execute on machines without a GPU),
 * ``Meta`` – shape/dtype propagation, so fake-tensor tracing of the joint graph works,
-* ``CUDA`` – the hand-written sm_100a kernels (registered by ``ops.cuda_impl`` once the
-  in-tree extension is loaded; a CUDA tensor reaching an op without it raises).
+* ``CUDA`` – the hand-written sm_100a kernels: until the in-tree extension is loaded an entry that loads it and calls the
+  function of ``ops.cuda_impl``, from then on the native entries of ``csrc/binding.cpp``, which go to that function for forms that
+  the kernels do not take and to whatever ``register_cuda_impl`` has installed (``gemm``, ``scaled_mm`` and attention have Python entries
+  alone; a CUDA tensor reaching an op without the extension raises).
 
 Backward formulas are themselves ``apb200`` ops, so a traced joint forward/backward graph
 contains only planner-visible nodes (the planner has a sharding rule per op, see
@@ -252,7 +254,7 @@ for _name, _fn in _META_IMPLS.items():
 
 
 # --------------------------------------------------------------------------------------
-# CUDA: a guard kernel until ops.cuda_impl installs the sm_100a kernels.
+# CUDA: the entry that loads the extension; most of them give way to native entries then (csrc/binding.cpp).
 # --------------------------------------------------------------------------------------
 _cuda_table: dict[str, object] = {}
 
