@@ -656,7 +656,8 @@ Tensor op_grouped_wgrad(const Tensor& a, const Tensor& b, at::ScalarType dtype) 
 }
 Tensor op_cast(const Tensor& x, at::ScalarType dtype) {
   if (x.scalar_type() == dtype && ours(DTYPE_CAST)) return x;
-  if (ours(DTYPE_CAST) && !native().shadows.load(std::memory_order_relaxed) && (dtype == at::kBFloat16 || (dtype == at::kFloat && x.scalar_type() == at::kBFloat16))) {
+  if (ours(DTYPE_CAST) && !native().shadows.load(std::memory_order_relaxed) &&
+      (dtype == at::kBFloat16 || (dtype == at::kFloat && x.scalar_type() == at::kBFloat16))) {
     auto y = cast_new(x, dtype == at::kBFloat16);
     if (y.has_value()) {
       count();
@@ -708,7 +709,8 @@ Tensor op_xent_bwd(const Tensor& dloss, const Tensor& logits_, const Tensor& lab
   return out;
 }
 Tensor op_embedding(const Tensor& weight, const Tensor& ids) {
-  if (ours(EMBEDDING) && weight.dim() == 2 && float_or_bf16(weight.scalar_type()) && weight.size(1) * weight.element_size() % 16 == 0 && ids.scalar_type() == at::kLong) {
+  if (ours(EMBEDDING) && weight.dim() == 2 && float_or_bf16(weight.scalar_type()) && weight.size(1) * weight.element_size() % 16 == 0 &&
+      ids.scalar_type() == at::kLong) {
     auto shape = ids.sizes().vec();
     shape.push_back(weight.size(1));
     Tensor out = at::empty(shape, weight.options());
@@ -743,7 +745,8 @@ Tensor op_moe_slots(const Tensor& idx, int64_t E, int64_t C, int64_t nb) {
   return in_python<Tensor>(MOE_SLOTS, idx, E, C, nb);
 }
 Tensor op_moe_scatter(const Tensor& src, const Tensor& slot, const Tensor& w, int64_t E, int64_t C, int64_t nb) {
-  if (ours(MOE_SCATTER) && moe_ok({&src, &slot, &w}) && float_or_bf16(src.scalar_type()) && src.dim() == 2 && nb > 0 && src.size(0) > 0 && src.size(0) % nb == 0) {
+  if (ours(MOE_SCATTER) && moe_ok({&src, &slot, &w}) && float_or_bf16(src.scalar_type()) && src.dim() == 2 && nb > 0 && src.size(0) > 0 &&
+      src.size(0) % nb == 0) {
     Tensor buf = at::empty({E, nb, C, src.size(1)}, src.options());
     moe_scatter(src.contiguous(), slot.contiguous(), gate_weights(w, src.scalar_type()), buf, E, C, nb);
     count(2);
@@ -752,8 +755,8 @@ Tensor op_moe_scatter(const Tensor& src, const Tensor& slot, const Tensor& w, in
   return in_python<Tensor>(MOE_SCATTER, src, slot, w, E, C, nb);
 }
 Tensor op_moe_gather(const Tensor& buf, const Tensor& slot, const Tensor& w) {
-  if (ours(MOE_GATHER) && moe_ok({&buf, &slot, &w}) && float_or_bf16(buf.scalar_type()) && buf.dim() == 4 && buf.size(1) > 0 && slot.dim() == 2 && slot.size(0) > 0 &&
-      slot.size(0) % buf.size(1) == 0) {
+  if (ours(MOE_GATHER) && moe_ok({&buf, &slot, &w}) && float_or_bf16(buf.scalar_type()) && buf.dim() == 4 && buf.size(1) > 0 &&
+      slot.dim() == 2 && slot.size(0) > 0 && slot.size(0) % buf.size(1) == 0) {
     Tensor out = at::empty({slot.size(0), buf.size(3)}, buf.options());
     moe_gather(buf.contiguous(), slot.contiguous(), gate_weights(w, buf.scalar_type()), out);
     count();
@@ -762,8 +765,8 @@ Tensor op_moe_gather(const Tensor& buf, const Tensor& slot, const Tensor& w) {
   return in_python<Tensor>(MOE_GATHER, buf, slot, w);
 }
 Tensor op_moe_gate_grad(const Tensor& buf, const Tensor& slot, const Tensor& g) {
-  if (ours(MOE_GATE_GRAD) && moe_ok({&buf, &slot, &g}) && float_or_bf16(buf.scalar_type()) && buf.dim() == 4 && g.scalar_type() == buf.scalar_type() && buf.size(1) > 0 &&
-      slot.dim() == 2 && slot.size(0) > 0 && slot.size(0) % buf.size(1) == 0) {
+  if (ours(MOE_GATE_GRAD) && moe_ok({&buf, &slot, &g}) && float_or_bf16(buf.scalar_type()) && buf.dim() == 4 &&
+      g.scalar_type() == buf.scalar_type() && buf.size(1) > 0 && slot.dim() == 2 && slot.size(0) > 0 && slot.size(0) % buf.size(1) == 0) {
     Tensor dw = at::empty(slot.sizes(), buf.options().dtype(at::kFloat));
     moe_gate_grad(buf.contiguous(), slot.contiguous(), g.contiguous(), dw);
     count();

@@ -360,8 +360,14 @@ struct SplitCosts {
   double l2, memory, memory_per_mb;                                                        // bytes per us; the last per megabyte in flight
   double long_chain, sum_width, sum_byte, sum_slice;                                       // us; per slice and 64 columns, per byte, per slice
 };
-constexpr SplitCosts EARLIER = {5.5, 0.5, 0.38, 5.5, 0.5, 0.35, 0.95, {0.27, 0.20, 0.27}, {5.6, 7.0, 9.0}, {5.6, 7.0, 9.0}, 9.5e6, 6.5e6, 0.62e6, 0.0, 0.05, 0.0, 0.0};
-constexpr SplitCosts FITTED = {3.35, 0.49, 0.45, 3.2, 0.87, 0.33, 1.0, {0.23, 0.26, 0.39}, {3.5, 4.0, 4.0}, {4.1, 4.1, 3.8}, 14.7e6, 8.6e6, 0.684e6, 0.31, 0.0, 1 / 18.7e3, 0.034};
+constexpr SplitCosts EARLIER = {5.5, 0.5, 0.38, 5.5, 0.5, 0.35, 0.95,
+                                {0.27, 0.20, 0.27}, {5.6, 7.0, 9.0}, {5.6, 7.0, 9.0},
+                                9.5e6, 6.5e6, 0.62e6,
+                                0.0, 0.05, 0.0, 0.0};
+constexpr SplitCosts FITTED = {3.35, 0.49, 0.45, 3.2, 0.87, 0.33, 1.0,
+                               {0.23, 0.26, 0.39}, {3.5, 4.0, 4.0}, {4.1, 4.1, 3.8},
+                               14.7e6, 8.6e6, 0.684e6,
+                               0.31, 0.0, 1 / 18.7e3, 0.034};
 
 // The fastest form by ``costs`` with at most ``max_chain`` k-blocks to a slice; the persistent kernels have them all.
 static SplitPlan split_pick(const SplitCosts& costs, int max_chain, int G, int M, int N, int K, int num_sms, int reserved) {
@@ -376,7 +382,8 @@ static SplitPlan split_pick(const SplitCosts& costs, int max_chain, int G, int M
   int units = pair ? apb_gemm_resident_pairs(num_sms) - reserved / 2 : usable;  // as the launches have it
   if (units < 1) units = 1;
   const double waves = (double)((tiles + units - 1) / units);
-  const double now = pair ? costs.pair_launch + waves * (costs.pair_wave + costs.pair_kb * kb) : costs.single_launch + waves * (costs.single_wave + costs.single_kb * kb);
+  const double now = pair ? costs.pair_launch + waves * (costs.pair_wave + costs.pair_kb * kb)
+                          : costs.single_launch + waves * (costs.single_wave + costs.single_kb * kb);
   const long long ctas = (tiles < units ? tiles : units) * (pair ? 2 : 1) * (kb <= 2 ? 2 : 1);
   const double operands = 2.0 * g * ((double)M * K + (double)N * K);
   const int* slots = split_slots(num_sms);

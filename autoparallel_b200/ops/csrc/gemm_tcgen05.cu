@@ -280,11 +280,13 @@ extern "C" int apb_gemm_grouped_bf16(const void* A, const void* B, void* C, int 
 
 // Footprint of the ``i``-th plain kernel that fills its SM's shared memory; -1 past the last.
 extern "C" int apb_gemm_footprint(int i, int* out) {
-#define APB_LAYOUTS(KERN, ...) \
-  (const void*)KERN<false, false __VA_ARGS__>, (const void*)KERN<false, true __VA_ARGS__>, (const void*)KERN<true, false __VA_ARGS__>, (const void*)KERN<true, true __VA_ARGS__>
+#define APB_LAYOUTS(KERN, ...)                                                                                      \
+  (const void*)KERN<false, false __VA_ARGS__>, (const void*)KERN<false, true __VA_ARGS__>,                          \
+      (const void*)KERN<true, false __VA_ARGS__>, (const void*)KERN<true, true __VA_ARGS__>
 #define APB_COMMA ,
-  static const void* const kernels[] = {APB_LAYOUTS(gemm_bf16_kernel), APB_LAYOUTS(gemm_bf16_pair_kernel), APB_LAYOUTS(gemm_bf16_pair_kernel, APB_COMMA 0 APB_COMMA true),
-                                        APB_LAYOUTS(gemm_grouped_kernel), APB_LAYOUTS(gemm_grouped_pair_kernel)};
+  static const void* const kernels[] = {APB_LAYOUTS(gemm_bf16_kernel), APB_LAYOUTS(gemm_bf16_pair_kernel),
+                                        APB_LAYOUTS(gemm_bf16_pair_kernel, APB_COMMA 0 APB_COMMA true), APB_LAYOUTS(gemm_grouped_kernel),
+                                        APB_LAYOUTS(gemm_grouped_pair_kernel)};
 #undef APB_LAYOUTS
 #undef APB_COMMA
   if (i < 0 || i >= (int)(sizeof(kernels) / sizeof(kernels[0]))) return -1;

@@ -497,8 +497,8 @@ def test_communication_kernels_fit_beside_a_gemm_cta(K):
                 assert gemm[2] + other[2] + 2 * 1024 <= sm.shared_memory_per_multiprocessor, (kind, gemm, other)
 
 
-@pytest.mark.parametrize("groups,M,N,K_,bn,slices", [(0, 2514, 256, 1096, 128, 2), (0, 2615, 176, 3416, 256, 4), (4, 1470, 200, 2024, 256, 2), (0, 155, 472, 7304, 128, 8),
-                                                     (0, 121, 10624, 2360, 256, 2)])
+@pytest.mark.parametrize("groups,M,N,K_,bn,slices", [
+    (0, 2514, 256, 1096, 128, 2), (0, 2615, 176, 3416, 256, 4), (4, 1470, 200, 2024, 256, 2), (0, 155, 472, 7304, 128, 8), (0, 121, 10624, 2360, 256, 2)])
 def test_a_faster_form_has_no_longer_chains(K, groups, M, N, K_, bn, slices):
     """The error of an fp32 result grows with the blocks that one chain of sums runs through; the form that the rule picks is as exact as
     the one given, which it took before the kernels got faster (a tenth for the order of the sums)."""

@@ -267,7 +267,8 @@ def test_an_installed_wrapper_is_what_the_next_call_runs(name):
 
     def equal(x, y):
         x, y = (x, y) if isinstance(x, tuple) else ((x,), (y,))
-        return all(torch.allclose(p, q, atol=1e-5) if name == "embedding_bwd" else torch.equal(p, q) for p, q in zip(x, y, strict=True))  # (atomics)
+        same = (lambda p, q: torch.allclose(p, q, atol=1e-5)) if name == "embedding_bwd" else torch.equal  # (atomics)
+        return all(map(same, x, y))
 
     register_cuda_impl(name, mine)
     try:
