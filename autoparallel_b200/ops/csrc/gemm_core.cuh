@@ -25,7 +25,6 @@
 //                   sums the n slots once every rank has signalled completion
 #pragma once
 #include "footprint.cuh"
-#include "footprint.cuh"
 #include "ptx.cuh"
 #include "symm_proto.cuh"
 
@@ -90,6 +89,7 @@ struct GemmParams {
   int* tile_counter = nullptr;
   // plain GEMM: divisors of the tile order, see plain_tile
   FastDiv div_group, div_tiles, div_tail;
+  int wide_tiles = 0, all_wide_tiles = 0;  // WIDE: tiles of two column tiles that stay whole, and all there are (see set_wide_tiles)
   int vec_store = 0;  // C leaves through shared memory in whole 128-byte lines (plain GEMM; needs 16-byte rows)
 };
 
@@ -126,10 +126,23 @@ __device__ __forceinline__ void tile_coords(int t, int num_m, int num_n, int& tm
 // Every tile goes through the contraction forwards, so that its bits depend neither on the launch (reserved SMs, pairs that are resident, tiles
 // handed out at run time) nor on where the tile lies: equal rows give equal results.  Backwards in every other round, for what L2 still holds
 // of the round before, saves power and with it time where a round reads more than L2 holds (8B feed-forward block 0 to 3 %), and gives that up.
-inline void set_tile_order(GemmParams& p, int num_m) {
-  p.div_group = FastDiv((uint32_t)GROUP_M * p.num_n_tiles);
-  p.div_tiles = FastDiv((uint32_t)num_m * p.num_n_tiles);
+inline void set_tile_order(GemmParams& p, int num_m, int num_n) {
+  p.div_group = FastDiv((uint32_t)GROUP_M * num_n);
+  p.div_tiles = FastDiv((uint32_t)num_m * num_n);
   p.div_tail = FastDiv(num_m % GROUP_M ? num_m % GROUP_M : GROUP_M);
+}
+// Whether a product of CTA pairs runs in wide tiles, and how many of them: whole waves of wide tiles, and the rest column tile by column tile
+// where that fits in half a wave.
+inline bool set_wide_tiles(GemmParams& p, int num_m, int units) {
+  const int num_n = (p.num_n_tiles + 1) / 2;
+  const long long all = (long long)num_m * num_n * p.groups;
+  if (2ll * (num_m < GROUP_M ? num_m : GROUP_M) * 2 * BM * p.K < 36000000ll) return false;
+  if (all < units || 2 * all > 0x7fffffffll) return false;
+  const int rest = (int)(all % units);
+  p.all_wide_tiles = (int)all;
+  p.wide_tiles = 2 * rest <= units ? (int)all - rest : (int)all;
+  set_tile_order(p, num_m, num_n);
+  return true;
 }
 __device__ __forceinline__ void plain_tile(const GemmParams& p, int num_m, bool grouped, int t, int& grp, int& tm, int& tn) {
   grp = grouped ? p.div_tiles.div(t) : 0;
@@ -401,16 +414,21 @@ __device__ __forceinline__ void gather_comm_warp(const GemmParams& p, const Fuse
 // persistent GEMM CTA), and that many pairs - never more than half of the launch - leave early; the tiles
 // they would have taken go to the pairs that stay.
 constexpr int TILE_RING = 4;
-template <bool A_MN, bool B_MN, int FUSE, bool PAIR = false, bool GROUPED = false, int ST_ARG = 0, bool DYN = false>
+constexpr int WIDE_RUN = 4;
+template <bool A_MN, bool B_MN, int FUSE, bool PAIR = false, bool GROUPED = false, int ST_ARG = 0, bool DYN = false, bool WIDE = false>
 __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p,
                                          const FuseParams& f, int cta, int num_ctas, uint8_t* smem_raw) {
   constexpr int STAGING = FUSE == FUSE_NONE && ST_ARG == 0 ? STAGING_BYTES : 0;  // (fewer stages: to leave shared memory free)
   constexpr int EPI = STAGING > 0 ? EPI_WARPS : 4;
   constexpr int EPI_COLS = BN * 4 / EPI;  // columns of the tile per epilogue warp
-  constexpr int ST = ST_ARG > 0 ? ST_ARG : (PAIR ? PAIR_STAGES : STAGES);
-  constexpr int A_BYTES = A_STAGE_BYTES;                          // 128 rows of A per CTA
-  constexpr int B_BYTES = PAIR ? B_STAGE_BYTES / 2 : B_STAGE_BYTES;  // PAIR: this CTA's 128 of the 256 B rows
+  constexpr int ST = ST_ARG > 0 ? ST_ARG : (PAIR && !WIDE ? PAIR_STAGES : STAGES);
+  constexpr int SUBS = WIDE ? 2 : 1;                                     // column tiles of BN that share their A
+  constexpr int A_BYTES = A_STAGE_BYTES;                                 // 128 rows of A per CTA
+  constexpr int SUB_BYTES = PAIR ? B_STAGE_BYTES / 2 : B_STAGE_BYTES;    // PAIR: this CTA's 128 of the 256 B rows
+  constexpr int B_BYTES = SUBS * SUB_BYTES;
   constexpr int B_ROWS = PAIR ? BN / 2 : BN;
+  constexpr bool NARROW = PAIR && FUSE == FUSE_NONE;  // column tiles with 128 columns or fewer take MMAs of 128
+  static_assert(!WIDE || (PAIR && FUSE == FUSE_NONE && ST_ARG == 0), "wide tiles: CTA pairs, plain GEMM");
   constexpr int TM = PAIR ? 2 * BM : BM;                          // tile rows
   static_assert(ST * (A_BYTES + B_BYTES) <= STAGES * (A_STAGE_BYTES + B_STAGE_BYTES), "stages must fit the launch's shared memory");
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -438,7 +456,7 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int tiles_per_group = num_m_units * p.num_n_tiles;
-  const int num_tiles = tiles_per_group * (GROUPED ? p.groups : 1);
+  const int num_tiles = WIDE ? 2 * p.all_wide_tiles - p.wide_tiles : tiles_per_group * (GROUPED ? p.groups : 1);
   const int num_kb = (p.K + BK - 1) / BK;
   // rotation that makes every rank start on data it already owns
   int m_rot = 0, n_rot = 0, k_rot = 0;
@@ -451,10 +469,18 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
     if (f.rows_per_shard % BN == 0 && p.num_n_tiles == (f.rows_per_shard / BN) * f.n) shard_n_tiles = f.rows_per_shard / BN;
     else n_rot = (f.rank * f.rows_per_shard) / BN;
   }
-  auto map_tile = [&](int t, int& grp, int& tm, int& tn) {
+  // Returns the number of column tiles, ``tn`` and the next one (WIDE; 0: the second half of a pair of columns that has only one).
+  auto map_tile = [&](int t, int& grp, int& tm, int& tn) -> int {
+    if (WIDE) {
+      const int r = t - p.wide_tiles;
+      const bool whole = r < 0;
+      plain_tile(p, num_m_units, GROUPED, whole ? t : p.wide_tiles + (r >> 1), grp, tm, tn);
+      tn = 2 * tn + (whole ? 0 : (r & 1));
+      return min(whole ? 2 : 1, p.num_n_tiles - tn);
+    }
     if (FUSE == FUSE_NONE) {
       plain_tile(p, num_m_units, GROUPED, t, grp, tm, tn);
-      return;
+      return 1;
     }
     grp = 0;
     if (shard_n_tiles > 0) {
@@ -467,7 +493,10 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
       tm = (tm + m_rot) % num_m_units;
       tn = (tn + n_rot) % p.num_n_tiles;
     }
+    return 1;
   };
+  // B rows that each CTA of a pair stages of a column tile
+  auto b_rows = [&](int tn) { return NARROW && p.N - tn * BN <= BN / 2 ? B_ROWS / 2 : B_ROWS; };
   if (FUSE == FUSE_GATHER_B && B_MN) k_rot = (f.rank * f.rows_per_shard) / BK;
   if (FUSE == FUSE_GATHER_A && A_MN) k_rot = (f.rank * f.rows_per_shard) / BK;
   if (FUSE == FUSE_REDUCE_SCATTER) m_rot = (((f.rank + 1) % f.n) * f.rows_per_rank) / TM;  // own rows last
@@ -590,9 +619,13 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
       for (int t = (DYN && half == 0) ? fetch_tile(tile_it) : read_tile(tile_it); t >= 0 && ok;
            t = (DYN && half == 0) ? fetch_tile(tile_it) : read_tile(tile_it)) {
         int grp, tm, tn;
-        map_tile(t, grp, tm, tn);
+        const int subs = map_tile(t, grp, tm, tn);
+        if (WIDE && subs <= 0) continue;
         // rows of A and of B that THIS CTA stages
-        const int m0 = tm * TM + (int)half * BM, n0 = tn * BN + (int)half * B_ROWS;
+        const int m0 = tm * TM + (int)half * BM, rows0 = b_rows(tn), n0 = tn * BN + (int)half * rows0;
+        const int rows1 = WIDE && subs > 1 ? b_rows(tn + 1) : 0, n1 = (tn + 1) * BN + (int)half * rows1;
+        // (a K-major box has 128 rows whatever the tile needs; MN-major boxes of 64 columns come one by one)
+        const uint32_t pair_bytes = 2 * (A_BYTES + (B_MN ? CHUNK_BYTES / 64 * (rows0 + rows1) : (rows1 > 0 ? 2 : 1) * SUB_BYTES));
         if ((FUSE == FUSE_GATHER_A && !A_MN) || (FUSE == FUSE_GATHER_B && !B_MN)) {
           // the tile's rows of the gathered operand must have landed
           const int r0 = (FUSE == FUSE_GATHER_A) ? m0 : n0;
@@ -635,7 +668,7 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
             }
           };
           if (PAIR) {
-            if (half == 0) mbar_expect_tx(&full[stage], 2 * (A_BYTES + B_BYTES));  // both CTAs' bytes land on the even CTA's barrier
+            if (half == 0) mbar_expect_tx(&full[stage], NARROW ? pair_bytes : 2 * (A_BYTES + B_BYTES));  // both CTAs' bytes land on the even CTA's barrier
           } else {
             mbar_expect_tx(&full[stage], A_BYTES + B_BYTES);
           }
@@ -647,9 +680,14 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
           }
           if (!B_MN) {
             load(b_dst, &tmB, kb * BK, n0);
+            if (WIDE && rows1 > 0) load(b_dst + SUB_BYTES, &tmB, kb * BK, n1);
           } else {
 #pragma unroll
-            for (int c = 0; c < B_ROWS / 64; ++c) load(b_dst + c * CHUNK_BYTES, &tmB, n0 + c * 64, kb * BK);
+            for (int c = 0; c < B_ROWS / 64; ++c)
+              if (!NARROW || c * 64 < rows0) load(b_dst + c * CHUNK_BYTES, &tmB, n0 + c * 64, kb * BK);
+#pragma unroll
+            for (int c = 0; WIDE && c < B_ROWS / 64; ++c)
+              if (c * 64 < rows1) load(b_dst + SUB_BYTES + c * CHUNK_BYTES, &tmB, n1 + c * 64, kb * BK);
           }
           if (++stage == ST) {
             stage = 0;
@@ -663,63 +701,90 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
     // One elected thread, descriptors as offsets from one base: the issue of a k-block cost about 300 ns before, more than its MMAs take.
     // 64 x 1280 x 2048 x 1408 387 -> 343 us, 8192 x 4096 x 4096 NN 194 -> 173, 2048 x 4096 x 4096 NN 59 -> 51.
     if (half == 0 && elect_one()) {
-      constexpr uint32_t idesc = make_idesc_bf16(TM, BN, A_MN ? 1u : 0u, B_MN ? 1u : 0u);
+      constexpr uint32_t idesc_full = make_idesc_bf16(TM, BN, A_MN ? 1u : 0u, B_MN ? 1u : 0u);
+      constexpr uint32_t idesc_half = make_idesc_bf16(TM, BN / 2, A_MN ? 1u : 0u, B_MN ? 1u : 0u);
       const uint64_t a_desc = make_smem_desc(smem_u32(sA), A_MN ? CHUNK_BYTES : 16, 1024);
       const uint64_t b_desc = make_smem_desc(smem_u32(sB), B_MN ? CHUNK_BYTES : 16, 1024);
       const uint32_t empty_even = PAIR ? map_to_cta(empty, 0) : 0u, empty_odd = PAIR ? map_to_cta(empty, 1) : 0u;
       int stage = 0;
       uint32_t phase = 0;
-      int buf = 0;
-      uint32_t buf_phase = 0;
+      uint32_t seq = 0;  // accumulators begun: the buffer is its last bit
       bool ok = true;
       int tile_it = 0;
       for (int t = read_tile(tile_it); t >= 0 && ok; t = read_tile(tile_it)) {
-        if (!mbar_wait(&tmem_empty[buf], buf_phase ^ 1, abort_flag)) {
-          atomicCAS(p.status, 0u, (uint32_t)ST_TIMEOUT_TMEM_EMPTY);
-          *abort_flag = 1;
-          break;
-        }
-        tc_fence_after();
-        const uint32_t d_tmem = tmem_base + buf * BN;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(&full[stage], phase, abort_flag)) {
-            ok = false;
-            atomicCAS(p.status, 0u, (uint32_t)ST_TIMEOUT_FULL);
-            *abort_flag = 1;
-            break;
-          }
-          tc_fence_after();
-          const uint64_t a_stage = a_desc + desc_offset(stage * A_BYTES), b_stage = b_desc + desc_offset(stage * B_BYTES);
+        int grp, tm, tn = 0, subs = 1;
+        if (NARROW) subs = map_tile(t, grp, tm, tn);
+        // WIDE: runs of k-blocks go through the first column tile and then through the second; one k-block a run, but for the first and the
+        // last of a tile, so that one accumulator is read out while the other one's run is under way.
+        for (int kb0 = 0; kb0 < num_kb && ok;) {
+          const int left = num_kb - kb0;
+          const int run = !WIDE ? 1 : kb0 == 0 ? min(WIDE_RUN, left) : left <= WIDE_RUN ? left : 1;
+          int end_stage = stage;
+          uint32_t end_phase = phase;
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            const uint64_t ad = a_stage + desc_offset(k * (A_MN ? UMMA_K * 128 : UMMA_K * 2));
-            const uint64_t bd = b_stage + desc_offset(k * (B_MN ? UMMA_K * 128 : UMMA_K * 2));
-            if (PAIR) umma_f16_pair(d_tmem, ad, bd, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-            else umma_f16(d_tmem, ad, bd, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          for (int sub = 0; sub < SUBS; ++sub) {
+            if (WIDE && (sub >= subs || !ok)) break;
+            const uint32_t buf = (seq + sub) & 1u;
+            if (kb0 == 0) {
+              if (!mbar_wait(&tmem_empty[buf], ((seq + sub) >> 1 & 1u) ^ 1u, abort_flag)) {
+                atomicCAS(p.status, 0u, (uint32_t)ST_TIMEOUT_TMEM_EMPTY);
+                *abort_flag = 1;
+                ok = false;
+                break;
+              }
+              tc_fence_after();
+            }
+            const uint32_t d_tmem = tmem_base + buf * BN;
+            const uint32_t idesc = NARROW && b_rows(tn + sub) < B_ROWS ? idesc_half : idesc_full;
+            end_stage = stage;
+            end_phase = phase;
+            for (int kb = kb0; kb < kb0 + run; ++kb) {
+              if (sub == 0) {
+                if (!mbar_wait(&full[end_stage], end_phase, abort_flag)) {
+                  ok = false;
+                  atomicCAS(p.status, 0u, (uint32_t)ST_TIMEOUT_FULL);
+                  *abort_flag = 1;
+                  break;
+                }
+                tc_fence_after();
+              }
+              const uint64_t a_stage = a_desc + desc_offset(end_stage * A_BYTES);
+              const uint64_t b_stage = b_desc + desc_offset(end_stage * B_BYTES + sub * SUB_BYTES);
+#pragma unroll
+              for (int k = 0; k < BK / UMMA_K; ++k) {
+                const uint64_t ad = a_stage + desc_offset(k * (A_MN ? UMMA_K * 128 : UMMA_K * 2));
+                const uint64_t bd = b_stage + desc_offset(k * (B_MN ? UMMA_K * 128 : UMMA_K * 2));
+                if (PAIR) umma_f16_pair(d_tmem, ad, bd, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                else umma_f16(d_tmem, ad, bd, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+              }
+              // stage reusable once these MMAs have read it (PAIR: in both CTAs)
+              if (!WIDE || sub == subs - 1) {
+                if (PAIR) {
+                  umma_commit_pair(empty_even + end_stage * 8);
+                  umma_commit_pair(empty_odd + end_stage * 8);
+                } else {
+                  umma_commit(&empty[end_stage]);
+                }
+              }
+              if (++end_stage == ST) {
+                end_stage = 0;
+                end_phase ^= 1;
+              }
+            }
+            if (ok && kb0 + run == num_kb) {  // the accumulator is complete
+              if (PAIR) {
+                umma_commit_pair(map_to_cta(&tmem_full[buf], 0));
+                umma_commit_pair(map_to_cta(&tmem_full[buf], 1));
+              } else {
+                umma_commit(&tmem_full[buf]);
+              }
+            }
           }
-          // stage reusable once these MMAs have read it (PAIR: in both CTAs)
-          if (PAIR) {
-            umma_commit_pair(empty_even + stage * 8);
-            umma_commit_pair(empty_odd + stage * 8);
-          } else {
-            umma_commit(&empty[stage]);
-          }
-          if (++stage == ST) {
-            stage = 0;
-            phase ^= 1;
-          }
+          stage = end_stage;
+          phase = end_phase;
+          kb0 += run;
         }
-        if (!ok) break;
-        if (PAIR) {
-          umma_commit_pair(map_to_cta(&tmem_full[buf], 0));
-          umma_commit_pair(map_to_cta(&tmem_full[buf], 1));
-        } else {
-          umma_commit(&tmem_full[buf]);
-        }
-        if (++buf == 2) {
-          buf = 0;
-          buf_phase ^= 1;
-        }
+        if (ok) seq += subs;
       }
     }
   } else if (GATHER && warp == 6) {
@@ -733,39 +798,43 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
     const int q = warp & 3;  // TMEM lane quarter this warp may read
     const int col0 = ((warp - 2) >> 2) * EPI_COLS;  // first of its columns
     const uint32_t tmem_empty_even = PAIR ? map_to_cta(tmem_empty, 0) : 0u;
-    int buf = 0;
-    uint32_t buf_phase = 0;
+    uint32_t seq = 0;  // accumulators read
+    bool ok = true;
     int tile_it = 0;
     auto next_epi_tile = [&]() -> int {  // lane 0 reads the sequence, the warp follows
       int t = 0;
       if (lane == 0) t = read_tile(tile_it);
       return __shfl_sync(0xffffffffu, t, 0);
     };
-    for (int t = next_epi_tile(); t >= 0; t = next_epi_tile()) {
+    for (int t = next_epi_tile(); t >= 0 && ok; t = next_epi_tile()) {
       int grp, tm, tn;
-      map_tile(t, grp, tm, tn);
+      const int subs = map_tile(t, grp, tm, tn);
+#pragma unroll 1
+      for (int sub = 0; sub < (WIDE ? subs : 1); ++sub, ++seq) {
+      const uint32_t buf = seq & 1u;
       const long long cta_row0 = (long long)tm * TM + (long long)half * BM;  // first of this CTA's 128 rows
       // (the TMEM loads are warp-wide: the warp goes on together or not at all)
-      if (!__all_sync(0xffffffffu, mbar_wait(&tmem_full[buf], buf_phase, abort_flag))) {
+      if (!__all_sync(0xffffffffu, mbar_wait(&tmem_full[buf], seq >> 1 & 1u, abort_flag))) {
         atomicCAS(p.status, 0u, (uint32_t)ST_TIMEOUT_TMEM_FULL);
         *abort_flag = 1;
+        ok = false;
         break;
       }
       tc_fence_after();
       const long long row = cta_row0 + q * 32 + lane;
-      const int n0 = tn * BN + col0;
+      const int n0 = (tn + sub) * BN + col0;
       const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + buf * BN + col0;
       float* rs_base = nullptr;
       if (FUSE == FUSE_REDUCE_SCATTER) {
         const int owner = (int)(cta_row0 / f.rows_per_rank);
         // the owner zeroes its accumulation buffer at the start of the step and then raises "ready"
-        bool ok = true;
+        bool raised = true;
         if (owner != f.rank) {
-          if (lane == 0) ok = apbs::wait_ge<true>(apbs::flag_ptr(f.peers.base[f.rank], apbs::OFF_READY, owner), f.epoch, p.status);
+          if (lane == 0) raised = apbs::wait_ge<true>(apbs::flag_ptr(f.peers.base[f.rank], apbs::OFF_READY, owner), f.epoch, p.status);
         } else {
-          if (lane == 0) ok = apbs::wait_ge<false>(apbs::flag_ptr(f.peers.base[f.rank], apbs::OFF_READY, owner), f.epoch, p.status);
+          if (lane == 0) raised = apbs::wait_ge<false>(apbs::flag_ptr(f.peers.base[f.rank], apbs::OFF_READY, owner), f.epoch, p.status);
         }
-        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+        ok = __shfl_sync(0xffffffffu, raised ? 1 : 0, 0) != 0;
         if (!ok) {
           *abort_flag = 1;
           break;
@@ -854,9 +923,6 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
         store_row_chunk(p, row, col, r, GROUPED ? (long long)grp * p.M * p.ldc : 0);
       }
       if (!staged) release();
-      if (++buf == 2) {
-        buf = 0;
-        buf_phase ^= 1;
       }
     }
   }

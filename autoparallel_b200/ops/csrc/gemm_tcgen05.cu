@@ -15,6 +15,8 @@
 // cuBLAS for the same nodes (autoparallel/graph_passes/graph_utils.py:320-412).
 #include "gemm_core.cuh"
 
+#include <type_traits>
+
 namespace apb {
 
 template <bool A_MN, bool B_MN>
@@ -25,12 +27,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   gemm_cta<A_MN, B_MN, FUSE_NONE>(tmA, tmB, p, f, blockIdx.x, gridDim.x, smem_raw);
 }
 
-template <bool A_MN, bool B_MN, int ST = 0, bool DYN = false>
+template <bool A_MN, bool B_MN, int ST = 0, bool DYN = false, bool WIDE = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ST == 0 ? GEMM_PLAIN_THREADS : GEMM_THREADS, ST == 0 ? GEMM_MIN_CTAS : 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
   FuseParams f{};
-  gemm_cta<A_MN, B_MN, FUSE_NONE, true, false, ST, DYN>(tmA, tmB, p, f, blockIdx.x, gridDim.x, smem_raw);
+  gemm_cta<A_MN, B_MN, FUSE_NONE, true, false, ST, DYN, WIDE>(tmA, tmB, p, f, blockIdx.x, gridDim.x, smem_raw);
 }
 
 // Grouped GEMM: G problems of one shape (the expert projections of a capacity-based MoE layer).
@@ -42,12 +44,12 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   gemm_cta<A_MN, B_MN, FUSE_NONE, false, true>(tmA, tmB, p, f, blockIdx.x, gridDim.x, smem_raw);
 }
 
-template <bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN, bool WIDE = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_PLAIN_THREADS, GEMM_MIN_CTAS)
 gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
   FuseParams f{};
-  gemm_cta<A_MN, B_MN, FUSE_NONE, true, true>(tmA, tmB, p, f, blockIdx.x, gridDim.x, smem_raw);
+  gemm_cta<A_MN, B_MN, FUSE_NONE, true, true, 0, false, WIDE>(tmA, tmB, p, f, blockIdx.x, gridDim.x, smem_raw);
 }
 
 static int g_pair_mode = 1;  // 0: one CTA per tile, 1: CTA pairs where the shape allows (default)
@@ -183,35 +185,36 @@ extern "C" int apb_gemm_bf16(const void* A, const void* B, void* C, int M, int N
     int resident = apb_gemm_resident_pairs(num_sms) - g_reserved_sms / 2;
     if (resident < 1) resident = 1;
     const int pairs = tiles2 < resident ? tiles2 : resident;
-    set_tile_order(p, (M + 2 * BM - 1) / (2 * BM));
+    const int num_m2 = (M + 2 * BM - 1) / (2 * BM);
+    const bool wide = g_pair_stages == PAIR_STAGES && set_wide_tiles(p, num_m2, resident);
+    if (!wide) set_tile_order(p, num_m2, p.num_n_tiles);
     const int smem2 = apb_gemm_pair_smem_bytes(g_pair_stages);
     const int threads2 = g_pair_stages == PAIR_STAGES ? GEMM_PLAIN_THREADS : GEMM_THREADS;
     auto launch2 = [&](auto kern) {
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2);
       kern<<<2 * pairs, threads2, smem2, stream>>>(tmA, tmB, p);
     };
-#define APB_LAUNCH_PAIR(ST)                                                              \
-  do {                                                                                   \
-    if (!a_mn_major && !b_mn_major) launch2(gemm_bf16_pair_kernel<false, false, ST>);    \
-    else if (!a_mn_major && b_mn_major) launch2(gemm_bf16_pair_kernel<false, true, ST>); \
-    else if (a_mn_major && !b_mn_major) launch2(gemm_bf16_pair_kernel<true, false, ST>); \
-    else launch2(gemm_bf16_pair_kernel<true, true, ST>);                                 \
+#define APB_LAUNCH_PAIR(...)                                                                      \
+  do {                                                                                            \
+    if (!a_mn_major && !b_mn_major) launch2(gemm_bf16_pair_kernel<false, false, __VA_ARGS__>);    \
+    else if (!a_mn_major && b_mn_major) launch2(gemm_bf16_pair_kernel<false, true, __VA_ARGS__>); \
+    else if (a_mn_major && !b_mn_major) launch2(gemm_bf16_pair_kernel<true, false, __VA_ARGS__>); \
+    else launch2(gemm_bf16_pair_kernel<true, true, __VA_ARGS__>);                                 \
   } while (0)
     int* counters = (g_dynamic_tiles && g_pair_stages == 6) ? tile_counters() : nullptr;
     if (counters != nullptr) {
       p.tile_counter = counters;
-      if (!a_mn_major && !b_mn_major) launch2(gemm_bf16_pair_kernel<false, false, 0, true>);
-      else if (!a_mn_major && b_mn_major) launch2(gemm_bf16_pair_kernel<false, true, 0, true>);
-      else if (a_mn_major && !b_mn_major) launch2(gemm_bf16_pair_kernel<true, false, 0, true>);
-      else launch2(gemm_bf16_pair_kernel<true, true, 0, true>);
+      if (wide) APB_LAUNCH_PAIR(0, true, true);
+      else APB_LAUNCH_PAIR(0, true);
     } else if (g_pair_stages == 4) APB_LAUNCH_PAIR(4);
     else if (g_pair_stages == 5) APB_LAUNCH_PAIR(5);
+    else if (wide) APB_LAUNCH_PAIR(0, false, true);
     else APB_LAUNCH_PAIR(0);
     return cudaGetLastError() == cudaSuccess ? 0 : 4;
   }
   const int tiles = p.num_m_tiles * p.num_n_tiles;
   const int grid = tiles < usable ? tiles : usable;
-  set_tile_order(p, p.num_m_tiles);
+  set_tile_order(p, p.num_m_tiles, p.num_n_tiles);
   auto launch = [&](auto kern) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_PLAIN_SMEM_BYTES);
     kern<<<grid, GEMM_PLAIN_THREADS, GEMM_PLAIN_SMEM_BYTES, stream>>>(tmA, tmB, p);
@@ -261,15 +264,24 @@ extern "C" int apb_gemm_grouped_bf16(const void* A, const void* B, void* C, int 
     int resident = apb_gemm_resident_pairs(num_sms) - g_reserved_sms / 2;
     if (resident < 1) resident = 1;
     const int grid = 2 * (int)(tiles2 < resident ? tiles2 : resident);
-    set_tile_order(p, (M + 2 * BM - 1) / (2 * BM));
-    if (!a_mn_major && !b_mn_major) launch(gemm_grouped_pair_kernel<false, false>, grid);
-    else if (!a_mn_major && b_mn_major) launch(gemm_grouped_pair_kernel<false, true>, grid);
-    else if (a_mn_major && !b_mn_major) launch(gemm_grouped_pair_kernel<true, false>, grid);
-    else launch(gemm_grouped_pair_kernel<true, true>, grid);
+    const int num_m2 = (M + 2 * BM - 1) / (2 * BM);
+    auto launch_layout = [&](auto wide) {
+      constexpr bool W = decltype(wide)::value;
+      if (!a_mn_major && !b_mn_major) launch(gemm_grouped_pair_kernel<false, false, W>, grid);
+      else if (!a_mn_major && b_mn_major) launch(gemm_grouped_pair_kernel<false, true, W>, grid);
+      else if (a_mn_major && !b_mn_major) launch(gemm_grouped_pair_kernel<true, false, W>, grid);
+      else launch(gemm_grouped_pair_kernel<true, true, W>, grid);
+    };
+    if (set_wide_tiles(p, num_m2, resident)) {
+      launch_layout(std::true_type{});
+    } else {
+      set_tile_order(p, num_m2, p.num_n_tiles);
+      launch_layout(std::false_type{});
+    }
   } else {
     const long long tiles = (long long)G * p.num_m_tiles * p.num_n_tiles;
     const int grid = (int)(tiles < usable ? tiles : usable);
-    set_tile_order(p, p.num_m_tiles);
+    set_tile_order(p, p.num_m_tiles, p.num_n_tiles);
     if (!a_mn_major && !b_mn_major) launch(gemm_grouped_kernel<false, false>, grid);
     else if (!a_mn_major && b_mn_major) launch(gemm_grouped_kernel<false, true>, grid);
     else if (a_mn_major && !b_mn_major) launch(gemm_grouped_kernel<true, false>, grid);
@@ -286,7 +298,10 @@ extern "C" int apb_gemm_footprint(int i, int* out) {
 #define APB_COMMA ,
   static const void* const kernels[] = {APB_LAYOUTS(gemm_bf16_kernel), APB_LAYOUTS(gemm_bf16_pair_kernel),
                                         APB_LAYOUTS(gemm_bf16_pair_kernel, APB_COMMA 0 APB_COMMA true), APB_LAYOUTS(gemm_grouped_kernel),
-                                        APB_LAYOUTS(gemm_grouped_pair_kernel)};
+                                        APB_LAYOUTS(gemm_grouped_pair_kernel),
+                                        APB_LAYOUTS(gemm_bf16_pair_kernel, APB_COMMA 0 APB_COMMA false APB_COMMA true),
+                                        APB_LAYOUTS(gemm_bf16_pair_kernel, APB_COMMA 0 APB_COMMA true APB_COMMA true),
+                                        APB_LAYOUTS(gemm_grouped_pair_kernel, APB_COMMA true)};
 #undef APB_LAYOUTS
 #undef APB_COMMA
   if (i < 0 || i >= (int)(sizeof(kernels) / sizeof(kernels[0]))) return -1;
