@@ -71,6 +71,21 @@ def test_gradients_match_the_portable_formulas(ops, name):
         assert ((a.cpu().double() - b.double()).norm() / b.double().norm()).item() <= 2**-6
 
 
+@pytest.mark.parametrize("name", ["rms_norm", "attention", "cross_entropy"])
+def test_the_second_output_has_no_gradient_of_its_own(ops, name):
+    """Used alone it gives zeros, as the zeros that stood for the first one's gradient did; used beside the first it adds nothing."""
+    (tensors, rest), _ = _case(name)
+    ins = [t.cuda() for t in tensors]
+    diff = [t.requires_grad_() for t in ins if t.is_floating_point()]
+    for x in torch.autograd.grad(_op(ops, name)(*ins, *rest)[1].sum(), diff):
+        assert x.abs().max().item() == 0
+    first, second = _op(ops, name)(*ins, *rest)
+    both = torch.autograd.grad(first.float().sum() + second.sum(), diff)
+    alone = torch.autograd.grad(_op(ops, name)(*ins, *rest)[0].float().sum(), diff)
+    # (one rounding apart at most: the library's attention backward may add up in another order)
+    assert all((a - b).float().norm() <= 2**-8 * b.float().norm() for a, b in zip(both, alone))
+
+
 @pytest.mark.parametrize("name", NAMES)
 def test_no_gradient_is_recorded_when_none_is_asked_for(ops, name):
     (tensors, rest), _ = _case(name)
