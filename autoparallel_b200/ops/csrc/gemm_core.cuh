@@ -8,7 +8,8 @@
 //                 32 KB per k-block instead of 48 KB and six stages fit.  TMA transaction bytes and
 //                 the epilogues' "accumulator free" arrivals go to the even CTA's barriers; "stage
 //                 free" and "accumulator full" are committed by the MMA thread to each CTA's barrier
-//                 separately (two plain commits; no multicast anywhere).
+//                 separately (two plain commits; no multicast anywhere).  A column tile with 128 columns or
+//                 fewer takes MMAs of 128 (64 x 1280 x 1408 x 2048, whose last one is half empty: 434 -> 427 us).
 //   warp 0: TMA producer | warp 1: TMEM owner + MMA issuer | warps 2..9 (2..5 in the fused kernels and with fewer stages): epilogue
 //   warp 6 (gather-fused kernels only): copy engine driver, see gather_comm_warp
 //
@@ -89,7 +90,7 @@ struct GemmParams {
   int* tile_counter = nullptr;
   // plain GEMM: divisors of the tile order, see plain_tile
   FastDiv div_group, div_tiles, div_tail;
-  int wide_tiles = 0, all_wide_tiles = 0;  // WIDE: tiles of two column tiles that stay whole, and all there are (see set_wide_tiles)
+  int whole_tiles = 0, all_tiles = 0;  // CTA pairs, plain GEMM: tiles that stay whole, and all there are (see set_pair_tiles)
   int vec_store = 0;  // C leaves through shared memory in whole 128-byte lines (plain GEMM; needs 16-byte rows)
 };
 
@@ -131,18 +132,27 @@ inline void set_tile_order(GemmParams& p, int num_m, int num_n) {
   p.div_tiles = FastDiv((uint32_t)num_m * num_n);
   p.div_tail = FastDiv(num_m % GROUP_M ? num_m % GROUP_M : GROUP_M);
 }
-// Whether a product of CTA pairs runs in wide tiles, and how many of them: whole waves of wide tiles, and the rest column tile by column tile
-// where that fits in half a wave.
-inline bool set_wide_tiles(GemmParams& p, int num_m, int units) {
-  const int num_n = (p.num_n_tiles + 1) / 2;
+// Tiles of a product of CTA pairs, and whether they are wide (256 x 512).
+//
+// Halves: whole waves of tiles, then the rest in halves of their columns where those fit in one wave, which then takes half the time (a little
+// more: a half tile brings in three quarters of the operands).  4096 x 1408 x 2048, 96 tiles on 74 pairs: 25.0 -> 21.9 us; 1500 x 4096 x 2048
+// 25.5 -> 22.1, 2048 x 5632 x 1024 21.5 -> 19.9, 64 x 160 x 1408 x 2048 81 -> 78.  Above half a wave of tiles the halves would take two.
+//
+// Wide tiles read A half as often: every wave of tiles goes through the row group's panel of A (16 tile rows) once, and where that no longer
+// stays in L2 from one wave to the next it comes from memory again.  The line lies where that begins, at 36 MB (4096 rows: K = 4394).
+// Narrow -> wide, us at the power cap: 4096 rows of A in a group, N = 4096, K = 4096 205 -> 204, 5120 262 -> 252, 8192 430 -> 401, 14336 747 ->
+// 700; N = 10240, K = 4608 291.9 -> 290.5, 8192 540 -> 511; 2048 rows, N = 14336, K = 5632 259 -> 261, 8192 380 -> 374, 11008 514 -> 496; 8192 x
+// 128256 x 8192 and its like gain 5 to 8 %.  Short contractions lose: K = 512 6 to 8 %, 256 2 to 8 %.
+inline bool set_pair_tiles(GemmParams& p, int num_m, int units, bool may_be_wide) {
+  const bool wide = may_be_wide && 2ll * (num_m < GROUP_M ? num_m : GROUP_M) * 2 * BM * p.K >= 36000000ll &&
+                    (long long)num_m * ((p.num_n_tiles + 1) / 2) * p.groups >= units;
+  const int num_n = wide ? (p.num_n_tiles + 1) / 2 : p.num_n_tiles;
   const long long all = (long long)num_m * num_n * p.groups;
-  if (2ll * (num_m < GROUP_M ? num_m : GROUP_M) * 2 * BM * p.K < 36000000ll) return false;
-  if (all < units || 2 * all > 0x7fffffffll) return false;
   const int rest = (int)(all % units);
-  p.all_wide_tiles = (int)all;
-  p.wide_tiles = 2 * rest <= units ? (int)all - rest : (int)all;
+  p.all_tiles = (int)all;
+  p.whole_tiles = 2 * rest <= units ? (int)all - rest : (int)all;
   set_tile_order(p, num_m, num_n);
-  return true;
+  return wide;
 }
 __device__ __forceinline__ void plain_tile(const GemmParams& p, int num_m, bool grouped, int t, int& grp, int& tm, int& tn) {
   grp = grouped ? p.div_tiles.div(t) : 0;
@@ -414,6 +424,9 @@ __device__ __forceinline__ void gather_comm_warp(const GemmParams& p, const Fuse
 // persistent GEMM CTA), and that many pairs - never more than half of the launch - leave early; the tiles
 // they would have taken go to the pairs that stay.
 constexpr int TILE_RING = 4;
+// WIDE: a tile of two column tiles, whose MMAs take turns on the stages (16 KB of A, 2 x 16 KB of B per CTA; four of them) and go to one TMEM
+// buffer each.  The turns are one k-block long, but WIDE_RUN at the ends of the contraction: the first accumulator is complete that much before
+// the second and is read out meanwhile, and the next tile begins with it.  Runs of 4 / 2 / 1 blocks: 8192 x 128256 x 4096 6129 / 6255 / 6348 us.
 constexpr int WIDE_RUN = 4;
 template <bool A_MN, bool B_MN, int FUSE, bool PAIR = false, bool GROUPED = false, int ST_ARG = 0, bool DYN = false, bool WIDE = false>
 __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p,
@@ -456,7 +469,7 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int tiles_per_group = num_m_units * p.num_n_tiles;
-  const int num_tiles = WIDE ? 2 * p.all_wide_tiles - p.wide_tiles : tiles_per_group * (GROUPED ? p.groups : 1);
+  const int num_tiles = NARROW ? 2 * p.all_tiles - p.whole_tiles : tiles_per_group * (GROUPED ? p.groups : 1);
   const int num_kb = (p.K + BK - 1) / BK;
   // rotation that makes every rank start on data it already owns
   int m_rot = 0, n_rot = 0, k_rot = 0;
@@ -469,34 +482,42 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
     if (f.rows_per_shard % BN == 0 && p.num_n_tiles == (f.rows_per_shard / BN) * f.n) shard_n_tiles = f.rows_per_shard / BN;
     else n_rot = (f.rank * f.rows_per_shard) / BN;
   }
-  // Returns the number of column tiles, ``tn`` and the next one (WIDE; 0: the second half of a pair of columns that has only one).
-  auto map_tile = [&](int t, int& grp, int& tm, int& tn) -> int {
-    if (WIDE) {
-      const int r = t - p.wide_tiles;
+  struct Tile {
+    int grp, tm, col;  // group, row tile, first column
+    int subs, width;   // column tiles (0: nothing, the second half of a tile whose columns end in the first), and columns of one
+  };
+  auto map_tile = [&](int t) -> Tile {
+    Tile x{0, 0, 0, 1, BN};
+    int tn;
+    if (NARROW) {
+      const int r = t - p.whole_tiles;
       const bool whole = r < 0;
-      plain_tile(p, num_m_units, GROUPED, whole ? t : p.wide_tiles + (r >> 1), grp, tm, tn);
-      tn = 2 * tn + (whole ? 0 : (r & 1));
-      return min(whole ? 2 : 1, p.num_n_tiles - tn);
+      plain_tile(p, num_m_units, GROUPED, whole ? t : p.whole_tiles + (r >> 1), x.grp, x.tm, tn);
+      if (!WIDE && !whole) x.width = BN / 2;
+      x.col = tn * SUBS * BN + (whole || !(r & 1) ? 0 : SUBS * BN / 2);
+      x.subs = x.col >= p.N ? 0 : WIDE && whole && x.col + BN < p.N ? 2 : 1;
+      return x;
     }
     if (FUSE == FUSE_NONE) {
-      plain_tile(p, num_m_units, GROUPED, t, grp, tm, tn);
-      return 1;
+      plain_tile(p, num_m_units, GROUPED, t, x.grp, x.tm, tn);
+      x.col = tn * BN;
+      return x;
     }
-    grp = 0;
     if (shard_n_tiles > 0) {
       const int per_shard = num_m_units * shard_n_tiles;
       const int s = t / per_shard;
-      tile_coords(t - s * per_shard, num_m_units, shard_n_tiles, tm, tn);
+      tile_coords(t - s * per_shard, num_m_units, shard_n_tiles, x.tm, tn);
       tn += ((s + f.rank) % f.n) * shard_n_tiles;
     } else {
-      tile_coords(t, num_m_units, p.num_n_tiles, tm, tn);
-      tm = (tm + m_rot) % num_m_units;
+      tile_coords(t, num_m_units, p.num_n_tiles, x.tm, tn);
+      x.tm = (x.tm + m_rot) % num_m_units;
       tn = (tn + n_rot) % p.num_n_tiles;
     }
-    return 1;
+    x.col = tn * BN;
+    return x;
   };
-  // B rows that each CTA of a pair stages of a column tile
-  auto b_rows = [&](int tn) { return NARROW && p.N - tn * BN <= BN / 2 ? B_ROWS / 2 : B_ROWS; };
+  // whether a column tile takes MMAs (and B rows) of half the width
+  auto narrow = [&](const Tile& x, int sub) { return NARROW && (x.width < BN || p.N - (x.col + sub * BN) <= BN / 2); };
   if (FUSE == FUSE_GATHER_B && B_MN) k_rot = (f.rank * f.rows_per_shard) / BK;
   if (FUSE == FUSE_GATHER_A && A_MN) k_rot = (f.rank * f.rows_per_shard) / BK;
   if (FUSE == FUSE_REDUCE_SCATTER) m_rot = (((f.rank + 1) % f.n) * f.rows_per_rank) / TM;  // own rows last
@@ -618,12 +639,12 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
       int tile_it = 0;
       for (int t = (DYN && half == 0) ? fetch_tile(tile_it) : read_tile(tile_it); t >= 0 && ok;
            t = (DYN && half == 0) ? fetch_tile(tile_it) : read_tile(tile_it)) {
-        int grp, tm, tn;
-        const int subs = map_tile(t, grp, tm, tn);
-        if (WIDE && subs <= 0) continue;
+        const Tile x = map_tile(t);
+        if (NARROW && x.subs == 0) continue;
+        const int grp = x.grp;
         // rows of A and of B that THIS CTA stages
-        const int m0 = tm * TM + (int)half * BM, rows0 = b_rows(tn), n0 = tn * BN + (int)half * rows0;
-        const int rows1 = WIDE && subs > 1 ? b_rows(tn + 1) : 0, n1 = (tn + 1) * BN + (int)half * rows1;
+        const int m0 = x.tm * TM + (int)half * BM, rows0 = narrow(x, 0) ? B_ROWS / 2 : B_ROWS, n0 = x.col + (int)half * rows0;
+        const int rows1 = !WIDE || x.subs < 2 ? 0 : narrow(x, 1) ? B_ROWS / 2 : B_ROWS, n1 = x.col + BN + (int)half * rows1;
         // (a K-major box has 128 rows whatever the tile needs; MN-major boxes of 64 columns come one by one)
         const uint32_t pair_bytes = 2 * (A_BYTES + (B_MN ? CHUNK_BYTES / 64 * (rows0 + rows1) : (rows1 > 0 ? 2 : 1) * SUB_BYTES));
         if ((FUSE == FUSE_GATHER_A && !A_MN) || (FUSE == FUSE_GATHER_B && !B_MN)) {
@@ -712,8 +733,10 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
       bool ok = true;
       int tile_it = 0;
       for (int t = read_tile(tile_it); t >= 0 && ok; t = read_tile(tile_it)) {
-        int grp, tm, tn = 0, subs = 1;
-        if (NARROW) subs = map_tile(t, grp, tm, tn);
+        Tile x{};
+        x.subs = 1;
+        if (NARROW) x = map_tile(t);
+        if (NARROW && x.subs == 0) continue;
         // WIDE: runs of k-blocks go through the first column tile and then through the second; one k-block a run, but for the first and the
         // last of a tile, so that one accumulator is read out while the other one's run is under way.
         for (int kb0 = 0; kb0 < num_kb && ok;) {
@@ -723,7 +746,7 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
           uint32_t end_phase = phase;
 #pragma unroll
           for (int sub = 0; sub < SUBS; ++sub) {
-            if (WIDE && (sub >= subs || !ok)) break;
+            if (WIDE && (sub >= x.subs || !ok)) break;
             const uint32_t buf = (seq + sub) & 1u;
             if (kb0 == 0) {
               if (!mbar_wait(&tmem_empty[buf], ((seq + sub) >> 1 & 1u) ^ 1u, abort_flag)) {
@@ -735,7 +758,7 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
               tc_fence_after();
             }
             const uint32_t d_tmem = tmem_base + buf * BN;
-            const uint32_t idesc = NARROW && b_rows(tn + sub) < B_ROWS ? idesc_half : idesc_full;
+            const uint32_t idesc = narrow(x, sub) ? idesc_half : idesc_full;
             end_stage = stage;
             end_phase = phase;
             for (int kb = kb0; kb < kb0 + run; ++kb) {
@@ -758,7 +781,7 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
                 else umma_f16(d_tmem, ad, bd, idesc, (kb > 0 || k > 0) ? 1u : 0u);
               }
               // stage reusable once these MMAs have read it (PAIR: in both CTAs)
-              if (!WIDE || sub == subs - 1) {
+              if (!WIDE || sub == x.subs - 1) {
                 if (PAIR) {
                   umma_commit_pair(empty_even + end_stage * 8);
                   umma_commit_pair(empty_odd + end_stage * 8);
@@ -784,7 +807,7 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
           phase = end_phase;
           kb0 += run;
         }
-        if (ok) seq += subs;
+        if (ok) seq += WIDE ? x.subs : 1;
       }
     }
   } else if (GATHER && warp == 6) {
@@ -796,7 +819,7 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
   } else {
     // ------------------------------------------------------------------ epilogue (warps 2..)
     const int q = warp & 3;  // TMEM lane quarter this warp may read
-    const int col0 = ((warp - 2) >> 2) * EPI_COLS;  // first of its columns
+    const int part = (warp - 2) >> 2;  // of the tile's columns
     const uint32_t tmem_empty_even = PAIR ? map_to_cta(tmem_empty, 0) : 0u;
     uint32_t seq = 0;  // accumulators read
     bool ok = true;
@@ -807,122 +830,122 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
       return __shfl_sync(0xffffffffu, t, 0);
     };
     for (int t = next_epi_tile(); t >= 0 && ok; t = next_epi_tile()) {
-      int grp, tm, tn;
-      const int subs = map_tile(t, grp, tm, tn);
+      const Tile x = map_tile(t);
 #pragma unroll 1
-      for (int sub = 0; sub < (WIDE ? subs : 1); ++sub, ++seq) {
-      const uint32_t buf = seq & 1u;
-      const long long cta_row0 = (long long)tm * TM + (long long)half * BM;  // first of this CTA's 128 rows
-      // (the TMEM loads are warp-wide: the warp goes on together or not at all)
-      if (!__all_sync(0xffffffffu, mbar_wait(&tmem_full[buf], seq >> 1 & 1u, abort_flag))) {
-        atomicCAS(p.status, 0u, (uint32_t)ST_TIMEOUT_TMEM_FULL);
-        *abort_flag = 1;
-        ok = false;
-        break;
-      }
-      tc_fence_after();
-      const long long row = cta_row0 + q * 32 + lane;
-      const int n0 = (tn + sub) * BN + col0;
-      const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + buf * BN + col0;
-      float* rs_base = nullptr;
-      if (FUSE == FUSE_REDUCE_SCATTER) {
-        const int owner = (int)(cta_row0 / f.rows_per_rank);
-        // the owner zeroes its accumulation buffer at the start of the step and then raises "ready"
-        bool raised = true;
-        if (owner != f.rank) {
-          if (lane == 0) raised = apbs::wait_ge<true>(apbs::flag_ptr(f.peers.base[f.rank], apbs::OFF_READY, owner), f.epoch, p.status);
-        } else {
-          if (lane == 0) raised = apbs::wait_ge<false>(apbs::flag_ptr(f.peers.base[f.rank], apbs::OFF_READY, owner), f.epoch, p.status);
-        }
-        ok = __shfl_sync(0xffffffffu, raised ? 1 : 0, 0) != 0;
-        if (!ok) {
+      for (int sub = 0; sub < (NARROW ? x.subs : 1); ++sub, ++seq) {
+        const uint32_t buf = seq & 1u;
+        const long long cta_row0 = (long long)x.tm * TM + (long long)half * BM;  // first of this CTA's 128 rows
+        // (the TMEM loads are warp-wide: the warp goes on together or not at all)
+        if (!__all_sync(0xffffffffu, mbar_wait(&tmem_full[buf], seq >> 1 & 1u, abort_flag))) {
+          atomicCAS(p.status, 0u, (uint32_t)ST_TIMEOUT_TMEM_FULL);
           *abort_flag = 1;
+          ok = false;
           break;
         }
-        // slot ``rank`` of the owner's staging area: [n][rows_per_rank][N], fp32 or bf16; rs_base is kept
-        // in units of fp32 elements of an fp32 slot and halved below for bf16 slots
-        rs_base = reinterpret_cast<float*>(f.peers.base[owner] + apbs::HEADER_BYTES) +
-                  ((long long)f.rank * f.rows_per_rank + (row - (long long)owner * f.rows_per_rank)) * p.N;
-      }
-      auto release = [&]() {  // this warp has read its rows of the accumulator
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) {
-          if (PAIR) mbar_arrive_cluster_plain(tmem_empty_even + buf * 8);
-          else mbar_arrive(&tmem_empty[buf]);
-        }
-      };
-      const bool staged = STAGING > 0 && p.vec_store;
-      if (staged) {
-        uint8_t* stg = smem + ST * (A_BYTES + B_BYTES) + (warp - 2) * STORE_BYTES;
-        const long long c_off = GROUPED ? (long long)grp * p.M * p.ldc : 0;
-        const int r0 = (int)cta_row0 + q * 32;
-        if (p.out_fp32) store_tile<true>(reinterpret_cast<float*>(p.C) + c_off, p.ldc, stg, taddr, r0, n0, EPI_COLS, p.M, p.N, lane, release);
-        else store_tile<false>(reinterpret_cast<__nv_bfloat16*>(p.C) + c_off, p.ldc, stg, taddr, r0, n0, EPI_COLS, p.M, p.N, lane, release);
-      }
-#pragma unroll 1
-      for (int c = 0; c < EPI_COLS / 32 && !staged; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32(taddr + c * 32, r);
-        tmem_ld_wait();
-        const int col = n0 + c * 32;
+        tc_fence_after();
+        const long long row = cta_row0 + q * 32 + lane;
+        const int cols = narrow(x, sub) ? EPI_COLS / 2 : EPI_COLS, col0 = part * cols;  // this warp's columns
+        const int n0 = x.col + sub * BN + col0;
+        const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + buf * BN + col0;
+        float* rs_base = nullptr;
         if (FUSE == FUSE_REDUCE_SCATTER) {
-          // Transpose the warp's 32x32 block through shared memory so that every store instruction
-          // writes four 128-byte row segments: NVLink moves full segments instead of 16-byte crumbs.
-          float* stg = reinterpret_cast<float*>(smem + ST * (A_BYTES + B_BYTES) + 256) + (warp - 2) * EPI_STAGE_FLOATS;
-#pragma unroll
-          for (int i = 0; i < 32; ++i) stg[lane * 33 + i] = __uint_as_float(r[i]);
+          const int owner = (int)(cta_row0 / f.rows_per_rank);
+          // the owner zeroes its accumulation buffer at the start of the step and then raises "ready"
+          bool raised = true;
+          if (owner != f.rank) {
+            if (lane == 0) raised = apbs::wait_ge<true>(apbs::flag_ptr(f.peers.base[f.rank], apbs::OFF_READY, owner), f.epoch, p.status);
+          } else {
+            if (lane == 0) raised = apbs::wait_ge<false>(apbs::flag_ptr(f.peers.base[f.rank], apbs::OFF_READY, owner), f.epoch, p.status);
+          }
+          ok = __shfl_sync(0xffffffffu, raised ? 1 : 0, 0) != 0;
+          if (!ok) {
+            *abort_flag = 1;
+            break;
+          }
+          // slot ``rank`` of the owner's staging area: [n][rows_per_rank][N], fp32 or bf16; rs_base is kept
+          // in units of fp32 elements of an fp32 slot and halved below for bf16 slots
+          rs_base = reinterpret_cast<float*>(f.peers.base[owner] + apbs::HEADER_BYTES) +
+                    ((long long)f.rank * f.rows_per_rank + (row - (long long)owner * f.rows_per_rank)) * p.N;
+        }
+        auto release = [&]() {  // this warp has read its rows of the accumulator
+          tc_fence_before();
           __syncwarp();
-          const long long row0 = cta_row0 + q * 32;  // first row of this warp's block
-          float* blk = rs_base - (long long)lane * p.N;         // rs_base points at this lane's row
-          if (f.slot_bf16) {
-            // 8 bf16 (16 bytes) per lane, 4 lanes per 64-byte row segment, 8 rows per instruction
-            __nv_bfloat16* blk16 = reinterpret_cast<__nv_bfloat16*>(f.peers.base[(int)(cta_row0 / f.rows_per_rank)] + apbs::HEADER_BYTES) +
-                                   (blk - reinterpret_cast<float*>(f.peers.base[(int)(cta_row0 / f.rows_per_rank)] + apbs::HEADER_BYTES));
-            const int sub8 = lane >> 2, seg8 = (lane & 3) * 8;
+          if (lane == 0) {
+            if (PAIR) mbar_arrive_cluster_plain(tmem_empty_even + buf * 8);
+            else mbar_arrive(&tmem_empty[buf]);
+          }
+        };
+        const bool staged = STAGING > 0 && p.vec_store;
+        if (staged) {
+          uint8_t* stg = smem + ST * (A_BYTES + B_BYTES) + (warp - 2) * STORE_BYTES;
+          const long long c_off = GROUPED ? (long long)x.grp * p.M * p.ldc : 0;
+          const int r0 = (int)cta_row0 + q * 32;
+          if (p.out_fp32) store_tile<true>(reinterpret_cast<float*>(p.C) + c_off, p.ldc, stg, taddr, r0, n0, cols, p.M, p.N, lane, release);
+          else store_tile<false>(reinterpret_cast<__nv_bfloat16*>(p.C) + c_off, p.ldc, stg, taddr, r0, n0, cols, p.M, p.N, lane, release);
+        }
+#pragma unroll 1
+        for (int c = 0; c < cols / 32 && !staged; ++c) {
+          uint32_t r[32];
+          tmem_ld_32x32(taddr + c * 32, r);
+          tmem_ld_wait();
+          const int col = n0 + c * 32;
+          if (FUSE == FUSE_REDUCE_SCATTER) {
+            // Transpose the warp's 32x32 block through shared memory so that every store instruction
+            // writes four 128-byte row segments: NVLink moves full segments instead of 16-byte crumbs.
+            float* stg = reinterpret_cast<float*>(smem + ST * (A_BYTES + B_BYTES) + 256) + (warp - 2) * EPI_STAGE_FLOATS;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const int rr = sub8 + 8 * j;
+            for (int i = 0; i < 32; ++i) stg[lane * 33 + i] = __uint_as_float(r[i]);
+            __syncwarp();
+            const long long row0 = cta_row0 + q * 32;  // first row of this warp's block
+            float* blk = rs_base - (long long)lane * p.N;         // rs_base points at this lane's row
+            if (f.slot_bf16) {
+              // 8 bf16 (16 bytes) per lane, 4 lanes per 64-byte row segment, 8 rows per instruction
+              __nv_bfloat16* blk16 = reinterpret_cast<__nv_bfloat16*>(f.peers.base[(int)(cta_row0 / f.rows_per_rank)] + apbs::HEADER_BYTES) +
+                                     (blk - reinterpret_cast<float*>(f.peers.base[(int)(cta_row0 / f.rows_per_rank)] + apbs::HEADER_BYTES));
+              const int sub8 = lane >> 2, seg8 = (lane & 3) * 8;
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const int rr = sub8 + 8 * j;
+                if (row0 + rr < p.M) {
+                  const float* sp = stg + rr * 33 + seg8;
+                  __nv_bfloat16* dst = blk16 + (long long)rr * p.N + col + seg8;
+                  if (col + seg8 + 8 <= p.N) {
+                    uint4 v;
+                    v.x = pack_bf16(sp[0], sp[1]);
+                    v.y = pack_bf16(sp[2], sp[3]);
+                    v.z = pack_bf16(sp[4], sp[5]);
+                    v.w = pack_bf16(sp[6], sp[7]);
+                    *reinterpret_cast<uint4*>(dst) = v;
+                  } else {
+                    for (int e = 0; e < 8; ++e)
+                      if (col + seg8 + e < p.N) dst[e] = __float2bfloat16(sp[e]);
+                  }
+                }
+              }
+              __syncwarp();
+              continue;
+            }
+            const int sub = lane >> 3, seg = (lane & 7) * 4;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const int rr = sub + 4 * j;
               if (row0 + rr < p.M) {
-                const float* sp = stg + rr * 33 + seg8;
-                __nv_bfloat16* dst = blk16 + (long long)rr * p.N + col + seg8;
-                if (col + seg8 + 8 <= p.N) {
-                  uint4 v;
-                  v.x = pack_bf16(sp[0], sp[1]);
-                  v.y = pack_bf16(sp[2], sp[3]);
-                  v.z = pack_bf16(sp[4], sp[5]);
-                  v.w = pack_bf16(sp[6], sp[7]);
-                  *reinterpret_cast<uint4*>(dst) = v;
+                const float* sp = stg + rr * 33 + seg;
+                float* dst = blk + (long long)rr * p.N + col + seg;
+                if (col + seg + 4 <= p.N) {
+                  *reinterpret_cast<float4*>(dst) = make_float4(sp[0], sp[1], sp[2], sp[3]);
                 } else {
-                  for (int e = 0; e < 8; ++e)
-                    if (col + seg8 + e < p.N) dst[e] = __float2bfloat16(sp[e]);
+                  for (int e = 0; e < 4; ++e)
+                    if (col + seg + e < p.N) dst[e] = sp[e];
                 }
               }
             }
             __syncwarp();
             continue;
           }
-          const int sub = lane >> 3, seg = (lane & 7) * 4;
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int rr = sub + 4 * j;
-            if (row0 + rr < p.M) {
-              const float* sp = stg + rr * 33 + seg;
-              float* dst = blk + (long long)rr * p.N + col + seg;
-              if (col + seg + 4 <= p.N) {
-                *reinterpret_cast<float4*>(dst) = make_float4(sp[0], sp[1], sp[2], sp[3]);
-              } else {
-                for (int e = 0; e < 4; ++e)
-                  if (col + seg + e < p.N) dst[e] = sp[e];
-              }
-            }
-          }
-          __syncwarp();
-          continue;
+          store_row_chunk(p, row, col, r, GROUPED ? (long long)x.grp * p.M * p.ldc : 0);
         }
-        store_row_chunk(p, row, col, r, GROUPED ? (long long)grp * p.M * p.ldc : 0);
-      }
-      if (!staged) release();
+        if (!staged) release();
       }
     }
   }

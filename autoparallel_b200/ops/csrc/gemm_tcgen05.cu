@@ -181,13 +181,11 @@ extern "C" int apb_gemm_bf16(const void* A, const void* B, void* C, int M, int N
     int e2 = 0;
     if (!b_mn_major) e2 = make_map(&tmB, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, BN / 2);
     if (e2) return e2;
-    const int tiles2 = ((M + 2 * BM - 1) / (2 * BM)) * p.num_n_tiles;
     int resident = apb_gemm_resident_pairs(num_sms) - g_reserved_sms / 2;
     if (resident < 1) resident = 1;
-    const int pairs = tiles2 < resident ? tiles2 : resident;
     const int num_m2 = (M + 2 * BM - 1) / (2 * BM);
-    const bool wide = g_pair_stages == PAIR_STAGES && set_wide_tiles(p, num_m2, resident);
-    if (!wide) set_tile_order(p, num_m2, p.num_n_tiles);
+    const bool wide = set_pair_tiles(p, num_m2, resident, g_pair_stages == PAIR_STAGES);
+    const int units = 2 * p.all_tiles - p.whole_tiles, pairs = units < resident ? units : resident;
     const int smem2 = apb_gemm_pair_smem_bytes(g_pair_stages);
     const int threads2 = g_pair_stages == PAIR_STAGES ? GEMM_PLAIN_THREADS : GEMM_THREADS;
     auto launch2 = [&](auto kern) {
@@ -260,24 +258,20 @@ extern "C" int apb_gemm_grouped_bf16(const void* A, const void* B, void* C, int 
     kern<<<grid, GEMM_PLAIN_THREADS, GEMM_PLAIN_SMEM_BYTES, stream>>>(tmA, tmB, p);
   };
   if (pair) {
-    const long long tiles2 = (long long)G * ((M + 2 * BM - 1) / (2 * BM)) * p.num_n_tiles;
     int resident = apb_gemm_resident_pairs(num_sms) - g_reserved_sms / 2;
     if (resident < 1) resident = 1;
-    const int grid = 2 * (int)(tiles2 < resident ? tiles2 : resident);
     const int num_m2 = (M + 2 * BM - 1) / (2 * BM);
-    auto launch_layout = [&](auto wide) {
-      constexpr bool W = decltype(wide)::value;
+    const bool wide = set_pair_tiles(p, num_m2, resident, true);
+    const int units = 2 * p.all_tiles - p.whole_tiles, grid = 2 * (units < resident ? units : resident);
+    auto launch_layout = [&](auto wide_form) {
+      constexpr bool W = decltype(wide_form)::value;
       if (!a_mn_major && !b_mn_major) launch(gemm_grouped_pair_kernel<false, false, W>, grid);
       else if (!a_mn_major && b_mn_major) launch(gemm_grouped_pair_kernel<false, true, W>, grid);
       else if (a_mn_major && !b_mn_major) launch(gemm_grouped_pair_kernel<true, false, W>, grid);
       else launch(gemm_grouped_pair_kernel<true, true, W>, grid);
     };
-    if (set_wide_tiles(p, num_m2, resident)) {
-      launch_layout(std::true_type{});
-    } else {
-      set_tile_order(p, num_m2, p.num_n_tiles);
-      launch_layout(std::false_type{});
-    }
+    if (wide) launch_layout(std::true_type{});
+    else launch_layout(std::false_type{});
   } else {
     const long long tiles = (long long)G * p.num_m_tiles * p.num_n_tiles;
     const int grid = (int)(tiles < usable ? tiles : usable);

@@ -455,6 +455,54 @@ def test_gemm_tiles_land_where_they_belong(K, G, M, N, Kd, a_mn, b_mn, out):
         assert bool((wide == 99.0).all())
 
 
+@pytest.mark.parametrize("G,M,N,Kd", [
+    (0, 1504, 4104, 72),    # 102 pair tiles: a wave of whole ones, the others in halves, a last column tile of 8 columns
+    (0, 1500, 4232, 72),    # a last column tile of 136 columns
+    (0, 4360, 4872, 6552),  # wide tiles, an odd number of column tiles, the rest of the waves column tile by column tile
+    (0, 4100, 1032, 72),    # whole tiles only, 8 columns in the last column tile
+    (64, 160, 1416, 136),   # grouped
+    (20, 2304, 2184, 8200),  # grouped, wide
+])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+@pytest.mark.parametrize("dynamic", [False, True])
+def test_whole_and_half_and_wide_tiles(K, G, M, N, Kd, a_mn, b_mn, dynamic):
+    """Whole numbers first: every sum is exact, and nothing is written past the result.  Then columns that repeat every 128 and rows that
+    repeat every 4: their results are the same bits in whatever kind of tile they lie."""
+    _, impl = K
+    ext = impl.extension()
+    if (a_mn and M % 8) or (dynamic and G):
+        pytest.skip("rows of 16 bytes; grouped products have no dynamic tiles")
+    gen = torch.Generator(device="cuda").manual_seed(M + N)
+    lead = (G,) if G else ()
+    prev = ext.gemm_get_dynamic_tiles()
+    ext.gemm_set_dynamic_tiles(dynamic)
+    try:
+        for random in (False, True):
+            if random:
+                a = torch.randn(*lead, 4, Kd, device="cuda", generator=gen).to(torch.bfloat16).repeat(*([1] * len(lead)), M // 4, 1)
+                b = torch.randn(*lead, 128, Kd, device="cuda", generator=gen).to(torch.bfloat16).repeat(*([1] * len(lead)), N // 128 + 1, 1)
+                b = b[..., :N, :].contiguous()
+            else:
+                a = torch.randint(-1, 2, (*lead, M, Kd), device="cuda", generator=gen).to(torch.bfloat16)
+                b = torch.randint(-1, 2, (*lead, N, Kd), device="cuda", generator=gen).to(torch.bfloat16)
+            x = a.transpose(-1, -2).contiguous() if a_mn else a
+            y = b.transpose(-1, -2).contiguous() if b_mn else b
+            flat = torch.full(((G or 1) * M * N + 4096,), 99.0, device="cuda")
+            c = flat[:-4096].view(*lead, M, N)
+            if G:
+                ext.gemm_grouped(x, y, c, a_mn, b_mn, impl.status_buffer(c.device))
+            else:
+                ext.gemm(x, y, c, a_mn, b_mn, impl.status_buffer(c.device))
+            assert bool((flat[-4096:] == 99.0).all())
+            if random:
+                first = c[..., :4, :128].repeat(*([1] * len(lead)), M // 4, N // 128 + 1)[..., :N]
+                assert torch.equal(c, first)
+            else:
+                assert torch.equal(c, a.float() @ b.float().transpose(-1, -2))
+    finally:
+        ext.gemm_set_dynamic_tiles(prev)
+
+
 @pytest.mark.parametrize("pair", [True, False])
 def test_gemm_bits_do_not_depend_on_the_launch(K, pair):
     """Products whose rounds of tiles read more than L2 holds: equal rows and columns of the operands give equal results wherever they lie,
