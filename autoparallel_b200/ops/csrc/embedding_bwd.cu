@@ -3,7 +3,7 @@
 // Two forms; ``apb_embedding_bwd_sorts`` says which one runs.
 //
 // Sorted, bound by memory: the table gradient is written once in its own type and dy is read once.  The tokens are grouped by row
-// first, so that every output row is summed in fp32 registers and stored once - no fp32 table, no zero fill of it, no second
+// first, so that every output row is summed in fp32 registers and stored once - no fp32 table, no second
 // pass that converts it, no atomics on row data.
 //
 //   emb_group_kernel    one cluster of 8 CTAs: counts per row (one atomic per warp and distinct id), segment starts, token
@@ -13,6 +13,11 @@
 //                       that no block walks a long list alone.  Of rows with more than EMB_DIRECT chunks the last block of a group adds
 //                       the group up, and the last group the row.
 //   emb_rows_kernel     every other row: zeros, the sum of its tokens, or of its chunks.
+//
+// Where the table has far more rows than there are tokens (``emb_zeros_first``), the whole of it is filled with zeros beside the grouping,
+// by the SMs that the cluster leaves idle, and the last kernel is
+//
+//   emb_tokens_kernel   only the rows that have tokens.
 //
 // Atomic: an fp32 table of zeros, one block per token, for bf16 a conversion.  Better where the table is small or the rows are
 // short (the grouping is a chain of latencies that a small table does not pay for), and for most fp32 tables, which the atomics
@@ -31,6 +36,7 @@ constexpr int EMB_CHUNK = 32;
 constexpr int EMB_DIRECT = 32;  // most chunks of a row that emb_rows_kernel adds up
 constexpr int EMB_GROUP = 16;   // chunks of a longer one that are added up by one block
 constexpr int EMB_CTAS = 8, EMB_GROUP_THREADS = 1024;
+constexpr int EMB_ZERO_VECS = 2048;  // 16-byte vectors of zeros that a block fills
 constexpr int EMB_ROWS = 8;  // most rows of one block of emb_rows_kernel
 
 // Workspace (32-bit words), carved from one allocation of the caller.
@@ -50,8 +56,16 @@ __host__ __device__ inline long long emb_max_longs(long long T) { return T / (EM
 __host__ __device__ inline long long emb_max_chunks(long long T) { return T / EMB_CHUNK + emb_max_longs(T); }
 static inline long long emb_round4(long long n) { return (n + 3) & ~3ll; }
 
+// Blocks of the clusters after the first fill EMB_ZERO_VECS of the ``nzero`` vectors of ``zeros`` each.
 __global__ void __cluster_dims__(EMB_CTAS, 1, 1) __launch_bounds__(EMB_GROUP_THREADS)
-emb_group_kernel(const long long* __restrict__ ids, EmbWs ws, int T, long long V, long long ndone) {
+emb_group_kernel(const long long* __restrict__ ids, EmbWs ws, int T, long long V, long long ndone, uint4* __restrict__ zeros, long long nzero) {
+  if (blockIdx.x >= EMB_CTAS) {
+    const long long i = (long long)(blockIdx.x - EMB_CTAS) * EMB_ZERO_VECS + threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < EMB_ZERO_VECS; k += EMB_GROUP_THREADS)
+      if (i + k < nzero) zeros[i + k] = make_uint4(0, 0, 0, 0);
+    return;
+  }
   const int tid = blockIdx.x * EMB_GROUP_THREADS + threadIdx.x, lane = threadIdx.x & 31;
   constexpr int nt = EMB_CTAS * EMB_GROUP_THREADS;
   for (long long v = tid; v < V; v += nt) ws.count[v] = 0;
@@ -233,6 +247,38 @@ __global__ void __launch_bounds__(128) emb_partial_kernel(const T* __restrict__ 
   }
 }
 
+// Columns of one row with ``c`` tokens; ``from``: its first entry in perm, or its first chunk.
+template <typename T, int W>
+__device__ __forceinline__ void emb_row(const T* __restrict__ dy, const EmbWs& ws, T* dst, int c, int from, int D, int col, int step) {
+  for (; col < D; col += step) {
+    float acc[W] = {};
+    if (c > EMB_CHUNK) {
+      const float* p = ws.part + (long long)from * D + col;
+      const int n = (c + EMB_CHUNK - 1) / EMB_CHUNK;
+#pragma unroll 4
+      for (int i = 0; i < n; ++i)
+#pragma unroll
+        for (int k = 0; k < W; ++k) acc[k] += p[(long long)i * D + k];
+    } else if (c > 0) {
+      emb_sum<T, W>(dy, ws.perm + from, c, D, col, acc);
+    }
+    EmbVec<T, W>::store(dst + col, acc);
+  }
+}
+
+// The first token of every row stores it; ``tx`` threads to a token, as below.
+template <typename T, int W>
+__global__ void __launch_bounds__(256) emb_tokens_kernel(const T* __restrict__ dy, const long long* __restrict__ ids, EmbWs ws, T* __restrict__ out,
+                                                         int tokens, long long V, int D, int tx) {
+  const int t = blockIdx.x * (256 / tx) + threadIdx.x / tx;
+  if (t >= tokens) return;
+  const long long v = ids[t];
+  if (v < 0 || v >= V || ws.rank[t] != 0) return;
+  const int c = ws.count[v];
+  if (c > EMB_CHUNK * EMB_DIRECT) return;
+  emb_row<T, W>(dy, ws, out + v * D, c, (c > EMB_CHUNK ? ws.chunk0 : ws.start)[v], D, (threadIdx.x & (tx - 1)) * W, tx * W);
+}
+
 // ``tx`` threads (a power of two, 32..256) walk a row, 256 / tx rows at a time; the block owns ``R`` consecutive rows
 template <typename T, int W>
 __global__ void __launch_bounds__(256) emb_rows_kernel(const T* __restrict__ dy, EmbWs ws, T* __restrict__ out, long long V, int D,
@@ -247,23 +293,9 @@ __global__ void __launch_bounds__(256) emb_rows_kernel(const T* __restrict__ dy,
   }
   __syncthreads();
   for (int r = threadIdx.x / tx; r < nrows; r += 256 / tx) {
-    T* dst = out + (row0 + r) * D;
     const int c = cnt[r];
     if (c > EMB_CHUNK * EMB_DIRECT) continue;
-    for (int col = (threadIdx.x & (tx - 1)) * W; col < D; col += tx * W) {
-      float acc[W] = {};
-      if (c > EMB_CHUNK) {
-        const float* p = ws.part + (long long)from[r] * D + col;
-        const int n = (c + EMB_CHUNK - 1) / EMB_CHUNK;
-#pragma unroll 4
-        for (int i = 0; i < n; ++i)
-#pragma unroll
-          for (int k = 0; k < W; ++k) acc[k] += p[(long long)i * D + k];
-      } else if (c > 0) {
-        emb_sum<T, W>(dy, ws.perm + from[r], c, D, col, acc);
-      }
-      EmbVec<T, W>::store(dst + col, acc);
-    }
+    emb_row<T, W>(dy, ws, out + (row0 + r) * D, c, from[r], D, (threadIdx.x & (tx - 1)) * W, tx * W);
   }
 }
 
@@ -316,16 +348,33 @@ static int emb_slices(int D, int w) {
   return n < 16 ? n : 16;
 }
 
+// Zeros first, beside the grouping (a chain of latencies on eight SMs, 20 us and more), in blocks that end with their 32 KB: those write 7.3 TB/s,
+// blocks that stay and take many pieces 6.2, emb_rows_kernel 7.8 in rows of 8 KB and 5.8 in shorter ones.  The rows that have tokens are written
+// twice, so the line lies where a table has four times as many rows as there are tokens, ten times in rows of more than 4 KB.  bf16, ids by Zipf's law /
+// at random, rows first -> zeros first: 128256 x 1024, 8000 tokens 85 / 78 -> 66 / 57 us, x 2048 127 / 125 -> 110 / 105, x 4096 210 / 195 -> 194 /
+// 186, 16000 tokens 221 / 215 -> 211 / 224; 32000 x 2048, 8000 tokens 57 / 52 -> 51 / 46, 16000 73 / 66 -> 72 / 72; 32000 x 4096, 2000 tokens 74 /
+// 63 -> 67 / 51, 8000 85 / 77 -> 89 / 79; 8000 x 2048, 2000 tokens 27 / 24 -> 23 / 21, 4000 26 / 25 -> 27 / 24.
+static bool emb_zeros_first(long long tokens, long long V, long long row_bytes) { return tokens <= V / (row_bytes > 4096 ? 10 : 4); }
+
 template <typename T, int W>
 static void emb_launch(const void* dy, const long long* ids, const EmbWs& ws, void* out, long long T_, long long V, int D, int num_sms,
                        cudaStream_t st) {
   const int nvec = D / W, slices = emb_slices(D, W);
   const long long chunks = emb_max_chunks(T_);
-  emb_group_kernel<<<EMB_CTAS, EMB_GROUP_THREADS, 0, st>>>(ids, ws, (int)T_, V, 2 * chunks * slices);
+  const bool zeros_first = W > 1 && emb_zeros_first(T_, V, (long long)D * sizeof(T));
+  const long long fill = (long long)EMB_CTAS * EMB_ZERO_VECS;  // vectors of a cluster
+  const unsigned clusters = 1 + (zeros_first ? (unsigned)((V * nvec + fill - 1) / fill) : 0u);
+  emb_group_kernel<<<EMB_CTAS * clusters, EMB_GROUP_THREADS, 0, st>>>(ids, ws, (int)T_, V, 2 * chunks * slices, reinterpret_cast<uint4*>(out),
+                                                                       V * nvec);
   if (emb_max_longs(T_) > 0)
     emb_partial_kernel<T, W><<<dim3((unsigned)chunks, (unsigned)slices), 128, 0, st>>>((const T*)dy, ws, (T*)out, chunks, D);
   int tx = 32;
   while (tx < nvec && tx < 256) tx *= 2;
+  if (zeros_first) {
+    const int per = 256 / tx;
+    if (T_ > 0) emb_tokens_kernel<T, W><<<(unsigned)((T_ + per - 1) / per), 256, 0, st>>>((const T*)dy, ids, ws, (T*)out, (int)T_, V, D, tx);
+    return;
+  }
   // rows per block: eight where the table is long (one 64-KB store stream per block), fewer where it would leave SMs idle,
   // but never fewer than the block takes at a time
   const long long want = V / ((long long)num_sms * 8);

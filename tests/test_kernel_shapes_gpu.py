@@ -86,6 +86,39 @@ def test_embedding_gradient_by_both_forms(K, dtype, V, D, T, ids, sorts):
     assert not out[torch.bincount(idx, minlength=V) == 0].any()
 
 
+@pytest.mark.parametrize("ids", ["same", "skewed", "random"])
+@pytest.mark.parametrize("dtype,V,D,T", [
+    (torch.bfloat16, 8003, 2048, 2000),  # the most tokens for which zeros come first, in rows of 4 KB; the last block of zeros is partial
+    (torch.bfloat16, 8003, 2048, 2001),
+    (torch.bfloat16, 32000, 2056, 3200),  # in longer rows
+    (torch.bfloat16, 32000, 2056, 3201),
+    (torch.bfloat16, 30000, 1032, 1),
+    (torch.float32, 40000, 4096, 4000),
+])
+def test_embedding_gradient_with_zeros_first(K, dtype, V, D, T, ids):
+    """Every row is written, whatever the buffer held; ids outside the table are skipped."""
+    _, impl = K
+    ext = impl.extension()
+    if not ext.embedding_bwd_sorts(T, V, D, dtype == torch.bfloat16):
+        pytest.skip("the other form")
+    g = torch.Generator(device="cuda").manual_seed(V + T)
+    idx = torch.randint(0, V, (T,), device="cuda", generator=g)
+    if ids == "same":
+        idx.fill_(V - 1)
+    elif ids == "skewed":
+        idx = (torch.rand(T, device="cuda", generator=g) ** 4 * V).long()
+    if T > 1:
+        idx[T // 2], idx[T // 3] = V, -1
+    dy = torch.randn(T, D, device="cuda", generator=g).to(dtype)
+    out = torch.full((V, D), float("nan"), device="cuda", dtype=dtype)
+    ext.embedding_bwd(dy, idx, out)
+    inside = (idx >= 0) & (idx < V)
+    ref = torch.zeros(V, D, device="cuda", dtype=torch.float64).index_add_(0, idx[inside], dy[inside].double())
+    err = ((out.double() - ref).norm() / ref.norm()).item()
+    assert err <= (2**-8 if dtype == torch.bfloat16 else 2**-24 * T ** 0.5 * 4)  # as above
+    assert not out[torch.bincount(idx[inside], minlength=V) == 0].any()
+
+
 def test_embedding_gradient_of_an_unaligned_view(K):
     lib, _ = K
     flat = torch.randn(1 + 12 * 16, device="cuda").to(torch.bfloat16)
