@@ -1,6 +1,10 @@
 // Bandwidth-bound kernels of the transformer step for sm_100a: RMSNorm fwd/bwd, RoPE, SwiGLU
 // fwd/bwd, cross-entropy fwd/bwd, dtype cast, embedding forward, multi-tensor AdamW.
-// All use 16-byte vector accesses, fp32 math, and grids sized as multiples of the 148 SMs.
+// All use 16-byte vector accesses and fp32 math.  Kernels without anything to carry from one element to the next (casts, SwiGLU, RoPE, RMSNorm
+// forward, AdamW) take one vector per thread and tensor, in blocks that end there: as many loads are under way as in loops over the tensor with 8
+// blocks an SM, but the memory sees one front that moves through every tensor.  Loop -> so: casts to fp32 of 2^28 elements 333 -> 235 us, to bf16 252 ->
+// 229; SwiGLU of 8192 x 14336 bf16 117 -> 100, its gradient 193 -> 170 (6.9 TB/s); AdamW over 218 M parameters 1067 -> 963.  Two and four vectors a thread
+// are no faster there and slower in small tensors (SwiGLU gradient of 999 x 1408 2.7 / 3.2 / 3.7 us).
 // They replace the ATen / Inductor-generated kernels the reference reaches for the same nodes
 // (autoparallel/_testing/models/llama3.py:187-213, 355-356, 396-397).
 #include <cuda_bf16.h>
@@ -83,19 +87,17 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 // ------------------------------------------------------------------------------------ RMSNorm
 // Forward.  A group of ``TPR`` threads owns a row and keeps its NVEC x 8 elements per thread in registers between the
 // sum of squares and the scaling, so x is read once.  TPR = 32: one warp per row, reduction by shuffles only, no
-// block barrier; several rows per block keep enough loads in flight.  TPR = blockDim.x: one block per row for wide rows.
+// block barrier; several rows per block keep enough loads in flight.  TPR = blockDim.x: a block takes a row at a time (see apb_rms_norm_fwd).
 // D % 8 == 0 and D <= TPR * 8 * NVEC.
-template <typename T, int NVEC, bool WARP_ROWS>
+template <typename T, int NVEC, bool WARP_ROWS, bool IN_TURN = false>
 __global__ void rms_norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ y,
                                     float* __restrict__ rstd, long long rows, int D, float eps) {
   __shared__ float red[32];
   const int tpr = WARP_ROWS ? 32 : blockDim.x;
   const int t = WARP_ROWS ? (threadIdx.x & 31) : threadIdx.x;
-  const long long rows_per_block = WARP_ROWS ? (blockDim.x >> 5) : 1;
-  const long long first = (long long)blockIdx.x * rows_per_block + (WARP_ROWS ? (threadIdx.x >> 5) : 0);
-  const long long step = (long long)gridDim.x * rows_per_block;
-  for (long long row = first; WARP_ROWS ? (row < rows) : (row - (WARP_ROWS ? (threadIdx.x >> 5) : 0) < rows); row += step) {
-    if (!WARP_ROWS && row >= rows) break;
+  long long row = WARP_ROWS ? blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5) : blockIdx.x;
+  if (row >= rows) return;
+  do {
     const T* xr = x + row * D;
     T* yr = y + row * D;
     Vec8<T> v[NVEC];
@@ -124,7 +126,7 @@ __global__ void rms_norm_fwd_kernel(const T* __restrict__ x, const T* __restrict
         Vec8<T> o; o.from_float(f); o.store(yr + c);
       }
     }
-  }
+  } while (IN_TURN && (row += gridDim.x) < rows);  // (the same for the whole block)
 }
 
 // block-wide sums of R values at once (one barrier pair for all of them); ``red`` holds 32 * R floats
@@ -401,105 +403,87 @@ __global__ void __launch_bounds__(1024) rms_dw_kernel(const float* __restrict__ 
   if ((threadIdx.x & 31) == 0 && co < D) dw[co] = T(s);
 }
 
-template <typename T>
-__global__ void cast_from_f32_kernel(const float* __restrict__ src, T* __restrict__ dst, long long n) {
-  long long i = (blockIdx.x * (long long)blockDim.x + threadIdx.x) * 8;
-  const long long stride = (long long)gridDim.x * blockDim.x * 8;
-  for (; i + 8 <= n; i += stride) {
-    Vec8<float> v; v.load(src + i);
+template <typename S, typename D>
+__global__ void __launch_bounds__(256) cast_kernel(const S* __restrict__ src, D* __restrict__ dst, long long n) {
+  const long long i = (blockIdx.x * 256ll + threadIdx.x) * 8;
+  if (i + 8 <= n) {
+    Vec8<S> v; v.load(src + i);
     float f[8]; v.to_float(f);
-    Vec8<T> o; o.from_float(f); o.store(dst + i);
+    Vec8<D> o; o.from_float(f); o.store(dst + i);
+  } else {
+    for (long long k = i; k < n; ++k) dst[k] = D(float(src[k]));
   }
-  if (i < n && i + 8 > n)
-    for (long long k = i; k < n; ++k) dst[k] = T(src[k]);
-}
-template <typename T>
-__global__ void cast_to_f32_kernel(const T* __restrict__ src, float* __restrict__ dst, long long n) {
-  long long i = (blockIdx.x * (long long)blockDim.x + threadIdx.x) * 8;
-  const long long stride = (long long)gridDim.x * blockDim.x * 8;
-  for (; i + 8 <= n; i += stride) {
-    Vec8<T> v; v.load(src + i);
-    float f[8]; v.to_float(f);
-    Vec8<float> o; o.from_float(f); o.store(dst + i);
-  }
-  if (i < n && i + 8 > n)
-    for (long long k = i; k < n; ++k) dst[k] = float(src[k]);
 }
 
 // ------------------------------------------------------------------------------------ RoPE
 // x [B, S, H, D] with interleaved pairs; cos/sin fp32 [S, D/2].  One thread owns eight consecutive elements of a
-// head (one 16-byte vector) at one position and walks over the heads: the 32 bytes of cos / sin it needs are read
-// once per position instead of once per head (the tables would otherwise be twice the traffic of x itself).
-template <typename T>
-__global__ void rope_kernel(const T* __restrict__ x, const float* __restrict__ cs, const float* __restrict__ sn,
-                            T* __restrict__ y, long long total_pos_vec, int S, int H, int D, float sign) {
+// head (one 16-byte vector) at one position, in HEADS neighbouring heads: the 32 bytes of cos / sin it needs are read
+// once for them (the tables would otherwise be twice the traffic of x itself).  Eight heads where that leaves the SMs 768 threads each, else
+// four; all heads of a position in one thread -> 8 / 4 heads a thread: 8192 x 32 x 128 33.4 -> 25.3 / 27.7 us, 8192 x 8 x 128 8.3 -> 8.2 / 9.0,
+// 8192 x 8 x 64 5.6 -> 5.5 / 4.2, 100 x 32 x 128 8.8 -> 3.6 / 2.7.
+template <typename T, int HEADS>
+__global__ void __launch_bounds__(128) rope_kernel(const T* __restrict__ x, const float* __restrict__ cs, const float* __restrict__ sn,
+                                                   T* __restrict__ y, long long total_pos_vec, int S, int H, int D, float sign) {
   const int vec_per_head = D / 8;
-  for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < total_pos_vec;
-       v += (long long)gridDim.x * blockDim.x) {
-    const int dv = v % vec_per_head;
-    const long long bs = v / vec_per_head;  // b * S + s
-    const int s = bs % S;
-    const float4 c = *reinterpret_cast<const float4*>(cs + (long long)s * (D / 2) + dv * 4);
-    const float4 n = *reinterpret_cast<const float4*>(sn + (long long)s * (D / 2) + dv * 4);
-    const float cc[4] = {c.x, c.y, c.z, c.w};
-    const float nn[4] = {n.x * sign, n.y * sign, n.z * sign, n.w * sign};
-    const long long base = (bs * H) * D + dv * 8;
-    int h = 0;
-    for (; h + 4 <= H; h += 4) {  // four independent loads in flight
-      Vec8<T> xv[4];
+  const unsigned groups = (H + HEADS - 1) / HEADS;  // of heads; neighbouring blocks take the groups of the same positions
+  const long long v = blockIdx.x / groups * 128ll + threadIdx.x;
+  if (v >= total_pos_vec) return;
+  const int dv = v % vec_per_head;
+  const long long bs = v / vec_per_head;  // b * S + s
+  const int s = bs % S;
+  const float4 c = *reinterpret_cast<const float4*>(cs + (long long)s * (D / 2) + dv * 4);
+  const float4 n = *reinterpret_cast<const float4*>(sn + (long long)s * (D / 2) + dv * 4);
+  const float cc[4] = {c.x, c.y, c.z, c.w};
+  const float nn[4] = {n.x * sign, n.y * sign, n.z * sign, n.w * sign};
+  const long long base = (bs * H) * D + dv * 8;
+  const int h0 = blockIdx.x % groups * HEADS, h1 = min(H, h0 + HEADS);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) xv[k].load(x + base + (long long)(h + k) * D);
+  for (int hg = 0; hg < HEADS; hg += 4) {  // four independent loads in flight
+    Vec8<T> xv[4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        float f[8], o[8];
-        xv[k].to_float(f);
+    for (int k = 0; k < 4; ++k)
+      if (h0 + hg + k < h1) xv[k].load(x + base + (long long)(h0 + hg + k) * D);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          o[2 * i] = f[2 * i] * cc[i] - f[2 * i + 1] * nn[i];
-          o[2 * i + 1] = f[2 * i] * nn[i] + f[2 * i + 1] * cc[i];
-        }
-        Vec8<T> ov; ov.from_float(o); ov.store(y + base + (long long)(h + k) * D);
-      }
-    }
-    for (; h < H; ++h) {
-      Vec8<T> xv; xv.load(x + base + (long long)h * D);
-      float f[8], o[8]; xv.to_float(f);
+    for (int k = 0; k < 4; ++k) {
+      if (h0 + hg + k >= h1) break;
+      float f[8], o[8];
+      xv[k].to_float(f);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         o[2 * i] = f[2 * i] * cc[i] - f[2 * i + 1] * nn[i];
         o[2 * i + 1] = f[2 * i] * nn[i] + f[2 * i + 1] * cc[i];
       }
-      Vec8<T> ov; ov.from_float(o); ov.store(y + base + (long long)h * D);
+      Vec8<T> ov; ov.from_float(o); ov.store(y + base + (long long)(h0 + hg + k) * D);
     }
   }
 }
 
 // ------------------------------------------------------------------------------------ SwiGLU
 template <typename T>
-__global__ void swiglu_fwd_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ y, long long nvec) {
-  for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < nvec; v += (long long)gridDim.x * blockDim.x) {
-    Vec8<T> av, bv; av.load(a + v * 8); bv.load(b + v * 8);
-    float fa[8], fb[8], o[8]; av.to_float(fa); bv.to_float(fb);
+__global__ void __launch_bounds__(256) swiglu_fwd_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ y, long long nvec) {
+  const long long v = blockIdx.x * 256ll + threadIdx.x;
+  if (v >= nvec) return;
+  Vec8<T> av, bv; av.load(a + v * 8); bv.load(b + v * 8);
+  float fa[8], fb[8], o[8]; av.to_float(fa); bv.to_float(fb);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) o[i] = fa[i] / (1.f + __expf(-fa[i])) * fb[i];
-    Vec8<T> ov; ov.from_float(o); ov.store(y + v * 8);
-  }
+  for (int i = 0; i < 8; ++i) o[i] = fa[i] / (1.f + __expf(-fa[i])) * fb[i];
+  Vec8<T> ov; ov.from_float(o); ov.store(y + v * 8);
 }
 template <typename T>
-__global__ void swiglu_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ a, const T* __restrict__ b,
-                                  T* __restrict__ da, T* __restrict__ db, long long nvec) {
-  for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < nvec; v += (long long)gridDim.x * blockDim.x) {
-    Vec8<T> gv, av, bv; gv.load(dy + v * 8); av.load(a + v * 8); bv.load(b + v * 8);
-    float g[8], fa[8], fb[8], oa[8], ob[8]; gv.to_float(g); av.to_float(fa); bv.to_float(fb);
+__global__ void __launch_bounds__(256) swiglu_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ a, const T* __restrict__ b,
+                                                         T* __restrict__ da, T* __restrict__ db, long long nvec) {
+  const long long v = blockIdx.x * 256ll + threadIdx.x;
+  if (v >= nvec) return;
+  Vec8<T> gv, av, bv; gv.load(dy + v * 8); av.load(a + v * 8); bv.load(b + v * 8);
+  float g[8], fa[8], fb[8], oa[8], ob[8]; gv.to_float(g); av.to_float(fa); bv.to_float(fb);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float sig = 1.f / (1.f + __expf(-fa[i]));
-      const float silu = fa[i] * sig;
-      oa[i] = g[i] * fb[i] * (sig * (1.f + fa[i] * (1.f - sig)));
-      ob[i] = g[i] * silu;
-    }
-    Vec8<T> o1, o2; o1.from_float(oa); o2.from_float(ob); o1.store(da + v * 8); o2.store(db + v * 8);
+  for (int i = 0; i < 8; ++i) {
+    const float sig = 1.f / (1.f + __expf(-fa[i]));
+    const float silu = fa[i] * sig;
+    oa[i] = g[i] * fb[i] * (sig * (1.f + fa[i] * (1.f - sig)));
+    ob[i] = g[i] * silu;
   }
+  Vec8<T> o1, o2; o1.from_float(oa); o2.from_float(ob); o1.store(da + v * 8); o2.store(db + v * 8);
 }
 
 // ------------------------------------------------------------------------------------ cross-entropy
@@ -613,8 +597,9 @@ __global__ void embedding_fwd_kernel(const T* __restrict__ weight, const long lo
 }
 
 // ------------------------------------------------------------------------------------ AdamW
-// Multi-tensor: ``table`` lists chunks (tensor id, offset); each block handles one chunk.  Where the parameter starts on a 16-byte boundary
-// so do the other three (the optimizer sees to it: as a test in here it cost 2 %); elsewhere elements are taken one by one.
+// Multi-tensor: ``chunks`` lists pieces of ADAM_CHUNK elements (tensor id, number); a block takes ADAM_PART of one, four elements a thread.  Bound by
+// memory, 28 or 30 bytes an element.  218 M elements: pieces of 65536 / 8192 / 4096 / 1024 to a block 1067 / 1003 / 992 / 963 us.  Where the parameter
+// starts on a 16-byte boundary so do the other three (the optimizer sees to it); elsewhere elements are taken one by one.
 struct AdamTensor {
   float* p;        // fp32 master / parameter
   const float* g;  // fp32 gradient
@@ -623,10 +608,10 @@ struct AdamTensor {
   __nv_bfloat16* p_lp;  // optional low-precision copy to emit (may be null)
   long long n;
 };
-constexpr int ADAM_CHUNK = 65536;
+constexpr int ADAM_CHUNK = 65536, ADAM_PART = 1024;
 // ``hyper`` (optional, device memory): {lr, bc1, bc2} read at run time instead of the launch arguments, so that a step
 // captured in a CUDA graph follows the learning-rate schedule and the bias corrections of the step it is replayed for.
-__global__ void adamw_kernel(const AdamTensor* __restrict__ tensors, const int2* __restrict__ chunks, float lr,
+__global__ void __launch_bounds__(ADAM_PART / 4) adamw_kernel(const AdamTensor* __restrict__ tensors, const int2* __restrict__ chunks, float lr,
                              float beta1, float beta2, float eps, float wd, float bc1, float bc2, float grad_scale,
                              const float* __restrict__ hyper) {
   if (hyper != nullptr) {
@@ -634,43 +619,45 @@ __global__ void adamw_kernel(const AdamTensor* __restrict__ tensors, const int2*
     bc1 = hyper[1];
     bc2 = hyper[2];
   }
-  const int2 ch = chunks[blockIdx.x];
+  const int2 ch = chunks[blockIdx.x / (ADAM_CHUNK / ADAM_PART)];
   const AdamTensor t = tensors[ch.x];
-  const long long base = (long long)ch.y * ADAM_CHUNK;
-  const long long end = min(base + (long long)ADAM_CHUNK, t.n);
-  for (long long i = base + threadIdx.x * 4; i < end; i += blockDim.x * 4) {
-    if (i + 4 <= end && ((reinterpret_cast<uintptr_t>(t.p + i) & 15) == 0)) {
-      float4 p = *reinterpret_cast<float4*>(t.p + i);
-      const float4 g4 = *reinterpret_cast<const float4*>(t.g + i);
-      float4 m = *reinterpret_cast<float4*>(t.m + i);
-      float4 v = *reinterpret_cast<float4*>(t.v + i);
-      float* pp = &p.x; const float* gg = &g4.x; float* mm = &m.x; float* vv = &v.x;
+  const long long i = (long long)ch.y * ADAM_CHUNK + (blockIdx.x % (ADAM_CHUNK / ADAM_PART)) * ADAM_PART + threadIdx.x * 4;
+  if (i >= t.n) return;
+  if (i + 4 <= t.n && ((reinterpret_cast<uintptr_t>(t.p + i) & 15) == 0)) {
+    float4 p = *reinterpret_cast<float4*>(t.p + i);
+    const float4 g4 = *reinterpret_cast<const float4*>(t.g + i);
+    float4 m = *reinterpret_cast<float4*>(t.m + i);
+    float4 v = *reinterpret_cast<float4*>(t.v + i);
+    float* pp = &p.x; const float* gg = &g4.x; float* mm = &m.x; float* vv = &v.x;
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const float g = gg[k] * grad_scale;
-        mm[k] = beta1 * mm[k] + (1.f - beta1) * g;
-        vv[k] = beta2 * vv[k] + (1.f - beta2) * g * g;
-        const float mh = mm[k] / bc1;
-        const float vh = vv[k] / bc2;
-        pp[k] = pp[k] * (1.f - lr * wd) - lr * mh / (sqrtf(vh) + eps);
-      }
-      *reinterpret_cast<float4*>(t.p + i) = p;
-      *reinterpret_cast<float4*>(t.m + i) = m;
-      *reinterpret_cast<float4*>(t.v + i) = v;
-      if (t.p_lp) {
+    for (int k = 0; k < 4; ++k) {
+      const float g = gg[k] * grad_scale;
+      mm[k] = beta1 * mm[k] + (1.f - beta1) * g;
+      vv[k] = beta2 * vv[k] + (1.f - beta2) * g * g;
+      const float mh = mm[k] / bc1;
+      const float vh = vv[k] / bc2;
+      pp[k] = pp[k] * (1.f - lr * wd) - lr * mh / (sqrtf(vh) + eps);
+    }
+    *reinterpret_cast<float4*>(t.p + i) = p;
+    *reinterpret_cast<float4*>(t.m + i) = m;
+    *reinterpret_cast<float4*>(t.v + i) = v;
+    if (t.p_lp) {
+      if ((reinterpret_cast<uintptr_t>(t.p_lp + i) & 7) == 0) {
+        *reinterpret_cast<uint2*>(t.p_lp + i) = make_uint2(pack_bf16(p.x, p.y), pack_bf16(p.z, p.w));
+      } else {
         t.p_lp[i] = __float2bfloat16(p.x); t.p_lp[i + 1] = __float2bfloat16(p.y);
         t.p_lp[i + 2] = __float2bfloat16(p.z); t.p_lp[i + 3] = __float2bfloat16(p.w);
       }
-    } else {
-      for (long long k = i; k < min(i + 4, end); ++k) {
-        const float g = t.g[k] * grad_scale;
-        const float m = beta1 * t.m[k] + (1.f - beta1) * g;
-        const float v = beta2 * t.v[k] + (1.f - beta2) * g * g;
-        t.m[k] = m; t.v[k] = v;
-        const float pn = t.p[k] * (1.f - lr * wd) - lr * (m / bc1) / (sqrtf(v / bc2) + eps);
-        t.p[k] = pn;
-        if (t.p_lp) t.p_lp[k] = __float2bfloat16(pn);
-      }
+    }
+  } else {
+    for (long long k = i; k < min(i + 4, t.n); ++k) {
+      const float g = t.g[k] * grad_scale;
+      const float m = beta1 * t.m[k] + (1.f - beta1) * g;
+      const float v = beta2 * t.v[k] + (1.f - beta2) * g * g;
+      t.m[k] = m; t.v[k] = v;
+      const float pn = t.p[k] * (1.f - lr * wd) - lr * (m / bc1) / (sqrtf(v / bc2) + eps);
+      t.p[k] = pn;
+      if (t.p_lp) t.p_lp[k] = __float2bfloat16(pn);
     }
   }
 }
@@ -745,11 +732,7 @@ static inline int launch_rms_norm_bwd(const void* dy, const void* x, const void*
   return -3;
 }
 
-static inline int grid_for(long long work_items, int threads, int num_sms) {
-  long long blocks = (work_items + threads - 1) / threads;
-  long long cap = (long long)num_sms * 8;
-  return (int)(blocks < cap ? (blocks > 0 ? blocks : 1) : cap);
-}
+static inline unsigned blocks_for(long long items, int per_block) { return (unsigned)((items + per_block - 1) / per_block); }
 
 // All kernels here read and write 16-byte vectors: the entries refuse (3) a base that is not on such a boundary.
 template <typename... P>
@@ -778,25 +761,38 @@ int apb_rms_norm_fwd(const void* x, const void* w, void* y, float* rstd, long lo
   if (!aligned16(x, w, y)) return 3;
   if (D % 8) return 3;
   if (rows == 0) return 0;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (D <= 32 * 8 * 4) {
     // one warp per row, eight rows per block
     const int nvec = (D + 255) / 256;
-    const long long blocks = (rows + 7) / 8, cap = (long long)sms * 8;
-    const unsigned grid = (unsigned)(blocks < cap ? blocks : cap);
+    const unsigned grid = blocks_for(rows, 8);
 #define APB_RMS_FWD_W(NV) DISPATCH(is_bf16, rms_norm_fwd_kernel<T, NV, true><<<grid, 256, 0, st>>>((const T*)x, (const T*)w, (T*)y, rstd, rows, D, eps))
     if (nvec == 1) { APB_RMS_FWD_W(1); } else if (nvec == 2) { APB_RMS_FWD_W(2); } else { APB_RMS_FWD_W(4); }
 #undef APB_RMS_FWD_W
   } else {
+    // Threads of a row's block and what it does after the row.  Few rows: one vector per thread, the row itself is the latency (64 x 4096 bf16,
+    // 256 -> 512 threads 2.8 -> 2.4 us).  Many short rows: two, and more blocks on an SM (8192 x 1536 bf16 192 -> 96 threads 11.1 -> 9.9 us,
+    // fp32 17.3 -> 16.3).  Blocks end with their row; only bf16 rows from 4096 on keep blocks that take rows in turn, 8 (or 2048 threads) to an
+    // SM: row by row -> in turn 8192 x 3072 bf16 20.5 -> 21.4 us, x 4096 26.8 -> 25.6, x 8192 49.3 -> 44.7; fp32 x 2048 23.6 -> 29.4, x 4096 42.0
+    // -> 52.7, x 8192 82.7 -> 87.9.
+    const int vecs = D / 8;
     int threads = 256;
+    if (rows <= 256 && vecs <= 1024) threads = (vecs + 31) / 32 * 32;
+    else if (D <= 3072 && rows >= (is_bf16 ? 1024 : 4096)) threads = (vecs + 63) / 64 * 32;
     while (threads * 8 * 4 < D && threads < 1024) threads *= 2;
-    const int nvec = (D + threads * 8 - 1) / (threads * 8);
+    const int nvec = (vecs + threads - 1) / threads;
     if (nvec > 4) return 3;
-    const long long cap = (long long)sms * (threads >= 1024 ? 2 : (threads >= 512 ? 4 : 8));
-    const unsigned grid = (unsigned)(rows < cap ? rows : cap);
-#define APB_RMS_FWD_B(NV) DISPATCH(is_bf16, rms_norm_fwd_kernel<T, NV, false><<<grid, threads, 0, st>>>((const T*)x, (const T*)w, (T*)y, rstd, rows, D, eps))
+    unsigned grid = (unsigned)rows;
+    const bool in_turn = is_bf16 && D >= 4096;
+    if (in_turn) {
+      int dev = 0, sms = 148;
+      cudaGetDevice(&dev);
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+      const long long cap = (long long)sms * (threads >= 1024 ? 2 : threads >= 512 ? 4 : 8);
+      if (rows > cap) grid = (unsigned)cap;
+    }
+#define APB_RMS_FWD_B(NV)                                                                                                                             \
+  if (in_turn) rms_norm_fwd_kernel<bf16, NV, false, true><<<grid, threads, 0, st>>>((const bf16*)x, (const bf16*)w, (bf16*)y, rstd, rows, D, eps); \
+  else DISPATCH(is_bf16, rms_norm_fwd_kernel<T, NV, false><<<grid, threads, 0, st>>>((const T*)x, (const T*)w, (T*)y, rstd, rows, D, eps))
     if (nvec == 1) { APB_RMS_FWD_B(1); } else if (nvec == 2) { APB_RMS_FWD_B(2); } else { APB_RMS_FWD_B(4); }
 #undef APB_RMS_FWD_B
   }
@@ -826,9 +822,9 @@ int apb_rms_norm_bwd(const void* dy, const void* x, const void* w, const float* 
 int apb_cast(const void* src, void* dst, long long n, int src_bf16, int dst_bf16, int num_sms, cudaStream_t st) {
   if (!aligned16(src, dst)) return 3;
   if (n == 0) return 0;
-  const int grid = grid_for((n + 7) / 8, 256, num_sms);
-  if (src_bf16 && !dst_bf16) cast_to_f32_kernel<bf16><<<grid, 256, 0, st>>>((const bf16*)src, (float*)dst, n);
-  else if (!src_bf16 && dst_bf16) cast_from_f32_kernel<bf16><<<grid, 256, 0, st>>>((const float*)src, (bf16*)dst, n);
+  const unsigned grid = blocks_for((n + 7) / 8, 256);
+  if (src_bf16 && !dst_bf16) cast_kernel<bf16, float><<<grid, 256, 0, st>>>((const bf16*)src, (float*)dst, n);
+  else if (!src_bf16 && dst_bf16) cast_kernel<float, bf16><<<grid, 256, 0, st>>>((const float*)src, (bf16*)dst, n);
   else return 3;
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
@@ -839,8 +835,14 @@ int apb_rope(const void* x, const float* cs, const float* sn, void* y, long long
   if (D % 8) return 3;
   const long long nvec = B * S * (D / 8);  // one thread per (position, 8-element group); the kernel walks the heads
   if (nvec == 0 || H == 0) return 0;
-  const int grid = grid_for(nvec, 128, num_sms);
-  DISPATCH(is_bf16, rope_kernel<T><<<grid, 128, 0, st>>>((const T*)x, cs, sn, (T*)y, nvec, S, H, D, conj ? -1.f : 1.f));
+  const float sign = conj ? -1.f : 1.f;
+  const int heads = nvec * ((H + 7) / 8) >= 768ll * num_sms ? 8 : 4;
+  const unsigned grid = blocks_for(nvec, 128) * (unsigned)((H + heads - 1) / heads);
+  if (heads == 8) {
+    DISPATCH(is_bf16, rope_kernel<T, 8><<<grid, 128, 0, st>>>((const T*)x, cs, sn, (T*)y, nvec, S, H, D, sign));
+  } else {
+    DISPATCH(is_bf16, rope_kernel<T, 4><<<grid, 128, 0, st>>>((const T*)x, cs, sn, (T*)y, nvec, S, H, D, sign));
+  }
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 
@@ -848,7 +850,7 @@ int apb_swiglu_fwd(const void* a, const void* b, void* y, long long n, int is_bf
   if (!aligned16(a, b, y)) return 3;
   if (n % 8) return 3;
   if (n == 0) return 0;
-  DISPATCH(is_bf16, swiglu_fwd_kernel<T><<<grid_for(n / 8, 256, num_sms), 256, 0, st>>>((const T*)a, (const T*)b, (T*)y, n / 8));
+  DISPATCH(is_bf16, swiglu_fwd_kernel<T><<<blocks_for(n / 8, 256), 256, 0, st>>>((const T*)a, (const T*)b, (T*)y, n / 8));
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 
@@ -857,7 +859,7 @@ int apb_swiglu_bwd(const void* dy, const void* a, const void* b, void* da, void*
   if (!aligned16(dy, a, b, da, db)) return 3;
   if (n % 8) return 3;
   if (n == 0) return 0;
-  DISPATCH(is_bf16, swiglu_bwd_kernel<T><<<grid_for(n / 8, 256, num_sms), 256, 0, st>>>((const T*)dy, (const T*)a, (const T*)b,
+  DISPATCH(is_bf16, swiglu_bwd_kernel<T><<<blocks_for(n / 8, 256), 256, 0, st>>>((const T*)dy, (const T*)a, (const T*)b,
                                                                                        (T*)da, (T*)db, n / 8));
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
@@ -907,7 +909,7 @@ int apb_embedding_fwd(const void* weight, const long long* ids, void* out, long 
 int apb_adamw(const void* tensors_dev, const void* chunks_dev, int num_chunks, float lr, float beta1, float beta2, float eps,
               float wd, float bc1, float bc2, float grad_scale, const float* hyper_dev, cudaStream_t st) {
   if (num_chunks == 0) return 0;
-  adamw_kernel<<<num_chunks, 256, 0, st>>>((const AdamTensor*)tensors_dev, (const int2*)chunks_dev, lr, beta1, beta2, eps, wd,
+  adamw_kernel<<<(unsigned)num_chunks * (ADAM_CHUNK / ADAM_PART), ADAM_PART / 4, 0, st>>>((const AdamTensor*)tensors_dev, (const int2*)chunks_dev, lr, beta1, beta2, eps, wd,
                                            bc1, bc2, grad_scale, hyper_dev);
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
@@ -983,7 +985,7 @@ extern "C" int apb_rms_norm_bwd_noalloc(const void* dy, const void* x, const voi
   if (shared > 1) {
     DISPATCH(is_bf16, rms_dw_kernel<T><<<(D + 31) / 32, 1024, 0, st>>>(acc, (T*)dw, shared, D));
   } else if (is_bf16) {
-    cast_from_f32_kernel<bf16><<<grid_for(D / 8, 256, num_sms), 256, 0, st>>>(acc, (bf16*)dw, D);
+    cast_kernel<float, bf16><<<blocks_for(D / 8, 256), 256, 0, st>>>(acc, (bf16*)dw, D);
   } else {
     if (cudaMemcpyAsync(dw, acc, sizeof(float) * D, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
       return APB_NOALLOC_ERR_LAUNCH;
