@@ -536,6 +536,34 @@ def test_whole_and_half_and_wide_tiles(K, G, M, N, Kd, a_mn, b_mn, dynamic):
         ext.gemm_set_dynamic_tiles(prev)
 
 
+@pytest.mark.parametrize("out", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("M", [1, 7, 8, 9, 16, 17, 31, 32])
+@pytest.mark.parametrize("N,Kd", [
+    (16, 8),       # one block, one warp with work, a step that is not full
+    (24, 40),      # a block with 8 of its 16 columns
+    (1000, 520),   # warps with one step and with two
+    (2376, 1024),  # more blocks than SMs
+    (1024, 2048),  # fewer, and a long contraction
+    (4096, 4096),
+    (56, 14344),
+])
+def test_gemm_of_a_few_rows(K, M, N, Kd, out):
+    """Around the blocks of 8 rows and of 16 columns; rows of the operands and of the result that lie further apart than they are long."""
+    _, impl = K
+    ext = impl.extension()
+    gen = torch.Generator(device="cuda").manual_seed(M + N + Kd)
+    a = torch.randn(M + 1, Kd + 8, device="cuda", generator=gen).to(torch.bfloat16)[:M, :Kd]
+    w = torch.randn(N, Kd + 16, device="cuda", generator=gen).to(torch.bfloat16)[:, :Kd]
+    whole = torch.full((M + 1, N + 8), 99.0, device="cuda", dtype=out)
+    c = whole[:M, :N]
+    ext.gemm(a, w, c, False, False, impl.status_buffer(c.device))
+    ref = a.double() @ w.double().t()
+    # fp32 accumulation of K products, then one rounding
+    assert _rel(c, ref) <= 2**-24 * 8 * Kd ** 0.5 + (2**-8 if out == torch.bfloat16 else 0)
+    c.fill_(99.0)
+    assert bool((whole == 99.0).all())
+
+
 @pytest.mark.parametrize("pair", [True, False])
 def test_gemm_bits_do_not_depend_on_the_launch(K, pair):
     """Products whose rounds of tiles read more than L2 holds: equal rows and columns of the operands give equal results wherever they lie,
