@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "launch.cuh"
 #include "ptx.cuh"
 
 namespace apb {
@@ -92,6 +93,7 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 template <typename T, int NVEC, bool WARP_ROWS, bool IN_TURN = false>
 __global__ void rms_norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ y,
                                     float* __restrict__ rstd, long long rows, int D, float eps) {
+  after_previous();
   __shared__ float red[32];
   const int tpr = WARP_ROWS ? 32 : blockDim.x;
   const int t = WARP_ROWS ? (threadIdx.x & 31) : threadIdx.x;
@@ -177,6 +179,7 @@ constexpr int RMS_BWD_MAX_VEC = 4;
 template <typename T, int NVEC, int ROWS, bool EXACT>
 __global__ void __launch_bounds__(512, 1) rms_norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ w,
                                                            const float* __restrict__ rstd, T* __restrict__ dx, RmsDw dw, long long rows, int D) {
+  after_previous();
   __shared__ float red[32 * ROWS];
   float wreg[NVEC][8];
   float dwreg[NVEC][8];
@@ -300,6 +303,7 @@ __global__ void __launch_bounds__(THREADS, NVEC == 2 && THREADS == 512 ? 2 : 1) 
     mbar_fence_init();
   }
   __syncthreads();
+  after_previous();
   const long long step = gridDim.x, first = blockIdx.x;
   auto issue = [&](long long it) {  // one thread: start the copies of this block's step ``it``
     const long long row = first + it * step;
@@ -389,6 +393,7 @@ __global__ void __launch_bounds__(THREADS, NVEC == 2 && THREADS == 512 ? 2 : 1) 
 // dw = column sums of the blocks' partial rows: 32 columns per block, 32 groups of partial rows
 template <typename T>
 __global__ void __launch_bounds__(1024) rms_dw_kernel(const float* __restrict__ part, T* __restrict__ dw, int nparts, int D) {
+  after_previous();
   __shared__ float red[32][33];
   const int c = blockIdx.x * 32 + (threadIdx.x & 31), g = threadIdx.x >> 5;
   float s = 0.f;
@@ -405,6 +410,7 @@ __global__ void __launch_bounds__(1024) rms_dw_kernel(const float* __restrict__ 
 
 template <typename S, typename D>
 __global__ void __launch_bounds__(256) cast_kernel(const S* __restrict__ src, D* __restrict__ dst, long long n) {
+  after_previous();
   const long long i = (blockIdx.x * 256ll + threadIdx.x) * 8;
   if (i + 8 <= n) {
     Vec8<S> v; v.load(src + i);
@@ -424,6 +430,7 @@ __global__ void __launch_bounds__(256) cast_kernel(const S* __restrict__ src, D*
 template <typename T, int HEADS>
 __global__ void __launch_bounds__(128) rope_kernel(const T* __restrict__ x, const float* __restrict__ cs, const float* __restrict__ sn,
                                                    T* __restrict__ y, long long total_pos_vec, int S, int H, int D, float sign) {
+  after_previous();
   const int vec_per_head = D / 8;
   const unsigned groups = (H + HEADS - 1) / HEADS;  // of heads; neighbouring blocks take the groups of the same positions
   const long long v = blockIdx.x / groups * 128ll + threadIdx.x;
@@ -461,6 +468,7 @@ __global__ void __launch_bounds__(128) rope_kernel(const T* __restrict__ x, cons
 // ------------------------------------------------------------------------------------ SwiGLU
 template <typename T>
 __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ y, long long nvec) {
+  after_previous();
   const long long v = blockIdx.x * 256ll + threadIdx.x;
   if (v >= nvec) return;
   Vec8<T> av, bv; av.load(a + v * 8); bv.load(b + v * 8);
@@ -472,6 +480,7 @@ __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const T* __restrict__ a
 template <typename T>
 __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ a, const T* __restrict__ b,
                                                          T* __restrict__ da, T* __restrict__ db, long long nvec) {
+  after_previous();
   const long long v = blockIdx.x * 256ll + threadIdx.x;
   if (v >= nvec) return;
   Vec8<T> gv, av, bv; gv.load(dy + v * 8); av.load(a + v * 8); bv.load(b + v * 8);
@@ -495,6 +504,7 @@ constexpr int XENT_UNROLL = 2;
 template <typename T>
 __global__ void __launch_bounds__(1024) xent_fwd_kernel(const T* __restrict__ logits, const long long* __restrict__ labels,
                                                         float* __restrict__ loss, float* __restrict__ lse, int V) {
+  after_previous();
   __shared__ float red[32];
   const long long row = blockIdx.x;
   const T* lr = logits + row * V;
@@ -548,6 +558,7 @@ template <typename T, bool PAIRS>
 __global__ void __launch_bounds__(1024) xent_bwd_kernel(const float* __restrict__ dloss, const T* __restrict__ logits,
                                                         const long long* __restrict__ labels, const float* __restrict__ lse,
                                                         T* __restrict__ dlogits, int V) {
+  after_previous();
   const long long row = blockIdx.x;
   const T* lr = logits + row * V;
   T* dr = dlogits + row * V;
@@ -587,6 +598,7 @@ __global__ void __launch_bounds__(1024) xent_bwd_kernel(const float* __restrict_
 template <typename T>
 __global__ void embedding_fwd_kernel(const T* __restrict__ weight, const long long* __restrict__ ids, T* __restrict__ out, int D,
                                      long long num_rows) {
+  after_previous();
   const long long tok = blockIdx.x;
   long long r = ids[tok];
   r = r < 0 ? 0 : (r >= num_rows ? num_rows - 1 : r);  // (an id outside the table is the caller's bug; never read outside)
@@ -614,6 +626,7 @@ constexpr int ADAM_CHUNK = 65536, ADAM_PART = 1024;
 __global__ void __launch_bounds__(ADAM_PART / 4) adamw_kernel(const AdamTensor* __restrict__ tensors, const int2* __restrict__ chunks, float lr,
                              float beta1, float beta2, float eps, float wd, float bc1, float bc2, float grad_scale,
                              const float* __restrict__ hyper) {
+  after_previous();
   if (hyper != nullptr) {
     lr = hyper[0];
     bc1 = hyper[1];
@@ -710,7 +723,7 @@ static inline int launch_rms_norm_bwd(const void* dy, const void* x, const void*
   if (plan.nvec == NV && plan.threads == TH) {                                                                           \
     auto kern = rms_norm_bwd_bulk_kernel<T, NV, TH>;                                                                     \
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -4;         \
-    kern<<<grid, TH, smem, st>>>((const T*)dy, (const T*)x, (const T*)w, rstd, (T*)dx, dw, rows, D);                     \
+    launch_after(kern, grid, TH, smem, st, (const T*)dy, (const T*)x, (const T*)w, rstd, (T*)dx, dw, rows, D);                     \
     return shared ? shared : grid;                                                                                       \
   }
     APB_RMS_BULK(1, 32)
@@ -726,7 +739,7 @@ static inline int launch_rms_norm_bwd(const void* dy, const void* x, const void*
   if constexpr (sizeof(T) == 4) {
     const int grid = (int)(rows < num_sms ? rows : num_sms);
     auto kern = D == 512 * 8 * RMS_BWD_MAX_VEC ? rms_norm_bwd_kernel<T, RMS_BWD_MAX_VEC, 1, true> : rms_norm_bwd_kernel<T, RMS_BWD_MAX_VEC, 1, false>;
-    kern<<<grid, 512, 0, st>>>((const T*)dy, (const T*)x, (const T*)w, rstd, (T*)dx, dw, rows, D);
+    launch_after(kern, grid, 512, 0, st, (const T*)dy, (const T*)x, (const T*)w, rstd, (T*)dx, dw, rows, D);
     return shared ? shared : grid;
   }
   return -3;
@@ -765,7 +778,7 @@ int apb_rms_norm_fwd(const void* x, const void* w, void* y, float* rstd, long lo
     // one warp per row, eight rows per block
     const int nvec = (D + 255) / 256;
     const unsigned grid = blocks_for(rows, 8);
-#define APB_RMS_FWD_W(NV) DISPATCH(is_bf16, rms_norm_fwd_kernel<T, NV, true><<<grid, 256, 0, st>>>((const T*)x, (const T*)w, (T*)y, rstd, rows, D, eps))
+#define APB_RMS_FWD_W(NV) DISPATCH(is_bf16, launch_after(rms_norm_fwd_kernel<T, NV, true>, grid, 256, 0, st, (const T*)x, (const T*)w, (T*)y, rstd, rows, D, eps))
     if (nvec == 1) { APB_RMS_FWD_W(1); } else if (nvec == 2) { APB_RMS_FWD_W(2); } else { APB_RMS_FWD_W(4); }
 #undef APB_RMS_FWD_W
   } else {
@@ -791,8 +804,8 @@ int apb_rms_norm_fwd(const void* x, const void* w, void* y, float* rstd, long lo
       if (rows > cap) grid = (unsigned)cap;
     }
 #define APB_RMS_FWD_B(NV)                                                                                                                             \
-  if (in_turn) rms_norm_fwd_kernel<bf16, NV, false, true><<<grid, threads, 0, st>>>((const bf16*)x, (const bf16*)w, (bf16*)y, rstd, rows, D, eps); \
-  else DISPATCH(is_bf16, rms_norm_fwd_kernel<T, NV, false><<<grid, threads, 0, st>>>((const T*)x, (const T*)w, (T*)y, rstd, rows, D, eps))
+  if (in_turn) launch_after(rms_norm_fwd_kernel<bf16, NV, false, true>, grid, threads, 0, st, (const bf16*)x, (const bf16*)w, (bf16*)y, rstd, rows, D, eps); \
+  else DISPATCH(is_bf16, launch_after(rms_norm_fwd_kernel<T, NV, false>, grid, threads, 0, st, (const T*)x, (const T*)w, (T*)y, rstd, rows, D, eps))
     if (nvec == 1) { APB_RMS_FWD_B(1); } else if (nvec == 2) { APB_RMS_FWD_B(2); } else { APB_RMS_FWD_B(4); }
 #undef APB_RMS_FWD_B
   }
@@ -815,7 +828,7 @@ int apb_rms_norm_bwd(const void* dy, const void* x, const void* w, const float* 
     DISPATCH(is_bf16, n = launch_rms_norm_bwd<T>(dy, x, w, rstd, dx, part, 0, rows, D, num_sms, st));
     if (n < 0) return -n;
   }
-  DISPATCH(is_bf16, rms_dw_kernel<T><<<(D + 31) / 32, 1024, 0, st>>>(part, (T*)dw, n, D));
+  DISPATCH(is_bf16, launch_after(rms_dw_kernel<T>, (D + 31) / 32, 1024, 0, st, part, (T*)dw, n, D));
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 
@@ -823,8 +836,8 @@ int apb_cast(const void* src, void* dst, long long n, int src_bf16, int dst_bf16
   if (!aligned16(src, dst)) return 3;
   if (n == 0) return 0;
   const unsigned grid = blocks_for((n + 7) / 8, 256);
-  if (src_bf16 && !dst_bf16) cast_kernel<bf16, float><<<grid, 256, 0, st>>>((const bf16*)src, (float*)dst, n);
-  else if (!src_bf16 && dst_bf16) cast_kernel<float, bf16><<<grid, 256, 0, st>>>((const float*)src, (bf16*)dst, n);
+  if (src_bf16 && !dst_bf16) launch_after(cast_kernel<bf16, float>, grid, 256, 0, st, (const bf16*)src, (float*)dst, n);
+  else if (!src_bf16 && dst_bf16) launch_after(cast_kernel<float, bf16>, grid, 256, 0, st, (const float*)src, (bf16*)dst, n);
   else return 3;
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
@@ -839,9 +852,9 @@ int apb_rope(const void* x, const float* cs, const float* sn, void* y, long long
   const int heads = nvec * ((H + 7) / 8) >= 768ll * num_sms ? 8 : 4;
   const unsigned grid = blocks_for(nvec, 128) * (unsigned)((H + heads - 1) / heads);
   if (heads == 8) {
-    DISPATCH(is_bf16, rope_kernel<T, 8><<<grid, 128, 0, st>>>((const T*)x, cs, sn, (T*)y, nvec, S, H, D, sign));
+    DISPATCH(is_bf16, launch_after(rope_kernel<T, 8>, grid, 128, 0, st, (const T*)x, cs, sn, (T*)y, nvec, S, H, D, sign));
   } else {
-    DISPATCH(is_bf16, rope_kernel<T, 4><<<grid, 128, 0, st>>>((const T*)x, cs, sn, (T*)y, nvec, S, H, D, sign));
+    DISPATCH(is_bf16, launch_after(rope_kernel<T, 4>, grid, 128, 0, st, (const T*)x, cs, sn, (T*)y, nvec, S, H, D, sign));
   }
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
@@ -850,7 +863,7 @@ int apb_swiglu_fwd(const void* a, const void* b, void* y, long long n, int is_bf
   if (!aligned16(a, b, y)) return 3;
   if (n % 8) return 3;
   if (n == 0) return 0;
-  DISPATCH(is_bf16, swiglu_fwd_kernel<T><<<blocks_for(n / 8, 256), 256, 0, st>>>((const T*)a, (const T*)b, (T*)y, n / 8));
+  DISPATCH(is_bf16, launch_after(swiglu_fwd_kernel<T>, blocks_for(n / 8, 256), 256, 0, st, (const T*)a, (const T*)b, (T*)y, n / 8));
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 
@@ -859,7 +872,7 @@ int apb_swiglu_bwd(const void* dy, const void* a, const void* b, void* da, void*
   if (!aligned16(dy, a, b, da, db)) return 3;
   if (n % 8) return 3;
   if (n == 0) return 0;
-  DISPATCH(is_bf16, swiglu_bwd_kernel<T><<<blocks_for(n / 8, 256), 256, 0, st>>>((const T*)dy, (const T*)a, (const T*)b,
+  DISPATCH(is_bf16, launch_after(swiglu_bwd_kernel<T>, blocks_for(n / 8, 256), 256, 0, st, (const T*)dy, (const T*)a, (const T*)b,
                                                                                        (T*)da, (T*)db, n / 8));
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
@@ -882,7 +895,7 @@ int apb_xent_fwd(const void* logits, const long long* labels, float* loss, float
   if (V % 8) return 3;
   if (rows == 0) return 0;
   const int threads = xent_fwd_threads(rows, V, is_bf16);
-  DISPATCH(is_bf16, xent_fwd_kernel<T><<<(unsigned)rows, threads, 0, st>>>((const T*)logits, labels, loss, lse, V));
+  DISPATCH(is_bf16, launch_after(xent_fwd_kernel<T>, (unsigned)rows, threads, 0, st, (const T*)logits, labels, loss, lse, V));
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 
@@ -892,8 +905,8 @@ int apb_xent_bwd(const float* dloss, const void* logits, const long long* labels
   if (V % 8) return 3;
   if (rows == 0) return 0;
   const int threads = xent_bwd_threads(V, is_bf16);
-  if (is_bf16) xent_bwd_kernel<bf16, true><<<(unsigned)rows, threads, 0, st>>>(dloss, (const bf16*)logits, labels, lse, (bf16*)dlogits, V);
-  else xent_bwd_kernel<float, false><<<(unsigned)rows, threads, 0, st>>>(dloss, (const float*)logits, labels, lse, (float*)dlogits, V);
+  if (is_bf16) launch_after(xent_bwd_kernel<bf16, true>, (unsigned)rows, threads, 0, st, dloss, (const bf16*)logits, labels, lse, (bf16*)dlogits, V);
+  else launch_after(xent_bwd_kernel<float, false>, (unsigned)rows, threads, 0, st, dloss, (const float*)logits, labels, lse, (float*)dlogits, V);
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 
@@ -902,14 +915,14 @@ int apb_embedding_fwd(const void* weight, const long long* ids, void* out, long 
   if (!aligned16(weight, out)) return 3;
   if (tokens == 0) return 0;
   if ((D * (is_bf16 ? 2 : 4)) % 16) return 3;
-  DISPATCH(is_bf16, embedding_fwd_kernel<T><<<(unsigned)tokens, 128, 0, st>>>((const T*)weight, ids, (T*)out, D, num_rows));
+  DISPATCH(is_bf16, launch_after(embedding_fwd_kernel<T>, (unsigned)tokens, 128, 0, st, (const T*)weight, ids, (T*)out, D, num_rows));
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 
 int apb_adamw(const void* tensors_dev, const void* chunks_dev, int num_chunks, float lr, float beta1, float beta2, float eps,
               float wd, float bc1, float bc2, float grad_scale, const float* hyper_dev, cudaStream_t st) {
   if (num_chunks == 0) return 0;
-  adamw_kernel<<<(unsigned)num_chunks * (ADAM_CHUNK / ADAM_PART), ADAM_PART / 4, 0, st>>>((const AdamTensor*)tensors_dev, (const int2*)chunks_dev, lr, beta1, beta2, eps, wd,
+  launch_after(adamw_kernel, (unsigned)num_chunks * (ADAM_CHUNK / ADAM_PART), ADAM_PART / 4, 0, st, (const AdamTensor*)tensors_dev, (const int2*)chunks_dev, lr, beta1, beta2, eps, wd,
                                            bc1, bc2, grad_scale, hyper_dev);
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
@@ -983,9 +996,9 @@ extern "C" int apb_rms_norm_bwd_noalloc(const void* dy, const void* x, const voi
     if (n < 0) return APB_NOALLOC_ERR_BAD_SHAPE;
   }
   if (shared > 1) {
-    DISPATCH(is_bf16, rms_dw_kernel<T><<<(D + 31) / 32, 1024, 0, st>>>(acc, (T*)dw, shared, D));
+    DISPATCH(is_bf16, launch_after(rms_dw_kernel<T>, (D + 31) / 32, 1024, 0, st, acc, (T*)dw, shared, D));
   } else if (is_bf16) {
-    cast_kernel<float, bf16><<<blocks_for(D / 8, 256), 256, 0, st>>>(acc, (bf16*)dw, D);
+    launch_after(cast_kernel<float, bf16>, blocks_for(D / 8, 256), 256, 0, st, acc, (bf16*)dw, D);
   } else {
     if (cudaMemcpyAsync(dw, acc, sizeof(float) * D, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
       return APB_NOALLOC_ERR_LAUNCH;

@@ -26,6 +26,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "launch.cuh"
 #include "ptx.cuh"
 
 extern "C" int apb_cast(const void* src, void* dst, long long n, int src_bf16, int dst_bf16, int num_sms, cudaStream_t st);  // elementwise.cu
@@ -59,6 +60,7 @@ static inline long long emb_round4(long long n) { return (n + 3) & ~3ll; }
 // Blocks of the clusters after the first fill EMB_ZERO_VECS of the ``nzero`` vectors of ``zeros`` each.
 __global__ void __cluster_dims__(EMB_CTAS, 1, 1) __launch_bounds__(EMB_GROUP_THREADS)
 emb_group_kernel(const long long* __restrict__ ids, EmbWs ws, int T, long long V, long long ndone, uint4* __restrict__ zeros, long long nzero) {
+  after_previous();
   if (blockIdx.x >= EMB_CTAS) {
     const long long i = (long long)(blockIdx.x - EMB_CTAS) * EMB_ZERO_VECS + threadIdx.x;
 #pragma unroll
@@ -216,6 +218,7 @@ __device__ __forceinline__ bool emb_last(int* counter, int n) {
 // Zipf's law, 128256 x 4096, 222 us with the sums here, 228 with a launch of their own, 206 so.
 template <typename T, int W>
 __global__ void __launch_bounds__(128) emb_partial_kernel(const T* __restrict__ dy, EmbWs ws, T* __restrict__ out, long long max_chunks, int D) {
+  after_previous();
   __shared__ int list[EMB_CHUNK];
   const int b = blockIdx.x, slices = gridDim.y, step = slices * 128 * W, col0 = (blockIdx.y * 128 + threadIdx.x) * W;
   if (b >= ws.ctr[1]) return;
@@ -270,6 +273,7 @@ __device__ __forceinline__ void emb_row(const T* __restrict__ dy, const EmbWs& w
 template <typename T, int W>
 __global__ void __launch_bounds__(256) emb_tokens_kernel(const T* __restrict__ dy, const long long* __restrict__ ids, EmbWs ws, T* __restrict__ out,
                                                          int tokens, long long V, int D, int tx) {
+  after_previous();
   const int t = blockIdx.x * (256 / tx) + threadIdx.x / tx;
   if (t >= tokens) return;
   const long long v = ids[t];
@@ -283,6 +287,7 @@ __global__ void __launch_bounds__(256) emb_tokens_kernel(const T* __restrict__ d
 template <typename T, int W>
 __global__ void __launch_bounds__(256) emb_rows_kernel(const T* __restrict__ dy, EmbWs ws, T* __restrict__ out, long long V, int D,
                                                        int R, int tx) {
+  after_previous();
   __shared__ int cnt[EMB_ROWS], from[EMB_ROWS];
   const long long row0 = (long long)blockIdx.x * R;
   const int nrows = (int)min((long long)R, V - row0);
@@ -304,6 +309,7 @@ __global__ void __launch_bounds__(256) emb_rows_kernel(const T* __restrict__ dy,
 template <typename T, int U>
 __global__ void __launch_bounds__(256) emb_atomic_kernel(const T* __restrict__ dy, const long long* __restrict__ ids, float* __restrict__ out,
                                                          long long V, int D) {
+  after_previous();
   const long long tok = blockIdx.x;
   const long long r = ids[tok];
   const bool ok = (unsigned long long)r < (unsigned long long)V;
@@ -330,12 +336,13 @@ __global__ void __launch_bounds__(256) emb_atomic_kernel(const T* __restrict__ d
 
 template <typename T>
 static void emb_atomic(const void* dy, const long long* ids, float* out, long long tokens, long long V, int D, cudaStream_t st) {
-  if (D <= 256) emb_atomic_kernel<T, 1><<<(unsigned)tokens, 256, 0, st>>>((const T*)dy, ids, out, V, D);
-  else emb_atomic_kernel<T, 4><<<(unsigned)tokens, 256, 0, st>>>((const T*)dy, ids, out, V, D);
+  if (D <= 256) launch_after(emb_atomic_kernel<T, 1>, (unsigned)tokens, 256, 0, st, (const T*)dy, ids, out, V, D);
+  else launch_after(emb_atomic_kernel<T, 4>, (unsigned)tokens, 256, 0, st, (const T*)dy, ids, out, V, D);
 }
 
 // (a memset of the same bytes takes 1 to 3 us more)
 __global__ void __launch_bounds__(256) emb_zero_kernel(float4* p, long long n) {
+  after_previous();
   const long long i = (long long)blockIdx.x * 1024 + threadIdx.x;
 #pragma unroll
   for (int k = 0; k < 4; ++k)
@@ -364,15 +371,15 @@ static void emb_launch(const void* dy, const long long* ids, const EmbWs& ws, vo
   const bool zeros_first = W > 1 && emb_zeros_first(T_, V, (long long)D * sizeof(T));
   const long long fill = (long long)EMB_CTAS * EMB_ZERO_VECS;  // vectors of a cluster
   const unsigned clusters = 1 + (zeros_first ? (unsigned)((V * nvec + fill - 1) / fill) : 0u);
-  emb_group_kernel<<<EMB_CTAS * clusters, EMB_GROUP_THREADS, 0, st>>>(ids, ws, (int)T_, V, 2 * chunks * slices, reinterpret_cast<uint4*>(out),
+  launch_after(emb_group_kernel, EMB_CTAS * clusters, EMB_GROUP_THREADS, 0, st, ids, ws, (int)T_, V, 2 * chunks * slices, reinterpret_cast<uint4*>(out),
                                                                        V * nvec);
   if (emb_max_longs(T_) > 0)
-    emb_partial_kernel<T, W><<<dim3((unsigned)chunks, (unsigned)slices), 128, 0, st>>>((const T*)dy, ws, (T*)out, chunks, D);
+    launch_after(emb_partial_kernel<T, W>, dim3((unsigned)chunks, (unsigned)slices), 128, 0, st, (const T*)dy, ws, (T*)out, chunks, D);
   int tx = 32;
   while (tx < nvec && tx < 256) tx *= 2;
   if (zeros_first) {
     const int per = 256 / tx;
-    if (T_ > 0) emb_tokens_kernel<T, W><<<(unsigned)((T_ + per - 1) / per), 256, 0, st>>>((const T*)dy, ids, ws, (T*)out, (int)T_, V, D, tx);
+    if (T_ > 0) launch_after(emb_tokens_kernel<T, W>, (unsigned)((T_ + per - 1) / per), 256, 0, st, (const T*)dy, ids, ws, (T*)out, (int)T_, V, D, tx);
     return;
   }
   // rows per block: eight where the table is long (one 64-KB store stream per block), fewer where it would leave SMs idle,
@@ -380,7 +387,7 @@ static void emb_launch(const void* dy, const long long* ids, const EmbWs& ws, vo
   const long long want = V / ((long long)num_sms * 8);
   int R = (int)(want < 1 ? 1 : (want > EMB_ROWS ? EMB_ROWS : want));
   if (R < 256 / tx) R = 256 / tx;
-  emb_rows_kernel<T, W><<<(unsigned)((V + R - 1) / R), 256, 0, st>>>((const T*)dy, ws, (T*)out, V, D, R, tx);
+  launch_after(emb_rows_kernel<T, W>, (unsigned)((V + R - 1) / R), 256, 0, st, (const T*)dy, ws, (T*)out, V, D, R, tx);
 }
 
 static long long emb_carve(EmbWs* ws, void* base, long long T, long long V, int D) {
@@ -451,7 +458,7 @@ extern "C" int apb_embedding_bwd(const void* dy, const long long* ids, void* out
     if (tokens >= (1ll << 31) || (is_bf16 && (reinterpret_cast<uintptr_t>(out) & 15))) return 3;
     float* acc = reinterpret_cast<float*>(is_bf16 ? workspace : out);
     const long long n = num_rows * D;
-    if (n % 4 == 0 && (reinterpret_cast<uintptr_t>(acc) & 15) == 0) emb_zero_kernel<<<(unsigned)((n / 4 + 1023) / 1024), 256, 0, st>>>(reinterpret_cast<float4*>(acc), n / 4);
+    if (n % 4 == 0 && (reinterpret_cast<uintptr_t>(acc) & 15) == 0) launch_after(emb_zero_kernel, (unsigned)((n / 4 + 1023) / 1024), 256, 0, st, reinterpret_cast<float4*>(acc), n / 4);
     else if (cudaMemsetAsync(acc, 0, sizeof(float) * n, st) != cudaSuccess) return 4;
     if (tokens > 0) {
       if (is_bf16) emb_atomic<__nv_bfloat16>(dy, ids, acc, tokens, num_rows, D, st);

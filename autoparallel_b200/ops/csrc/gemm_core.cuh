@@ -26,6 +26,7 @@
 //                   sums the n slots once every rank has signalled completion
 #pragma once
 #include "footprint.cuh"
+#include "launch.cuh"
 #include "ptx.cuh"
 #include "symm_proto.cuh"
 
@@ -620,6 +621,7 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
   }
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (FUSE == FUSE_NONE) wait_previous();
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -716,6 +718,8 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
           }
         }
       }
+      // (not earlier: the next kernel's blocks would take the registers that are left beside this CTA for a communication kernel)
+      if (FUSE == FUSE_NONE) let_next_in();
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer

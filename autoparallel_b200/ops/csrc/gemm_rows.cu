@@ -13,6 +13,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "launch.cuh"
+
 namespace apb {
 
 constexpr int ROWS_WARPS = 16, ROWS_MAX = 32, ROWS_TILE = 16;
@@ -33,6 +35,7 @@ template <int MB, int U, int MIN_BLOCKS>
 __global__ void __launch_bounds__(32 * ROWS_WARPS, MIN_BLOCKS)
 gemm_rows_kernel(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restrict__ W, void* __restrict__ C, int M, int N, int K, long long ldx,
                  long long ldw, long long ldc, int out_fp32) {
+  after_previous();
   constexpr int TM = 8 * MB;
   __shared__ float part[ROWS_WARPS][TM * ROWS_TILE];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = (lane & 3) * 8;
@@ -120,7 +123,7 @@ extern "C" int apb_gemm_rows(const void* X, const void* W, void* C, int M, int N
   if (M > ROWS_MAX || K <= 0 || (K & 7) || (ldx & 7) || (ldw & 7) || ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(W)) & 15)) return 3;
   const unsigned grid = (unsigned)((N + ROWS_TILE - 1) / ROWS_TILE);
   auto launch = [&](auto kern) {
-    kern<<<grid, 32 * ROWS_WARPS, 0, st>>>((const __nv_bfloat16*)X, (const __nv_bfloat16*)W, C, M, N, K, ldx, ldw, ldc, out_fp32);
+    launch_after(kern, grid, 32 * ROWS_WARPS, 0, st, (const __nv_bfloat16*)X, (const __nv_bfloat16*)W, C, M, N, K, ldx, ldw, ldc, out_fp32);
   };
   // Two blocks to an SM and three steps under way; where there is no second block and K is long enough for it, four (8 x 2048 x 2048 4.0 -> 3.7 us, 32
   // x 2048 x 2048 6.4 -> 5.3; 8 x 512 x 512 2.0 -> 2.2).

@@ -86,6 +86,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
     __syncwarp();
     named_arrive(1, SPLIT_THREADS);
+    wait_previous();
   } else {
     if (warp == 1) {
       tmem_alloc(tmem_slot, BN_T);
@@ -98,6 +99,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     named_sync(1, SPLIT_THREADS);
     tc_fence_after();
     tmem_base = *tmem_slot;
+    wait_previous();
   }
   auto fail = [&](uint32_t code) {
     atomicCAS(p.status, 0u, code);
@@ -142,6 +144,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           }
         }
       }
+      let_next_in();
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -478,13 +481,14 @@ extern "C" int apb_gemm_split(const void* A, const void* B, void* C, int G, int 
   cfg.blockDim = dim3(SPLIT_THREADS);
   cfg.dynamicSmemBytes = SPLIT_SMEM_BYTES;
   cfg.stream = stream;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = (unsigned)s;
-  attr.val.clusterDim.y = 1;
-  attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cudaLaunchAttribute attrs[2];
+  attrs[0].id = cudaLaunchAttributeClusterDimension;
+  attrs[0].val.clusterDim.x = (unsigned)s;
+  attrs[0].val.clusterDim.y = 1;
+  attrs[0].val.clusterDim.z = 1;
+  attrs[1] = overlap_attribute();
+  cfg.attrs = attrs;
+  cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, kern, tmA, tmB, p) == cudaSuccess && cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 

@@ -198,7 +198,7 @@ extern "C" int apb_gemm_bf16(const void* A, const void* B, void* C, int M, int N
     const int threads2 = g_pair_stages == PAIR_STAGES ? GEMM_PLAIN_THREADS : GEMM_THREADS;
     auto launch2 = [&](auto kern) {
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2);
-      kern<<<2 * pairs, threads2, smem2, stream>>>(tmA, tmB, p);
+      launch_after(kern, 2 * pairs, threads2, smem2, stream, tmA, tmB, p);
     };
 #define APB_LAUNCH_PAIR(...)                                                                      \
   do {                                                                                            \
@@ -223,7 +223,7 @@ extern "C" int apb_gemm_bf16(const void* A, const void* B, void* C, int M, int N
   set_tile_order(p, p.num_m_tiles, p.num_n_tiles);
   auto launch = [&](auto kern) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_PLAIN_SMEM_BYTES);
-    kern<<<grid, GEMM_PLAIN_THREADS, GEMM_PLAIN_SMEM_BYTES, stream>>>(tmA, tmB, p);
+    launch_after(kern, grid, GEMM_PLAIN_THREADS, GEMM_PLAIN_SMEM_BYTES, stream, tmA, tmB, p);
   };
   if (!a_mn_major && !b_mn_major) launch(gemm_bf16_kernel<false, false>);
   else if (!a_mn_major && b_mn_major) launch(gemm_bf16_kernel<false, true>);
@@ -263,7 +263,7 @@ extern "C" int apb_gemm_grouped_bf16(const void* A, const void* B, void* C, int 
   p.vec_store = 1;  // (N % 8 == 0: rows of 16-byte vectors in both output types)
   auto launch = [&](auto kern, int grid) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_PLAIN_SMEM_BYTES);
-    kern<<<grid, GEMM_PLAIN_THREADS, GEMM_PLAIN_SMEM_BYTES, stream>>>(tmA, tmB, p);
+    launch_after(kern, grid, GEMM_PLAIN_THREADS, GEMM_PLAIN_SMEM_BYTES, stream, tmA, tmB, p);
   };
   if (pair) {
     int resident = apb_gemm_resident_pairs(num_sms) - g_reserved_sms / 2;

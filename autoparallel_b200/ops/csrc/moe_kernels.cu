@@ -19,6 +19,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "launch.cuh"
+
 namespace apb {
 
 // Slots: latency bound.  The arrival rank of an assignment is the number of earlier ones of its token block with the same
@@ -29,6 +31,7 @@ constexpr int SLOT_THREADS = 512;
 
 __global__ void __launch_bounds__(SLOT_THREADS) moe_count_kernel(const long long* __restrict__ gate_idx, int* __restrict__ counts,
                                                                  int per_block, int chunk, int nchunks, int E) {
+  after_previous();
   extern __shared__ int smem_i[];
   const int blk = blockIdx.x / nchunks, ch = blockIdx.x % nchunks;
   for (int e = threadIdx.x; e < E; e += blockDim.x) smem_i[e] = 0;
@@ -48,6 +51,7 @@ __global__ void __launch_bounds__(SLOT_THREADS) moe_count_kernel(const long long
 __global__ void __launch_bounds__(SLOT_THREADS) moe_slots_kernel(const long long* __restrict__ gate_idx, long long* __restrict__ slot,
                                                                  const int* __restrict__ counts, int per_block, int chunk, int nchunks, int E,
                                                                  int C) {
+  after_previous();
   extern __shared__ int smem_i[];
   const int blk = blockIdx.x / nchunks, ch = blockIdx.x % nchunks;
   int* base = smem_i;
@@ -148,6 +152,7 @@ __device__ __forceinline__ long long buf_row(long long s, int blk, int E, int C,
 // 136 -> 69 us (zero fill and 2-byte copies before).
 __global__ void moe_inverse_kernel(const long long* __restrict__ slot, long long* __restrict__ inv, long long n, int k, long long tokens_per_block,
                                    int E, int C, int nb) {
+  after_previous();
   const long long a = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= n) return;
   const long long row = buf_row(slot[a], (int)(a / k / tokens_per_block), E, C, nb);
@@ -159,6 +164,7 @@ template <typename T, int W>
 __global__ void __launch_bounds__(256) moe_scatter_kernel(const T* __restrict__ src, const long long* __restrict__ slot, const void* __restrict__ w,
                                                           int w_bf16, const long long* __restrict__ inv, T* __restrict__ buf, long long n, int k,
                                                           long long tokens_per_block, int d, long long rows, int E, int C, int nb) {
+  after_previous();
   const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= rows) return;
@@ -206,6 +212,7 @@ template <typename T, int W>
 __global__ void __launch_bounds__(128) moe_gather_kernel(const T* __restrict__ buf, const long long* __restrict__ slot, const void* __restrict__ w,
                                                          int w_bf16, T* __restrict__ out, long long Tn, int k, long long tokens_per_block, int d,
                                                          int E, int C, int nb) {
+  after_previous();
   const long long t = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (t >= Tn) return;  // (a whole warp)
@@ -249,6 +256,7 @@ template <typename T, int W>
 __global__ void __launch_bounds__(256) moe_gate_grad_kernel(const T* __restrict__ buf, const long long* __restrict__ slot, const T* __restrict__ g,
                                                             float* __restrict__ dw, long long n, int k, long long tokens_per_block, int d, int E, int C,
                                                             int nb) {
+  after_previous();
   const long long a = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (a >= n) return;
@@ -306,9 +314,9 @@ extern "C" int apb_moe_slots(const long long* gate_idx, long long* slot, int* co
   const int chunk = slot_chunk(num_blocks, per_block, num_sms);
   const int nchunks = (per_block + chunk - 1) / chunk;
   const unsigned grid = (unsigned)((long long)nchunks * num_blocks);
-  if (nchunks > 1) moe_count_kernel<<<grid, threads, (size_t)E * sizeof(int), st>>>(gate_idx, counts, per_block, chunk, nchunks, E);
+  if (nchunks > 1) launch_after(moe_count_kernel, grid, threads, (size_t)E * sizeof(int), st, gate_idx, counts, per_block, chunk, nchunks, E);
   const size_t smem = (size_t)E * ((threads >> 5) + 1) * sizeof(int);
-  moe_slots_kernel<<<grid, threads, smem, st>>>(gate_idx, slot, counts, per_block, chunk, nchunks, E, C);
+  launch_after(moe_slots_kernel, grid, threads, smem, st, gate_idx, slot, counts, per_block, chunk, nchunks, E, C);
   return launch_status();
 }
 
@@ -334,9 +342,9 @@ extern "C" int apb_moe_scatter(const void* src, const long long* slot, const voi
   const long long n = T_ * k, rows = (long long)E * nb * C;
   if (rows <= 0) return 0;
   const long long tpb = T_ / nb;
-  moe_inverse_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(slot, inv, n, k, tpb, E, C, nb);
+  launch_after(moe_inverse_kernel, (unsigned)((n + 255) / 256), 256, 0, st, slot, inv, n, k, tpb, E, C, nb);
   APB_MOE_DISPATCH(is_bf16, vec_rows(d, sizeof(T), src, buf),
-                   moe_scatter_kernel<T, W><<<(unsigned)((rows + 7) / 8), 256, 0, st>>>((const T*)src, slot, w, w_bf16, inv, (T*)buf, n, k, tpb, d,
+                   launch_after(moe_scatter_kernel<T, W>, (unsigned)((rows + 7) / 8), 256, 0, st, (const T*)src, slot, w, w_bf16, inv, (T*)buf, n, k, tpb, d,
                                                                                        rows, E, C, nb));
   return launch_status();
 }
@@ -350,7 +358,7 @@ extern "C" int apb_moe_gather(const void* buf, const long long* slot, const void
     const int pieces = (d + 32 * W - 1) / (32 * W);
     const long long want = (64ll * num_sms + T_ - 1) / T_;
     const dim3 grid((unsigned)((T_ + 3) / 4), (unsigned)(want < pieces ? want : pieces));
-    moe_gather_kernel<T, W><<<grid, 128, 0, st>>>((const T*)buf, slot, w, w_bf16, (T*)out, T_, k, tpb, d, E, C, nb);
+    launch_after(moe_gather_kernel<T, W>, grid, 128, 0, st, (const T*)buf, slot, w, w_bf16, (T*)out, T_, k, tpb, d, E, C, nb);
   });
   return launch_status();
 }
@@ -360,7 +368,7 @@ extern "C" int apb_moe_gate_grad(const void* buf, const long long* slot, const v
   if (T_ <= 0 || k <= 0 || d <= 0 || nb <= 0 || T_ % nb) return (int)cudaErrorInvalidValue;
   const long long n = T_ * k;
   APB_MOE_DISPATCH(is_bf16, vec_rows(d, sizeof(T), buf, g),
-                   moe_gate_grad_kernel<T, W><<<(unsigned)((n + 7) / 8), 256, 0, st>>>((const T*)buf, slot, (const T*)g, dw, n, k, T_ / nb, d, E,
+                   launch_after(moe_gate_grad_kernel<T, W>, (unsigned)((n + 7) / 8), 256, 0, st, (const T*)buf, slot, (const T*)g, dw, n, k, T_ / nb, d, E,
                                                                                        C, nb));
   return launch_status();
 }
