@@ -76,3 +76,46 @@ def test_init_weights_shape_change_is_refused(mesh_1d):
     wrap_init_weights(pm, mode="materialize")
     with pytest.raises(RuntimeError, match="changed the shape"):
         pm.init_weights()
+
+
+def test_gradients_of_all_shards_come_from_one_node(mesh_1d):
+    """What one ``to_local`` per parameter gave: placements, partial and frozen gradients, hooks, no recording without gradients."""
+    from autoparallel_b200.api import _as_shard, _local_params
+
+    pm = _build(mesh_1d)
+    names = [n for n, _ in pm.named_parameters()]
+    params = [p for _, p in pm.named_parameters()]
+    with torch.no_grad():
+        for p in params:
+            p.to_local().copy_(torch.arange(p.to_local().numel()).view_as(p.to_local()))
+        assert all(t is p._local_tensor for t, p in zip(_local_params(params), params))  # nothing is recorded
+    pm.mid.bias.requires_grad_(False)
+    seen = []
+    pm.mid.weight.register_hook(lambda g: seen.append(type(g)))
+    shards = _local_params(params)
+    assert len({id(s.grad_fn) for s in shards if s.requires_grad}) == 1
+    for s, p in zip(shards, params):
+        assert torch.equal(s, p.to_local()) and s.data_ptr() == p.to_local().data_ptr()
+    sum((i + 2) * s.sum() for i, s in enumerate(shards)).backward(retain_graph=True)
+    for i, (n, p) in enumerate(zip(names, params)):
+        if n == "mid.bias":
+            assert p.grad is None
+            continue
+        assert isinstance(p.grad, DTensor) and p.grad.placements == p.placements and p.grad.shape == p.shape and p.grad.stride() == p.stride()
+        assert torch.all(p.grad.to_local() == i + 2)
+    assert seen == [DTensor]
+    w = names.index("mid.weight")
+    (g,) = torch.autograd.grad(shards[w].square().sum(), [params[w]])
+    assert torch.equal(g.to_local(), 2 * params[w].to_local())
+    with torch.no_grad():
+        shards = _local_params(params)
+    assert not any(s.requires_grad for s in shards)
+    y = _local_params(params)[w].square().sum()
+    with torch.no_grad():
+        params[w].to_local().add_(1)  # a change between forward and backward is noticed
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        y.backward()
+    local = params[w].to_local()
+    turned = _as_shard(torch.ones(local.shape[::-1]).t(), params[w]._spec, local.stride())  # a gradient laid out otherwise
+    assert turned.to_local().is_contiguous() and turned.shape == params[w].shape and turned.stride() == params[w].stride()
+
