@@ -159,8 +159,16 @@ __global__ void moe_inverse_kernel(const long long* __restrict__ slot, long long
   if (row >= 0) inv[row] = a;
 }
 
-// one warp per buffer row
-template <typename T, int W>
+// 16-byte vectors may be stored to leave L2 first
+template <bool STREAM, typename T, int W>
+__device__ __forceinline__ void put(T* p, const Pack<T, W>& v) {
+  if constexpr (STREAM && W > 1) __stcs(reinterpret_cast<uint4*>(p), *reinterpret_cast<const uint4*>(&v));
+  else *reinterpret_cast<Pack<T, W>*>(p) = v;
+}
+
+// one warp per buffer row.  STREAM (buffers of more than half of L2): the rows leave L2 first, which keeps the tokens in it; they were read from memory
+// three times over.  64 x 1280 x 2048, 8192 tokens 71.7 -> 65.1 us, 32 x 1280 x 1024 19.3 -> 18.0; 8 x 2560 x 128 7.5 -> 7.7.
+template <typename T, int W, bool STREAM>
 __global__ void __launch_bounds__(256) moe_scatter_kernel(const T* __restrict__ src, const long long* __restrict__ slot, const void* __restrict__ w,
                                                           int w_bf16, const long long* __restrict__ inv, T* __restrict__ buf, long long n, int k,
                                                           long long tokens_per_block, int d, long long rows, int E, int C, int nb) {
@@ -172,7 +180,7 @@ __global__ void __launch_bounds__(256) moe_scatter_kernel(const T* __restrict__ 
   T* y = buf + row * d;
   if (a < 0 || a >= n || buf_row(slot[a], (int)(a / k / tokens_per_block), E, C, nb) != row) {
     const Pack<T, W> zero{};
-    for (int i = lane * W; i < d; i += 32 * W) *reinterpret_cast<Pack<T, W>*>(y + i) = zero;
+    for (int i = lane * W; i < d; i += 32 * W) put<STREAM>(y + i, zero);
     return;
   }
   const T* x = src + a / k * d;
@@ -183,7 +191,7 @@ __global__ void __launch_bounds__(256) moe_scatter_kernel(const T* __restrict__ 
     Pack<T, W> out;
 #pragma unroll
     for (int c = 0; c < W; ++c) out.v[c] = from_f<T>(to_f<T>(in.v[c]) * wt);
-    *reinterpret_cast<Pack<T, W>*>(y + i) = out;
+    put<STREAM>(y + i, out);
   }
 }
 
@@ -191,7 +199,7 @@ __global__ void __launch_bounds__(256) moe_scatter_kernel(const T* __restrict__ 
 // 32 choices at once and pass them round by shuffles, and the loads of eight choices are under way together for every 512 bytes of the
 // result, without a branch (a dropped choice loads nothing and adds zero).  Blocks of 256 threads that shared rows and weights of one
 // token through shared memory spent most of their life waiting for the slots, and 2-byte values in registers cost as much as the loads:
-// 97 -> 65 us, 4.6 TB/s; 32768 tokens 370 -> 230.  (Before that: 371 us, one row address per element.)
+// 97 -> 65 us; 32768 tokens 370 -> 230.  (Before that: 371 us, one row address per element.)
 constexpr int GATHER_K = 8;
 // acc += wt * v, element by element
 __device__ __forceinline__ void add_weighted(float (&acc)[8], float wt, const Pack<__nv_bfloat16, 8>& v) {
@@ -208,8 +216,10 @@ __device__ __forceinline__ void add_weighted(float (&acc)[W], float wt, const Pa
 #pragma unroll
   for (int c = 0; c < W; ++c) acc[c] += wt * to_f<T>(v.v[c]);
 }
-template <typename T, int W>
-__global__ void __launch_bounds__(128) moe_gather_kernel(const T* __restrict__ buf, const long long* __restrict__ slot, const void* __restrict__ w,
+// MIN_BLOCKS: 8 hold the kernel to 64 registers (80 without), a third more loads under way: 8192 tokens 62.5 -> 53.6 us (5.6 TB/s), 1000 10.9 -> 8.7;
+// where the launch does not fill the SMs it is the latency of one token that counts, 333 tokens 3.6 -> 4.3.
+template <typename T, int W, int MIN_BLOCKS>
+__global__ void __launch_bounds__(128, MIN_BLOCKS) moe_gather_kernel(const T* __restrict__ buf, const long long* __restrict__ slot, const void* __restrict__ w,
                                                          int w_bf16, T* __restrict__ out, long long Tn, int k, long long tokens_per_block, int d,
                                                          int E, int C, int nb) {
   after_previous();
@@ -343,9 +353,11 @@ extern "C" int apb_moe_scatter(const void* src, const long long* slot, const voi
   if (rows <= 0) return 0;
   const long long tpb = T_ / nb;
   launch_after(moe_inverse_kernel, (unsigned)((n + 255) / 256), 256, 0, st, slot, inv, n, k, tpb, E, C, nb);
-  APB_MOE_DISPATCH(is_bf16, vec_rows(d, sizeof(T), src, buf),
-                   launch_after(moe_scatter_kernel<T, W>, (unsigned)((rows + 7) / 8), 256, 0, st, (const T*)src, slot, w, w_bf16, inv, (T*)buf, n, k, tpb, d,
-                                                                                       rows, E, C, nb));
+  const bool stream = rows * d * (is_bf16 ? 2 : 4) > 64000000ll;
+  APB_MOE_DISPATCH(is_bf16, vec_rows(d, sizeof(T), src, buf), {
+    auto kern = stream ? moe_scatter_kernel<T, W, true> : moe_scatter_kernel<T, W, false>;
+    launch_after(kern, (unsigned)((rows + 7) / 8), 256, 0, st, (const T*)src, slot, w, w_bf16, inv, (T*)buf, n, k, tpb, d, rows, E, C, nb);
+  });
   return launch_status();
 }
 
@@ -358,7 +370,8 @@ extern "C" int apb_moe_gather(const void* buf, const long long* slot, const void
     const int pieces = (d + 32 * W - 1) / (32 * W);
     const long long want = (64ll * num_sms + T_ - 1) / T_;
     const dim3 grid((unsigned)((T_ + 3) / 4), (unsigned)(want < pieces ? want : pieces));
-    launch_after(moe_gather_kernel<T, W>, grid, 128, 0, st, (const T*)buf, slot, w, w_bf16, (T*)out, T_, k, tpb, d, E, C, nb);
+    auto kern = (long long)grid.x * grid.y >= 6ll * num_sms ? moe_gather_kernel<T, W, 8> : moe_gather_kernel<T, W, 1>;
+    launch_after(kern, grid, 128, 0, st, (const T*)buf, slot, w, w_bf16, (T*)out, T_, k, tpb, d, E, C, nb);
   });
   return launch_status();
 }

@@ -182,6 +182,28 @@ def test_moe_slots_around_one_and_two_rounds(K, T, k, nb, launches, E):
     assert impl.launch_count - before == launches and impl.library_fallbacks == fallbacks
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_moe_rows_of_a_buffer_of_more_than_half_of_l2(K, dtype):
+    """66 and 132 MB: rows that are stored to leave L2 first, and a gather that fills the SMs."""
+    lib, _ = K
+    T, k, E, C, d = 6001, 4, 32, 1000, 1032
+    g = torch.Generator(device="cuda").manual_seed(5)
+    idx = torch.rand(T, E, device="cuda", generator=g).topk(k).indices
+    w = torch.rand(T, k, device="cuda", generator=g).to(dtype)
+    x = torch.randn(T, d, device="cuda", generator=g).to(dtype)
+    slot = lib.ops.moe_slots(idx, E, C, 1)
+    buf = lib.ops.moe_scatter(x, slot, w, E, C, 1)
+    kept = (slot >= 0) & (slot < E * C)
+    assert kept.any() and (slot[kept].unique().numel() == int(kept.sum()))
+    ref = torch.zeros(E * C, d, device="cuda", dtype=dtype)
+    ref[slot[kept]] = (x.float().unsqueeze(1) * w.float().unsqueeze(2)).to(dtype)[kept]
+    assert torch.equal(buf.view(E * C, d), ref)
+    out = lib.ops.moe_gather(buf, slot, w)
+    rows = torch.where(kept.unsqueeze(2), ref[slot.clamp(0, E * C - 1)].double(), 0.0)
+    # fp32 sums of four products, one rounding
+    assert _rel(out, (rows * w.double().unsqueeze(2)).sum(1)) <= 2**-22 + (2**-8 if dtype == torch.bfloat16 else 0)
+
+
 def test_moe_dispatch_leaves_nothing_of_the_old_buffer(K):
     """Every row of the buffer is written, also those no assignment names, whatever the memory held before."""
     lib, _ = K
