@@ -152,7 +152,6 @@ __device__ __forceinline__ long long buf_row(long long s, int blk, int E, int C,
 // 136 -> 69 us (zero fill and 2-byte copies before).
 __global__ void moe_inverse_kernel(const long long* __restrict__ slot, long long* __restrict__ inv, long long n, int k, long long tokens_per_block,
                                    int E, int C, int nb) {
-  after_previous();
   const long long a = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= n) return;
   const long long row = buf_row(slot[a], (int)(a / k / tokens_per_block), E, C, nb);
@@ -352,7 +351,9 @@ extern "C" int apb_moe_scatter(const void* src, const long long* slot, const voi
   const long long n = T_ * k, rows = (long long)E * nb * C;
   if (rows <= 0) return 0;
   const long long tpb = T_ / nb;
-  launch_after(moe_inverse_kernel, (unsigned)((n + 255) / 256), 256, 0, st, slot, inv, n, k, tpb, E, C, nb);
+  // (launched in the ordinary way: where two choices name one row, the one whose warp starts later counts, and warps that waited for the kernel before
+  // them go on in any order)
+  moe_inverse_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(slot, inv, n, k, tpb, E, C, nb);
   const bool stream = rows * d * (is_bf16 ? 2 : 4) > 64000000ll;
   APB_MOE_DISPATCH(is_bf16, vec_rows(d, sizeof(T), src, buf), {
     auto kern = stream ? moe_scatter_kernel<T, W, true> : moe_scatter_kernel<T, W, false>;
