@@ -38,6 +38,7 @@ long long apb_rms_norm_bwd_workspace(long long rows, int D, int is_bf16, int num
 int apb_rms_norm_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx, void* dw, float* part,
                      long long rows, int D, int is_bf16, int num_sms, cudaStream_t st);
 int apb_cast(const void* src, void* dst, long long n, int src_bf16, int dst_bf16, int num_sms, cudaStream_t st);
+int apb_cast_many(const void* const* src, void* const* dst, const long long* n, int count, int* launches, cudaStream_t st);
 int apb_rope(const void* x, const float* cs, const float* sn, void* y, long long B, int S, int H, int D, int conj, int is_bf16,
              int num_sms, cudaStream_t st);
 int apb_swiglu_fwd(const void* a, const void* b, void* y, long long n, int is_bf16, int num_sms, cudaStream_t st);
@@ -555,11 +556,11 @@ std::map<std::string, std::vector<std::array<int, 3>>> kernel_footprints() {
 // ask for, and every call of an operator for which register_cuda_impl has installed another function go to the table of ops/library.py.
 enum Entry : int {
   MM_ND, MM_WGRAD, GROUPED_MM, GROUPED_MM_WGRAD, DTYPE_CAST, RMS_NORM, RMS_NORM_BWD, ROPE, SWIGLU, SWIGLU_BWD, CROSS_ENTROPY, CROSS_ENTROPY_BWD,
-  EMBEDDING, EMBEDDING_BWD, MOE_SLOTS, MOE_SCATTER, MOE_GATHER, MOE_GATE_GRAD, NUM_ENTRIES
+  EMBEDDING, EMBEDDING_BWD, MOE_SLOTS, MOE_SCATTER, MOE_GATHER, MOE_GATE_GRAD, CAST_MANY, NUM_ENTRIES
 };
 constexpr const char* ENTRY_NAMES[NUM_ENTRIES] = {
     "mm_nd", "mm_wgrad", "grouped_mm", "grouped_mm_wgrad", "dtype_cast", "rms_norm", "rms_norm_bwd", "rope", "swiglu", "swiglu_bwd", "cross_entropy",
-    "cross_entropy_bwd", "embedding", "embedding_bwd", "moe_slots", "moe_scatter", "moe_gather", "moe_gate_grad"};
+    "cross_entropy_bwd", "embedding", "embedding_bwd", "moe_slots", "moe_scatter", "moe_gather", "moe_gate_grad", "cast_many"};
 struct Native {
   py::object table;  // operator name -> Python function, as it is at the time of a call
   py::object status_buffer;
@@ -666,6 +667,37 @@ Tensor op_cast(const Tensor& x, at::ScalarType dtype) {
   }
   py::gil_scoped_acquire gil;
   return in_python<Tensor>(DTYPE_CAST, x, py_dtype(dtype));
+}
+// dtype_cast of every tensor; those that its kernel would take are cast together.
+std::vector<Tensor> op_cast_many(at::TensorList xs, at::ScalarType dtype) {
+  if (!ours(CAST_MANY)) {
+    py::gil_scoped_acquire gil;
+    return in_python<std::vector<Tensor>>(CAST_MANY, xs.vec(), py_dtype(dtype));
+  }
+  const bool together = dtype == at::kBFloat16 && ours(DTYPE_CAST) && !native().shadows.load(std::memory_order_relaxed);
+  std::vector<Tensor> out;
+  std::vector<const void*> src;
+  std::vector<void*> dst;
+  std::vector<long long> n;
+  out.reserve(xs.size());
+  for (const Tensor& x : xs) {
+    if (!together || x.scalar_type() != at::kFloat || x.get_device() != xs[0].get_device() || !x.is_contiguous() ||
+        reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 != 0 || x.numel() > (int64_t(1) << 31)) {
+      out.push_back(op_cast(x, dtype));
+      continue;
+    }
+    out.push_back(at::empty(x.sizes(), x.options().dtype(at::kBFloat16)));
+    src.push_back(x.data_ptr());
+    dst.push_back(out.back().data_ptr());
+    n.push_back(x.numel());
+  }
+  if (!src.empty()) {
+    c10::cuda::CUDAGuard g(xs[0].device());
+    int launches = 0;
+    check(apb_cast_many(src.data(), dst.data(), n.data(), (int)src.size(), &launches, stream()), "apb_cast_many");
+    count(launches);
+  }
+  return out;
 }
 Two op_rms_norm(const Tensor& x, const Tensor& w, double eps) {
   if (!ours(RMS_NORM)) return in_python<Two>(RMS_NORM, x, w, eps);
@@ -815,6 +847,7 @@ void register_native(py::dict table, py::object status_buffer, bool diag_library
   lib->impl(ENTRY_NAMES[MOE_SCATTER], op_moe_scatter);
   lib->impl(ENTRY_NAMES[MOE_GATHER], op_moe_gather);
   lib->impl(ENTRY_NAMES[MOE_GATE_GRAD], op_moe_gate_grad);
+  lib->impl(ENTRY_NAMES[CAST_MANY], op_cast_many);
 }
 
 }  // namespace

@@ -324,6 +324,10 @@ def _dtype_cast(x, dtype):
     return x.to(dtype)
 
 
+def _cast_many(xs, dtype):
+    return [_dtype_cast(x, dtype) for x in xs]
+
+
 def _rms_norm(x, w, eps):
     _count()
     return _C.rms_norm(x, w, eps)
@@ -479,6 +483,7 @@ def _register() -> None:
     R("moe_gate_grad", _moe_gate_grad)
     R("grouped_mm_wgrad", _grouped_mm_wgrad)
     R("dtype_cast", _dtype_cast)
+    R("cast_many", _cast_many)
     R("rms_norm", _rms_norm)
     R("rms_norm_bwd", _rms_norm_bwd)
     R("rope", _rope)

@@ -52,6 +52,8 @@ def _cast_ref(x, dtype):
     hit = shadow.lookup(x, dtype) if x.dtype != dtype else None
     return hit if hit is not None else x.to(dtype)
 
+# dtype_cast of every tensor of a list; for graphs that have been planned (parallel/passes/peephole.py), there is no sharding rule
+lib.define("cast_many(Tensor[] xs, ScalarType dtype) -> Tensor[]")
 lib.define("rms_norm(Tensor x, Tensor weight, float eps) -> (Tensor, Tensor)")
 lib.define("rms_norm_bwd(Tensor dy, Tensor x, Tensor weight, Tensor rstd) -> (Tensor, Tensor)")
 lib.define("rope(Tensor x, Tensor cos, Tensor sin, bool conj) -> Tensor")
@@ -195,6 +197,7 @@ def _embedding_bwd_ref(dy, ids, num_rows):
 
 _CPU_IMPLS = {
     "dtype_cast": lambda x, dtype: _cast_ref(x, dtype),
+    "cast_many": lambda xs, dtype: [_cast_ref(x, dtype) for x in xs],
     "rms_norm": _rms_norm_ref,
     "rms_norm_bwd": _rms_norm_bwd_ref,
     "rope": _rope_ref,
@@ -230,6 +233,7 @@ def _gemm_meta(a, b, trans_a, trans_b, out_dtype):
 
 _META_IMPLS = {
     "dtype_cast": lambda x, dtype: _meta_like(x, dtype=dtype),
+    "cast_many": lambda xs, dtype: [_meta_like(x, dtype=dtype) for x in xs],
     "rms_norm": lambda x, w, eps: (_meta_like(x), _meta_like(x, torch.float32, x.shape[:-1])),
     "rms_norm_bwd": lambda dy, x, w, rstd: (_meta_like(x), _meta_like(w)),
     "rope": lambda x, cos, sin, conj: _meta_like(x),

@@ -24,6 +24,7 @@ import torch.fx as fx
 
 from ..parallel.lower.apply import LoweredGraph
 from ..parallel.lower.partition import PartitionedGraph
+from ..parallel.passes.peephole import merge_parameter_casts
 
 
 class Runtime:
@@ -69,6 +70,8 @@ class Runtime:
                                 if kind == "buffer" and bnames[i] in getattr(joint, "buffer_updates", {})}
         self._graph_device = torch.device("cpu")  # device constants inside the graphs (planning happens on CPU fake tensors)
         self._fn = _make_function(self)
+        for gm in (self.fw, self.bw, self.fwd_only):
+            merge_parameter_casts(gm)
         if self.executor == "streams":
             from ..parallel.passes.overlap import schedule_for_streams
 

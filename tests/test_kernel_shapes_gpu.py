@@ -667,3 +667,18 @@ def test_gemm_split_rows_that_are_no_whole_vectors(K, M, N, K_, bn, slices, out)
         assert torch.equal(c, ref), ld
         c.fill_(99.0)
         assert bool((flat == 99.0).all()), ld
+
+
+@pytest.mark.parametrize("sizes", [[1], [0, 5, 0], [2047, 2048, 2049, 8], [16] * 48, [24] * 49 + [1 << 20, 3]])
+def test_cast_many(K, sizes):
+    """Blocks that are not full, empty tensors, as many tensors as one launch takes and more; tensors that go one by one."""
+    lib, impl = K
+    g = torch.Generator(device="cuda").manual_seed(len(sizes))
+    xs = [torch.randn(n, device="cuda", generator=g) for n in sizes]
+    before = impl.launch_count
+    out = lib.ops.cast_many(xs, torch.bfloat16)
+    assert impl.launch_count - before == -(-sum(n > 0 for n in sizes) // 48)
+    assert all(o.dtype == torch.bfloat16 and torch.equal(o, x.to(torch.bfloat16)) for o, x in zip(out, xs))
+    odd = [torch.randn(9, device="cuda")[1:], torch.randn(4, 6, device="cuda").t(), torch.randn(8, device="cuda").bfloat16(), *xs[:1]]
+    assert all(o.dtype == torch.bfloat16 and torch.equal(o, x.to(torch.bfloat16)) for o, x in zip(lib.ops.cast_many(odd, torch.bfloat16), odd))
+    assert all(torch.equal(o, x.float()) for o, x in zip(lib.ops.cast_many(out, torch.float32), out))

@@ -274,3 +274,38 @@ def test_reductions_whose_results_are_added_up_are_not_deferred_as_a_unit(mesh_1
             n_after = sum(1 for n in sched.graph.nodes if n.op == "call_function")
             assert n_after >= n_before  # (split collectives add their waits; nothing is lost or doubled beyond that)
             sched.graph.lint()
+
+
+def test_small_parameter_casts_become_one_node():
+    """Casts of graph inputs to bf16, up to a size, in a graph without collectives; the others stay."""
+    import torch.fx as fx
+
+    import autoparallel_b200.ops  # noqa: F401
+    from autoparallel_b200.parallel.passes import peephole
+    from autoparallel_b200.runtime import comm_ops  # noqa: F401
+
+    cast, many = torch.ops.apb200.dtype_cast.default, torch.ops.apb200.cast_many.default
+
+    def graph(shapes, collective=False):
+        g = fx.Graph()
+        ins = [g.placeholder(f"p{i}") for i in range(len(shapes))]
+        for p, s in zip(ins, shapes):
+            p.meta["val"] = torch.empty(s, device="meta")
+        outs = [g.call_function(cast, (p, torch.bfloat16)) for p in ins]
+        wide = g.call_function(cast, (outs[0], torch.float32))  # not of an input
+        neg = g.call_function(torch.ops.aten.neg.default, (outs[1],))
+        if collective:
+            neg = g.call_function(next(iter(comm_ops.COLLECTIVE_OPS)), (neg,))
+        g.output((wide, neg, *outs))
+        return fx.GraphModule(torch.nn.Module(), g)
+
+    small, large = (3, 4), (1025, 1024)
+    gm = graph([small, (7,), large, (0,)])
+    assert peephole.merge_parameter_casts(gm) == 3
+    assert [n.target for n in gm.graph.nodes].count(many) == 1 and [n.target for n in gm.graph.nodes].count(cast) == 2
+    xs = [torch.randn(small), torch.randn(7), torch.randn(large), torch.randn(0)]
+    got, ref = gm(*xs), graph([small, (7,), large, (0,)])(*xs)
+    assert all(torch.equal(a, b) and a.dtype == b.dtype for a, b in zip(got, ref))
+    assert peephole.merge_parameter_casts(graph([small, small], collective=True)) == 0
+    assert peephole.merge_parameter_casts(graph([large, small])) == 0  # one alone
+    assert peephole.merge_parameter_casts(graph([(1024, 1024)] * 20)) == 16  # what a graph casts at its head is bounded
