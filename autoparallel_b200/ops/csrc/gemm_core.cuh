@@ -142,8 +142,8 @@ inline void set_tile_order(GemmParams& p, int num_m, int num_n) {
 // Wide tiles read A half as often: every wave of tiles goes through the row group's panel of A (16 tile rows) once, and where that no longer
 // stays in L2 from one wave to the next it comes from memory again.  The line lies where that begins, at 36 MB (4096 rows: K = 4394).
 // Narrow -> wide, us at the power cap: 4096 rows of A in a group, N = 4096, K = 4096 205 -> 204, 5120 262 -> 252, 8192 430 -> 401, 14336 747 ->
-// 700; N = 10240, K = 4608 291.9 -> 290.5, 8192 540 -> 511; 2048 rows, N = 14336, K = 5632 259 -> 261, 8192 380 -> 374, 11008 514 -> 496; 8192 x
-// 128256 x 8192 and its like gain 5 to 8 %.  Short contractions lose: K = 512 6 to 8 %, 256 2 to 8 %.
+// 700; N = 10240, K = 4608 291.9 -> 290.5, 8192 540 -> 511; 2048 rows, N = 14336, K = 5632 259 -> 261, 8192 380 -> 374, 11008 514 -> 496; the
+// vocabulary head of 8192 tokens, forward and backward, 21598 -> 20036.  Short contractions lose: K = 512 6 to 8 %, 256 2 to 8 %.
 inline bool set_pair_tiles(GemmParams& p, int num_m, int units, bool may_be_wide) {
   const bool wide = may_be_wide && 2ll * (num_m < GROUP_M ? num_m : GROUP_M) * 2 * BM * p.K >= 36000000ll &&
                     (long long)num_m * ((p.num_n_tiles + 1) / 2) * p.groups >= units;
