@@ -314,6 +314,7 @@ struct SplitPlan {
   int bn, s;
 };
 extern "C" int apb_gemm_resident_pairs(int num_sms);
+extern "C" int apb_gemm_makes_room();
 
 static SplitKernel split_kernel_any() { return gemm_split_kernel<false, false, 64, false>; }
 
@@ -488,7 +489,7 @@ extern "C" int apb_gemm_split(const void* A, const void* B, void* C, int G, int 
   attrs[0].val.clusterDim.z = 1;
   attrs[1] = overlap_attribute();
   cfg.attrs = attrs;
-  cfg.numAttrs = 2;
+  cfg.numAttrs = apb_gemm_makes_room() ? 1 : 2;
   return cudaLaunchKernelEx(&cfg, kern, tmA, tmB, p) == cudaSuccess && cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 

@@ -148,6 +148,17 @@ extern "C" int apb_gemm_get_reserved_sms() { return g_reserved_sms; }
 extern "C" void apb_gemm_set_pair_mode(int on) { g_pair_mode = on ? 1 : 0; }
 extern "C" int apb_gemm_get_pair_mode() { return g_pair_mode; }
 
+// Where the GEMMs are set to make room for communication kernels, they start as ever, after the end of the kernel before them: the gap between two kernels is
+// where such a kernel becomes resident.
+extern "C" int apb_gemm_makes_room() { return g_dynamic_tiles || g_pair_stages != PAIR_STAGES || g_reserved_sms > 0; }
+template <typename Kernel>
+static void launch_gemm(Kernel kern, int grid, int threads, int smem, cudaStream_t stream, const CUtensorMap& tmA, const CUtensorMap& tmB,
+                        const GemmParams& p) {
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (apb_gemm_makes_room()) kern<<<grid, threads, smem, stream>>>(tmA, tmB, p);
+  else launch_after(kern, grid, threads, smem, stream, tmA, tmB, p);
+}
+
 // gemm_split.cu: products with few tiles; -1 = the kernels here are the better choice
 extern "C" int apb_gemm_split_auto(const void* A, const void* B, void* C, int G, int M, int N, int K, long long lda, long long ldb,
                                    long long ldc, int a_mn, int b_mn, int out_fp32, uint32_t* status, int num_sms, int reserved,
@@ -196,10 +207,7 @@ extern "C" int apb_gemm_bf16(const void* A, const void* B, void* C, int M, int N
     const int units = 2 * p.all_tiles - p.whole_tiles, pairs = units < resident ? units : resident;
     const int smem2 = apb_gemm_pair_smem_bytes(g_pair_stages);
     const int threads2 = g_pair_stages == PAIR_STAGES ? GEMM_PLAIN_THREADS : GEMM_THREADS;
-    auto launch2 = [&](auto kern) {
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2);
-      launch_after(kern, 2 * pairs, threads2, smem2, stream, tmA, tmB, p);
-    };
+    auto launch2 = [&](auto kern) { launch_gemm(kern, 2 * pairs, threads2, smem2, stream, tmA, tmB, p); };
 #define APB_LAUNCH_PAIR(...)                                                                      \
   do {                                                                                            \
     if (!a_mn_major && !b_mn_major) launch2(gemm_bf16_pair_kernel<false, false, __VA_ARGS__>);    \
@@ -221,10 +229,7 @@ extern "C" int apb_gemm_bf16(const void* A, const void* B, void* C, int M, int N
   const int tiles = p.num_m_tiles * p.num_n_tiles;
   const int grid = tiles < usable ? tiles : usable;
   set_tile_order(p, p.num_m_tiles, p.num_n_tiles);
-  auto launch = [&](auto kern) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_PLAIN_SMEM_BYTES);
-    launch_after(kern, grid, GEMM_PLAIN_THREADS, GEMM_PLAIN_SMEM_BYTES, stream, tmA, tmB, p);
-  };
+  auto launch = [&](auto kern) { launch_gemm(kern, grid, GEMM_PLAIN_THREADS, GEMM_PLAIN_SMEM_BYTES, stream, tmA, tmB, p); };
   if (!a_mn_major && !b_mn_major) launch(gemm_bf16_kernel<false, false>);
   else if (!a_mn_major && b_mn_major) launch(gemm_bf16_kernel<false, true>);
   else if (a_mn_major && !b_mn_major) launch(gemm_bf16_kernel<true, false>);
@@ -261,10 +266,7 @@ extern "C" int apb_gemm_grouped_bf16(const void* A, const void* B, void* C, int 
   p.status = status;
   p.groups = G;
   p.vec_store = 1;  // (N % 8 == 0: rows of 16-byte vectors in both output types)
-  auto launch = [&](auto kern, int grid) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_PLAIN_SMEM_BYTES);
-    launch_after(kern, grid, GEMM_PLAIN_THREADS, GEMM_PLAIN_SMEM_BYTES, stream, tmA, tmB, p);
-  };
+  auto launch = [&](auto kern, int grid) { launch_gemm(kern, grid, GEMM_PLAIN_THREADS, GEMM_PLAIN_SMEM_BYTES, stream, tmA, tmB, p); };
   if (pair) {
     int resident = apb_gemm_resident_pairs(num_sms) - g_reserved_sms / 2;
     if (resident < 1) resident = 1;
