@@ -539,7 +539,8 @@ def _as_shard(grad: torch.Tensor, spec, stride: tuple) -> DTensor:
     """The gradient of a shard as a DTensor that is placed like its parameter."""
     if grad.stride() == stride:
         return DTensor(grad, spec, requires_grad=grad.requires_grad)
-    return DTensor.from_local(grad.contiguous(), spec.mesh, spec.placements, run_check=False, shape=spec.shape, stride=_contig_stride(spec.shape))
+    return DTensor.from_local(grad.contiguous(), spec.mesh, spec.placements, run_check=False, shape=spec.shape,
+                              stride=_contig_stride(spec.shape))
 
 
 def _local_params(params: list) -> list:

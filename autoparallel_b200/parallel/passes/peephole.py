@@ -58,7 +58,9 @@ def merge_parameter_casts(gm: fx.GraphModule) -> int:
         return 0
     casts, elements = [], 0
     for n in nodes:
-        if n.op != "call_function" or n.target is not apb.dtype_cast.default or n.args[1] is not torch.bfloat16 or n.args[0].op != "placeholder":
+        if n.op != "call_function" or n.target is not apb.dtype_cast.default:
+            continue
+        if n.args[1] is not torch.bfloat16 or n.args[0].op != "placeholder":
             continue
         val = n.args[0].meta.get("val")
         if not isinstance(val, torch.Tensor) or val.dtype is not torch.float32 or not all(isinstance(d, int) for d in val.shape):

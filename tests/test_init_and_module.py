@@ -101,7 +101,8 @@ def test_gradients_of_all_shards_come_from_one_node(mesh_1d):
         if n == "mid.bias":
             assert p.grad is None
             continue
-        assert isinstance(p.grad, DTensor) and p.grad.placements == p.placements and p.grad.shape == p.shape and p.grad.stride() == p.stride()
+        assert isinstance(p.grad, DTensor) and p.grad.placements == p.placements
+        assert p.grad.shape == p.shape and p.grad.stride() == p.stride()
         assert torch.all(p.grad.to_local() == i + 2)
     assert seen == [DTensor]
     w = names.index("mid.weight")

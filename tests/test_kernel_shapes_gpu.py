@@ -680,5 +680,6 @@ def test_cast_many(K, sizes):
     assert impl.launch_count - before == -(-sum(n > 0 for n in sizes) // 48)
     assert all(o.dtype == torch.bfloat16 and torch.equal(o, x.to(torch.bfloat16)) for o, x in zip(out, xs))
     odd = [torch.randn(9, device="cuda")[1:], torch.randn(4, 6, device="cuda").t(), torch.randn(8, device="cuda").bfloat16(), *xs[:1]]
-    assert all(o.dtype == torch.bfloat16 and torch.equal(o, x.to(torch.bfloat16)) for o, x in zip(lib.ops.cast_many(odd, torch.bfloat16), odd))
+    got = lib.ops.cast_many(odd, torch.bfloat16)
+    assert all(o.dtype == torch.bfloat16 and torch.equal(o, x.to(torch.bfloat16)) for o, x in zip(got, odd))
     assert all(torch.equal(o, x.float()) for o, x in zip(lib.ops.cast_many(out, torch.float32), out))
