@@ -90,10 +90,9 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 // sum of squares and the scaling, so x is read once.  TPR = 32: one warp per row, reduction by shuffles only, no
 // block barrier; several rows per block keep enough loads in flight.  TPR = blockDim.x: a block takes a row at a time (see apb_rms_norm_fwd).
 // D % 8 == 0 and D <= TPR * 8 * NVEC.
-template <typename T, int NVEC, bool WARP_ROWS, bool IN_TURN = false>
-__global__ void rms_norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ y,
-                                    float* __restrict__ rstd, long long rows, int D, float eps) {
-  after_previous();
+template <typename T, int NVEC, bool WARP_ROWS, bool IN_TURN>
+__device__ __forceinline__ void rms_norm_fwd(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ y, float* __restrict__ rstd, long long rows,
+                                             int D, float eps) {
   __shared__ float red[32];
   const int tpr = WARP_ROWS ? 32 : blockDim.x;
   const int t = WARP_ROWS ? (threadIdx.x & 31) : threadIdx.x;
@@ -129,6 +128,11 @@ __global__ void rms_norm_fwd_kernel(const T* __restrict__ x, const T* __restrict
       }
     }
   } while (IN_TURN && (row += gridDim.x) < rows);  // (the same for the whole block)
+}
+template <typename T, int NVEC, bool WARP_ROWS, bool IN_TURN = false>
+__global__ void rms_norm_fwd_kernel(const T* x, const T* w, T* y, float* rstd, long long rows, int D, float eps) {
+  after_previous();
+  rms_norm_fwd<T, NVEC, WARP_ROWS, IN_TURN>(x, w, y, rstd, rows, D, eps);
 }
 
 // block-wide sums of R values at once (one barrier pair for all of them); ``red`` holds 32 * R floats
@@ -177,8 +181,8 @@ struct RmsDw {
 // Requires D <= blockDim.x * 8 * RMS_BWD_MAX_VEC.
 constexpr int RMS_BWD_MAX_VEC = 4;
 template <typename T, int NVEC, int ROWS, bool EXACT>
-__global__ void __launch_bounds__(512, 1) rms_norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ w,
-                                                           const float* __restrict__ rstd, T* __restrict__ dx, RmsDw dw, long long rows, int D) {
+__global__ void __launch_bounds__(512, 1) rms_norm_bwd_kernel(const T* dy, const T* x, const T* w, const float* rstd, T* dx, RmsDw dw, long long rows,
+                                                             int D) {
   after_previous();
   __shared__ float red[32 * ROWS];
   float wreg[NVEC][8];
@@ -286,9 +290,8 @@ __global__ void __launch_bounds__(512, 1) rms_norm_bwd_kernel(const T* __restric
 constexpr int RMS_STAGES = 3;
 __host__ __device__ inline int rms_ring_bytes(int row_bytes) { return RMS_STAGES * 2 * row_bytes + 128; }
 template <typename T, int NVEC, int THREADS>
-__global__ void __launch_bounds__(THREADS, NVEC == 2 && THREADS == 512 ? 2 : 1) rms_norm_bwd_bulk_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ w,
-                                                                    const float* __restrict__ rstd, T* __restrict__ dx, RmsDw dw,
-                                                                    long long rows, int D) {
+__global__ void __launch_bounds__(THREADS, NVEC == 2 && THREADS == 512 ? 2 : 1) rms_norm_bwd_bulk_kernel(const T* dy, const T* x,
+                                                                    const T* w, const float* rstd, T* dx, RmsDw dw, long long rows, int D) {
   extern __shared__ uint8_t rms_smem_raw[];
   __shared__ uint64_t bars[RMS_STAGES];
   __shared__ float red[2][THREADS / 32];
@@ -392,7 +395,7 @@ __global__ void __launch_bounds__(THREADS, NVEC == 2 && THREADS == 512 ? 2 : 1) 
 
 // dw = column sums of the blocks' partial rows: 32 columns per block, 32 groups of partial rows
 template <typename T>
-__global__ void __launch_bounds__(1024) rms_dw_kernel(const float* __restrict__ part, T* __restrict__ dw, int nparts, int D) {
+__global__ void __launch_bounds__(1024) rms_dw_kernel(const float* part, T* dw, int nparts, int D) {
   after_previous();
   __shared__ float red[32][33];
   const int c = blockIdx.x * 32 + (threadIdx.x & 31), g = threadIdx.x >> 5;
@@ -409,7 +412,7 @@ __global__ void __launch_bounds__(1024) rms_dw_kernel(const float* __restrict__ 
 }
 
 template <typename S, typename D>
-__global__ void __launch_bounds__(256) cast_kernel(const S* __restrict__ src, D* __restrict__ dst, long long n) {
+__global__ void __launch_bounds__(256) cast_kernel(const S* src, D* dst, long long n) {
   after_previous();
   const long long i = (blockIdx.x * 256ll + threadIdx.x) * 8;
   if (i + 8 <= n) {
@@ -455,10 +458,10 @@ __global__ void __launch_bounds__(256) cast_many_kernel(const __grid_constant__ 
 // head (one 16-byte vector) at one position, in HEADS neighbouring heads: the 32 bytes of cos / sin it needs are read
 // once for them (the tables would otherwise be twice the traffic of x itself).  Eight heads where that leaves the SMs 768 threads each, else
 // four; all heads of a position in one thread -> 8 / 4 heads a thread: 8192 x 32 x 128 33.4 -> 25.3 / 27.7 us, 8192 x 8 x 128 8.3 -> 8.2 / 9.0,
-// 8192 x 8 x 64 5.6 -> 5.5 / 4.2, 100 x 32 x 128 8.8 -> 3.6 / 2.7.
+// 8192 x 8 x 64 5.6 -> 5.5 / 4.2, 100 x 32 x 128 8.8 -> 3.6 / 2.7.  Eight loads under way instead of four: 8192 x 8 x 128 8.0 -> 7.6, fp32 16.9 -> 15.4.
 template <typename T, int HEADS>
-__global__ void __launch_bounds__(128) rope_kernel(const T* __restrict__ x, const float* __restrict__ cs, const float* __restrict__ sn,
-                                                   T* __restrict__ y, long long total_pos_vec, int S, int H, int D, float sign) {
+__global__ void __launch_bounds__(128) rope_kernel(const T* x, const float* cs, const float* sn, T* y, long long total_pos_vec, int S, int H,
+                                                   int D, float sign) {
   after_previous();
   const int vec_per_head = D / 8;
   const unsigned groups = (H + HEADS - 1) / HEADS;  // of heads; neighbouring blocks take the groups of the same positions
@@ -473,30 +476,27 @@ __global__ void __launch_bounds__(128) rope_kernel(const T* __restrict__ x, cons
   const float nn[4] = {n.x * sign, n.y * sign, n.z * sign, n.w * sign};
   const long long base = (bs * H) * D + dv * 8;
   const int h0 = blockIdx.x % groups * HEADS, h1 = min(H, h0 + HEADS);
+  Vec8<T> xv[HEADS];  // (all loads before the first store)
 #pragma unroll
-  for (int hg = 0; hg < HEADS; hg += 4) {  // four independent loads in flight
-    Vec8<T> xv[4];
+  for (int k = 0; k < HEADS; ++k)
+    if (h0 + k < h1) xv[k].load(x + base + (long long)(h0 + k) * D);
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
-      if (h0 + hg + k < h1) xv[k].load(x + base + (long long)(h0 + hg + k) * D);
+  for (int k = 0; k < HEADS; ++k) {
+    if (h0 + k >= h1) break;
+    float f[8], o[8];
+    xv[k].to_float(f);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (h0 + hg + k >= h1) break;
-      float f[8], o[8];
-      xv[k].to_float(f);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        o[2 * i] = f[2 * i] * cc[i] - f[2 * i + 1] * nn[i];
-        o[2 * i + 1] = f[2 * i] * nn[i] + f[2 * i + 1] * cc[i];
-      }
-      Vec8<T> ov; ov.from_float(o); ov.store(y + base + (long long)(h0 + hg + k) * D);
+    for (int i = 0; i < 4; ++i) {
+      o[2 * i] = f[2 * i] * cc[i] - f[2 * i + 1] * nn[i];
+      o[2 * i + 1] = f[2 * i] * nn[i] + f[2 * i + 1] * cc[i];
     }
+    Vec8<T> ov; ov.from_float(o); ov.store(y + base + (long long)(h0 + k) * D);
   }
 }
 
 // ------------------------------------------------------------------------------------ SwiGLU
 template <typename T>
-__global__ void __launch_bounds__(256) swiglu_fwd_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ y, long long nvec) {
+__global__ void __launch_bounds__(256) swiglu_fwd_kernel(const T* a, const T* b, T* y, long long nvec) {
   after_previous();
   const long long v = blockIdx.x * 256ll + threadIdx.x;
   if (v >= nvec) return;
@@ -507,8 +507,7 @@ __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const T* __restrict__ a
   Vec8<T> ov; ov.from_float(o); ov.store(y + v * 8);
 }
 template <typename T>
-__global__ void __launch_bounds__(256) swiglu_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ a, const T* __restrict__ b,
-                                                         T* __restrict__ da, T* __restrict__ db, long long nvec) {
+__global__ void __launch_bounds__(256) swiglu_bwd_kernel(const T* dy, const T* a, const T* b, T* da, T* db, long long nvec) {
   after_previous();
   const long long v = blockIdx.x * 256ll + threadIdx.x;
   if (v >= nvec) return;
@@ -531,8 +530,7 @@ __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const T* __restrict__ d
 // The maximum moves once per step of all its vectors, not once per vector.
 constexpr int XENT_UNROLL = 2;
 template <typename T>
-__global__ void __launch_bounds__(1024) xent_fwd_kernel(const T* __restrict__ logits, const long long* __restrict__ labels,
-                                                        float* __restrict__ loss, float* __restrict__ lse, int V) {
+__global__ void __launch_bounds__(1024) xent_fwd_kernel(const T* logits, const long long* labels, float* loss, float* lse, int V) {
   after_previous();
   __shared__ float red[32];
   const long long row = blockIdx.x;
@@ -584,9 +582,8 @@ __global__ void __launch_bounds__(1024) xent_fwd_kernel(const T* __restrict__ lo
   }
 }
 template <typename T, bool PAIRS>
-__global__ void __launch_bounds__(1024) xent_bwd_kernel(const float* __restrict__ dloss, const T* __restrict__ logits,
-                                                        const long long* __restrict__ labels, const float* __restrict__ lse,
-                                                        T* __restrict__ dlogits, int V) {
+__global__ void __launch_bounds__(1024) xent_bwd_kernel(const float* dloss, const T* logits, const long long* labels, const float* lse,
+                                                        T* dlogits, int V) {
   after_previous();
   const long long row = blockIdx.x;
   const T* lr = logits + row * V;
@@ -624,17 +621,16 @@ __global__ void __launch_bounds__(1024) xent_bwd_kernel(const float* __restrict_
 
 // ------------------------------------------------------------------------------------ embedding forward
 // out[token] = weight[ids[token]]: one block per token, 16-byte vectors (D % 8 == 0 for bf16, % 4 for fp32).
+__device__ __forceinline__ void copy_row(const uint4* __restrict__ src, uint4* __restrict__ dst, int nvec) {
+  for (int c = threadIdx.x; c < nvec; c += blockDim.x) dst[c] = src[c];
+}
 template <typename T>
-__global__ void embedding_fwd_kernel(const T* __restrict__ weight, const long long* __restrict__ ids, T* __restrict__ out, int D,
-                                     long long num_rows) {
+__global__ void embedding_fwd_kernel(const T* weight, const long long* ids, T* out, int D, long long num_rows) {
   after_previous();
   const long long tok = blockIdx.x;
   long long r = ids[tok];
   r = r < 0 ? 0 : (r >= num_rows ? num_rows - 1 : r);  // (an id outside the table is the caller's bug; never read outside)
-  const uint4* src = reinterpret_cast<const uint4*>(weight + r * D);
-  uint4* dst = reinterpret_cast<uint4*>(out + tok * D);
-  const int nvec = D * (int)sizeof(T) / 16;
-  for (int c = threadIdx.x; c < nvec; c += blockDim.x) dst[c] = src[c];
+  copy_row(reinterpret_cast<const uint4*>(weight + r * D), reinterpret_cast<uint4*>(out + tok * D), D * (int)sizeof(T) / 16);
 }
 
 // ------------------------------------------------------------------------------------ AdamW
@@ -652,9 +648,8 @@ struct AdamTensor {
 constexpr int ADAM_CHUNK = 65536, ADAM_PART = 1024;
 // ``hyper`` (optional, device memory): {lr, bc1, bc2} read at run time instead of the launch arguments, so that a step
 // captured in a CUDA graph follows the learning-rate schedule and the bias corrections of the step it is replayed for.
-__global__ void __launch_bounds__(ADAM_PART / 4) adamw_kernel(const AdamTensor* __restrict__ tensors, const int2* __restrict__ chunks, float lr,
-                             float beta1, float beta2, float eps, float wd, float bc1, float bc2, float grad_scale,
-                             const float* __restrict__ hyper) {
+__global__ void __launch_bounds__(ADAM_PART / 4) adamw_kernel(const AdamTensor* tensors, const int2* chunks, float lr,
+                             float beta1, float beta2, float eps, float wd, float bc1, float bc2, float grad_scale, const float* hyper) {
   after_previous();
   if (hyper != nullptr) {
     lr = hyper[0];

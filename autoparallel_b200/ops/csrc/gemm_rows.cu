@@ -21,7 +21,7 @@ constexpr int ROWS_WARPS = 16, ROWS_MAX = 32, ROWS_TILE = 16;
 
 __device__ __forceinline__ uint4 ld_stream(const __nv_bfloat16* p) {
   uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
 __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -33,7 +33,7 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
 // MB: blocks of 8 rows of X; U: steps of 32 elements of K whose loads are under way together
 template <int MB, int U, int MIN_BLOCKS>
 __global__ void __launch_bounds__(32 * ROWS_WARPS, MIN_BLOCKS)
-gemm_rows_kernel(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restrict__ W, void* __restrict__ C, int M, int N, int K, long long ldx,
+gemm_rows_kernel(const __nv_bfloat16* X, const __nv_bfloat16* W, void* C, int M, int N, int K, long long ldx,
                  long long ldw, long long ldc, int out_fp32) {
   after_previous();
   constexpr int TM = 8 * MB;
@@ -69,7 +69,7 @@ gemm_rows_kernel(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __res
 #pragma unroll
       for (int i = 0; i < MB; ++i) {
         xv[u][i] = make_uint4(0, 0, 0, 0);
-        if (in && xk[i]) xv[u][i] = __ldg(reinterpret_cast<const uint4*>(x[i] + k));
+        if (in && xk[i]) xv[u][i] = *reinterpret_cast<const uint4*>(x[i] + k);
       }
     }
 #pragma unroll

@@ -6,6 +6,11 @@
 // then at most two kernels of a stream overlap, and the earlier of them has seen everything before it complete.  A kernel that is launched in the
 // ordinary way waits for all of its predecessor as ever, whether that one let it in or not.
 //
+// What such a kernel reads may still be written when it is resident already, so its loads carry no promise that data stays the same for the life of
+// the kernel: no __restrict__ on its parameters, no __ldg, no ld.global.nc - with those the compiler may move a load above the wait.  Where a loop has to
+// know that its stores do not touch what it loads, a function that is called behind the wait has the __restrict__ parameters, or the loads of several
+// steps are written out before the stores.
+//
 // Worth it where kernels are short: without it the GPU starts the next kernel of a stream one to two microseconds after the end of the last, on
 // a grid of 2.05 us (16 x 4096 x 4096, 8.8 us in a captured graph: 10.24 a launch, with it 8.6; 8 x 4096 x 4096 9.6 -> 7.4).
 #pragma once

@@ -29,8 +29,8 @@ namespace apb {
 // 170 -> 7.4 us (one CTA walked the block in rounds of 1024 before).
 constexpr int SLOT_THREADS = 512;
 
-__global__ void __launch_bounds__(SLOT_THREADS) moe_count_kernel(const long long* __restrict__ gate_idx, int* __restrict__ counts,
-                                                                 int per_block, int chunk, int nchunks, int E) {
+__global__ void __launch_bounds__(SLOT_THREADS) moe_count_kernel(const long long* gate_idx, int* counts, int per_block, int chunk, int nchunks,
+                                                                 int E) {
   after_previous();
   extern __shared__ int smem_i[];
   const int blk = blockIdx.x / nchunks, ch = blockIdx.x % nchunks;
@@ -48,9 +48,8 @@ __global__ void __launch_bounds__(SLOT_THREADS) moe_count_kernel(const long long
 }
 
 // Shared memory: base[E] (assignments of each expert seen so far) and wcnt[warps][E] (those of each warp in this round).
-__global__ void __launch_bounds__(SLOT_THREADS) moe_slots_kernel(const long long* __restrict__ gate_idx, long long* __restrict__ slot,
-                                                                 const int* __restrict__ counts, int per_block, int chunk, int nchunks, int E,
-                                                                 int C) {
+__global__ void __launch_bounds__(SLOT_THREADS) moe_slots_kernel(const long long* gate_idx, long long* slot, const int* counts, int per_block,
+                                                                 int chunk, int nchunks, int E, int C) {
   after_previous();
   extern __shared__ int smem_i[];
   const int blk = blockIdx.x / nchunks, ch = blockIdx.x % nchunks;
@@ -150,12 +149,28 @@ __device__ __forceinline__ long long buf_row(long long s, int blk, int E, int C,
 // not zero-filled first.  ``inv`` names the assignment of a row; rows that none names hold whatever the memory held, so a
 // row's entry counts only if that assignment's slot leads back to the row.
 // 136 -> 69 us (zero fill and 2-byte copies before).
-__global__ void moe_inverse_kernel(const long long* __restrict__ slot, long long* __restrict__ inv, long long n, int k, long long tokens_per_block,
+__global__ void moe_inverse_kernel(const long long* slot, long long* inv, long long n, int k, long long tokens_per_block,
                                    int E, int C, int nb) {
   const long long a = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= n) return;
   const long long row = buf_row(slot[a], (int)(a / k / tokens_per_block), E, C, nb);
   if (row >= 0) inv[row] = a;
+}
+
+// The words of a Pack: the bf16 values of a vector that waits for its turn stay in 4 registers (as values they take 8).
+template <typename T, int W>
+struct RawOf { typedef uint4 type; };
+template <typename T>
+struct RawOf<T, 1> { typedef T type; };
+template <typename T, int W>
+using Raw = typename RawOf<T, W>::type;
+template <typename T, int W>
+__device__ __forceinline__ Pack<T, W> weighted(const Raw<T, W>& raw, float wt) {
+  Pack<T, W> out;
+  const Pack<T, W> in = *reinterpret_cast<const Pack<T, W>*>(&raw);
+#pragma unroll
+  for (int c = 0; c < W; ++c) out.v[c] = from_f<T>(to_f<T>(in.v[c]) * wt);
+  return out;
 }
 
 // 16-byte vectors may be stored to leave L2 first
@@ -168,29 +183,32 @@ __device__ __forceinline__ void put(T* p, const Pack<T, W>& v) {
 // one warp per buffer row.  STREAM (buffers of more than half of L2): the rows leave L2 first, which keeps the tokens in it; they were read from memory
 // three times over.  64 x 1280 x 2048, 8192 tokens 71.7 -> 65.1 us, 32 x 1280 x 1024 19.3 -> 18.0; 8 x 2560 x 128 7.5 -> 7.7.
 template <typename T, int W, bool STREAM>
-__global__ void __launch_bounds__(256) moe_scatter_kernel(const T* __restrict__ src, const long long* __restrict__ slot, const void* __restrict__ w,
-                                                          int w_bf16, const long long* __restrict__ inv, T* __restrict__ buf, long long n, int k,
-                                                          long long tokens_per_block, int d, long long rows, int E, int C, int nb) {
+__global__ void __launch_bounds__(256, 8) moe_scatter_kernel(const T* src, const long long* slot, const void* w, int w_bf16, const long long* inv, T* buf,
+                                                          long long n, int k, long long tokens_per_block, int d, long long rows, int E, int C, int nb) {
   after_previous();
   const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= rows) return;
   const long long a = inv[row];
   T* y = buf + row * d;
-  if (a < 0 || a >= n || buf_row(slot[a], (int)(a / k / tokens_per_block), E, C, nb) != row) {
+  const bool named = a >= 0 && a < n;
+  const long long to = named ? slot[a] : -1;
+  const float wt = named ? gate_weight<T>(w, a, w_bf16) : 0.f;  // (under way with the slot)
+  if (!named || buf_row(to, (int)(a / k / tokens_per_block), E, C, nb) != row) {
     const Pack<T, W> zero{};
     for (int i = lane * W; i < d; i += 32 * W) put<STREAM>(y + i, zero);
     return;
   }
   const T* x = src + a / k * d;
-  const float wt = gate_weight<T>(w, a, w_bf16);
-#pragma unroll 4
-  for (int i = lane * W; i < d; i += 32 * W) {
-    const Pack<T, W> in = *reinterpret_cast<const Pack<T, W>*>(x + i);
-    Pack<T, W> out;
+#pragma unroll 1
+  for (int i = lane * W; i < d; i += 4 * 32 * W) {  // four loads under way
+    Raw<T, W> v[4];
 #pragma unroll
-    for (int c = 0; c < W; ++c) out.v[c] = from_f<T>(to_f<T>(in.v[c]) * wt);
-    put<STREAM>(y + i, out);
+    for (int q = 0; q < 4; ++q)
+      if (i + q * 32 * W < d) v[q] = *reinterpret_cast<const Raw<T, W>*>(x + i + q * 32 * W);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (i + q * 32 * W < d) put<STREAM>(y + i + q * 32 * W, weighted<T, W>(v[q], wt));
   }
 }
 
@@ -218,9 +236,8 @@ __device__ __forceinline__ void add_weighted(float (&acc)[W], float wt, const Pa
 // MIN_BLOCKS: 8 hold the kernel to 64 registers (80 without), a third more loads under way: 8192 tokens 62.5 -> 53.6 us (5.6 TB/s), 1000 10.9 -> 8.7;
 // where the launch does not fill the SMs it is the latency of one token that counts, 333 tokens 3.6 -> 4.3.
 template <typename T, int W, int MIN_BLOCKS>
-__global__ void __launch_bounds__(128, MIN_BLOCKS) moe_gather_kernel(const T* __restrict__ buf, const long long* __restrict__ slot, const void* __restrict__ w,
-                                                         int w_bf16, T* __restrict__ out, long long Tn, int k, long long tokens_per_block, int d,
-                                                         int E, int C, int nb) {
+__global__ void __launch_bounds__(128, MIN_BLOCKS) moe_gather_kernel(const T* buf, const long long* slot, const void* w, int w_bf16, T* out,
+                                                         long long Tn, int k, long long tokens_per_block, int d, int E, int C, int nb) {
   after_previous();
   const long long t = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -262,9 +279,8 @@ __global__ void __launch_bounds__(128, MIN_BLOCKS) moe_gather_kernel(const T* __
 // one warp per assignment; the choices of a token sit in one block, so its gradient row comes from cache after the first
 // 118 -> 61 us (2-byte loads before)
 template <typename T, int W>
-__global__ void __launch_bounds__(256) moe_gate_grad_kernel(const T* __restrict__ buf, const long long* __restrict__ slot, const T* __restrict__ g,
-                                                            float* __restrict__ dw, long long n, int k, long long tokens_per_block, int d, int E, int C,
-                                                            int nb) {
+__global__ void __launch_bounds__(256) moe_gate_grad_kernel(const T* buf, const long long* slot, const T* g, float* dw, long long n, int k,
+                                                            long long tokens_per_block, int d, int E, int C, int nb) {
   after_previous();
   const long long a = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
