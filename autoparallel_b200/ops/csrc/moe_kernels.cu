@@ -147,14 +147,23 @@ __device__ __forceinline__ long long buf_row(long long s, int blk, int E, int C,
 
 // Scatter: every buffer row is written exactly once, with its assignment's weighted token or with zeros, so the buffer is
 // not zero-filled first.  ``inv`` names the assignment of a row; rows that none names hold whatever the memory held, so a
-// row's entry counts only if that assignment's slot leads back to the row.
+// row's entry counts only if that assignment's slot leads back to the row.  Where several do, the last of them has the row, as if they were stored in
+// order: an entry gives way to a later assignment, or where it does not count, in whatever order the threads come.
 // 136 -> 69 us (zero fill and 2-byte copies before).
-__global__ void moe_inverse_kernel(const long long* slot, long long* inv, long long n, int k, long long tokens_per_block,
-                                   int E, int C, int nb) {
+__global__ void moe_inverse_kernel(const long long* slot, long long* inv, long long n, int k, long long tokens_per_block, int E, int C, int nb) {
+  after_previous();
   const long long a = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= n) return;
-  const long long row = buf_row(slot[a], (int)(a / k / tokens_per_block), E, C, nb);
-  if (row >= 0) inv[row] = a;
+  auto row_of = [&](long long i) { return buf_row(slot[i], (int)(i / k / tokens_per_block), E, C, nb); };
+  const long long row = row_of(a);
+  if (row < 0) return;
+  unsigned long long* entry = reinterpret_cast<unsigned long long*>(inv) + row;
+  long long held = (long long)__ldcg(entry);
+  while (held < a || held >= n || row_of(held) != row) {  // (once more for every other assignment of the row at most)
+    const long long was = (long long)atomicCAS(entry, (unsigned long long)held, (unsigned long long)a);
+    if (was == held) break;
+    held = was;
+  }
 }
 
 // The words of a Pack: the bf16 values of a vector that waits for its turn stay in 4 registers (as values they take 8).
@@ -367,9 +376,7 @@ extern "C" int apb_moe_scatter(const void* src, const long long* slot, const voi
   const long long n = T_ * k, rows = (long long)E * nb * C;
   if (rows <= 0) return 0;
   const long long tpb = T_ / nb;
-  // (launched in the ordinary way: where two choices name one row, the one whose warp starts later counts, and warps that waited for the kernel before
-  // them go on in any order)
-  moe_inverse_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(slot, inv, n, k, tpb, E, C, nb);
+  launch_after(moe_inverse_kernel, (unsigned)((n + 255) / 256), 256, 0, st, slot, inv, n, k, tpb, E, C, nb);
   const bool stream = rows * d * (is_bf16 ? 2 : 4) > 64000000ll;
   APB_MOE_DISPATCH(is_bf16, vec_rows(d, sizeof(T), src, buf), {
     auto kern = stream ? moe_scatter_kernel<T, W, true> : moe_scatter_kernel<T, W, false>;

@@ -204,6 +204,26 @@ def test_moe_rows_of_a_buffer_of_more_than_half_of_l2(K, dtype):
     assert _rel(out, (rows * w.double().unsqueeze(2)).sum(1)) <= 2**-22 + (2**-8 if dtype == torch.bfloat16 else 0)
 
 
+@pytest.mark.parametrize("T,k,rows,nb", [(32, 2, 40, 1), (6000, 8, 40, 1), (6000, 8, 40000, 1), (3000, 3, 600, 3)])
+def test_moe_scatter_of_repeated_slots(K, T, k, rows, nb):
+    """The last choice that names a row has it, as if they were stored in order, whatever the table of rows held before and however often it is repeated."""
+    lib, _ = K
+    E, d = 8, 8
+    C = rows // E
+    g = torch.Generator(device="cuda").manual_seed(T)
+    slot = torch.randint(0, E * C + 1, (T, k), device="cuda", generator=g)
+    x = torch.randn(T, d, device="cuda", generator=g)
+    w = torch.rand(T, k, device="cuda", generator=g)
+    flat = torch.zeros(nb, E * C + 1, d).numpy()
+    block = (torch.arange(T) // (T // nb)).unsqueeze(1).expand(T, k)
+    flat[block.reshape(-1).numpy(), slot.reshape(-1).cpu().numpy()] = (x.unsqueeze(1) * w.unsqueeze(2)).reshape(T * k, d).cpu().numpy()  # (in order)
+    ref = torch.from_numpy(flat)[:, :E * C].view(nb, E, C, d).transpose(0, 1).contiguous()
+    for i in range(100):
+        junk = torch.randint(-3, T * k + 3, (E * nb * C,), device="cuda", generator=g) if i % 2 else torch.full((E * nb * C,), T * k - 1, device="cuda")
+        del junk  # (the table takes its memory)
+        assert torch.equal(lib.ops.moe_scatter(x, slot, w, E, C, nb).cpu(), ref)
+
+
 def test_moe_dispatch_leaves_nothing_of_the_old_buffer(K):
     """Every row of the buffer is written, also those no assignment names, whatever the memory held before."""
     lib, _ = K
