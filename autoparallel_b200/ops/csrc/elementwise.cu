@@ -806,20 +806,18 @@ int apb_rms_norm_fwd(const void* x, const void* w, void* y, float* rstd, long lo
     if (nvec == 1) { APB_RMS_FWD_W(1); } else if (nvec == 2) { APB_RMS_FWD_W(2); } else { APB_RMS_FWD_W(4); }
 #undef APB_RMS_FWD_W
   } else {
-    // Threads of a row's block and what it does after the row.  Few rows: one vector per thread, the row itself is the latency (64 x 4096 bf16,
-    // 256 -> 512 threads 2.8 -> 2.4 us).  Many short rows: two, and more blocks on an SM (8192 x 1536 bf16 192 -> 96 threads 11.1 -> 9.9 us,
-    // fp32 17.3 -> 16.3).  Blocks end with their row; only bf16 rows from 4096 on keep blocks that take rows in turn, 8 (or 2048 threads) to an
-    // SM: row by row -> in turn 8192 x 3072 bf16 20.5 -> 21.4 us, x 4096 26.8 -> 25.6, x 8192 49.3 -> 44.7; fp32 x 2048 23.6 -> 29.4, x 4096 42.0
-    // -> 52.7, x 8192 82.7 -> 87.9.
-    const int vecs = D / 8;
+    // The threads of a row's block, and with them the order of its sum, follow from D alone: a row gives the same bits whatever other rows are in the
+    // call (a rule by rows as well was faster, 64 x 4096 bf16 1.8 -> 1.6 us, 8192 x 1536 13.3 -> 11.3, but changed the bits and, with 16 squares to a
+    // thread instead of 8, made the error of the sum 1 to 2 % larger).
+    // Blocks end with their row, or, for bf16, take rows in turn, 8 (or 2048 threads) to an SM: row by row -> in turn 1024 x 1032 2.0 -> 2.3 us, 4096 x 1032
+    // 7.1 -> 6.8, 32768 x 1032 43 -> 38, 1024 x 2048 3.1 -> 3.2, 4096 x 2048 8.6 -> 8.5, 512 x 2560 2.5 -> 2.3, 8192 x 3072 22.1 -> 18.6, x 4096 26.8 -> 25.6,
+    // x 8192 49.3 -> 44.7; fp32 8192 x 2048 23.6 -> 29.4, x 4096 42.0 -> 52.7, x 8192 82.7 -> 87.9.
     int threads = 256;
-    if (rows <= 256 && vecs <= 1024) threads = (vecs + 31) / 32 * 32;
-    else if (D <= 3072 && rows >= (is_bf16 ? 1024 : 4096)) threads = (vecs + 63) / 64 * 32;
     while (threads * 8 * 4 < D && threads < 1024) threads *= 2;
-    const int nvec = (vecs + threads - 1) / threads;
+    const int nvec = (D + threads * 8 - 1) / (threads * 8);
     if (nvec > 4) return 3;
     unsigned grid = (unsigned)rows;
-    const bool in_turn = is_bf16 && D >= 4096;
+    const bool in_turn = is_bf16 && (D > 2048 || rows >= 4096);
     if (in_turn) {
       int dev = 0, sms = 148;
       cudaGetDevice(&dev);

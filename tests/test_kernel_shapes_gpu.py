@@ -119,6 +119,19 @@ def test_embedding_gradient_with_zeros_first(K, dtype, V, D, T, ids):
     assert not out[torch.bincount(idx[inside], minlength=V) == 0].any()
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("D", [8, 1024, 1032, 1536, 2048, 3072, 4096, 8192, 8200])
+def test_a_row_is_normalised_to_the_same_bits_in_any_call(K, D, dtype):
+    lib, _ = K
+    g = torch.Generator(device="cuda").manual_seed(D)
+    x, w = torch.randn(4100, D, device="cuda", generator=g).to(dtype), torch.randn(D, device="cuda", generator=g).to(dtype)
+    y, rstd = lib.ops.rms_norm(x, w, 1e-5)
+    for rows in (1, 256, 257, 1023, 1024, 4095, 4096):
+        part = x[-rows:].clone()
+        got = lib.ops.rms_norm(part, w, 1e-5)
+        assert torch.equal(got[0], y[-rows:]) and torch.equal(got[1].view(-1), rstd.view(-1)[-rows:]), rows
+
+
 def test_embedding_gradient_of_an_unaligned_view(K):
     lib, _ = K
     flat = torch.randn(1 + 12 * 16, device="cuda").to(torch.bfloat16)
