@@ -314,7 +314,6 @@ struct SplitPlan {
   int bn, s;
 };
 extern "C" int apb_gemm_resident_pairs(int num_sms);
-extern "C" int apb_gemm_makes_room();
 
 static SplitKernel split_kernel_any() { return gemm_split_kernel<false, false, 64, false>; }
 

@@ -148,15 +148,12 @@ extern "C" int apb_gemm_get_reserved_sms() { return g_reserved_sms; }
 extern "C" void apb_gemm_set_pair_mode(int on) { g_pair_mode = on ? 1 : 0; }
 extern "C" int apb_gemm_get_pair_mode() { return g_pair_mode; }
 
-// Where the GEMMs are set to make room for communication kernels, they start as ever, after the end of the kernel before them: the gap between two kernels is
-// where such a kernel becomes resident.
 extern "C" int apb_gemm_makes_room() { return g_dynamic_tiles || g_pair_stages != PAIR_STAGES || g_reserved_sms > 0; }
 template <typename Kernel>
 static void launch_gemm(Kernel kern, int grid, int threads, int smem, cudaStream_t stream, const CUtensorMap& tmA, const CUtensorMap& tmB,
                         const GemmParams& p) {
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (apb_gemm_makes_room()) kern<<<grid, threads, smem, stream>>>(tmA, tmB, p);
-  else launch_after(kern, grid, threads, smem, stream, tmA, tmB, p);
+  launch_after(kern, grid, threads, smem, stream, tmA, tmB, p);
 }
 
 // gemm_split.cu: products with few tiles; -1 = the kernels here are the better choice

@@ -18,6 +18,10 @@
 
 #include <utility>
 
+// Whether the GEMMs are set to make room for communication kernels (gemm_tcgen05.cu).  Then no launch overlaps: the gap between two kernels is where a
+// communication kernel becomes resident, and blocks that come early would take its place.
+extern "C" int apb_gemm_makes_room();
+
 namespace apb {
 
 __device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -43,7 +47,7 @@ inline cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, siz
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = apb_gemm_makes_room() ? 0 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 

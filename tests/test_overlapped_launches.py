@@ -158,3 +158,46 @@ def test_captured_chains(ops):
             graph.replay()
         torch.cuda.synchronize()
         assert all(torch.equal(a, b) for a, b in zip(got, ref))
+
+
+def _edges(fn):
+    """Edges between the launches of a captured graph: (overlapping, all)."""
+    cudart = pytest.importorskip("cuda.bindings.runtime")
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        fn()
+    raw = cudart.cudaGraph_t(graph.raw_cuda_graph())
+    get = getattr(cudart, "cudaGraphGetEdges_v2", cudart.cudaGraphGetEdges)
+    n = get(raw)[-1]
+    err, _, _, data, _ = get(raw, n)
+    assert err == cudart.cudaError_t.cudaSuccess
+    kind = cudart.cudaGraphDependencyType.cudaGraphDependencyTypeProgrammatic
+    return sum(int(d.type) == int(kind) for d in data[:n]), n
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["dynamic", "stages", "reserved"])
+def test_no_launch_overlaps_where_room_is_made(ops, mode):
+    """Neither the products, nor those of a few rows, nor anything between them."""
+    from autoparallel_b200.ops import cuda_impl
+
+    ext = cuda_impl.extension()
+    get, put, value = {"dynamic": (ext.gemm_get_dynamic_tiles, ext.gemm_set_dynamic_tiles, True),
+                       "stages": (ext.gemm_get_pair_stages, ext.gemm_set_pair_stages, 5),
+                       "reserved": (ext.gemm_get_reserved_sms, ext.gemm_set_reserved_sms, 8)}[mode]
+    state, large = _state(0), torch.randn(2048, 512, device="cuda").to(torch.bfloat16)
+
+    def work():
+        _chain(ops, state, lambda: None)
+        ops.swiglu(ops.mm_nd(large, state[1], True, torch.bfloat16), large)
+
+    work()
+    before = get()
+    overlapping, n = _edges(work)
+    assert overlapping > n // 2
+    put(value)
+    try:
+        work()
+        assert _edges(work)[0] == 0
+    finally:
+        put(before)
