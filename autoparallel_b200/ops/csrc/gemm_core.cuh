@@ -140,19 +140,26 @@ inline void set_tile_order(GemmParams& p, int num_m, int num_n) {
 // 25.5 -> 22.1, 2048 x 5632 x 1024 21.5 -> 19.9, 64 x 160 x 1408 x 2048 81 -> 78.  Above half a wave of tiles the halves would take two.
 //
 // Wide tiles read A half as often: every wave of tiles goes through the row group's panel of A (16 tile rows) once, and where that no longer
-// stays in L2 from one wave to the next it comes from memory again.  The line lies where that begins, at 36 MB (4096 rows: K = 4394).
-// Narrow -> wide, us at the power cap: 4096 rows of A in a group, N = 4096, K = 4096 205 -> 204, 5120 262 -> 252, 8192 430 -> 401, 14336 747 ->
-// 700; N = 10240, K = 4608 291.9 -> 290.5, 8192 540 -> 511; 2048 rows, N = 14336, K = 5632 259 -> 261, 8192 380 -> 374, 11008 514 -> 496; the
-// vocabulary head of 8192 tokens, forward and backward, 21598 -> 20036.  Short contractions lose: K = 512 6 to 8 %, 256 2 to 8 %.
+// stays in L2 from one wave to the next it comes from memory again.  The line lies where that begins, at 36 MB (4096 rows: K = 4394), and only where
+// wide tiles take hardly more waves: of two column tiles each, a last wave with few of them costs twice as much.  Where the waves are equal they
+// take 2 % longer by themselves, but save the power that bounds a long run.  Narrow -> wide, us, in runs of half a second (power cap): 8192 x 4096, K
+// = 4608 230 -> 229, 5120 256 -> 254, 8192 419 -> 402, 14336 724 -> 692; 8192 x 10240 x 8192 1050 -> 996, 8192 x 4096 x 128256 6716 -> 6200, 128256 x
+// 4096 x 8192 6631 -> 6268.  With 1.08 times the waves 2048 x 14336 x 8192 374 -> 374, 16384 x 1792 x 6144 291 -> 294, with 1.2 8192 x 1280 x 8192 147 ->
+// 157, with 2 32768 x 256 x 8192 110 -> 119.  Short contractions lose: K = 512 6 to 8 %, 256 2 to 8 %.
 inline bool set_pair_tiles(GemmParams& p, int num_m, int units, bool may_be_wide) {
-  const bool wide = may_be_wide && 2ll * (num_m < GROUP_M ? num_m : GROUP_M) * 2 * BM * p.K >= 36000000ll &&
-                    (long long)num_m * ((p.num_n_tiles + 1) / 2) * p.groups >= units;
-  const int num_n = wide ? (p.num_n_tiles + 1) / 2 : p.num_n_tiles;
-  const long long all = (long long)num_m * num_n * p.groups;
+  const long long narrow_tiles = (long long)num_m * p.num_n_tiles * p.groups, wide_tiles = (long long)num_m * ((p.num_n_tiles + 1) / 2) * p.groups;
+  // halves of column tiles that a unit goes through; the last wave runs in halves where those fit in one
+  auto halves = [&](long long tiles, int columns) {
+    const long long rest = tiles % units;
+    return tiles / units * 2 * columns + (rest == 0 ? 0 : 2 * rest <= units ? columns : 2 * columns);
+  };
+  const bool wide = may_be_wide && 2ll * (num_m < GROUP_M ? num_m : GROUP_M) * 2 * BM * p.K >= 36000000ll && wide_tiles >= units &&
+                    20 * halves(wide_tiles, 2) <= 21 * halves(narrow_tiles, 1);
+  const long long all = wide ? wide_tiles : narrow_tiles;
   const int rest = (int)(all % units);
   p.all_tiles = (int)all;
   p.whole_tiles = 2 * rest <= units ? (int)all - rest : (int)all;
-  set_tile_order(p, num_m, num_n);
+  set_tile_order(p, num_m, wide ? (p.num_n_tiles + 1) / 2 : p.num_n_tiles);
   return wide;
 }
 __device__ __forceinline__ void plain_tile(const GemmParams& p, int num_m, bool grouped, int t, int& grp, int& tm, int& tn) {
@@ -428,7 +435,7 @@ constexpr int TILE_RING = 4;
 // WIDE: a tile of two column tiles, whose MMAs take turns on the stages (16 KB of A, 2 x 16 KB of B per CTA; four of them) and go to one TMEM
 // buffer each.  The turns are one k-block long, but WIDE_RUN at the ends of the contraction: the first accumulator is complete that much before
 // the second and is read out meanwhile, and the next tile begins with it.  Runs of 4 / 2 / 1 blocks: 8192 x 128256 x 4096 6129 / 6255 / 6348 us.
-constexpr int WIDE_RUN = 4;
+constexpr int WIDE_RUN = 4;  // (stages that the first accumulator takes before the second gives one back: no more than there are)
 template <bool A_MN, bool B_MN, int FUSE, bool PAIR = false, bool GROUPED = false, int ST_ARG = 0, bool DYN = false, bool WIDE = false>
 __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p,
                                          const FuseParams& f, int cta, int num_ctas, uint8_t* smem_raw) {
@@ -443,6 +450,7 @@ __device__ __forceinline__ void gemm_cta(const CUtensorMap& tmA, const CUtensorM
   constexpr int B_ROWS = PAIR ? BN / 2 : BN;
   constexpr bool NARROW = PAIR && FUSE == FUSE_NONE;  // column tiles with 128 columns or fewer take MMAs of 128
   static_assert(!WIDE || (PAIR && FUSE == FUSE_NONE && ST_ARG == 0), "wide tiles: CTA pairs, plain GEMM");
+  static_assert(!WIDE || WIDE_RUN <= ST, "a run waits for more stages than there are");
   constexpr int TM = PAIR ? 2 * BM : BM;                          // tile rows
   static_assert(ST * (A_BYTES + B_BYTES) <= STAGES * (A_STAGE_BYTES + B_STAGE_BYTES), "stages must fit the launch's shared memory");
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));

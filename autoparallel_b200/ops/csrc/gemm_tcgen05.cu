@@ -156,6 +156,17 @@ static void launch_gemm(Kernel kern, int grid, int threads, int smem, cudaStream
   launch_after(kern, grid, threads, smem, stream, tmA, tmB, p);
 }
 
+// How ``units`` resident CTA pairs go through a product: {wide tiles?, tiles, tiles that stay whole} (see set_pair_tiles; for tests).
+extern "C" void apb_gemm_pair_tiles(int G, int M, int N, int K, int units, int* out) {
+  GemmParams p{};
+  p.K = K;
+  p.groups = G > 0 ? G : 1;
+  p.num_n_tiles = (N + BN - 1) / BN;
+  out[0] = set_pair_tiles(p, (M + 2 * BM - 1) / (2 * BM), units, true);
+  out[1] = p.all_tiles;
+  out[2] = p.whole_tiles;
+}
+
 // gemm_split.cu: products with few tiles; -1 = the kernels here are the better choice
 extern "C" int apb_gemm_split_auto(const void* A, const void* B, void* C, int G, int M, int N, int K, long long lda, long long ldb,
                                    long long ldc, int a_mn, int b_mn, int out_fp32, uint32_t* status, int num_sms, int reserved,

@@ -35,6 +35,35 @@ def test_slot_workspace_of_an_empty_dispatch():
 
 
 @needs_ext
+def test_wide_tiles_take_hardly_more_waves():
+    """A product goes to tiles of two column tiles only where a pair's share of them is at most a twentieth larger (74 pairs)."""
+    import random
+
+    def halves(tiles, columns, units):  # of column tiles that a pair goes through; a last wave that fits runs in halves
+        whole, rest = divmod(tiles, units)
+        return 2 * columns * whole + (0 if rest == 0 else columns if 2 * rest <= units else 2 * columns)
+
+    rng = random.Random(7)
+    wide = [(0, 8192, 4096, 8192), (0, 8192, 4096, 128256), (0, 128256, 4096, 8192), (0, 8192, 10240, 8192), (0, 5896, 4104, 6552), (10, 2304, 4104, 8200)]
+    narrow = [(0, 32768, 256, 8192), (0, 16384, 768, 8192), (0, 8192, 1280, 8192), (0, 4096, 2304, 5120), (0, 4096, 3328, 8192), (0, 8192, 4096, 4096)]
+    drawn = [(rng.choice((0, 0, 4, 16)), rng.randrange(256, 40000), rng.randrange(64, 20000), rng.randrange(4096, 20000)) for _ in range(400)]
+    shapes = wide + narrow + drawn
+    code = "i3 = (ctypes.c_int * 3)()\n" + f"for s in {shapes!r}:\n    so.apb_gemm_pair_tiles(*s, 74, i3)\n    print(*i3)\n"
+    out = [int(x) for x in _run(code)]
+    taken = 0
+    for i, (G, M, N, K) in enumerate(shapes):
+        is_wide, tiles, whole = out[3 * i:3 * i + 3]
+        m, n = -(-M // 256) * max(G, 1), -(-N // 256)
+        assert tiles == m * (-(-n // 2) if is_wide else n) and 0 <= whole <= tiles and 2 * tiles - whole >= tiles
+        assert whole == tiles or (whole % 74 == 0 and 2 * (tiles - whole) <= 74)
+        taken += is_wide
+        if is_wide:
+            assert n > 1 and 20 * halves(tiles, 2, 74) <= 21 * halves(m * n, 1, 74), (G, M, N, K)
+    assert out[:3 * len(wide):3] == [1] * len(wide) and not any(out[3 * len(wide):3 * len(wide + narrow):3])
+    assert 20 < taken < 380
+
+
+@needs_ext
 def test_the_extension_brings_no_cxx_library_of_its_own():
     """With a static copy inside, an error with a number in its message ends the process (see ops/build.py)."""
     with open(build.so_path(), "rb") as f:

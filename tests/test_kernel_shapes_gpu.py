@@ -546,10 +546,12 @@ def test_gemm_tiles_land_where_they_belong(K, G, M, N, Kd, a_mn, b_mn, out):
 @pytest.mark.parametrize("G,M,N,Kd", [
     (0, 1504, 4104, 72),    # 102 pair tiles: a wave of whole ones, the others in halves, a last column tile of 8 columns
     (0, 1500, 4232, 72),    # a last column tile of 136 columns
-    (0, 4360, 4872, 6552),  # wide tiles, an odd number of column tiles, the rest of the waves column tile by column tile
+    (0, 4360, 4872, 6552),  # wide tiles, a last column tile of 8 columns, the rest of the waves column tile by column tile
+    (0, 5896, 4104, 6552),  # wide tiles, an odd number of column tiles: the last wide one has 8 columns
     (0, 4100, 1032, 72),    # whole tiles only, 8 columns in the last column tile
     (64, 160, 1416, 136),   # grouped
-    (20, 2304, 2184, 8200),  # grouped, wide
+    (20, 2304, 2184, 8200),  # grouped, a long contraction in column tiles of their own
+    (10, 2304, 4104, 8200),  # grouped, wide
 ])
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
 @pytest.mark.parametrize("dynamic", [False, True])
