@@ -362,7 +362,9 @@ static int emb_slices(int D, int w) {
 // at random, rows first -> zeros first: 128256 x 1024, 8000 tokens 85 / 78 -> 66 / 57 us, x 2048 127 / 125 -> 110 / 105, x 4096 210 / 195 -> 194 /
 // 186, 16000 tokens 221 / 215 -> 211 / 224; 32000 x 2048, 8000 tokens 57 / 52 -> 51 / 46, 16000 73 / 66 -> 72 / 72; 32000 x 4096, 2000 tokens 74 /
 // 63 -> 67 / 51, 8000 85 / 77 -> 89 / 79; 8000 x 2048, 2000 tokens 27 / 24 -> 23 / 21, 4000 26 / 25 -> 27 / 24.
-static bool emb_zeros_first(long long tokens, long long V, long long row_bytes) { return tokens <= V / (row_bytes > 4096 ? 10 : 4); }
+static bool emb_zeros_first(long long tokens, long long V, long long row_bytes) {
+  return tokens > 0 && tokens <= V / (row_bytes > 4096 ? 10 : 4);  // (without tokens emb_rows_kernel writes the zeros)
+}
 
 template <typename T, int W>
 static void emb_launch(const void* dy, const long long* ids, const EmbWs& ws, void* out, long long T_, long long V, int D, int num_sms,
@@ -378,10 +380,12 @@ static void emb_launch(const void* dy, const long long* ids, const EmbWs& ws, vo
     launch_after(emb_partial_kernel<T, W>, dim3((unsigned)chunks, (unsigned)slices), 128, 0, st, (const T*)dy, ws, (T*)out, chunks, D);
   int tx = 32;
   while (tx < nvec && tx < 256) tx *= 2;
-  if (zeros_first) {
-    const int per = 256 / tx;
-    if (T_ > 0) launch_after(emb_tokens_kernel<T, W>, (unsigned)((T_ + per - 1) / per), 256, 0, st, (const T*)dy, ids, ws, (T*)out, (int)T_, V, D, tx);
-    return;
+  if constexpr (W > 1) {
+    if (zeros_first) {
+      const int per = 256 / tx;
+      launch_after(emb_tokens_kernel<T, W>, (unsigned)((T_ + per - 1) / per), 256, 0, st, (const T*)dy, ids, ws, (T*)out, (int)T_, V, D, tx);
+      return;
+    }
   }
   // rows per block: eight where the table is long (one 64-KB store stream per block), fewer where it would leave SMs idle,
   // but never fewer than the block takes at a time

@@ -119,6 +119,27 @@ def test_embedding_gradient_with_zeros_first(K, dtype, V, D, T, ids):
     assert not out[torch.bincount(idx[inside], minlength=V) == 0].any()
 
 
+@pytest.mark.parametrize("dtype,V,D,T", [
+    (torch.bfloat16, 30000, 1032, 0),
+    (torch.bfloat16, 30000, 1032, 1),
+    (torch.bfloat16, 8000, 2048, 2001),
+    (torch.bfloat16, 100, 64, 0),  # by atomics
+    (torch.float32, 40000, 4096, 0),
+])
+def test_embedding_gradient_counts_what_it_launches(K, dtype, V, D, T):
+    _, impl = K
+    cudart = pytest.importorskip("cuda.bindings.runtime")
+    ext = impl.extension()
+    dy, ids = torch.ones(T, D, device="cuda", dtype=dtype), torch.arange(T, device="cuda")
+    out = torch.full((V, D), float("nan"), device="cuda", dtype=dtype)
+    ext.embedding_bwd(dy, ids, out)
+    assert torch.equal(out.sum(1), torch.where(torch.arange(V, device="cuda") < T, float(D), 0.0).to(dtype))
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        said = ext.embedding_bwd(dy, ids, out)
+    assert cudart.cudaGraphGetNodes(cudart.cudaGraph_t(graph.raw_cuda_graph()))[-1] == said
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("D", [8, 1024, 1032, 1536, 2048, 3072, 4096, 8192, 8200])
 def test_a_row_is_normalised_to_the_same_bits_in_any_call(K, D, dtype):
