@@ -110,7 +110,8 @@ class AdamW(torch.optim.Optimizer):
         # drained the whole backward pass).  The chunk list only depends on the sizes and is kept.
         nbytes = len(recs)
         capturing = lp_dev_capturing()
-        stage = cached[4] if cached is not None and cached[4].numel() == nbytes else None
+        sizes = tuple(_local(p).numel() for p in plist)
+        stage = cached[4] if cached is not None and cached[6] == sizes else None
         if stage is None:
             stage = {"host": torch.empty(nbytes, dtype=torch.uint8, pin_memory=True),
                      "dev": torch.empty(nbytes, dtype=torch.uint8, device=dev), "ev": None}
@@ -131,7 +132,7 @@ class AdamW(torch.optim.Optimizer):
             self._graph_keepalive.append((stage, ch))
             self._tables.pop(gi, None)
         else:
-            self._tables[gi] = (key, table, ch, len(chunks), stage["host"], stage)
+            self._tables[gi] = (key, table, ch, len(chunks), stage["host"], stage, sizes)
         return table, ch, len(chunks)
 
     def _hyper_buffers(self, gi: int, device):

@@ -162,6 +162,24 @@ def test_adamw_steps_on_the_loaded_state(K):
         assert torch.equal(opt.state[p][k], other.state[q][k])
 
 
+def test_adamw_where_other_parameters_have_gradients_each_step(K):
+    """One at a time, large after small and small after large."""
+    from autoparallel_b200.optim import AdamW
+
+    g = torch.Generator().manual_seed(4)
+    sizes = [5, 200000, 1024, 70001]
+    own = [torch.nn.Parameter(torch.randn(n, generator=g).cuda()) for n in sizes]
+    ref = [torch.nn.Parameter(p.detach().cpu().double()) for p in own]
+    opt, std = (cls(ps, lr=1e-2, betas=(0.9, 0.95), eps=1e-8, weight_decay=0.1) for cls, ps in ((AdamW, own), (torch.optim.AdamW, ref)))
+    for i in (0, 1, 0, 2, 3, 2, 1):
+        grad = torch.randn(sizes[i], generator=g)
+        for j, (p, q) in enumerate(zip(own, ref)):
+            p.grad, q.grad = (grad.cuda(), grad.double()) if j == i else (None, None)
+        opt.step(), std.step()
+    for p, q in zip(own, ref):
+        assert _rel(p.detach(), q.detach()) <= 2**-20  # fp32 steps of the size of lr
+
+
 @pytest.mark.parametrize("odd", ["param", "grad", "exp_avg", "exp_avg_sq"])
 def test_adamw_takes_views_off_a_16_byte_boundary(K, odd):
     """A parameter, gradient or state out of a flat buffer: the same step as on tensors of their own."""

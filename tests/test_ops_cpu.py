@@ -247,3 +247,47 @@ def test_device_neutral_attention_matches_the_planning_hosts_operator(causal, ma
             assert torch.allclose(l.to(rl.dtype), rl, atol=1e-6)
         dq, dk, dv = P.sdpa_backward(go, q, k, v, o, l.double(), 0.0, causal, attn_mask=m)
         assert torch.allclose(dq, rdq, atol=1e-8) and torch.allclose(dk, rdk, atol=1e-8) and torch.allclose(dv, rdv, atol=1e-8)
+
+
+def _adamw_pieces(opt, params):
+    """[(parameter, first element, elements)] of the launch for ``params``, in the order of its blocks."""
+    table, chunks, n = opt._table(0, params)
+    assert chunks.shape == (n, 2)
+    return [(t, c * opt.CHUNK, min(opt.CHUNK, params[t].numel() - c * opt.CHUNK)) for t, c in chunks.tolist()]
+
+
+def test_adamw_pieces_follow_the_parameters_that_have_gradients(monkeypatch):
+    """As many parameters as in the step before, but of other sizes: every element of them is in the list, and nothing else."""
+    from autoparallel_b200.optim import AdamW
+
+    class Event:
+        def record(self):
+            pass
+
+        synchronize = record
+
+    empty = torch.empty
+    monkeypatch.setattr(torch, "empty", lambda *a, pin_memory=False, **k: empty(*a, **k))
+    monkeypatch.setattr(torch.cuda, "Event", Event)
+    sizes = [5, 70000, 1, 200000, 65536, 1024, 1025, 131072]
+    params = [torch.nn.Parameter(torch.zeros(n)) for n in sizes]
+    opt = AdamW(params, lr=1e-3)
+    for p in params:
+        p.grad = torch.zeros_like(p)
+        opt._init_state(p)
+    for pick in ([0], [1], [2], [3, 4], [5, 6], [0, 7], [0, 7], list(range(8))):
+        plist = [params[i] for i in pick]
+        pieces = _adamw_pieces(opt, plist)
+        for t, p in enumerate(plist):
+            assert sorted((a, n) for q, a, n in pieces if q == t) == _cut(pieces, t, p.numel())
+        assert all(n > 0 for _, _, n in pieces)
+
+
+def _cut(pieces, t, total):
+    """The pieces of ``t`` end to end."""
+    out, at = [], 0
+    for a, n in sorted((a, n) for q, a, n in pieces if q == t):
+        out.append((at, n))
+        at += n
+    assert at == total
+    return out
