@@ -92,7 +92,7 @@ int apb_gemm_footprint(int i, int* out);
 int apb_gemm_split_footprint(int i, int* out);
 int apb_symm_footprint(int mode, int* out);
 int apb_dma_sum_footprint(int n, int* out);
-int apb_adamw(const void* tensors_dev, const void* chunks_dev, int num_chunks, float lr, float beta1, float beta2, float eps,
+int apb_adamw(const void* tensors_dev, const void* pieces_dev, int num_pieces, int whole, float lr, float beta1, float beta2, float eps,
               float wd, float bc1, float bc2, float grad_scale, const float* hyper_dev, cudaStream_t st);
 }
 
@@ -345,7 +345,7 @@ void moe_gate_grad(const at::Tensor& buf, const at::Tensor& slot, const at::Tens
         "apb_moe_gate_grad");
 }
 
-void adamw(const at::Tensor& table, const at::Tensor& chunks, int64_t num_chunks, double lr, double b1, double b2, double eps,
+void adamw(const at::Tensor& table, const at::Tensor& pieces, int64_t whole, double lr, double b1, double b2, double eps,
            double wd, double bc1, double bc2, double grad_scale, const c10::optional<at::Tensor>& hyper) {
   c10::cuda::CUDAGuard g(table.device());
   const float* hp = nullptr;
@@ -353,7 +353,9 @@ void adamw(const at::Tensor& table, const at::Tensor& chunks, int64_t num_chunks
     TORCH_CHECK(hyper->scalar_type() == at::kFloat && hyper->numel() >= 3 && hyper->is_cuda(), "adamw: hyper = fp32 [3] on the device");
     hp = hyper->data_ptr<float>();
   }
-  check(apb_adamw(table.data_ptr(), chunks.data_ptr(), (int)num_chunks, (float)lr, (float)b1, (float)b2, (float)eps, (float)wd,
+  TORCH_CHECK(pieces.dim() == 2 && pieces.size(1) == 2 && pieces.scalar_type() == at::kInt && whole >= 0 && whole <= pieces.size(0),
+              "adamw: pieces = int32 [n, 2], the first ``whole`` of them whole runs");
+  check(apb_adamw(table.data_ptr(), pieces.data_ptr(), (int)pieces.size(0), (int)whole, (float)lr, (float)b1, (float)b2, (float)eps, (float)wd,
                   (float)bc1, (float)bc2, (float)grad_scale, hp, stream()),
         "apb_adamw");
 }

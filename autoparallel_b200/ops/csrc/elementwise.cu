@@ -634,8 +634,9 @@ __global__ void embedding_fwd_kernel(const T* weight, const long long* ids, T* o
 }
 
 // ------------------------------------------------------------------------------------ AdamW
-// Multi-tensor: ``chunks`` lists pieces of ADAM_CHUNK elements (tensor id, number); a block takes ADAM_PART of one, four elements a thread.  Bound by
-// memory, 28 or 30 bytes an element.  218 M elements: pieces of 65536 / 8192 / 4096 / 1024 to a block 1067 / 1003 / 992 / 963 us.  Where the parameter
+// Multi-tensor: a block takes ADAM_PART elements of a tensor, four a thread.  ``pieces`` lists {tensor, first part}: ``whole`` entries of ADAM_RUN parts each,
+// then entries of one part, the ends of tensors and small ones (64 blocks for every tensor, however small: 2000 of 128 elements 134 us, so 4.5).
+// Bound by memory, 28 or 30 bytes an element.  218 M elements: 65536 / 8192 / 4096 / 1024 to a block 1067 / 1003 / 992 / 963 us.  Where the parameter
 // starts on a 16-byte boundary so do the other three (the optimizer sees to it); elsewhere elements are taken one by one.
 struct AdamTensor {
   float* p;        // fp32 master / parameter
@@ -645,10 +646,10 @@ struct AdamTensor {
   __nv_bfloat16* p_lp;  // optional low-precision copy to emit (may be null)
   long long n;
 };
-constexpr int ADAM_CHUNK = 65536, ADAM_PART = 1024;
+constexpr int ADAM_PART = 1024, ADAM_RUN = 64;  // (optim.py makes the list by both)
 // ``hyper`` (optional, device memory): {lr, bc1, bc2} read at run time instead of the launch arguments, so that a step
 // captured in a CUDA graph follows the learning-rate schedule and the bias corrections of the step it is replayed for.
-__global__ void __launch_bounds__(ADAM_PART / 4) adamw_kernel(const AdamTensor* tensors, const int2* chunks, float lr,
+__global__ void __launch_bounds__(ADAM_PART / 4) adamw_kernel(const AdamTensor* tensors, const int2* pieces, int whole, float lr,
                              float beta1, float beta2, float eps, float wd, float bc1, float bc2, float grad_scale, const float* hyper) {
   after_previous();
   if (hyper != nullptr) {
@@ -656,9 +657,10 @@ __global__ void __launch_bounds__(ADAM_PART / 4) adamw_kernel(const AdamTensor* 
     bc1 = hyper[1];
     bc2 = hyper[2];
   }
-  const int2 ch = chunks[blockIdx.x / (ADAM_CHUNK / ADAM_PART)];
-  const AdamTensor t = tensors[ch.x];
-  const long long i = (long long)ch.y * ADAM_CHUNK + (blockIdx.x % (ADAM_CHUNK / ADAM_PART)) * ADAM_PART + threadIdx.x * 4;
+  const int b = blockIdx.x, in_runs = whole * ADAM_RUN;
+  const int2 piece = pieces[b < in_runs ? b / ADAM_RUN : whole + b - in_runs];
+  const AdamTensor t = tensors[piece.x];
+  const long long i = (piece.y + (b < in_runs ? b % ADAM_RUN : 0ll)) * ADAM_PART + threadIdx.x * 4;
   if (i >= t.n) return;
   if (i + 4 <= t.n && ((reinterpret_cast<uintptr_t>(t.p + i) & 15) == 0)) {
     float4 p = *reinterpret_cast<float4*>(t.p + i);
@@ -968,11 +970,11 @@ int apb_embedding_fwd(const void* weight, const long long* ids, void* out, long 
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 
-int apb_adamw(const void* tensors_dev, const void* chunks_dev, int num_chunks, float lr, float beta1, float beta2, float eps,
-              float wd, float bc1, float bc2, float grad_scale, const float* hyper_dev, cudaStream_t st) {
-  if (num_chunks == 0) return 0;
-  launch_after(adamw_kernel, (unsigned)num_chunks * (ADAM_CHUNK / ADAM_PART), ADAM_PART / 4, 0, st, (const AdamTensor*)tensors_dev, (const int2*)chunks_dev, lr, beta1, beta2, eps, wd,
-                                           bc1, bc2, grad_scale, hyper_dev);
+int apb_adamw(const void* tensors_dev, const void* pieces_dev, int num_pieces, int whole, float lr, float beta1, float beta2, float eps, float wd,
+              float bc1, float bc2, float grad_scale, const float* hyper_dev, cudaStream_t st) {
+  if (num_pieces == 0) return 0;
+  launch_after(adamw_kernel, (unsigned)whole * ADAM_RUN + (unsigned)(num_pieces - whole), ADAM_PART / 4, 0, st, (const AdamTensor*)tensors_dev,
+               (const int2*)pieces_dev, whole, lr, beta1, beta2, eps, wd, bc1, bc2, grad_scale, hyper_dev);
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 

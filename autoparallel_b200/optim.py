@@ -25,7 +25,8 @@ def lp_dev_capturing() -> bool:
 
 
 class AdamW(torch.optim.Optimizer):
-    CHUNK = 65536
+    #: what a block of the kernel takes, and how many such parts an entry for a whole run of them stands for (csrc/elementwise.cu)
+    PART, RUN = 1024, 64
 
     def __init__(self, params: Iterable, lr=3e-4, betas=(0.9, 0.95), eps=1e-8, weight_decay=0.1, grad_scale: float = 1.0,
                  emit_bf16: bool = False, shadow_arena=None):
@@ -87,13 +88,14 @@ class AdamW(torch.optim.Optimizer):
         return st
 
     def _table(self, gi: int, plist):
-        """Device table of (p, g, m, v, p_lp, n) records + chunk list; rebuilt if a pointer moved.  ``None`` where the kernel's 16-byte
-        accesses, which go by the parameter's address, would meet a gradient or moment at an odd offset."""
+        """Device table of (p, g, m, v, p_lp, n) records, list of (record, first part) pieces and the number of whole runs that it begins
+        with; rebuilt if a pointer moved.  ``None`` where the kernel's 16-byte accesses, which go by the parameter's address, would meet a
+        gradient or moment at an odd offset."""
         key = tuple((_local(p).data_ptr(), _local(p.grad).data_ptr()) for p in plist)
         cached = self._tables.get(gi)
         if cached is not None and cached[0] == key:
             return cached[1], cached[2], cached[3]
-        recs, chunks = bytearray(), []
+        recs, runs, parts = bytearray(), [], []
         for ti, p in enumerate(plist):
             st = self.state[p]
             lp, lg = _local(p), _local(p.grad)
@@ -103,11 +105,13 @@ class AdamW(torch.optim.Optimizer):
             if (ptrs[1] | ptrs[2] | ptrs[3]) & 15 and not ptrs[0] & 15:
                 return None
             recs += struct.pack("<QQQQQq", *ptrs, lp_ptr, n)
-            chunks += [(ti, c) for c in range((n + self.CHUNK - 1) // self.CHUNK)]
+            in_runs = n // (self.PART * self.RUN) * self.RUN
+            runs += [(ti, c) for c in range(0, in_runs, self.RUN)]
+            parts += [(ti, c) for c in range(in_runs, (n + self.PART - 1) // self.PART)]
         dev = _local(plist[0]).device
         # Gradients are fresh tensors every step, so the record table changes every step: stage it in
         # pinned memory and copy asynchronously (a pageable copy would stall the host until the GPU has
-        # drained the whole backward pass).  The chunk list only depends on the sizes and is kept.
+        # drained the whole backward pass).  The list of pieces only depends on the sizes and is kept.
         nbytes = len(recs)
         capturing = lp_dev_capturing()
         sizes = tuple(_local(p).numel() for p in plist)
@@ -115,7 +119,7 @@ class AdamW(torch.optim.Optimizer):
         if stage is None:
             stage = {"host": torch.empty(nbytes, dtype=torch.uint8, pin_memory=True),
                      "dev": torch.empty(nbytes, dtype=torch.uint8, device=dev), "ev": None}
-            ch = torch.tensor(chunks, dtype=torch.int32).reshape(-1, 2).to(dev)
+            ch = torch.tensor(runs + parts, dtype=torch.int32).reshape(-1, 2).to(dev)
         else:
             stage, ch = cached[5], cached[2]
         if stage["ev"] is not None and not capturing:
@@ -127,13 +131,13 @@ class AdamW(torch.optim.Optimizer):
             stage["ev"].record()
         table = stage["dev"]
         if capturing:
-            # the captured copy re-reads this pinned table on every replay: keep it (and the chunk list) alive and out
+            # the captured copy re-reads this pinned table on every replay: keep it (and the list of pieces) alive and out
             # of reach of later eager steps, which build their own
             self._graph_keepalive.append((stage, ch))
             self._tables.pop(gi, None)
         else:
-            self._tables[gi] = (key, table, ch, len(chunks), stage["host"], stage, sizes)
-        return table, ch, len(chunks)
+            self._tables[gi] = (key, table, ch, len(runs), stage["host"], stage, sizes)
+        return table, ch, len(runs)
 
     def _hyper_buffers(self, gi: int, device):
         h = self._hyper.get(gi)
@@ -213,9 +217,9 @@ class AdamW(torch.optim.Optimizer):
                 from .ops import cuda_impl
 
                 cuda_impl.ensure_loaded()
-                table, ch, n = tabled
+                table, ch, whole = tabled
                 hyper = self._hyper_buffers(gi, lp0.device)["dev"] if capturing else None
-                cuda_impl.extension().adamw(table, ch, n, group["lr"], b1, b2, group["eps"], group["weight_decay"], bc1, bc2,
+                cuda_impl.extension().adamw(table, ch, whole, group["lr"], b1, b2, group["eps"], group["weight_decay"], bc1, bc2,
                                             self.grad_scale, hyper)
                 cuda_impl._count()
             else:

@@ -251,9 +251,9 @@ def test_device_neutral_attention_matches_the_planning_hosts_operator(causal, ma
 
 def _adamw_pieces(opt, params):
     """[(parameter, first element, elements)] of the launch for ``params``, in the order of its blocks."""
-    table, chunks, n = opt._table(0, params)
-    assert chunks.shape == (n, 2)
-    return [(t, c * opt.CHUNK, min(opt.CHUNK, params[t].numel() - c * opt.CHUNK)) for t, c in chunks.tolist()]
+    _, pieces, whole = opt._table(0, params)
+    parts = [(t, c + k) for t, c in pieces[:whole].tolist() for k in range(opt.RUN)] + [tuple(x) for x in pieces[whole:].tolist()]
+    return [(t, c * opt.PART, min(opt.PART, params[t].numel() - c * opt.PART)) for t, c in parts]
 
 
 def test_adamw_pieces_follow_the_parameters_that_have_gradients(monkeypatch):
@@ -280,7 +280,7 @@ def test_adamw_pieces_follow_the_parameters_that_have_gradients(monkeypatch):
         pieces = _adamw_pieces(opt, plist)
         for t, p in enumerate(plist):
             assert sorted((a, n) for q, a, n in pieces if q == t) == _cut(pieces, t, p.numel())
-        assert all(n > 0 for _, _, n in pieces)
+        assert all(n > 0 for _, _, n in pieces)  # no block without work
 
 
 def _cut(pieces, t, total):
