@@ -69,7 +69,7 @@ gemm_rows_kernel(const __nv_bfloat16* X, const __nv_bfloat16* W, void* C, int M,
 #pragma unroll
       for (int i = 0; i < MB; ++i) {
         xv[u][i] = make_uint4(0, 0, 0, 0);
-        if (in && xk[i]) xv[u][i] = *reinterpret_cast<const uint4*>(x[i] + k);
+        if (in && xk[i]) xv[u][i] = __ldca(reinterpret_cast<const uint4*>(x[i] + k));
       }
     }
 #pragma unroll
