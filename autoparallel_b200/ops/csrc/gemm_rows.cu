@@ -104,16 +104,23 @@ gemm_rows_kernel(const __nv_bfloat16* X, const __nv_bfloat16* W, void* C, int M,
 
 using namespace apb;
 
-// Whether the product is this kernel's.  Up to 8 rows it is the faster one at every size that was timed (64 <= N <= 32064, 256 <= K <= 14336).  With more, X
-// comes from L2 once per 16 columns and makes up half of what a block reads and more: split kernel against this one, us: 16 rows, 4096 x 4096 10.3 / 8.7,
-// 6144 x 1024 7.4 / 6.6, 4096 x 14336 22.9 / 23.2, 8192 x 8192 25.3 / 27.0, 64 x 8192 6.1 / 6.9; 32 rows, 512 x 512 4.4 / 3.3, 2048 x 2048 6.2 / 5.3, 6144 x
-// 1024 7.3 / 8.5, 1024 x 4096 6.9 / 8.0.
-extern "C" int apb_gemm_rows_takes(int M, int N, int K) {
+// Whether the product is this kernel's: where it is no slower than the split kernel, both launched to overlap.  Fitted to 3478 sizes (1 to 32 rows,
+// 64 <= N <= 32768, 64 <= K <= 14336): the mean loss against the better one of both is 0.2, 0.6 and 1.3 % with up to 8, 16 and 32 rows (as the line was
+// drawn with launches that did not overlap: 4, 5 and 9 %, at worst a factor of four).  us in a captured graph, split / this one:
+//   up to 8 rows  8 x 256 x 256 2.7 / 1.6, 8 x 4096 x 4096 10.7 / 7.4, 8 x 32064 x 4096 51 / 43.  Every round of the blocks that are resident together
+//                 (two to an SM) costs as much as a launch, so that many columns need some K: 8 x 14336 x 256 5.4 / 6.3, x 1024 10.7 / 8.4.  With few
+//                 columns and a long K there are too few blocks: 8 x 256 x 8192 4.9 / 6.6, 8 x 1024 x 8192 8.5 / 8.3, 1 x 512 x 8192 8.4 / 7.8.
+//   up to 16      X comes from L2 once per 16 columns and is half of what a block reads: 16 x 2048 x 2048 6.1 / 4.1, 16 x 4096 x 4096 8.8 / 8.3, 16 x 512
+//                 x 4096 4.2 / 5.3, 16 x 6144 x 512 5.8 / 4.8, 16 x 14336 x 512 7.2 / 8.8, x 1024 10.8 / 10.1, 16 x 4096 x 8192 15 / 16.
+//   up to 32      32 x 1024 x 1024 4.1 / 3.4, 24 x 2048 x 2048 6.4 / 4.7, 32 x 4096 x 1024 6.0 / 5.8; 32 x 1024 x 2048 4.2 / 4.8, 32 x 4096 x 512 4.6 /
+//                 5.3 (here it is one of the losses), 32 x 6144 x 256 4.0 / 6.4, 32 x 14336 x 256 5.5 / 11.6.
+extern "C" int apb_gemm_rows_takes(int M, int N, int K, int num_sms) {
   if (M <= 0 || N <= 0 || K <= 0 || K % 8) return 0;
-  const long long size = (long long)N * K;
-  if (M <= 8) return 1;
-  if (M <= 16) return K <= 4096 && size <= 4096ll * 4096;
-  return M <= ROWS_MAX && K <= 2048 && size <= 2048ll * 2048;
+  const long long round = 2ll * ROWS_TILE * num_sms;  // columns of the blocks that are resident together
+  const long long size = (long long)N * K, x = (long long)M * K;
+  if (M <= 8) return K <= 6144 ? N <= 2 * round || N <= 32ll * K : N >= 512 && N <= round && x <= 65536;
+  if (M <= 16) return K <= 3072 ? N <= (K >= 192 ? 2 : 1) * round || N <= 20ll * K : K <= 6144 && N >= 1024 && N <= round;
+  return M <= ROWS_MAX && (size <= 8192 || (K >= 192 && x <= 49152 && size <= 2048 * 2048 && N <= 8ll * K));
 }
 
 // X, W: 16-byte bases and rows.  Returns 0, or an argument / launch error (nothing launched).

@@ -173,7 +173,7 @@ extern "C" int apb_gemm_split_auto(const void* A, const void* B, void* C, int G,
                                    cudaStream_t stream);
 
 // gemm_rows.cu: products with a handful of rows
-extern "C" int apb_gemm_rows_takes(int M, int N, int K);
+extern "C" int apb_gemm_rows_takes(int M, int N, int K, int num_sms);
 extern "C" int apb_gemm_rows(const void* X, const void* W, void* C, int M, int N, int K, long long ldx, long long ldw, long long ldc, int out_fp32,
                              int num_sms, cudaStream_t st);
 
@@ -185,7 +185,7 @@ extern "C" int apb_gemm_bf16(const void* A, const void* B, void* C, int M, int N
   if (reinterpret_cast<uintptr_t>(C) & 15) return 3;
   if (K <= 0) return zero_result(C, M, N, ldc, out_fp32, stream);
   // (its blocks come to every SM: where some are reserved, the kernels that keep off them)
-  if (!a_mn_major && !b_mn_major && g_reserved_sms == 0 && apb_gemm_rows_takes(M, N, K))
+  if (!a_mn_major && !b_mn_major && g_reserved_sms == 0 && apb_gemm_rows_takes(M, N, K, num_sms))
     return apb_gemm_rows(A, B, C, M, N, K, lda, ldb, ldc, out_fp32, num_sms, stream);
   const int usable = num_sms - g_reserved_sms > 0 ? num_sms - g_reserved_sms : 1;
   // Pairs with dynamic tiles answer the requests for SMs, pairs with fewer stages leave shared memory free: those products stay theirs.

@@ -64,6 +64,18 @@ def test_wide_tiles_take_hardly_more_waves():
 
 
 @needs_ext
+def test_products_of_a_few_rows_go_to_the_faster_kernel():
+    """Sizes on both sides of the line, each timed with both kernels (148 SMs); what the few-row kernel cannot take stays out."""
+    rows = [(8, 256, 256), (8, 4096, 4096), (8, 32064, 4096), (8, 14336, 1024), (1, 512, 8192), (8, 1024, 8192), (16, 256, 2048), (16, 2048, 2048),
+            (16, 4096, 4096), (16, 6144, 512), (16, 14336, 1024), (32, 1024, 1024), (24, 2048, 2048), (32, 4096, 1024), (17, 64, 64)]
+    split = [(8, 14336, 256), (8, 32064, 512), (8, 256, 8192), (8, 6144, 8192), (1, 256, 14336), (16, 512, 4096), (16, 14336, 512), (16, 4096, 8192),
+             (32, 1024, 2048), (32, 6144, 256), (32, 14336, 256), (32, 2048, 4096), (17, 1024, 64)]
+    never = [(33, 1024, 1024), (8, 256, 252), (0, 256, 256), (8, 0, 256), (8, 256, 0), (8, 256, -8)]
+    out = _run(f"for s in {rows + split + never!r}:\n    print(so.apb_gemm_rows_takes(*s, 148))\n")
+    assert out == ["1"] * len(rows) + ["0"] * len(split + never)
+
+
+@needs_ext
 def test_the_extension_brings_no_cxx_library_of_its_own():
     """With a static copy inside, an error with a number in its message ends the process (see ops/build.py)."""
     with open(build.so_path(), "rb") as f:
