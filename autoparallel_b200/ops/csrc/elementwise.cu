@@ -411,10 +411,10 @@ __global__ void __launch_bounds__(1024) rms_dw_kernel(const float* part, T* dw, 
   if ((threadIdx.x & 31) == 0 && co < D) dw[co] = T(s);
 }
 
+// One vector of a thread: the ``vec``-th of ``n`` elements, or the end of them.
 template <typename S, typename D>
-__global__ void __launch_bounds__(256) cast_kernel(const S* src, D* dst, long long n) {
-  after_previous();
-  const long long i = (blockIdx.x * 256ll + threadIdx.x) * 8;
+__device__ __forceinline__ void cast_vec(const S* src, D* dst, long long n, long long vec) {
+  const long long i = vec * 8;
   if (i + 8 <= n) {
     Vec8<S> v; v.load(src + i);
     float f[8]; v.to_float(f);
@@ -422,6 +422,11 @@ __global__ void __launch_bounds__(256) cast_kernel(const S* src, D* dst, long lo
   } else {
     for (long long k = i; k < n; ++k) dst[k] = D(float(src[k]));
   }
+}
+template <typename S, typename D>
+__global__ void __launch_bounds__(256) cast_kernel(const S* src, D* dst, long long n) {
+  after_previous();
+  cast_vec(src, dst, n, blockIdx.x * 256ll + threadIdx.x);
 }
 
 // Many small casts to bf16 in one launch: a block finds its tensor in the table that travels with the launch.  21 parameters of a debug-sized decoder:
@@ -441,16 +446,7 @@ __global__ void __launch_bounds__(256) cast_many_kernel(const __grid_constant__ 
     if (t.first[mid] <= (int)blockIdx.x) lo = mid;
     else hi = mid;
   }
-  const float* src = t.src[lo];
-  __nv_bfloat16* dst = t.dst[lo];
-  const long long n = t.n[lo], i = ((long long)((int)blockIdx.x - t.first[lo]) * 256 + threadIdx.x) * 8;
-  if (i + 8 <= n) {
-    Vec8<float> v; v.load(src + i);
-    float f[8]; v.to_float(f);
-    Vec8<__nv_bfloat16> o; o.from_float(f); o.store(dst + i);
-  } else {
-    for (long long k = i; k < n; ++k) dst[k] = __float2bfloat16(src[k]);
-  }
+  cast_vec(t.src[lo], t.dst[lo], t.n[lo], ((int)blockIdx.x - t.first[lo]) * 256ll + threadIdx.x);
 }
 
 // ------------------------------------------------------------------------------------ RoPE
