@@ -623,7 +623,9 @@ def test_whole_and_half_and_wide_tiles(K, G, M, N, Kd, a_mn, b_mn, dynamic):
     (2376, 1024),  # more blocks than SMs
     (1024, 2048),  # fewer, and a long contraction
     (4096, 4096),
-    (56, 14344),
+    (520, 8192),   # the longest contraction with up to 8 rows
+    (9480, 304),   # three rounds of blocks
+    (56, 14344),   # the split kernel's
 ])
 def test_gemm_of_a_few_rows(K, M, N, Kd, out):
     """Around the blocks of 8 rows and of 16 columns; rows of the operands and of the result that lie further apart than they are long."""
