@@ -454,11 +454,10 @@ __global__ void __launch_bounds__(256) cast_many_kernel(const __grid_constant__ 
 // head (one 16-byte vector) at one position, in HEADS neighbouring heads: the 32 bytes of cos / sin it needs are read
 // once for them (the tables would otherwise be twice the traffic of x itself).  Eight heads where that leaves the SMs 768 threads each, else
 // four; all heads of a position in one thread -> 8 / 4 heads a thread: 8192 x 32 x 128 33.4 -> 25.3 / 27.7 us, 8192 x 8 x 128 8.3 -> 8.2 / 9.0,
-// 8192 x 8 x 64 5.6 -> 5.5 / 4.2, 100 x 32 x 128 8.8 -> 3.6 / 2.7.  Eight loads under way instead of four: 8192 x 8 x 128 8.0 -> 7.6, fp32 16.9 -> 15.4.
+// 8192 x 8 x 64 5.6 -> 5.5 / 4.2, 100 x 32 x 128 8.8 -> 3.6 / 2.7.
 template <typename T, int HEADS>
-__global__ void __launch_bounds__(128) rope_kernel(const T* x, const float* cs, const float* sn, T* y, long long total_pos_vec, int S, int H,
-                                                   int D, float sign) {
-  after_previous();
+__device__ __forceinline__ void rope(const T* __restrict__ x, const float* __restrict__ cs, const float* __restrict__ sn, T* __restrict__ y,
+                                     long long total_pos_vec, int S, int H, int D, float sign) {
   const int vec_per_head = D / 8;
   const unsigned groups = (H + HEADS - 1) / HEADS;  // of heads; neighbouring blocks take the groups of the same positions
   const long long v = blockIdx.x / groups * 128ll + threadIdx.x;
@@ -472,22 +471,31 @@ __global__ void __launch_bounds__(128) rope_kernel(const T* x, const float* cs, 
   const float nn[4] = {n.x * sign, n.y * sign, n.z * sign, n.w * sign};
   const long long base = (bs * H) * D + dv * 8;
   const int h0 = blockIdx.x % groups * HEADS, h1 = min(H, h0 + HEADS);
-  Vec8<T> xv[HEADS];  // (all loads before the first store)
 #pragma unroll
-  for (int k = 0; k < HEADS; ++k)
-    if (h0 + k < h1) xv[k].load(x + base + (long long)(h0 + k) * D);
+  for (int hg = 0; hg < HEADS; hg += 4) {  // four independent loads in flight
+    Vec8<T> xv[4];
 #pragma unroll
-  for (int k = 0; k < HEADS; ++k) {
-    if (h0 + k >= h1) break;
-    float f[8], o[8];
-    xv[k].to_float(f);
+    for (int k = 0; k < 4; ++k)
+      if (h0 + hg + k < h1) xv[k].load(x + base + (long long)(h0 + hg + k) * D);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      o[2 * i] = f[2 * i] * cc[i] - f[2 * i + 1] * nn[i];
-      o[2 * i + 1] = f[2 * i] * nn[i] + f[2 * i + 1] * cc[i];
+    for (int k = 0; k < 4; ++k) {
+      if (h0 + hg + k >= h1) break;
+      float f[8], o[8];
+      xv[k].to_float(f);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        o[2 * i] = f[2 * i] * cc[i] - f[2 * i + 1] * nn[i];
+        o[2 * i + 1] = f[2 * i] * nn[i] + f[2 * i + 1] * cc[i];
+      }
+      Vec8<T> ov; ov.from_float(o); ov.store(y + base + (long long)(h0 + hg + k) * D);
     }
-    Vec8<T> ov; ov.from_float(o); ov.store(y + base + (long long)(h0 + k) * D);
   }
+}
+template <typename T, int HEADS>
+__global__ void __launch_bounds__(128) rope_kernel(const T* x, const float* cs, const float* sn, T* y, long long total_pos_vec, int S, int H, int D,
+                                                   float sign) {
+  after_previous();
+  rope<T, HEADS>(x, cs, sn, y, total_pos_vec, S, H, D, sign);
 }
 
 // ------------------------------------------------------------------------------------ SwiGLU
