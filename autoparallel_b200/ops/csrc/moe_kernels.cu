@@ -145,24 +145,27 @@ __device__ __forceinline__ long long buf_row(long long s, int blk, int E, int C,
   return (e * nb + blk) * C + c;
 }
 
+// token block of assignment ``a`` (64-bit divisions only where there is more than one block)
+__device__ __forceinline__ int block_of(long long a, int k, long long tokens_per_block, int nb) { return nb == 1 ? 0 : (int)(a / k / tokens_per_block); }
+
 // Scatter: every buffer row is written exactly once, with its assignment's weighted token or with zeros, so the buffer is
 // not zero-filled first.  ``inv`` names the assignment of a row; rows that none names hold whatever the memory held, so a
 // row's entry counts only if that assignment's slot leads back to the row.  Where several do, the last of them has the row, as if they were stored in
-// order: an entry gives way to a later assignment, or where it does not count, in whatever order the threads come.
+// order: whoever takes a later one out of the entry puts it back, so that of all that name the row none but the last is left, in whatever order
+// the threads come.
 // 136 -> 69 us (zero fill and 2-byte copies before).
 __global__ void moe_inverse_kernel(const long long* slot, long long* inv, long long n, int k, long long tokens_per_block, int E, int C, int nb) {
   after_previous();
   const long long a = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= n) return;
-  auto row_of = [&](long long i) { return buf_row(slot[i], (int)(i / k / tokens_per_block), E, C, nb); };
+  auto row_of = [&](long long i) { return buf_row(slot[i], block_of(i, k, tokens_per_block, nb), E, C, nb); };
   const long long row = row_of(a);
   if (row < 0) return;
   unsigned long long* entry = reinterpret_cast<unsigned long long*>(inv) + row;
-  long long held = (long long)__ldcg(entry);
-  while (held < a || held >= n || row_of(held) != row) {  // (once more for every other assignment of the row at most)
-    const long long was = (long long)atomicCAS(entry, (unsigned long long)held, (unsigned long long)a);
-    if (was == held) break;
-    held = was;
+  for (long long put = a;;) {  // (``put`` grows: it ends)
+    const long long was = (long long)atomicExch(entry, (unsigned long long)put);
+    if (was <= put || was >= n || row_of(was) != row) break;
+    put = was;  // a later assignment of the row: back with it
   }
 }
 
@@ -203,7 +206,7 @@ __global__ void __launch_bounds__(256, 8) moe_scatter_kernel(const T* src, const
   const bool named = a >= 0 && a < n;
   const long long to = named ? slot[a] : -1;
   const float wt = named ? gate_weight<T>(w, a, w_bf16) : 0.f;  // (under way with the slot)
-  if (!named || buf_row(to, (int)(a / k / tokens_per_block), E, C, nb) != row) {
+  if (!named || buf_row(to, block_of(a, k, tokens_per_block, nb), E, C, nb) != row) {
     const Pack<T, W> zero{};
     for (int i = lane * W; i < d; i += 32 * W) put<STREAM>(y + i, zero);
     return;
