@@ -141,11 +141,13 @@ inline void set_tile_order(GemmParams& p, int num_m, int num_n) {
 //
 // Wide tiles read A half as often: every wave of tiles goes through the row group's panel of A (16 tile rows) once, and where that no longer
 // stays in L2 from one wave to the next it comes from memory again.  The line lies where that begins, at 36 MB (4096 rows: K = 4394), and only where
-// wide tiles take hardly more waves: of two column tiles each, a last wave with few of them costs twice as much.  Where the waves are equal they
-// take 2 % longer by themselves, but save the power that bounds a long run.  Narrow -> wide, us, in runs of half a second (power cap): 8192 x 4096, K
-// = 4608 230 -> 229, 5120 256 -> 254, 8192 419 -> 402, 14336 724 -> 692; 8192 x 10240 x 8192 1050 -> 996, 8192 x 4096 x 128256 6716 -> 6200, 128256 x
-// 4096 x 8192 6631 -> 6268.  With 1.08 times the waves 2048 x 14336 x 8192 374 -> 374, 16384 x 1792 x 6144 291 -> 294, with 1.2 8192 x 1280 x 8192 147 ->
-// 157, with 2 32768 x 256 x 8192 110 -> 119.  Short contractions lose: K = 512 6 to 8 %, 256 2 to 8 %.
+// wide tiles do not take many more waves: of two column tiles each, a last wave with few of them costs twice as much.  By themselves they take 2 %
+// longer where the waves are equal and 10 % where they are 8 to 7, but save the power that bounds a long run.  Narrow -> wide, us, in runs of half a
+// second (power cap): 8192 x 4096, K = 4608 230 -> 229, 5120 256 -> 254, 8192 419 -> 402, 14336 724 -> 692; 8192 x 10240 x 8192 1050 -> 996, 8192 x
+// 4096 x 128256 6716 -> 6200, 128256 x 4096 x 8192 6631 -> 6268; at 8 to 7 4096 x 4096 x 8192 221 -> 213, 16384 x 1024 x 6144 175 -> 166.  Beyond it 4096 x
+// 2560 x 8192 147 -> 151, 2048 x 5120 x 11008 194 -> 206.  With an odd number of column tiles the last wide one of a row shares nothing: 16384 x 5376
+// x 6144 (1.08 times the waves) 841 -> 854, 8192 x 1792 x 8192 (8 to 7) 204 -> 206, 4096 x 3328 x 8192 (4 to 3) 179 -> 197, 32768 x 256 x 8192 110 -> 119; so
+// there the line is 21 to 20.  Short contractions lose: K = 512 6 to 8 %, 256 2 to 8 %.
 inline bool set_pair_tiles(GemmParams& p, int num_m, int units, bool may_be_wide) {
   const long long narrow_tiles = (long long)num_m * p.num_n_tiles * p.groups, wide_tiles = (long long)num_m * ((p.num_n_tiles + 1) / 2) * p.groups;
   // halves of column tiles that a unit goes through; the last wave runs in halves where those fit in one
@@ -154,7 +156,7 @@ inline bool set_pair_tiles(GemmParams& p, int num_m, int units, bool may_be_wide
     return tiles / units * 2 * columns + (rest == 0 ? 0 : 2 * rest <= units ? columns : 2 * columns);
   };
   const bool wide = may_be_wide && 2ll * (num_m < GROUP_M ? num_m : GROUP_M) * 2 * BM * p.K >= 36000000ll && wide_tiles >= units &&
-                    20 * halves(wide_tiles, 2) <= 21 * halves(narrow_tiles, 1);
+                    (p.num_n_tiles % 2 ? 20 * halves(wide_tiles, 2) <= 21 * halves(narrow_tiles, 1) : 7 * halves(wide_tiles, 2) <= 8 * halves(narrow_tiles, 1));
   const long long all = wide ? wide_tiles : narrow_tiles;
   const int rest = (int)(all % units);
   p.all_tiles = (int)all;
