@@ -36,8 +36,8 @@ def test_slot_workspace_of_an_empty_dispatch():
 
 @needs_ext
 def test_wide_tiles_take_hardly_more_waves():
-    """A product goes to tiles of two column tiles only where a pair's share of them is at most a seventh larger, with an odd number of column
-    tiles a twentieth (74 pairs)."""
+    """A product goes to tiles of two column tiles only where a pair's share of them is at most a seventh larger, with an odd number
+    of column tiles a twentieth (74 pairs)."""
     import random
 
     def halves(tiles, columns, units):  # of column tiles that a pair goes through; a last wave that fits runs in halves
@@ -45,11 +45,12 @@ def test_wide_tiles_take_hardly_more_waves():
         return 2 * columns * whole + (0 if rest == 0 else columns if 2 * rest <= units else 2 * columns)
 
     rng = random.Random(7)
-    wide = [(0, 8192, 4096, 8192), (0, 8192, 4096, 128256), (0, 128256, 4096, 8192), (0, 8192, 10240, 8192), (0, 5896, 4104, 6552), (10, 2304, 4104, 8200),
-            (0, 4096, 4096, 8192), (0, 16384, 1024, 6144)]
-    narrow = [(0, 32768, 256, 8192), (0, 16384, 768, 8192), (0, 8192, 1280, 8192), (0, 4096, 2304, 5120), (0, 4096, 3328, 8192), (0, 8192, 4096, 4096),
-              (0, 4096, 2560, 8192), (0, 8192, 1792, 8192), (0, 2048, 5120, 11008)]
-    drawn = [(rng.choice((0, 0, 4, 16)), rng.randrange(256, 40000), rng.randrange(64, 20000), rng.randrange(4096, 20000)) for _ in range(400)]
+    wide = [(0, 8192, 4096, 8192), (0, 8192, 4096, 128256), (0, 128256, 4096, 8192), (0, 8192, 10240, 8192), (0, 5896, 4104, 6552),
+            (10, 2304, 4104, 8200), (0, 4096, 4096, 8192), (0, 16384, 1024, 6144)]
+    narrow = [(0, 32768, 256, 8192), (0, 16384, 768, 8192), (0, 8192, 1280, 8192), (0, 4096, 2304, 5120), (0, 4096, 3328, 8192),
+              (0, 8192, 4096, 4096), (0, 4096, 2560, 8192), (0, 8192, 1792, 8192), (0, 2048, 5120, 11008)]
+    drawn = [(rng.choice((0, 0, 4, 16)), rng.randrange(256, 40000), rng.randrange(64, 20000), rng.randrange(4096, 20000))
+             for _ in range(400)]
     shapes = wide + narrow + drawn
     code = "i3 = (ctypes.c_int * 3)()\n" + f"for s in {shapes!r}:\n    so.apb_gemm_pair_tiles(*s, 74, i3)\n    print(*i3)\n"
     out = [int(x) for x in _run(code)]
@@ -70,10 +71,11 @@ def test_wide_tiles_take_hardly_more_waves():
 @needs_ext
 def test_products_of_a_few_rows_go_to_the_faster_kernel():
     """Sizes on both sides of the line, each timed with both kernels (148 SMs); what the few-row kernel cannot take stays out."""
-    rows = [(8, 256, 256), (8, 4096, 4096), (8, 32064, 4096), (8, 14336, 1024), (1, 512, 8192), (8, 1024, 8192), (16, 256, 2048), (16, 2048, 2048),
-            (16, 4096, 4096), (16, 6144, 512), (16, 14336, 1024), (32, 1024, 1024), (24, 2048, 2048), (32, 4096, 1024), (17, 64, 64)]
-    split = [(8, 14336, 256), (8, 32064, 512), (8, 256, 8192), (8, 6144, 8192), (1, 256, 14336), (16, 512, 4096), (16, 14336, 512), (16, 4096, 8192),
-             (32, 1024, 2048), (32, 6144, 256), (32, 14336, 256), (32, 2048, 4096), (17, 1024, 64)]
+    rows = [(8, 256, 256), (8, 4096, 4096), (8, 32064, 4096), (8, 14336, 1024), (1, 512, 8192), (8, 1024, 8192), (16, 256, 2048),
+            (16, 2048, 2048), (16, 4096, 4096), (16, 6144, 512), (16, 14336, 1024), (32, 1024, 1024), (24, 2048, 2048),
+            (32, 4096, 1024), (17, 64, 64)]
+    split = [(8, 14336, 256), (8, 32064, 512), (8, 256, 8192), (8, 6144, 8192), (1, 256, 14336), (16, 512, 4096), (16, 14336, 512),
+             (16, 4096, 8192), (32, 1024, 2048), (32, 6144, 256), (32, 14336, 256), (32, 2048, 4096), (17, 1024, 64)]
     never = [(33, 1024, 1024), (8, 256, 252), (0, 256, 256), (8, 0, 256), (8, 256, 0), (8, 256, -8)]
     out = _run(f"for s in {rows + split + never!r}:\n    print(so.apb_gemm_rows_takes(*s, 148))\n")
     assert out == ["1"] * len(rows) + ["0"] * len(split + never)

@@ -240,7 +240,8 @@ def test_moe_rows_of_a_buffer_of_more_than_half_of_l2(K, dtype):
 
 @pytest.mark.parametrize("T,k,rows,nb", [(32, 2, 40, 1), (6000, 8, 40, 1), (6000, 8, 40000, 1), (3000, 3, 600, 3)])
 def test_moe_scatter_of_repeated_slots(K, T, k, rows, nb):
-    """The last choice that names a row has it, as if they were stored in order, whatever the table of rows held before and however often it is repeated."""
+    """The last choice that names a row has it, as if they were stored in order, whatever the table of rows held before and however
+    often it is repeated."""
     lib, _ = K
     E, d = 8, 8
     C = rows // E
@@ -250,10 +251,13 @@ def test_moe_scatter_of_repeated_slots(K, T, k, rows, nb):
     w = torch.rand(T, k, device="cuda", generator=g)
     flat = torch.zeros(nb, E * C + 1, d).numpy()
     block = (torch.arange(T) // (T // nb)).unsqueeze(1).expand(T, k)
-    flat[block.reshape(-1).numpy(), slot.reshape(-1).cpu().numpy()] = (x.unsqueeze(1) * w.unsqueeze(2)).reshape(T * k, d).cpu().numpy()  # (in order)
+    rows_of_x = (x.unsqueeze(1) * w.unsqueeze(2)).reshape(T * k, d).cpu().numpy()
+    flat[block.reshape(-1).numpy(), slot.reshape(-1).cpu().numpy()] = rows_of_x  # (in order)
     ref = torch.from_numpy(flat)[:, :E * C].view(nb, E, C, d).transpose(0, 1).contiguous()
     for i in range(100):
-        junk = torch.randint(-3, T * k + 3, (E * nb * C,), device="cuda", generator=g) if i % 2 else torch.full((E * nb * C,), T * k - 1, device="cuda")
+        junk = torch.full((E * nb * C,), T * k - 1, device="cuda")
+        if i % 2:
+            junk.random_(-3, T * k + 3, generator=g)
         del junk  # (the table takes its memory)
         assert torch.equal(lib.ops.moe_scatter(x, slot, w, E, C, nb).cpu(), ref)
 

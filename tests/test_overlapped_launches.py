@@ -73,7 +73,8 @@ def _state(seed, rows=8, d=512):
     bf = torch.bfloat16
     ids = torch.randperm(300, device="cuda", generator=g)[:rows]  # (one token a row: sums in one order)
     slots = torch.randperm(32, device="cuda", generator=g)[:2 * rows].view(rows, 2)
-    return (r(rows, d), (r(d, d) / d**0.5).to(bf), (r(d, d) / d**0.5).to(bf), (1 + 0.1 * r(d)).to(bf), r(rows, d // 8), r(rows, d // 8), ids, slots,
+    w1, w2 = ((r(d, d) / d**0.5).to(bf) for _ in range(2))
+    return (r(rows, d), w1, w2, (1 + 0.1 * r(d)).to(bf), r(rows, d // 8), r(rows, d // 8), ids, slots,
             torch.rand(rows, 2, device="cuda", generator=g).to(bf))
 
 
